@@ -70,8 +70,9 @@ typedef struct {
     int32_t nan_seen;
     int64_t total_sweeps_psi, total_sweeps_A;
     uint32_t rand_t;        /* Langevin seed after the call */
-    int32_t used_graph;     /* 1: device-side loop (CUDA graph), 0: host-driven loop */
-    int64_t sweep_launches; /* Jacobi sweep kernel launches (psi and A) */
+    int32_t used_graph;     /* 1: device-side loop (CUDA graph or one resident launch), 0: host-driven loop */
+    int64_t sweep_launches; /* Jacobi sweep kernel launches (psi and A); 1 where the whole call is one
+                             * launch (domains that fit on chip) */
 } glgpu_td_stats;
 
 /* --- lifetime: GLSolver construction / destruction (svirl/__init__.py:30-179,

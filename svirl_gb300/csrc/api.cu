@@ -85,6 +85,8 @@ void upload_inst(glgpu_handle* h) {
     I.flang_psi = (float)I.lang_psi;
     I.flang_A = (float)I.lang_A;
     I.lang_psi_on = (h->dtype == 4 ? (double)I.flang_psi : I.lang_psi) > 1.0e-32 ? 1 : 0;
+    I.thr_psi = res_threshold(h->dtype, I.stop_psi);
+    I.thr_A = res_threshold(h->dtype, I.stop_A);
     I.lang_A_on = (h->dtype == 4 ? (double)I.flang_A : I.lang_A) > 1.0e-32 ? 1 : 0;
     I.dt = h->inst_h.dt;
     I.fdt = (float)I.dt;
@@ -118,6 +120,7 @@ static void free_all(glgpu_handle* h) {
                     h->dscal, h->out, h->vort, h->vort_n, h->flush};
     for (void* p : ptrs)
         if (p) cudaFree(p);
+    res_free(&h->res);
     if (h->hscal) cudaFreeHost(h->hscal);
     if (h->pin) cudaFreeHost(h->pin);
     if (h->stream) cudaStreamDestroy(h->stream);
@@ -603,6 +606,7 @@ int glgpu_batch_destroy(glgpu_batch* b) {
     for (int q = 0; q < kTDGraphs; ++q)
         if (b->td_exec[q]) cudaGraphExecDestroy(b->td_exec[q]);
     if (b->cg_exec) cudaGraphExecDestroy(b->cg_exec);
+    res_free(&b->res);
     void* ptrs[] = {b->insts, b->gather, b->tiles, b->atiles, b->items, b->loop, b->cg_partials, b->cg_loop, b->cg_tiles};
     for (void* p : ptrs)
         if (p) cudaFree(p);

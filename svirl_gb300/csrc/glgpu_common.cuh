@@ -47,16 +47,18 @@ template <typename T> __device__ __forceinline__ C2<T> link_U(T ph) {
     return cmk<T>(c, -s);
 }
 
-// Im(conj(psi0) U(ph) psi1) (svirl/cuda/common.h:66-73).
 // a * b rounded once, never fused into a neighbouring add
 __device__ __forceinline__ float mul_rn_t(float a, float b) { return __fmul_rn(a, b); }
 __device__ __forceinline__ double mul_rn_t(double a, double b) { return __dmul_rn(a, b); }
 template <typename T> __device__ __forceinline__ T mul_rn(T a, T b) { return mul_rn_t(a, b); }
 
+// Im(conj(psi0) U(ph) psi1) (svirl/cuda/common.h:66-73); fused operations written out,
+// so that every kernel rounds alike.
 template <typename T> __device__ __forceinline__ T js_of(C2<T> p0, T ph, C2<T> p1) {
     T s, c;
     sincos_t(ph, &s, &c);
-    return (p0.x * p1.y - p0.y * p1.x) * c - (p0.x * p1.x + p0.y * p1.y) * s;
+    const T im = fma(p0.x, p1.y, -mul_rn<T>(p0.y, p1.x)), re = fma(p0.x, p1.x, mul_rn<T>(p0.y, p1.y));
+    return fma(im, c, -mul_rn<T>(re, s));
 }
 
 // |psi1 U(ph) - psi0|^2 (svirl/cuda/observables.h:238-247).

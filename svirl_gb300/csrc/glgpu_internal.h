@@ -97,6 +97,7 @@ struct Inst {
     int cg_exact;             // batched device CG: exact dF/dA on boundary links
     double cg_target;         // batched device CG: stop once E <= cg_target + cg_target_tol |cg_target| (NaN: off)
     double cg_target_tol;
+    unsigned long long thr_psi, thr_A;  // largest residual that meets the stop rule, as IEEE bits (res_threshold)
 };
 
 // Global state of one batched Jacobi/time loop.
@@ -114,6 +115,39 @@ struct LoopState {
 
 constexpr int kErrLoopGuard = 1;
 constexpr int kErrCopyWait = 2;  // a wait for a bulk copy into shared memory ran out (psi sweep)
+constexpr int kErrBarrier = 4;   // a wait at an instance's barrier ran out (resident time loop)
+
+// Resident time loop (tdr.cu).  An instance's barrier: CTAs arrived so far in the
+// call, and the residual maxima and NaN bits of the last three rounds.
+constexpr int kResSweeps = 8;    // at most this many sweeps per round
+struct ResGroup {
+    unsigned arrived, pad;
+    unsigned long long res[3][kResSweeps];
+    int nan[3], pad2;
+};
+// One CTA's tile of an instance: origin of its own nodes, the instance's CTAs, where
+// the instance's tiles start in the owner table, tiles per row.
+struct ResTile {
+    int inst, x0, y0, ncta, own0, ntx;
+};
+// Schedule of a call: CTA c works on tiles[first[c]] .. tiles[first[c + 1] - 1];
+// owner: the CTA of every tile of every instance.
+struct ResPlan {
+    void* fn = nullptr;
+    int threads = 0, smem = 0;
+    size_t scratch = 0;  // exchange slots of a CTA, bytes
+    std::vector<ResTile> tiles;
+    std::vector<int> first, owner;
+};
+// A handle's or batch's schedule and its device copies.
+struct ResState {
+    int ready = 0;  // 0: not made, 1: made, -1: the domain does not fit on chip
+    ResPlan plan;
+    ResTile* tiles = nullptr;
+    int *first = nullptr, *owner = nullptr;
+    ResGroup* groups = nullptr;
+    void* scratch = nullptr;
+};
 
 // A tile = 256 consecutive nodes of one instance.
 struct Tile {
@@ -227,6 +261,7 @@ struct glgpu_handle {
     // host pinned staging for small results
     double* hscal = nullptr;
     void* pin = nullptr;                // PinStage (pinned host memory)
+    glgpu::ResState res;                // resident time loop
 };
 
 // A batch: several handles (instances of any sizes and parameters, one dtype,
@@ -272,6 +307,7 @@ struct glgpu_batch {
     double cg_target_tol = 0.0;
     int cg_window = 0;                   // energy-window stop: iterations (0: off) and relative decrease
     double cg_window_tol = 0.0;
+    glgpu::ResState res;                 // resident time loop
     std::string last_error;
 };
 
@@ -294,6 +330,11 @@ int choose_strip_rows(int dtype, const Geo* const* geos, int n);
 inline int psi_kind(int dtype, int select) { return dtype == 8 ? 8 : (select == 1 ? 5 : 4); }
 int psi_sweep_grid(int kind, int rows, int nitems);
 std::vector<Item> make_items(const Geo& g, int inst, int rows);
+// tdr.cu
+bool res_prepare(ResState* r, glgpu_handle* const* hs, int n);
+void res_free(ResState* r);
+cudaError_t res_launch(const ResState& r, const Inst* insts, int ninst, LoopState* loop, int Nt, int eqn, cudaStream_t s);
+unsigned long long res_threshold(int dtype, double stop);
 // obs.cu
 int obs_free_energy(glgpu_handle* h, double* out);
 int obs_magnetic_field(glgpu_handle* h, void* host_out);

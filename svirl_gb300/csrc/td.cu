@@ -26,6 +26,7 @@
 
 #include "glgpu_bulk.cuh"
 #include "glgpu_internal.h"
+#include "glgpu_td.cuh"
 
 namespace glgpu {
 
@@ -158,62 +159,6 @@ template <typename T> __device__ __forceinline__ C2<T> shfl_up_c(C2<T> v, int d)
 }
 template <typename T> __device__ __forceinline__ C2<T> shfl_down_c(C2<T> v, int d) {
     return cmk<T>(__shfl_down_sync(0xffffffffu, v.x, d), __shfl_down_sync(0xffffffffu, v.y, d));
-}
-
-// The backward-Euler Jacobi update of one node (svirl/cuda/td.h:4-133 with the
-// Winecki-Adams link weights of td.h:159-163, coded as bits of cd: 0 left,
-// 1 right, 2 lower, 3 upper link), in two parts.  The diagonal depends only on
-// the right-hand side (with the Langevin term, rq), the linear coefficient and
-// the link weights, which are fixed during a Jacobi loop, so its reciprocal is
-// formed once per node and launch (psi_diag_inv) and each sweep only forms the
-// neighbour sums (psi_node).  A node with neither a left nor a right link gets 0.
-// The link table holds U scaled by dt/dx^2 (x links) or dt/dy^2 (y links), and
-// 0 on links of weight 0, so the neighbour sum is one FMA chain per component
-// with no branch per link.
-template <typename T>
-__device__ __forceinline__ T psi_diag_inv(C2<T> rq, T eps, unsigned cd, T dt, T idx2, T idy2) {
-    // FP64: the link-count terms by selects, keeping conversions off the FP64 pipe
-    if constexpr (sizeof(T) == 8) {
-        const unsigned nx = (cd & 1u) + ((cd >> 1) & 1u), ny = ((cd >> 2) & 1u) + ((cd >> 3) & 1u);
-        const T cx = nx == 0u ? T(0) : (nx == 1u ? idx2 : idx2 + idx2);
-        const T cy = ny == 0u ? T(0) : (ny == 1u ? idy2 : idy2 + idy2);
-        const T diag = T(1) + dt * (rq.x * rq.x + rq.y * rq.y - eps + (cx + cy));
-        return T(1) / diag;
-    } else {
-        const bool rm0 = cd & 1u, rp0 = cd & 2u, r0m = cd & 4u, r0p = cd & 8u;
-        const T wx = T(rm0) + T(rp0), wy = T(r0m) + T(r0p);
-        const T diag = T(1) + dt * (rq.x * rq.x + rq.y * rq.y - eps + (idx2 * wx + idy2 * wy));
-        return T(1) / diag;
-    }
-}
-
-// rq + conj(ua_left) p_left + ua p_right + conj(ub_down) p_prev + ub p_next as one
-// FMA chain per component, the link factors already scaled; p_next, the row the
-// previous sweep produced last, enters at the end of the chain.
-template <typename T>
-__device__ __forceinline__ C2<T> psi_node(C2<T> p_left, C2<T> p_right, C2<T> p_prev, C2<T> p_next, C2<T> ua_left,
-                                          C2<T> ua, C2<T> ub_down, C2<T> ub, C2<T> rq, T inv, unsigned cd) {
-    const C2<T> z = cmk<T>(T(0), T(0));
-    C2<T> out = z;
-    T ax = fma(ua_left.x, p_left.x, rq.x);
-    ax = fma(ua_left.y, p_left.y, ax);
-    ax = fma(ua.x, p_right.x, ax);
-    ax = fma(-ua.y, p_right.y, ax);
-    T ay = fma(ua_left.x, p_left.y, rq.y);
-    ay = fma(-ua_left.y, p_left.x, ay);
-    ay = fma(ua.x, p_right.y, ay);
-    ay = fma(ua.y, p_right.x, ay);
-    ax = fma(ub_down.x, p_prev.x, ax);
-    ax = fma(ub_down.y, p_prev.y, ax);
-    ax = fma(ub.x, p_next.x, ax);
-    ax = fma(-ub.y, p_next.y, ax);
-    ay = fma(ub_down.x, p_prev.y, ay);
-    ay = fma(-ub_down.y, p_prev.x, ay);
-    ay = fma(ub.x, p_next.y, ay);
-    ay = fma(ub.y, p_next.x, ay);
-    const T vx = ax * inv, vy = ay * inv;
-    if (cd & 3u) out = cmk<T>(vx, vy);
-    return out;
 }
 
 // Per-row inputs of the psi update besides psi itself, as loaded: the link
@@ -377,8 +322,8 @@ k_psi_sweep(const Inst* __restrict__ insts, const Item* __restrict__ items, int 
             r.rq = q.rr;
             if (lang && calc_lane && y >= 0 && y < Ny) {
                 const uint32_t n = (uint32_t)(i + Nx * y);
-                r.rq.x += lc * (rand_1<T>(n, rt) - T(0.5));
-                r.rq.y += lc * (rand_2<T>(n, rt) - T(0.5));
+                r.rq.x = add_noise<T>(r.rq.x, lc, rand_1<T>(n, rt));
+                r.rq.y = add_noise<T>(r.rq.y, lc, rand_2<T>(n, rt));
             }
             if (load_inv) {
                 r.inv = q.eps;
@@ -627,8 +572,8 @@ k_psi_sweep_bulk(const Inst* __restrict__ insts, const Item* __restrict__ items,
             r.rq = q.rr;
             if (lang && calc_lane && y >= 0 && y < Ny) {
                 const uint32_t n = (uint32_t)(i + Nx * y);
-                r.rq.x += lc * (rand_1<T>(n, rt) - T(0.5));
-                r.rq.y += lc * (rand_2<T>(n, rt) - T(0.5));
+                r.rq.x = add_noise<T>(r.rq.x, lc, rand_1<T>(n, rt));
+                r.rq.y = add_noise<T>(r.rq.y, lc, rand_2<T>(n, rt));
             }
             r.inv = (q.cd & 3u) ? psi_diag_inv<T>(r.rq, q.eps, q.cd, dt, idx2, idy2) : T(0);
             return r;
@@ -925,6 +870,9 @@ k_A_sweep(const Inst* __restrict__ insts, const ATile* __restrict__ atiles, Loop
             const bool fresh = k == 0 || (!I.vpi && (k & 1) == 0);
             T* Xc = (T*)I.U;
             T* Gc = Xc + g.Nab;
+            const T c2 = gsel<T>(I.dt, I.fdt) * gsel<T>(I.rho, I.frho) * gsel<T>(I.kappa2, I.fkappa2);
+            const T den_a = T(1) + T(2) * c2 * GT(g, idy2), den_b = T(1) + T(2) * c2 * GT(g, idx2);
+            const T rden_a = T(1) / den_a, rden_b = T(1) / den_b;
             T res = T(0);
             bool nan = false;
             // the node loop compiled twice, for the sweeps that compute the fixed parts and
@@ -939,110 +887,18 @@ k_A_sweep(const Inst* __restrict__ insts, const ATile* __restrict__ atiles, Loop
                     T va = T(0), vb = T(0), ca = T(0), cbv = T(0);
                     bool has_a = false, has_b = false;
                     int na = 0, nb = 0;
-                    if constexpr (kDelta) {
-                        // The same Jacobi iteration as the FP64 branch, written for delta: with
-                        // A^(k) = A^(0) + delta^(k) the update of a link is
-                        //   delta' = (noise + dt rho (js + rh) + dt rho k2 (dd nbs(A^(0)) - 2 d^-2 A^(0))
-                        //            + dt rho k2 dd nbs(delta^(k))) / D,
-                        // and the stop rule's |A^(k+1) - A^(k)| = |delta^(k+1) - delta^(k)|.  In FP32 the
-                        // iterates of A itself differ by whole units in the last place once |A| > 8
-                        // (the Landau gauge reaches H L), which the absolute stop rule of 1e-6
-                        // (svirl/solvers/td.py:53-57) never accepts; delta is small, so the loop
-                        // converges.  The supercurrent phase is that of A^(0) + delta^(2 floor(k/2)).
-                        // The division by a link's constant diagonal is a multiplication by
-                        // its reciprocal here; FP64 divides as the reference does.
-                        if (n < g.N) {
-                            const int i = ti, j = tj;
-                            const int Nxa = g.Nx - 1, Na = g.Na;
-                            has_a = i < g.Nx - 1;
-                            has_b = j < g.Ny - 1;
-                            na = i + Nxa * j;
-                            nb = Na + i + g.Nx * j;
-                            auto dlx = [&](int ii, int jj) -> T { return cur ? cx(ii, jj) : T(0); };
-                            auto dly = [&](int ii, int jj) -> T { return cur ? cy(ii, jj) : T(0); };
-                            const T idx2 = GT(g, idx2), idy2 = GT(g, idy2), idxy = GT(g, idxy);
-                            const T k2 = I.fkappa2;
-                            const T dt_rho_k2 = I.fdt * I.frho * k2;
-                            T xa = T(0), xb = T(0);
-                            if constexpr (kFresh) {
-                                const T* al = (I.vpi || k < 2) ? nullptr : (const T*)I.ab[(R + 2) % 3];  // delta of the phase
-                                const T ph_a = has_a ? (I.vpi ? abi[na] : rhs[na] + (al ? al[na] : T(0))) : T(0);
-                                const T ph_b = has_b ? (I.vpi ? abi[nb] : rhs[nb] + (al ? al[nb] : T(0))) : T(0);
-                                const unsigned cb = cell_bits(g, I.mt, i, j);
-                                const C2<T> psi0 = psi[n];
-                                const T dx = GT(g, dx), dy = GT(g, dy);
-                                const T idx = GT(g, idx), idy = GT(g, idy);
-                                const T H = I.fH;
-                                const T dt_rho = I.fdt * I.frho;
-                                const T lc = I.flang_A;
-                                const bool lang = I.lang_A_on != 0;
-                                if (has_a) {
-                                    const T noise = lang ? lc * (rand_1<T>((uint32_t)na, s_rt) - T(0.5)) : T(0);
-                                    T rh = T(0), dd = T(1);
-                                    if (j == 0) { rh = T(2) * k2 * H * idy; dd = T(2); }
-                                    else if (j == g.Ny - 1) { rh = -T(2) * k2 * H * idy; dd = T(2); }
-                                    T jl = T(0);
-                                    if (GL_PM(cb) || GL_PP(cb)) jl = idx * js_of<T>(psi0, dx * ph_a, psi[n + 1]);
-                                    T ga;
-                                    if (k == 0) {
-                                        T nr = T(0);
-                                        if (j > 0)
-                                            nr += idy2 * rhs[i + Nxa * (j - 1)] - idxy * rhs[Na + i + g.Nx * (j - 1)] +
-                                                  idxy * rhs[Na + i + 1 + g.Nx * (j - 1)];
-                                        if (j < g.Ny - 1)
-                                            nr += idy2 * rhs[i + Nxa * (j + 1)] + idxy * rhs[Na + i + g.Nx * j] - idxy * rhs[Na + i + 1 + g.Nx * j];
-                                        ga = mul_rn<T>(dt_rho_k2, dd * nr - T(2) * idy2 * rhs[na]);
-                                        Gc[na] = ga;
-                                    } else {
-                                        ga = Gc[na];
-                                    }
-                                    xa = noise + dt_rho * (jl + rh) + ga;
-                                    Xc[na] = xa;
-                                }
-                                if (has_b) {
-                                    const T noise = lang ? lc * (rand_2<T>((uint32_t)nb, s_rt) - T(0.5)) : T(0);
-                                    T rh = T(0), dd = T(1);
-                                    if (i == 0) { rh = -T(2) * k2 * H * idx; dd = T(2); }
-                                    else if (i == g.Nx - 1) { rh = T(2) * k2 * H * idx; dd = T(2); }
-                                    T jl = T(0);
-                                    if (GL_MP(cb) || GL_PP(cb)) jl = idy * js_of<T>(psi0, dy * ph_b, psi[n + g.Nx]);
-                                    T gb;
-                                    if (k == 0) {
-                                        T nr = T(0);
-                                        if (i > 0)
-                                            nr += idx2 * rhs[Na + (i - 1) + g.Nx * j] - idxy * rhs[(i - 1) + Nxa * j] + idxy * rhs[(i - 1) + Nxa * (j + 1)];
-                                        if (i < g.Nx - 1)
-                                            nr += idx2 * rhs[Na + (i + 1) + g.Nx * j] + idxy * rhs[i + Nxa * j] - idxy * rhs[i + Nxa * (j + 1)];
-                                        gb = mul_rn<T>(dt_rho_k2, dd * nr - T(2) * idx2 * rhs[nb]);
-                                        Gc[nb] = gb;
-                                    } else {
-                                        gb = Gc[nb];
-                                    }
-                                    xb = noise + dt_rho * (jl + rh) + gb;
-                                    Xc[nb] = xb;
-                                }
-                            } else {
-                                if (has_a) xa = Xc[na];
-                                if (has_b) xb = Xc[nb];
-                            }
-                            if (has_a) {
-                                const T dd = (j == 0 || j == g.Ny - 1) ? T(2) : T(1);
-                                T nd = T(0);
-                                if (j > 0) nd += idy2 * dlx(i, j - 1) - idxy * dly(i, j - 1) + idxy * dly(i + 1, j - 1);
-                                if (j < g.Ny - 1) nd += idy2 * dlx(i, j + 1) + idxy * dly(i, j) - idxy * dly(i + 1, j);
-                                va = (xa + dt_rho_k2 * dd * nd) * (T(1) / (T(1) + T(2) * dt_rho_k2 * idy2));
-                                ca = dlx(i, j);
-                            }
-                            if (has_b) {
-                                const T dd = (i == 0 || i == g.Nx - 1) ? T(2) : T(1);
-                                T nd = T(0);
-                                if (i > 0) nd += idx2 * dly(i - 1, j) - idxy * dlx(i - 1, j) + idxy * dlx(i - 1, j + 1);
-                                if (i < g.Nx - 1) nd += idx2 * dly(i + 1, j) + idxy * dlx(i, j) - idxy * dlx(i, j + 1);
-                                vb = (xb + dt_rho_k2 * dd * nd) * (T(1) / (T(1) + T(2) * dt_rho_k2 * idx2));
-                                cbv = dly(i, j);
-                            }
-                        }
-                    } else
+                    // FP64 iterates A; FP32 the offset delta.  FP32:
+                    // The same Jacobi iteration as the FP64 branch, written for delta: with
+                    // A^(k) = A^(0) + delta^(k) the update of a link is
+                    //   delta' = (noise + dt rho (js + rh) + dt rho k2 (dd nbs(A^(0)) - 2 d^-2 A^(0))
+                    //            + dt rho k2 dd nbs(delta^(k))) / D,
+                    // and the stop rule's |A^(k+1) - A^(k)| = |delta^(k+1) - delta^(k)|.  In FP32 the
+                    // iterates of A itself differ by whole units in the last place once |A| > 8
+                    // (the Landau gauge reaches H L), which the absolute stop rule of 1e-6
+                    // (svirl/solvers/td.py:53-57) never accepts; delta is small, so the loop
+                    // converges.  The supercurrent phase is that of A^(0) + delta^(2 floor(k/2)).
+                    // The division by a link's constant diagonal is a multiplication by
+                    // its reciprocal here; FP64 divides as the reference does.
                     if (n < g.N) {
                         const int i = ti, j = tj;
                         const int Nxa = g.Nx - 1, Na = g.Na;
@@ -1050,15 +906,20 @@ k_A_sweep(const Inst* __restrict__ insts, const ATile* __restrict__ atiles, Loop
                         has_b = j < g.Ny - 1;
                         na = i + Nxa * j;
                         nb = Na + i + g.Nx * j;
+                        auto dlx = [&](int ii, int jj) -> T { return cur ? cx(ii, jj) : T(0); };
+                        auto dly = [&](int ii, int jj) -> T { return cur ? cy(ii, jj) : T(0); };
                         const T idx2 = GT(g, idx2), idy2 = GT(g, idy2), idxy = GT(g, idxy);
                         const T k2 = gsel<T>(I.kappa2, I.fkappa2);
-                        const T dt_rho = gsel<T>(I.dt, I.fdt) * gsel<T>(I.rho, I.frho);
-                        const T dt_rho_k2 = dt_rho * k2;
+                        const T dt_rho = gsel<T>(I.dt, I.fdt) * gsel<T>(I.rho, I.frho), dt_rho_k2 = dt_rho * k2;
+                        const T dda = (j == 0 || j == g.Ny - 1) ? T(2) : T(1), ddb = (i == 0 || i == g.Nx - 1) ? T(2) : T(1);
                         T xa = T(0), xb = T(0);
                         if constexpr (kFresh) {
-                            // read the supercurrent phases before anything is stored (aliasing, see top)
-                            const T ph_a = has_a ? abi[na] : T(0);
-                            const T ph_b = has_b ? abi[nb] : T(0);
+                            // read the supercurrent phases before anything is stored (aliasing, see top);
+                            // FP32: A^(0) + delta^(2 floor(k/2))
+                            const T* al = (!kDelta || I.vpi || k < 2) ? nullptr : (const T*)I.ab[(R + 2) % 3];
+                            const bool base = kDelta && !I.vpi;
+                            const T ph_a = has_a ? (base ? rhs[na] + (al ? al[na] : T(0)) : abi[na]) : T(0);
+                            const T ph_b = has_b ? (base ? rhs[nb] + (al ? al[nb] : T(0)) : abi[nb]) : T(0);
                             const unsigned cb = cell_bits(g, I.mt, i, j);
                             const C2<T> psi0 = psi[n];
                             const T dx = GT(g, dx), dy = GT(g, dy);
@@ -1066,26 +927,52 @@ k_A_sweep(const Inst* __restrict__ insts, const ATile* __restrict__ atiles, Loop
                             const T H = gsel<T>(I.H, I.fH);
                             const T lc = gsel<T>(I.lang_A, I.flang_A);
                             const bool lang = I.lang_A_on != 0;
+                            auto rx = [&](int ii, int jj) -> T { return ii >= 0 && ii < Nxa && jj >= 0 && jj < g.Ny ? rhs[ii + Nxa * jj] : T(0); };
+                            auto ry = [&](int ii, int jj) -> T { return ii >= 0 && ii < g.Nx && jj >= 0 && jj < g.Ny - 1 ? rhs[Na + ii + g.Nx * jj] : T(0); };
                             if (has_a) {
-                                T r = rhs[na];
-                                if (lang) r += lc * (rand_1<T>((uint32_t)na, s_rt) - T(0.5));
+                                T first = kDelta ? T(0) : rhs[na];
+                                if (lang) first = add_noise<T>(first, lc, rand_1<T>((uint32_t)na, s_rt));
                                 T rh = T(0);
                                 if (j == 0) rh = T(2) * k2 * H * idy;
                                 else if (j == g.Ny - 1) rh = -T(2) * k2 * H * idy;
                                 T jl = T(0);
-                                if (GL_PM(cb) || GL_PP(cb)) jl = idx * js_of<T>(psi0, dx * ph_a, psi[n + 1]);
-                                xa = r + dt_rho * (jl + rh);
+                                if (GL_PM(cb) || GL_PP(cb)) jl = mul_rn<T>(idx, js_of<T>(psi0, dx * ph_a, psi[n + 1]));
+                                xa = A_fixed<T>(first, dt_rho, jl, rh);
+                                if constexpr (kDelta) {
+                                    T ga;
+                                    if (k == 0) {
+                                        ga = A_base<T>(dt_rho_k2, dda,
+                                                       A_nbs_x<T>(idy2, idxy, rx(i, j - 1), rx(i, j + 1), ry(i, j - 1), ry(i + 1, j - 1),
+                                                                  ry(i, j), ry(i + 1, j)), idy2, rhs[na]);
+                                        Gc[na] = ga;
+                                    } else {
+                                        ga = Gc[na];
+                                    }
+                                    xa += ga;
+                                }
                                 Xc[na] = xa;
                             }
                             if (has_b) {
-                                T r = rhs[nb];
-                                if (lang) r += lc * (rand_2<T>((uint32_t)nb, s_rt) - T(0.5));
+                                T first = kDelta ? T(0) : rhs[nb];
+                                if (lang) first = add_noise<T>(first, lc, rand_2<T>((uint32_t)nb, s_rt));
                                 T rh = T(0);
                                 if (i == 0) rh = -T(2) * k2 * H * idx;
                                 else if (i == g.Nx - 1) rh = T(2) * k2 * H * idx;
                                 T jl = T(0);
-                                if (GL_MP(cb) || GL_PP(cb)) jl = idy * js_of<T>(psi0, dy * ph_b, psi[n + g.Nx]);
-                                xb = r + dt_rho * (jl + rh);
+                                if (GL_MP(cb) || GL_PP(cb)) jl = mul_rn<T>(idy, js_of<T>(psi0, dy * ph_b, psi[n + g.Nx]));
+                                xb = A_fixed<T>(first, dt_rho, jl, rh);
+                                if constexpr (kDelta) {
+                                    T gb;
+                                    if (k == 0) {
+                                        gb = A_base<T>(dt_rho_k2, ddb,
+                                                       A_nbs_y<T>(idx2, idxy, ry(i - 1, j), ry(i + 1, j), rx(i - 1, j), rx(i - 1, j + 1),
+                                                                  rx(i, j), rx(i, j + 1)), idx2, rhs[nb]);
+                                        Gc[nb] = gb;
+                                    } else {
+                                        gb = Gc[nb];
+                                    }
+                                    xb += gb;
+                                }
                                 Xc[nb] = xb;
                             }
                         } else {
@@ -1093,20 +980,16 @@ k_A_sweep(const Inst* __restrict__ insts, const ATile* __restrict__ atiles, Loop
                             if (has_b) xb = Xc[nb];
                         }
                         if (has_a) {
-                            const T dd = (j == 0 || j == g.Ny - 1) ? T(2) : T(1);
-                            T nbs = T(0);
-                            if (j > 0) nbs += idy2 * cx(i, j - 1) - idxy * cy(i, j - 1) + idxy * cy(i + 1, j - 1);
-                            if (j < g.Ny - 1) nbs += idy2 * cx(i, j + 1) + idxy * cy(i, j) - idxy * cy(i + 1, j);
-                            va = (xa + dt_rho_k2 * dd * nbs) / (T(1) + T(2) * dt_rho_k2 * idy2);
-                            ca = cx(i, j);
+                            const T nd = A_nbs_x<T>(idy2, idxy, dlx(i, j - 1), dlx(i, j + 1), dly(i, j - 1), dly(i + 1, j - 1),
+                                                    dly(i, j), dly(i + 1, j));
+                            va = div_by(fma(dt_rho_k2 * dda, nd, xa), den_a, rden_a);
+                            ca = dlx(i, j);
                         }
                         if (has_b) {
-                            const T dd = (i == 0 || i == g.Nx - 1) ? T(2) : T(1);
-                            T nbs = T(0);
-                            if (i > 0) nbs += idx2 * cy(i - 1, j) - idxy * cx(i - 1, j) + idxy * cx(i - 1, j + 1);
-                            if (i < g.Nx - 1) nbs += idx2 * cy(i + 1, j) + idxy * cx(i, j) - idxy * cx(i, j + 1);
-                            vb = (xb + dt_rho_k2 * dd * nbs) / (T(1) + T(2) * dt_rho_k2 * idx2);
-                            cbv = cy(i, j);
+                            const T nd = A_nbs_y<T>(idx2, idxy, dly(i - 1, j), dly(i + 1, j), dlx(i - 1, j), dlx(i - 1, j + 1),
+                                                    dlx(i, j), dlx(i, j + 1));
+                            vb = div_by(fma(dt_rho_k2 * ddb, nd, xb), den_b, rden_b);
+                            cbv = dly(i, j);
                         }
                     }
                     if (n < g.N) {
@@ -1458,6 +1341,7 @@ struct TDLaunch {
     int psi_cn;       // psi time stepping: 0 backward Euler, 1 Crank-Nicolson, 2 its kernel as written
     bool any_solveA;
     bool any_fv;  // an instance has fixed vortices (irregular potential or phase lock)
+    const ResState* res;  // the resident loop (tdr.cu), or null: a launch per sweep
 };
 
 static void* fv_psi_pre_fn(int dt) { return dt == 8 ? (void*)k_fv_psi_pre<double> : (void*)k_fv_psi_pre<float>; }
@@ -1909,8 +1793,14 @@ static TDOutcome td_core(cudaStream_t s, const TDLaunch& L, int Nt, int eqn, cud
     LoopState& hl = *hl_pinned;
     memset(&hl, 0, sizeof(hl));
     if (Nt > 0) {
+        if (L.res) {
+            if (ev0) cudaEventRecord(ev0, s);
+            o.err = res_launch(*L.res, L.insts, L.ninst, L.loop, Nt, eqn, s);
+            if (o.err != cudaSuccess) return o;
+            o.used_graph = 1;
+        }
         const int slot = eqn * 4 + (L.any_solveA ? 2 : 0) + (L.any_fv ? 1 : 0);
-        if (use_graphs && !*graph_failed) {
+        if (!o.used_graph && use_graphs && !*graph_failed) {
             if (execs[slot] == nullptr) {
                 if (build_td_graph(L, eqn, &execs[slot]) != cudaSuccess) {
                     *graph_failed = true;
@@ -1965,8 +1855,16 @@ static void fill_stats(glgpu_td_stats* stats, const InstState* hs, int n, const 
     }
 }
 
+// The resident loop runs backward Euler with the default sweep kernel selection; the
+// fixed-vortex steps, the Crank-Nicolson schemes, a loop guard in launches and the
+// host-driven loop keep a launch per sweep.
+static bool resident_ok(const glgpu_handle* h, bool use_graphs, int guard) {
+    return use_graphs && guard == 0 && h->psi_scheme == 0 && h->psi_select == 0 && !h->vpi && h->lock_n == 0;
+}
+
 int td_run(glgpu_handle* h, double dt, int Nt, int eqn, glgpu_td_stats* stats, double* elapsed_ms) {
     if (eqn < 0 || eqn > 2 || Nt < 0) return set_error(h, GLGPU_E_ARG, "glgpu_td: bad eqn or Nt");
+    const bool resident = Nt > 0 && resident_ok(h, h->use_graphs, h->loop_guard) && res_prepare(&h->res, &h, 1);
     // dt of the order-parameter iterator; the A kernel also receives it (td.py:278)
     h->inst_h.dt = dt;
     h->inst_h.fdt = (float)dt;
@@ -1985,6 +1883,7 @@ int td_run(glgpu_handle* h, double dt, int Nt, int eqn, glgpu_td_stats* stats, d
     L.psi_cn = h->psi_scheme;
     L.any_solveA = h->inst_h.solveA != 0;
     L.any_fv = h->vpi != nullptr || h->lock_n > 0;
+    L.res = resident ? &h->res : nullptr;
     TDOutcome o = td_core(h->stream, L, Nt, eqn, h->td_exec, &h->td_graph_failed, h->use_graphs, h->loop_guard,
                           elapsed_ms != nullptr,
                           h->st_gather, &ps->st, &ps->loop);
@@ -1994,6 +1893,7 @@ int td_run(glgpu_handle* h, double dt, int Nt, int eqn, glgpu_td_stats* stats, d
     h->p.rand_t = hs.rand_t;
     fill_stats(stats, &hs, 1, o);
     if (o.loop_err & kErrLoopGuard) return set_error(h, GLGPU_E_TIMEOUT, "td: Jacobi loop guard reached");
+    if (o.loop_err & kErrBarrier) return set_error(h, GLGPU_E_TIMEOUT, "td: a wait at a barrier of the time loop ran out");
     if (o.loop_err & kErrCopyWait) return set_error(h, GLGPU_E_TIMEOUT, "td: psi sweep: a bulk-copy wait ran out");
     if (hs.nan_seen) return set_error(h, GLGPU_E_NAN, "td: NaN residual (the state was updated as the reference does)");
     return GLGPU_OK;
@@ -2003,9 +1903,13 @@ int batch_td(glgpu_batch* b, double dt, int Nt, int eqn, glgpu_td_stats* stats, 
     if (eqn < 0 || eqn > 2 || Nt < 0) return batch_error(b, GLGPU_E_ARG, "batch_td: bad eqn or Nt");
     std::vector<Inst> insts(b->ninst);
     bool any_solveA = false, any_fv = false;
-    for (int q = 0; q < b->ninst; ++q)
+    bool resident = Nt > 0;
+    for (int q = 0; q < b->ninst; ++q) {
         if (b->hs[q]->psi_scheme != 0)
             return batch_error(b, GLGPU_E_ARG, "batch_td: Crank-Nicolson instances run on their own handle");
+        resident = resident && resident_ok(b->hs[q], b->use_graphs, b->loop_guard);
+    }
+    resident = resident && res_prepare(&b->res, b->hs.data(), b->ninst);
     for (int q = 0; q < b->ninst; ++q) {
         glgpu_handle* h = b->hs[q];
         cudaStreamSynchronize(h->stream);
@@ -2028,6 +1932,7 @@ int batch_td(glgpu_batch* b, double dt, int Nt, int eqn, glgpu_td_stats* stats, 
     L.psi_cn = 0;
     L.any_solveA = any_solveA;
     L.any_fv = any_fv;
+    L.res = resident ? &b->res : nullptr;
     TDOutcome o = td_core(b->stream, L, Nt, eqn, b->td_exec, &b->td_graph_failed, b->use_graphs, b->loop_guard,
                           elapsed_ms != nullptr,
                           b->gather, b->gather_pin, b->loop_pin);
@@ -2041,6 +1946,7 @@ int batch_td(glgpu_batch* b, double dt, int Nt, int eqn, glgpu_td_stats* stats, 
     }
     fill_stats(stats, b->gather_h.data(), b->ninst, o);
     if (o.loop_err & kErrLoopGuard) return batch_error(b, GLGPU_E_TIMEOUT, "batch_td: Jacobi loop guard reached");
+    if (o.loop_err & kErrBarrier) return batch_error(b, GLGPU_E_TIMEOUT, "batch_td: a wait at a barrier of the time loop ran out");
     if (o.loop_err & kErrCopyWait) return batch_error(b, GLGPU_E_TIMEOUT, "batch_td: psi sweep: a bulk-copy wait ran out");
     if (nan) return batch_error(b, GLGPU_E_NAN, "batch_td: NaN residual in at least one instance");
     return GLGPU_OK;
