@@ -504,7 +504,14 @@ void glnn_tc_wgrad_plan(int n, int h, int w, int cin, int cout, int* nz, int* ch
 int glnn_tc_wgrad(const void* dy, const void* y, int relu, const void* x1, int c1, const void* x2, int c2, float* ws,
                   void* dy_masked, int n, int h, int w, int cout, int* err, cudaStream_t s);
 
-// work layout: [split partial sums (the larger of the two plans)][bias partials]
+// nn_tile.cu: the weight gradient for the other shapes (the ReLU derivative applied to dy
+// before), its largest number of splits, and whether the switch allows it
+int glnn_tile_wgrad(const void* dy, const void* x1, int c1, const void* x2, int c2, float* ws, int n, int h, int w,
+                    int cout, int* nz, int* err, cudaStream_t s);
+int glnn_tile_wgrad_splits(int n, int h, int w, int cin, int cout);
+bool glnn_tc_tiles();
+
+// work layout: [split partial sums (the largest of the plans)][bias partials]
 // [dy * relu'(y) in bf16, for the tcgen05 path], each part 256-byte aligned
 struct WLayout {
     long long ws, bias_off, dym_off, total;
@@ -515,7 +522,8 @@ static WLayout wlayout(int n, int h, int w, int cin, int cout) {
     glnn_tc_wgrad_plan(n, h, w, cin, cout, &nz_tc, &chunk_tc);
     auto up = [](long long v) { return (v + 63) / 64 * 64; };
     WLayout L;
-    L.ws = up(std::max(q.ws_floats, (long long)nz_tc * cout * 9 * cin));
+    const int nz = std::max(nz_tc, glnn_tile_wgrad_splits(n, h, w, cin, cout));
+    L.ws = up(std::max(q.ws_floats, (long long)nz * cout * 9 * cin));
     L.bias_off = L.ws;
     L.dym_off = L.bias_off + up(q.bias_floats);
     L.total = L.dym_off + up(((long long)n * h * w * cout + 1) / 2);
@@ -548,7 +556,11 @@ int glnn_conv3x3_bwd_weight(const void* dy, const void* y, int32_t relu, const v
     if (glnn_tc_wgrad(dy, y, relu, x1, c1, x2, c2, work, work + L.dym_off, n, h, w, cout, err, s)) {
         int chunk_tc = 0;
         glnn_tc_wgrad_plan(n, h, w, cin, cout, &nz, &chunk_tc);
+    } else if (glnn_tc_tiles() &&
+               (!relu || glnn_relu_mask(dy, y, work + L.dym_off, P * cout, stream) == GLGPU_OK) &&
+               glnn_tile_wgrad(relu ? (const void*)(work + L.dym_off) : dy, x1, c1, x2, c2, work, n, h, w, cout, &nz, err, s)) {
     } else {
+        nz = q.nz;
         dim3 grid((unsigned)((cout + BM - 1) / BM), (unsigned)((9 * cin + BN - 1) / BN), (unsigned)q.nz);
         if (relu)
             k_conv_bwd_weight<1><<<grid, NT, 0, s>>>((const bf16*)dy, (const bf16*)y, (const bf16*)x1, c1, (const bf16*)x2, c2, work, n, h, w, cout, q.chunk);

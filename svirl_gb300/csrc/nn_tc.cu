@@ -14,18 +14,12 @@
 // bias, applies the ReLU and stores bfloat16.  Every wait is bounded; on a
 // timeout the kernel records an error, skips its stores and still frees its
 // tensor memory.  The weight gradient (K = pixels) is in nn.cu.
-#include <cuda.h>
-#include <cuda_bf16.h>
-#include <cuda_runtime.h>
-#include <cudaTypedefs.h>
-#include <stdint.h>
+#include "nn_tc.cuh"
 
 #include "../../include/glgpu.h"
 #include "../../include/glgpu_nn.h"
 
 namespace glnn_tc {
-
-typedef __nv_bfloat16 bf16;
 
 constexpr int TM = 128, TN = 64, TK = 64, NTH = 128;
 constexpr int A_BYTES = TM * TK * 2;        // 16 KB
@@ -37,13 +31,12 @@ constexpr int kStages = GLNN_TC_STAGES;       // operand stages in shared memory
 constexpr int STAGE_BYTES = A_BYTES + B_BYTES;
 constexpr int SMEM_BYTES = kStages * STAGE_BYTES + 32;  // stages, a barrier per stage, the TMEM address
 constexpr uint32_t kTmemCols = 64;          // FP32 accumulator: TN columns
-constexpr uint32_t kSpinLimit = 1u << 20;   // mbarrier polls before giving up
 // instruction descriptor (kind::f16): D f32 (bits 4-5 = 1), A bf16 (7-9 = 1),
 // B bf16 (10-12 = 1), both K-major (bits 15, 16 = 0), N >> 3 at 17-22, M >> 4 at 24-28
 constexpr uint32_t kIdesc = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(TN >> 3) << 17) |
                             ((uint32_t)(TM >> 4) << 24);
 
-__device__ __forceinline__ uint32_t saddr(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
+constexpr uint32_t kHi = desc_hi(1024);  // the TMA kernels' operands: eight-row groups 1 KB apart
 
 // Byte offset of element (row, k) of a K-major tile with `kb` core matrices along K:
 // core matrix (row / 8, k / 8) at ((row / 8) * kb + k / 8) * 128 B, rows of 16 B inside.
@@ -60,27 +53,6 @@ __device__ __forceinline__ uint64_t smem_desc(uint32_t start, uint32_t lbo, uint
     d |= (uint64_t)((sbo >> 4) & 0x3FFFu) << 32;
     d |= (uint64_t)1u << 46;
     return d;
-}
-
-__device__ __forceinline__ void mma_f16(uint32_t tmem_d, uint64_t adesc, uint64_t bdesc, uint32_t idesc, uint32_t acc) {
-    asm volatile(
-        "{\n .reg .pred p;\n setp.ne.b32 p, %4, 0;\n"
-        " tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n}\n" ::"r"(tmem_d),
-        "l"(adesc), "l"(bdesc), "r"(idesc), "r"(acc)
-        : "memory");
-}
-
-__device__ __forceinline__ bool wait_parity(uint32_t bar, uint32_t phase) {
-    for (uint32_t it = 0; it < kSpinLimit; ++it) {
-        uint32_t done;
-        asm volatile(
-            "{\n .reg .pred p;\n mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n selp.u32 %0, 1, 0, p;\n}\n"
-            : "=r"(done)
-            : "r"(bar), "r"(phase)
-            : "memory");
-        if (done) return true;
-    }
-    return false;
 }
 
 __device__ __forceinline__ uint4 load_cat8(const bf16* x1, int C1, const bf16* x2, int C2, int n, int sy, int sx,
@@ -299,44 +271,6 @@ constexpr int TMA_SMEM = TMA_STAGES * STAGE_BYTES + 1024 + (2 * TMA_STAGES + 2) 
 constexpr uint32_t kStageTx = (uint32_t)STAGE_BYTES;
 static_assert(TMA_STAGES >= 1 && TMA_SMEM <= 227 * 1024, "TMA conv stages exceed shared memory");
 
-// SM100 shared-memory matrix descriptor, K-major with the 128-byte swizzle:
-// start >> 4 (bits 0-13), leading offset 16 B (unused for this layout), stride
-// offset 1024 B between 8-row groups (32-45), version 1 (46-47), layout type
-// 2 = 128-byte swizzle (61-63).  A K step of 16 elements advances the start by 32 B.
-__device__ __forceinline__ uint64_t smem_desc_sw128(uint32_t start) {
-    uint64_t d = (uint64_t)((start >> 4) & 0x3FFFu);
-    d |= (uint64_t)1u << 16;
-    d |= (uint64_t)(1024u >> 4) << 32;
-    d |= (uint64_t)1u << 46;
-    d |= (uint64_t)2u << 61;
-    return d;
-}
-
-__device__ __forceinline__ void tma_load_4d(uint32_t dst, const CUtensorMap* map, int c0, int c1, int c2, int c3,
-                                            uint32_t bar) {
-    asm volatile(
-        "cp.async.bulk.tensor.4d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3, %4, %5}], "
-        "[%6];\n" ::"r"(dst),
-        "l"((uint64_t)map), "r"(c0), "r"(c1), "r"(c2), "r"(c3), "r"(bar)
-        : "memory");
-}
-
-__device__ __forceinline__ void tma_load_2d(uint32_t dst, const CUtensorMap* map, int c0, int c1, uint32_t bar) {
-    asm volatile(
-        "cp.async.bulk.tensor.2d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];\n" ::"r"(
-            dst),
-        "l"((uint64_t)map), "r"(c0), "r"(c1), "r"(bar)
-        : "memory");
-}
-
-__device__ __forceinline__ void tma_load_3d(uint32_t dst, const CUtensorMap* map, int c0, int c1, int c2, uint32_t bar) {
-    asm volatile(
-        "cp.async.bulk.tensor.3d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3, %4}], "
-        "[%5];\n" ::"r"(dst),
-        "l"((uint64_t)map), "r"(c0), "r"(c1), "r"(c2), "r"(bar)
-        : "memory");
-}
-
 // MODE 0 (forward): A = [x1 | x2] (C1 + C2 channels) shifted by +tap, B = Wb as the
 // 2-D tensor [cout][9 cin] (box: 64 rows of 64 k), out = y (Co1 = cout channels,
 // + bias, ReLU).  MODE 1 (data gradient): A = dy' (C1 = cout channels, C2 = 0: dy
@@ -354,7 +288,7 @@ k_conv_fwd_tma(const __grid_constant__ CUtensorMap ta1, const __grid_constant__ 
     uint64_t* empty = full + TMA_STAGES;
     uint64_t* done = empty + TMA_STAGES;
     uint32_t* tslot = (uint32_t*)(done + 1);
-    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    const int tid = threadIdx.x, warp = warp_id(), lane = tid & 31;
     const int m0 = blockIdx.x * TM, n0 = blockIdx.y * TN;
     const int img = m0 / (H * W), rem = m0 - img * H * W, y0 = rem / W, x0 = rem - y0 * W;
     const int nck = (C1 + C2) / TK, nk = 9 * nck;
@@ -376,7 +310,7 @@ k_conv_fwd_tma(const __grid_constant__ CUtensorMap ta1, const __grid_constant__ 
     asm volatile("tcgen05.fence::before_thread_sync;\n" ::: "memory");
     __syncthreads();
     asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
-    const uint32_t tmem = *tslot;
+    const uint32_t tmem = __shfl_sync(0xffffffffu, *tslot, 0);
     bool ok = true;
 
     // warp 0, lane 0: producer; warp 1, lane 0: MMA issuer.  The other lanes of those
@@ -404,27 +338,22 @@ k_conv_fwd_tma(const __grid_constant__ CUtensorMap ta1, const __grid_constant__ 
         }
         __syncwarp();
     } else if (warp == 1) {
-        if (lane == 0) {
+        // the whole warp in step, an elected lane issues (mma_f16)
         // MMA issuer
         for (int kc = 0; kc < nk && ok; ++kc) {
             const int st = kc % TMA_STAGES, use = kc / TMA_STAGES;
-            if (!wait_parity(saddr(full + st), (uint32_t)(use & 1))) {
+            if (!wait_parity_warp(saddr(full + st), (uint32_t)(use & 1))) {
                 ok = false;
                 break;
             }
             asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
-            const uint32_t a0 = saddr(smem + st * STAGE_BYTES), b0 = a0 + A_BYTES;
+            const uint32_t a = desc_lo(saddr(smem + st * STAGE_BYTES)), b = a + (A_BYTES >> 4);
 #pragma unroll
             for (int j = 0; j < TK / 16; ++j)
-                mma_f16(tmem, smem_desc_sw128(a0 + 32 * j), smem_desc_sw128(b0 + 32 * j), kIdesc,
-                        (kc > 0 || j > 0) ? 1u : 0u);
-            asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];\n" ::"r"(
-                             saddr(empty + st))
-                         : "memory");
+                mma_f16(tmem, a + 2 * j, kHi, b + 2 * j, kHi, kIdesc, j > 0 || kc > 0 ? 1u : 0u);
+            mma_commit(saddr(empty + st));
         }
-        asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];\n" ::"r"(saddr(done))
-                     : "memory");
-        }
+        mma_commit(saddr(done));
         __syncwarp();
     }
     // everyone: the accumulator is complete when `done` fires (the issuer commits it
@@ -444,24 +373,9 @@ k_conv_fwd_tma(const __grid_constant__ CUtensorMap ta1, const __grid_constant__ 
                 : "r"(tmem + ((uint32_t)(warp * 32) << 16) + (uint32_t)c)
                 : "memory");
             asm volatile("tcgen05.wait::ld.sync.aligned;\n" ::: "memory");
-            if (MODE == 0) {
-#pragma unroll
-                for (int q = 0; q < 16; q += 2) {
-                    const int col = n0 + c + q;
-                    float v0 = __uint_as_float(r[q]) + bias[col], v1 = __uint_as_float(r[q + 1]) + bias[col + 1];
-                    if (RELU) {
-                        v0 = fmaxf(v0, 0.f);
-                        v1 = fmaxf(v1, 0.f);
-                    }
-                    *(__nv_bfloat162*)(y + (size_t)p * Cout + col) = __floats2bfloat162_rn(v0, v1);
-                }
-            } else {
-                // output channel tile n0 lies in [o1 | o2]: both channel counts are multiples of TN
-                bf16* out = n0 < Cout ? y + (size_t)p * Cout + n0 : o2 + (size_t)p * Co2 + (n0 - Cout);
-#pragma unroll
-                for (int q = 0; q < 16; q += 2)
-                    *(__nv_bfloat162*)(out + c + q) = __floats2bfloat162_rn(__uint_as_float(r[q]), __uint_as_float(r[q + 1]));
-            }
+            // output channel tile n0 lies in [y | o2]: both channel counts are multiples of TN (forward: all in y)
+            bf16* out = MODE == 0 || n0 < Cout ? y + (size_t)p * Cout + n0 : o2 + (size_t)p * Co2 + (n0 - Cout);
+            store_cols16<MODE == 0, MODE == 0 && RELU>(r, MODE == 0 ? bias + n0 + c : nullptr, out + c);
         }
     } else if (tid == 0) {
         atomicExch(err, 1);
@@ -507,7 +421,7 @@ k_conv_tma_persist(const __grid_constant__ CUtensorMap ta1, const __grid_constan
     uint64_t* acc_full = empty + P_STAGES;
     uint64_t* acc_empty = acc_full + 2;
     uint32_t* tslot = (uint32_t*)(acc_empty + 2);
-    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    const int tid = threadIdx.x, warp = warp_id(), lane = tid & 31;
     const int nck = (C1 + C2) / TK, nk = 9 * nck;
 
     if (warp == 0) {
@@ -530,7 +444,7 @@ k_conv_tma_persist(const __grid_constant__ CUtensorMap ta1, const __grid_constan
     asm volatile("tcgen05.fence::before_thread_sync;\n" ::: "memory");
     __syncthreads();
     asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
-    const uint32_t tmem = *tslot;
+    const uint32_t tmem = __shfl_sync(0xffffffffu, *tslot, 0);
     bool ok = true;
 
     if (warp == 0) {
@@ -568,38 +482,38 @@ k_conv_tma_persist(const __grid_constant__ CUtensorMap ta1, const __grid_constan
         }
         __syncwarp();
     } else if (warp == 1) {
-        if (lane == 0) {
-            int g = 0, lt = 0;
-            for (int t = blockIdx.x; t < ntiles && ok; t += gridDim.x, ++lt) {
-                const int acc = lt & 1, ause = lt >> 1;
-                if (ause > 0 && !wait_parity(saddr(acc_empty + acc), (uint32_t)((ause + 1) & 1))) {
+        // the whole warp in step, an elected lane issues (mma_f16); stage, accumulator and
+        // parities are carried along (this warp's instructions set the MMA rate)
+        const uint32_t a0 = desc_lo(saddr(smem)), full0 = saddr(full), empty0 = saddr(empty);
+        int st = 0, acc = 0, lt = 0;
+        uint32_t ph = 0u, aph = 1u;
+        for (int t = blockIdx.x; t < ntiles && ok; t += gridDim.x, ++lt) {
+            if (lt >= 2 && !wait_parity_warp(saddr(acc_empty + acc), aph)) {
+                ok = false;
+                break;
+            }
+            const uint32_t d = tmem + (uint32_t)(acc * TN);
+            for (int kc = 0; kc < nk; ++kc) {
+                if (!wait_parity_warp(full0 + 8 * st, ph)) {
                     ok = false;
                     break;
                 }
                 asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
-                const uint32_t d = tmem + (uint32_t)(acc * TN);
-                for (int kc = 0; kc < nk; ++kc, ++g) {
-                    const int st = g % P_STAGES, use = g / P_STAGES;
-                    if (!wait_parity(saddr(full + st), (uint32_t)(use & 1))) {
-                        ok = false;
-                        break;
-                    }
-                    asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
-                    const uint32_t a0 = saddr(smem + st * STAGE_BYTES), b0 = a0 + A_BYTES;
+                const uint32_t a = a0 + (uint32_t)st * (STAGE_BYTES >> 4), b = a + (A_BYTES >> 4);
 #pragma unroll
-                    for (int j = 0; j < TK / 16; ++j)
-                        mma_f16(d, smem_desc_sw128(a0 + 32 * j), smem_desc_sw128(b0 + 32 * j), kIdesc,
-                                (kc > 0 || j > 0) ? 1u : 0u);
-                    asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];\n" ::"r"(
-                                     saddr(empty + st))
-                                 : "memory");
+                for (int j = 0; j < TK / 16; ++j)
+                    mma_f16(d, a + 2 * j, kHi, b + 2 * j, kHi, kIdesc, j > 0 || kc > 0 ? 1u : 0u);
+                mma_commit(empty0 + 8 * st);
+                if (++st == P_STAGES) {
+                    st = 0;
+                    ph ^= 1u;
                 }
-                // the tile's accumulator is complete once its MMAs are (committed even
-                // after a failed wait, so the epilogue's wait ends)
-                asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];\n" ::"r"(
-                                 saddr(acc_full + acc))
-                             : "memory");
             }
+            // the tile's accumulator is complete once its MMAs are (committed even
+            // after a failed wait, so the epilogue's wait ends)
+            mma_commit(saddr(acc_full + acc));
+            acc ^= 1;
+            if (acc == 0) aph ^= 1u;
         }
         __syncwarp();
     } else {
@@ -626,423 +540,11 @@ k_conv_tma_persist(const __grid_constant__ CUtensorMap ta1, const __grid_constan
                     : "r"(tmem + ((uint32_t)(quarter * 32) << 16) + (uint32_t)(acc * TN + c))
                     : "memory");
                 asm volatile("tcgen05.wait::ld.sync.aligned;\n" ::: "memory");
-                if (MODE == 0) {
-#pragma unroll
-                    for (int q = 0; q < 16; q += 2) {
-                        const int col = n0 + c + q;
-                        float v0 = __uint_as_float(r[q]) + bias[col], v1 = __uint_as_float(r[q + 1]) + bias[col + 1];
-                        if (RELU) {
-                            v0 = fmaxf(v0, 0.f);
-                            v1 = fmaxf(v1, 0.f);
-                        }
-                        *(__nv_bfloat162*)(y + (size_t)p * Cout + col) = __floats2bfloat162_rn(v0, v1);
-                    }
-                } else {
-                    bf16* out = n0 < Cout ? y + (size_t)p * Cout + n0 : o2 + (size_t)p * Co2 + (n0 - Cout);
-#pragma unroll
-                    for (int q = 0; q < 16; q += 2)
-                        *(__nv_bfloat162*)(out + c + q) =
-                            __floats2bfloat162_rn(__uint_as_float(r[q]), __uint_as_float(r[q + 1]));
-                }
+                // output channel tile n0 lies in [y | o2]: both channel counts are multiples of TN (forward: all in y)
+                bf16* out = MODE == 0 || n0 < Cout ? y + (size_t)p * Cout + n0 : o2 + (size_t)p * Co2 + (n0 - Cout);
+                store_cols16<MODE == 0, MODE == 0 && RELU>(r, MODE == 0 ? bias + n0 + c : nullptr, out + c);
             }
             // this warp has read the accumulator: the MMAs of the tile after next may use it
-            asm volatile("tcgen05.fence::before_thread_sync;\n" ::: "memory");
-            __syncwarp();
-            if (lane == 0)
-                asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];\n" ::"r"(saddr(acc_empty + acc)) : "memory");
-        }
-    }
-    if (!ok) atomicExch(err, 1);
-    asm volatile("tcgen05.fence::before_thread_sync;\n" ::: "memory");
-    __syncthreads();
-    if (warp == 0)
-        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;\n" ::"r"(tmem), "r"(kTmemColsP) : "memory");
-}
-
-// ---------------------------------------------------------------------------
-// k_conv_tma_persist with the B operand resident: a CTA works on one output-channel
-// tile (n-tile = blockIdx.x % NT) and loops over pixel tiles; it loads the n-tile's
-// weights (all 9 taps x input-channel chunks, 8 KB each) into shared memory once,
-// and only the shifted activation boxes (16 KB per chunk) stream through the ring.
-// This removes the weight re-reads, a third of the bytes that move from L2 into the
-// SMs.  Used when the weights of an n-tile fit (at most two 64-channel input
-// chunks); the same MMAs in the same order, so the same values bitwise.
-// ---------------------------------------------------------------------------
-constexpr int BR_MAX_CHUNKS = 18;  // 9 taps x 2 input-channel chunks
-__host__ __device__ constexpr int br_smem_bytes(int nk) {
-    return P_STAGES * A_BYTES + nk * B_BYTES + 1024 + (2 * P_STAGES + 5) * 8 + 16;
-}
-static_assert(br_smem_bytes(BR_MAX_CHUNKS) <= 227 * 1024, "resident-weight conv exceeds shared memory");
-
-template <int MODE, int RELU>
-__global__ void __launch_bounds__(P_THREADS)
-k_conv_tma_bres(const __grid_constant__ CUtensorMap ta1, const __grid_constant__ CUtensorMap ta2,
-                const __grid_constant__ CUtensorMap tb, const float* __restrict__ bias, bf16* __restrict__ y, int Cout,
-                bf16* __restrict__ o2, int Co2, int C1, int C2, int H, int W, int nmt, int NT, int* err) {
-    extern __shared__ unsigned char smem_raw[];
-    unsigned char* smem = (unsigned char*)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
-    const int nck = (C1 + C2) / TK, nk = 9 * nck;
-    unsigned char* bres = smem + P_STAGES * A_BYTES;
-    uint64_t* full = (uint64_t*)(bres + nk * B_BYTES);
-    uint64_t* empty = full + P_STAGES;
-    uint64_t* acc_full = empty + P_STAGES;
-    uint64_t* acc_empty = acc_full + 2;
-    uint64_t* b_full = acc_empty + 2;
-    uint32_t* tslot = (uint32_t*)(b_full + 1);
-    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-    const int cpn = gridDim.x / NT;  // CTAs per n-tile
-    const int nt = blockIdx.x % NT, mt0 = blockIdx.x / NT, n0 = nt * TN;
-
-    if (warp == 0) {
-        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;\n" ::"r"(saddr(tslot)),
-                     "r"(kTmemColsP)
-                     : "memory");
-        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;\n" ::: "memory");
-    }
-    if (tid == 0) {
-        for (int q = 0; q < P_STAGES; ++q) {
-            asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;\n" ::"r"(saddr(full + q)) : "memory");
-            asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;\n" ::"r"(saddr(empty + q)) : "memory");
-        }
-        for (int q = 0; q < 2; ++q) {
-            asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;\n" ::"r"(saddr(acc_full + q)) : "memory");
-            asm volatile("mbarrier.init.shared::cta.b64 [%0], 4;\n" ::"r"(saddr(acc_empty + q)) : "memory");
-        }
-        asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;\n" ::"r"(saddr(b_full)) : "memory");
-        asm volatile("fence.mbarrier_init.release.cluster;\n" ::: "memory");
-    }
-    asm volatile("tcgen05.fence::before_thread_sync;\n" ::: "memory");
-    __syncthreads();
-    asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
-    const uint32_t tmem = *tslot;
-    bool ok = true;
-
-    if (warp == 0) {
-        if (lane == 0) {
-            // the n-tile's weights, once
-            asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;\n" ::"r"(saddr(b_full)),
-                         "r"((uint32_t)(nk * B_BYTES))
-                         : "memory");
-            for (int kc = 0; kc < nk; ++kc) {
-                const int tap = kc / nck, c = (kc - tap * nck) * TK;
-                const uint32_t b_dst = saddr(bres + kc * B_BYTES);
-                if (MODE == 0) tma_load_2d(b_dst, &tb, tap * (C1 + C2) + c, n0, saddr(b_full));
-                else tma_load_3d(b_dst, &tb, c, n0, tap, saddr(b_full));
-            }
-            int g = 0;
-            for (int mt = mt0; mt < nmt && ok; mt += cpn) {
-                const int m0 = mt * TM;
-                const int img = m0 / (H * W), rem = m0 - img * H * W, y0 = rem / W, x0 = rem - y0 * W;
-                for (int kc = 0; kc < nk; ++kc, ++g) {
-                    const int st = g % P_STAGES, use = g / P_STAGES;
-                    if (use > 0 && !wait_parity(saddr(empty + st), (uint32_t)((use + 1) & 1))) {
-                        ok = false;
-                        break;
-                    }
-                    const int tap = kc / nck, cc = kc - tap * nck;
-                    const int sgn = MODE == 0 ? 1 : -1;
-                    const int dy = sgn * (tap / 3 - 1), dx = sgn * (tap % 3 - 1);
-                    const int c = cc * TK;
-                    const uint32_t a_dst = saddr(smem + st * A_BYTES);
-                    asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;\n" ::"r"(saddr(full + st)),
-                                 "r"((uint32_t)A_BYTES)
-                                 : "memory");
-                    if (c < C1) tma_load_4d(a_dst, &ta1, c, x0 + dx, y0 + dy, img, saddr(full + st));
-                    else tma_load_4d(a_dst, &ta2, c - C1, x0 + dx, y0 + dy, img, saddr(full + st));
-                }
-            }
-            // copies still in flight land before the CTA leaves (bounded waits)
-            wait_parity(saddr(b_full), 0u);
-            for (int q = 0; q < P_STAGES && q < g; ++q) {
-                const int gg = g - 1 - q, st = gg % P_STAGES, use = gg / P_STAGES;
-                wait_parity(saddr(full + st), (uint32_t)(use & 1));
-            }
-        }
-        __syncwarp();
-    } else if (warp == 1) {
-        if (lane == 0) {
-            if (!wait_parity(saddr(b_full), 0u)) ok = false;
-            asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
-            int g = 0, lt = 0;
-            for (int mt = mt0; mt < nmt && ok; mt += cpn, ++lt) {
-                const int acc = lt & 1, ause = lt >> 1;
-                if (ause > 0 && !wait_parity(saddr(acc_empty + acc), (uint32_t)((ause + 1) & 1))) {
-                    ok = false;
-                    break;
-                }
-                asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
-                const uint32_t d = tmem + (uint32_t)(acc * TN);
-                for (int kc = 0; kc < nk; ++kc, ++g) {
-                    const int st = g % P_STAGES, use = g / P_STAGES;
-                    if (!wait_parity(saddr(full + st), (uint32_t)(use & 1))) {
-                        ok = false;
-                        break;
-                    }
-                    asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
-                    const uint32_t a0 = saddr(smem + st * A_BYTES), b0 = saddr(bres + kc * B_BYTES);
-#pragma unroll
-                    for (int j = 0; j < TK / 16; ++j)
-                        mma_f16(d, smem_desc_sw128(a0 + 32 * j), smem_desc_sw128(b0 + 32 * j), kIdesc,
-                                (kc > 0 || j > 0) ? 1u : 0u);
-                    asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];\n" ::"r"(
-                                     saddr(empty + st))
-                                 : "memory");
-                }
-                asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];\n" ::"r"(
-                                 saddr(acc_full + acc))
-                             : "memory");
-            }
-        }
-        __syncwarp();
-    } else {
-        const int quarter = warp & 3;
-        int lt = 0;
-        for (int mt = mt0; mt < nmt; mt += cpn, ++lt) {
-            const int acc = lt & 1, ause = lt >> 1;
-            const bool got = wait_parity(saddr(acc_full + acc), (uint32_t)(ause & 1));
-            asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
-            if (!got) {
-                ok = false;
-                break;
-            }
-            const int p = mt * TM + quarter * 32 + lane;
-#pragma unroll
-            for (int c = 0; c < TN; c += 16) {
-                uint32_t r[16];
-                asm volatile(
-                    "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%16];\n"
-                    : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]),
-                      "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
-                    : "r"(tmem + ((uint32_t)(quarter * 32) << 16) + (uint32_t)(acc * TN + c))
-                    : "memory");
-                asm volatile("tcgen05.wait::ld.sync.aligned;\n" ::: "memory");
-                if (MODE == 0) {
-#pragma unroll
-                    for (int q = 0; q < 16; q += 2) {
-                        const int col = n0 + c + q;
-                        float v0 = __uint_as_float(r[q]) + bias[col], v1 = __uint_as_float(r[q + 1]) + bias[col + 1];
-                        if (RELU) {
-                            v0 = fmaxf(v0, 0.f);
-                            v1 = fmaxf(v1, 0.f);
-                        }
-                        *(__nv_bfloat162*)(y + (size_t)p * Cout + col) = __floats2bfloat162_rn(v0, v1);
-                    }
-                } else {
-                    bf16* out = n0 < Cout ? y + (size_t)p * Cout + n0 : o2 + (size_t)p * Co2 + (n0 - Cout);
-#pragma unroll
-                    for (int q = 0; q < 16; q += 2)
-                        *(__nv_bfloat162*)(out + c + q) =
-                            __floats2bfloat162_rn(__uint_as_float(r[q]), __uint_as_float(r[q + 1]));
-                }
-            }
-            asm volatile("tcgen05.fence::before_thread_sync;\n" ::: "memory");
-            __syncwarp();
-            if (lane == 0)
-                asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];\n" ::"r"(saddr(acc_empty + acc)) : "memory");
-        }
-    }
-    if (!ok) atomicExch(err, 1);
-    asm volatile("tcgen05.fence::before_thread_sync;\n" ::: "memory");
-    __syncthreads();
-    if (warp == 0)
-        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;\n" ::"r"(tmem), "r"(kTmemColsP) : "memory");
-}
-
-// ---------------------------------------------------------------------------
-// k_conv_tma_bres with each input row loaded once: for 128-pixel tiles that lie in
-// one image row (w a multiple of 128), a stage holds one tap row dy of the tile, i.e.
-// for every input-channel chunk one box of 130 pixels (the tile and a one-pixel halo
-// on each side, zeros outside the image) x 64 channels.  The three taps dx of that row
-// read the same box from pixel 0, 1 or 2: the A descriptor starts 0, 128 or 256 bytes
-// into the 1024-byte swizzle atom (see smem_desc_sw128_at).  The activation bytes
-// moved from L2 per tile fall from 9 x 16 KB to 3 x 16.25 KB per channel chunk.  The
-// MMAs run in the order of the other kernels (tap-major, channel chunk inner), so
-// the results are the same bitwise.
-// ---------------------------------------------------------------------------
-constexpr int HALO_PX = TM + 2;                        // 130 pixels per box
-constexpr int HALO_BOX = HALO_PX * TK * 2;             // 16,640 bytes
-constexpr int HALO_SLOT = 17 * 1024;                   // a box's 1024-aligned slot
-__host__ __device__ constexpr int halo_stages(int nck) { return nck == 1 ? 3 : 2; }
-__host__ __device__ constexpr int halo_smem_bytes(int nck) {
-    return halo_stages(nck) * nck * HALO_SLOT + 9 * nck * B_BYTES + 1024 + (2 * 3 + 5) * 8 + 16;
-}
-static_assert(halo_smem_bytes(1) <= 227 * 1024 && halo_smem_bytes(2) <= 227 * 1024, "halo conv exceeds shared memory");
-
-// A view starting 128 or 256 bytes into a swizzle atom: the MMA applies the 128-byte
-// swizzle by the absolute shared-memory address bits, as the TMA copy that wrote the
-// box did, so the descriptor is the plain one (its base-offset field stays 0; set to
-// (start >> 7) & 7 it gave wrong products, measured).
-__device__ __forceinline__ uint64_t smem_desc_sw128_at(uint32_t start) { return smem_desc_sw128(start); }
-
-template <int MODE, int RELU>
-__global__ void __launch_bounds__(P_THREADS)
-k_conv_tma_halo(const __grid_constant__ CUtensorMap ta1, const __grid_constant__ CUtensorMap ta2,
-                const __grid_constant__ CUtensorMap tb, const float* __restrict__ bias, bf16* __restrict__ y, int Cout,
-                bf16* __restrict__ o2, int Co2, int C1, int C2, int H, int W, int nmt, int NT, int* err) {
-    extern __shared__ unsigned char smem_raw[];
-    unsigned char* smem = (unsigned char*)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
-    const int nck = (C1 + C2) / TK, nk = 9 * nck, S = halo_stages(nck);
-    const int stage_bytes = nck * HALO_SLOT;
-    unsigned char* bres = smem + S * stage_bytes;
-    uint64_t* full = (uint64_t*)(bres + nk * B_BYTES);
-    uint64_t* empty = full + 3;
-    uint64_t* acc_full = empty + 3;
-    uint64_t* acc_empty = acc_full + 2;
-    uint64_t* b_full = acc_empty + 2;
-    uint32_t* tslot = (uint32_t*)(b_full + 1);
-    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-    const int cpn = gridDim.x / NT;
-    const int nt = blockIdx.x % NT, mt0 = blockIdx.x / NT, n0 = nt * TN;
-    const int sgn = MODE == 0 ? 1 : -1;
-
-    if (warp == 0) {
-        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;\n" ::"r"(saddr(tslot)),
-                     "r"(kTmemColsP)
-                     : "memory");
-        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;\n" ::: "memory");
-    }
-    if (tid == 0) {
-        for (int q = 0; q < S; ++q) {
-            asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;\n" ::"r"(saddr(full + q)) : "memory");
-            asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;\n" ::"r"(saddr(empty + q)) : "memory");
-        }
-        for (int q = 0; q < 2; ++q) {
-            asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;\n" ::"r"(saddr(acc_full + q)) : "memory");
-            asm volatile("mbarrier.init.shared::cta.b64 [%0], 4;\n" ::"r"(saddr(acc_empty + q)) : "memory");
-        }
-        asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;\n" ::"r"(saddr(b_full)) : "memory");
-        asm volatile("fence.mbarrier_init.release.cluster;\n" ::: "memory");
-    }
-    asm volatile("tcgen05.fence::before_thread_sync;\n" ::: "memory");
-    __syncthreads();
-    asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
-    const uint32_t tmem = *tslot;
-    bool ok = true;
-
-    if (warp == 0) {
-        if (lane == 0) {
-            asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;\n" ::"r"(saddr(b_full)),
-                         "r"((uint32_t)(nk * B_BYTES))
-                         : "memory");
-            for (int kc = 0; kc < nk; ++kc) {
-                const int tap = kc / nck, c = (kc - tap * nck) * TK;
-                const uint32_t b_dst = saddr(bres + kc * B_BYTES);
-                if (MODE == 0) tma_load_2d(b_dst, &tb, tap * (C1 + C2) + c, n0, saddr(b_full));
-                else tma_load_3d(b_dst, &tb, c, n0, tap, saddr(b_full));
-            }
-            int g = 0;  // stages filled, across tiles
-            for (int mt = mt0; mt < nmt && ok; mt += cpn) {
-                const int m0 = mt * TM;
-                const int img = m0 / (H * W), rem = m0 - img * H * W, y0 = rem / W, x0 = rem - y0 * W;
-                for (int ty = 0; ty < 3; ++ty, ++g) {
-                    const int st = g % S, use = g / S;
-                    if (use > 0 && !wait_parity(saddr(empty + st), (uint32_t)((use + 1) & 1))) {
-                        ok = false;
-                        break;
-                    }
-                    asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;\n" ::"r"(saddr(full + st)),
-                                 "r"((uint32_t)(nck * HALO_BOX))
-                                 : "memory");
-                    const int yy = y0 + sgn * (ty - 1);
-                    for (int cc = 0; cc < nck; ++cc) {
-                        const int c = cc * TK;
-                        const uint32_t dst = saddr(smem + st * stage_bytes + cc * HALO_SLOT);
-                        if (c < C1) tma_load_4d(dst, &ta1, c, x0 - 1, yy, img, saddr(full + st));
-                        else tma_load_4d(dst, &ta2, c - C1, x0 - 1, yy, img, saddr(full + st));
-                    }
-                }
-            }
-            wait_parity(saddr(b_full), 0u);
-            for (int q = 0; q < S && q < g; ++q) {
-                const int gg = g - 1 - q, st = gg % S, use = gg / S;
-                wait_parity(saddr(full + st), (uint32_t)(use & 1));
-            }
-        }
-        __syncwarp();
-    } else if (warp == 1) {
-        if (lane == 0) {
-            if (!wait_parity(saddr(b_full), 0u)) ok = false;
-            asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
-            int g = 0, lt = 0;
-            for (int mt = mt0; mt < nmt && ok; mt += cpn, ++lt) {
-                const int acc = lt & 1, ause = lt >> 1;
-                if (ause > 0 && !wait_parity(saddr(acc_empty + acc), (uint32_t)((ause + 1) & 1))) {
-                    ok = false;
-                    break;
-                }
-                asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
-                const uint32_t d = tmem + (uint32_t)(acc * TN);
-                for (int ty = 0; ty < 3; ++ty, ++g) {
-                    const int st = g % S, use = g / S;
-                    if (!wait_parity(saddr(full + st), (uint32_t)(use & 1))) {
-                        ok = false;
-                        break;
-                    }
-                    asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
-                    for (int tx = 0; tx < 3; ++tx) {
-                        // pixel offset of the view in the box: +tx-1 (forward) or -(tx-1) (data gradient)
-                        const int off = MODE == 0 ? tx : 2 - tx;
-                        for (int cc = 0; cc < nck; ++cc) {
-                            const int kc = (ty * 3 + tx) * nck + cc;
-                            const uint32_t a0 = saddr(smem + st * stage_bytes + cc * HALO_SLOT) + 128u * off;
-                            const uint32_t b0 = saddr(bres + kc * B_BYTES);
-#pragma unroll
-                            for (int j = 0; j < TK / 16; ++j)
-                                mma_f16(d, smem_desc_sw128_at(a0 + 32 * j), smem_desc_sw128(b0 + 32 * j), kIdesc,
-                                        (kc > 0 || j > 0) ? 1u : 0u);
-                        }
-                    }
-                    asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];\n" ::"r"(
-                                     saddr(empty + st))
-                                 : "memory");
-                }
-                asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];\n" ::"r"(
-                                 saddr(acc_full + acc))
-                             : "memory");
-            }
-        }
-        __syncwarp();
-    } else {
-        const int quarter = warp & 3;
-        int lt = 0;
-        for (int mt = mt0; mt < nmt; mt += cpn, ++lt) {
-            const int acc = lt & 1, ause = lt >> 1;
-            const bool got = wait_parity(saddr(acc_full + acc), (uint32_t)(ause & 1));
-            asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
-            if (!got) {
-                ok = false;
-                break;
-            }
-            const int p = mt * TM + quarter * 32 + lane;
-#pragma unroll
-            for (int c = 0; c < TN; c += 16) {
-                uint32_t r[16];
-                asm volatile(
-                    "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%16];\n"
-                    : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]),
-                      "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
-                    : "r"(tmem + ((uint32_t)(quarter * 32) << 16) + (uint32_t)(acc * TN + c))
-                    : "memory");
-                asm volatile("tcgen05.wait::ld.sync.aligned;\n" ::: "memory");
-                if (MODE == 0) {
-#pragma unroll
-                    for (int q = 0; q < 16; q += 2) {
-                        const int col = n0 + c + q;
-                        float v0 = __uint_as_float(r[q]) + bias[col], v1 = __uint_as_float(r[q + 1]) + bias[col + 1];
-                        if (RELU) {
-                            v0 = fmaxf(v0, 0.f);
-                            v1 = fmaxf(v1, 0.f);
-                        }
-                        *(__nv_bfloat162*)(y + (size_t)p * Cout + col) = __floats2bfloat162_rn(v0, v1);
-                    }
-                } else {
-                    bf16* out = n0 < Cout ? y + (size_t)p * Cout + n0 : o2 + (size_t)p * Co2 + (n0 - Cout);
-#pragma unroll
-                    for (int q = 0; q < 16; q += 2)
-                        *(__nv_bfloat162*)(out + c + q) =
-                            __floats2bfloat162_rn(__uint_as_float(r[q]), __uint_as_float(r[q + 1]));
-                }
-            }
             asm volatile("tcgen05.fence::before_thread_sync;\n" ::: "memory");
             __syncwarp();
             if (lane == 0)
@@ -1088,18 +590,6 @@ static_assert(WG_STAGES >= 1 && WG_SMEM <= 227 * 1024, "weight-gradient stages e
 // kIdesc (M = 128, N = 64, bf16 -> f32) with A and B MN-major (bits 15, 16)
 constexpr uint32_t kIdescMN = kIdesc | (1u << 15) | (1u << 16);
 
-// SM100 shared-memory matrix descriptor, MN-major with the 128-byte swizzle:
-// leading byte offset = distance between 64-element atoms along M or N, stride
-// byte offset = distance between 8-row groups along K (1024 B here).
-__device__ __forceinline__ uint64_t smem_desc_sw128_mn(uint32_t start, uint32_t lbo) {
-    uint64_t d = (uint64_t)((start >> 4) & 0x3FFFu);
-    d |= (uint64_t)((lbo >> 4) & 0x3FFFu) << 16;
-    d |= (uint64_t)(1024u >> 4) << 32;
-    d |= (uint64_t)1u << 46;
-    d |= (uint64_t)2u << 61;
-    return d;
-}
-
 __global__ void __launch_bounds__(NTH)
 k_conv_wgrad_tma(const __grid_constant__ CUtensorMap tx1, const __grid_constant__ CUtensorMap tx2,
                  const __grid_constant__ CUtensorMap tdy, float* __restrict__ ws, int C1, int C2, int Cout, int H,
@@ -1110,7 +600,7 @@ k_conv_wgrad_tma(const __grid_constant__ CUtensorMap tx1, const __grid_constant_
     uint64_t* empty = full + WG_STAGES;
     uint64_t* done = empty + WG_STAGES;
     uint32_t* tslot = (uint32_t*)(done + 1);
-    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    const int tid = threadIdx.x, warp = warp_id(), lane = tid & 31;
     const int Cin = C1 + C2, nco = Cout / 64, nci = Cin / 64;
     int t = blockIdx.x;
     const int oc = t % nco;
@@ -1140,7 +630,7 @@ k_conv_wgrad_tma(const __grid_constant__ CUtensorMap tx1, const __grid_constant_
     asm volatile("tcgen05.fence::before_thread_sync;\n" ::: "memory");
     __syncthreads();
     asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
-    const uint32_t tmem = *tslot;
+    const uint32_t tmem = __shfl_sync(0xffffffffu, *tslot, 0);
     bool ok = true;
 
     if (nk > 0) {
@@ -1166,27 +656,21 @@ k_conv_wgrad_tma(const __grid_constant__ CUtensorMap tx1, const __grid_constant_
             }
             __syncwarp();
         } else if (warp == 1) {
-            if (lane == 0) {
+            // the whole warp in step, an elected lane issues (mma_f16)
             for (int kc = 0; kc < nk && ok; ++kc) {
                 const int st = kc % WG_STAGES, use = kc / WG_STAGES;
-                if (!wait_parity(saddr(full + st), (uint32_t)(use & 1))) {
+                if (!wait_parity_warp(saddr(full + st), (uint32_t)(use & 1))) {
                     ok = false;
                     break;
                 }
                 asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
-                const uint32_t a0 = saddr(smem + st * WG_STAGE), b0 = a0 + 2 * WG_BOX;
+                const uint32_t a = desc_lo_mn(saddr(smem + st * WG_STAGE), WG_BOX), b = a + ((2 * WG_BOX) >> 4);
 #pragma unroll
                 for (int j = 0; j < WG_PX / 16; ++j)
-                    mma_f16(tmem, smem_desc_sw128_mn(a0 + 2048 * j, WG_BOX), smem_desc_sw128_mn(b0 + 2048 * j, WG_BOX),
-                            kIdescMN, (kc > 0 || j > 0) ? 1u : 0u);
-                asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];\n" ::"r"(
-                                 saddr(empty + st))
-                             : "memory");
+                    mma_f16(tmem, a + 128 * j, kHi, b + 128 * j, kHi, kIdescMN, j > 0 || kc > 0 ? 1u : 0u);
+                mma_commit(saddr(empty + st));
             }
-            asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];\n" ::"r"(
-                             saddr(done))
-                         : "memory");
-            }
+            mma_commit(saddr(done));
             __syncwarp();
         }
         if (!wait_parity(saddr(done), 0u)) ok = false;
@@ -1249,20 +733,6 @@ template <int MODE, int RELU> static cudaError_t conv_tc_smem_attr() {
 // --- TMA forward: tensor maps and the shapes it takes -------------------------
 static int g_conv_tma = 2;  // glnn_set_conv_tma: 0 thread gather, 1 TMA per tile, 2 TMA persistent
 
-static PFN_cuTensorMapEncodeTiled_v12000 tmap_encoder() {
-    static PFN_cuTensorMapEncodeTiled_v12000 fn = nullptr;
-    static bool tried = false;
-    if (!tried) {
-        tried = true;
-        void* p = nullptr;
-        cudaDriverEntryPointQueryResult q;
-        if (cudaGetDriverEntryPointByVersion("cuTensorMapEncodeTiled", &p, 12000, cudaEnableDefault, &q) == cudaSuccess &&
-            q == cudaDriverEntryPointSuccess)
-            fn = (PFN_cuTensorMapEncodeTiled_v12000)p;
-    }
-    return fn;
-}
-
 // activations [n][h][w][c] (bf16), box = 64 channels x one tile of `px` pixels
 // (whole rows or a run of one row)
 static bool act_map(CUtensorMap* m, const void* base, int c, int n, int h, int w, int px = TM) {
@@ -1272,20 +742,6 @@ static bool act_map(CUtensorMap* m, const void* base, int c, int n, int h, int w
     cuuint64_t dims[4] = {(cuuint64_t)c, (cuuint64_t)w, (cuuint64_t)h, (cuuint64_t)n};
     cuuint64_t strides[3] = {(cuuint64_t)c * 2, (cuuint64_t)w * c * 2, (cuuint64_t)h * w * c * 2};
     cuuint32_t box[4] = {(cuuint32_t)TK, (cuuint32_t)wb, (cuuint32_t)hb, 1u};
-    cuuint32_t es[4] = {1u, 1u, 1u, 1u};
-    return enc(m, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 4, const_cast<void*>(base), dims, strides, box, es,
-               CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
-               CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
-}
-
-// activations [n][h][w][c] (bf16), box = 64 channels x 130 pixels of one row (a
-// 128-pixel tile with a one-pixel halo on each side)
-static bool act_map_halo(CUtensorMap* m, const void* base, int c, int n, int h, int w) {
-    PFN_cuTensorMapEncodeTiled_v12000 enc = tmap_encoder();
-    if (!enc) return false;
-    cuuint64_t dims[4] = {(cuuint64_t)c, (cuuint64_t)w, (cuuint64_t)h, (cuuint64_t)n};
-    cuuint64_t strides[3] = {(cuuint64_t)c * 2, (cuuint64_t)w * c * 2, (cuuint64_t)h * w * c * 2};
-    cuuint32_t box[4] = {(cuuint32_t)TK, (cuuint32_t)HALO_PX, 1u, 1u};
     cuuint32_t es[4] = {1u, 1u, 1u, 1u};
     return enc(m, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 4, const_cast<void*>(base), dims, strides, box, es,
                CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
@@ -1310,6 +766,14 @@ static bool weight_map(CUtensorMap* m, const void* base, long long k, long long 
 static bool conv_tma_shape_ok(int c1, int c2, int h, int w, int cout) {
     return c1 % TK == 0 && c2 % TK == 0 && cout % TN == 0 && ((long long)h * w) % TM == 0 && (w % TM == 0 || TM % w == 0);
 }
+
+// Up to two 64-channel input chunks go to the tile kernel (nn_tile.cu), which loads an
+// input box once for all taps: 64 images, us, nine boxes per tile with the weights resident
+// / tile kernel: 64 -> 64 at 64^2 45 / 23, 64 -> 128 at 32^2 27 / 15, 128 -> 128 at 32^2 45 /
+// 27, at 16^2 17 / 13; one box per tap row (w = 128), 32 images 64 -> 64: 47 / 47.  With more
+// chunks its weights leave room for 32 or 16 output channels per CTA and the input is read
+// again for each: 128 + 64 -> 64 at 64^2 here 119, there 147; 128 + 128 -> 128 at 32^2 76 / 166.
+static bool tile_better(int cin) { return g_conv_tma == 2 && cin <= 2 * TK; }
 
 template <int MODE, int RELU> static cudaError_t conv_tma_smem_attr() {
     static cudaError_t e =
@@ -1336,41 +800,6 @@ template <int MODE, int RELU> static cudaError_t conv_persist_smem_attr() {
     return e;
 }
 
-template <int MODE, int RELU> static cudaError_t conv_bres_smem_attr() {
-    static cudaError_t e = cudaFuncSetAttribute(k_conv_tma_bres<MODE, RELU>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                                br_smem_bytes(BR_MAX_CHUNKS));
-    return e;
-}
-
-template <int MODE, int RELU> static cudaError_t conv_halo_smem_attr() {
-    static cudaError_t e = cudaFuncSetAttribute(k_conv_tma_halo<MODE, RELU>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                                halo_smem_bytes(2));
-    return e;
-}
-template <int MODE, int RELU> static int halo_grid(int NT, int nmt, int smem) {
-    int dev = 0, sms = 0, per = 0;
-    cudaGetDevice(&dev);
-    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, k_conv_tma_halo<MODE, RELU>, P_THREADS, smem);
-    int cpn = (sms > 0 ? sms : 152) * (per > 0 ? per : 1) / NT;
-    cpn = cpn < 1 ? 1 : (cpn > nmt ? nmt : cpn);
-    return NT * cpn;
-}
-// the halo kernel takes 128-pixel tiles inside one image row and at most two input chunks
-static bool halo_ok(int w, int nck) { return g_conv_tma == 2 && w % TM == 0 && nck >= 1 && nck <= 2; }
-
-// grid of the resident-weight kernel: NT x (CTAs per n-tile), the CTAs that fit on
-// all SMs at this shared-memory size, at most one per pixel tile of an n-tile
-template <int MODE, int RELU> static int bres_grid(int NT, int nmt, int smem) {
-    int dev = 0, sms = 0, per = 0;
-    cudaGetDevice(&dev);
-    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, k_conv_tma_bres<MODE, RELU>, P_THREADS, smem);
-    int cpn = (sms > 0 ? sms : 152) * (per > 0 ? per : 1) / NT;
-    cpn = cpn < 1 ? 1 : (cpn > nmt ? nmt : cpn);
-    return NT * cpn;
-}
-
 // grid of the persistent kernel: its resident CTAs on every SM, at most one per tile
 static int persist_grid(int ntiles) {
     static int ctas = 0;
@@ -1388,25 +817,10 @@ static int persist_grid(int ntiles) {
 // data gradient without a ReLU derivative (dy already masked) by TMA: 1 launched, 0 not taken
 static int conv_bwd_data_tma(const void* dy, const void* wt, void* dx1, int c1, void* dx2, int c2, int n, int h, int w,
                              int cout, int* err, cudaStream_t s) {
-    if (!g_conv_tma || !conv_tma_shape_ok(c1, c2, h, w, cout)) return 0;
+    if (!g_conv_tma || !conv_tma_shape_ok(c1, c2, h, w, cout) || tile_better(cout)) return 0;
     CUtensorMap ta, tb;
     if (!act_map(&ta, dy, cout, n, h, w) || !weight_t_map(&tb, wt, c1 + c2, cout)) return 0;
     const long long P = (long long)n * h * w;
-    if (halo_ok(w, cout / TK)) {
-        CUtensorMap th;
-        if (!act_map_halo(&th, dy, cout, n, h, w) || conv_halo_smem_attr<1, 0>() != cudaSuccess) return 0;
-        const int nmt = (int)(P / TM), NT = (c1 + c2) / TN, smem = halo_smem_bytes(cout / TK);
-        k_conv_tma_halo<1, 0><<<halo_grid<1, 0>(NT, nmt, smem), P_THREADS, smem, s>>>(
-            th, th, tb, nullptr, (bf16*)dx1, c1, (bf16*)dx2, c2, cout, 0, h, w, nmt, NT, err);
-        return 1;
-    }
-    if (g_conv_tma == 2 && 9 * (cout / TK) <= BR_MAX_CHUNKS) {
-        if (conv_bres_smem_attr<1, 0>() != cudaSuccess) return 0;
-        const int nmt = (int)(P / TM), NT = (c1 + c2) / TN, smem = br_smem_bytes(9 * (cout / TK));
-        k_conv_tma_bres<1, 0><<<bres_grid<1, 0>(NT, nmt, smem), P_THREADS, smem, s>>>(
-            ta, ta, tb, nullptr, (bf16*)dx1, c1, (bf16*)dx2, c2, cout, 0, h, w, nmt, NT, err);
-        return 1;
-    }
     if (g_conv_tma == 2) {
         if (conv_persist_smem_attr<1, 0>() != cudaSuccess) return 0;
         const int nmt = (int)(P / TM), ntiles = nmt * ((c1 + c2) / TN);
@@ -1424,7 +838,7 @@ static int conv_bwd_data_tma(const void* dy, const void* wt, void* dx1, int c1, 
 // 1: launched; 0: shape or tensor maps not available (the caller uses the gather kernel)
 static int conv_fwd_tma(const void* x1, int c1, const void* x2, int c2, const void* wb, const float* bias, void* y, int n,
                         int h, int w, int cout, int relu, int* err, cudaStream_t s) {
-    if (!g_conv_tma || !conv_tma_shape_ok(c1, c2, h, w, cout)) return 0;
+    if (!g_conv_tma || !conv_tma_shape_ok(c1, c2, h, w, cout) || tile_better(c1 + c2)) return 0;
     CUtensorMap t1, t2, tb;
     if (!act_map(&t1, x1, c1, n, h, w)) return 0;
     if (c2 > 0) {
@@ -1434,35 +848,6 @@ static int conv_fwd_tma(const void* x1, int c1, const void* x2, int c2, const vo
     }
     if (!weight_map(&tb, wb, 9LL * (c1 + c2), cout)) return 0;
     const long long P = (long long)n * h * w;
-    if (halo_ok(w, (c1 + c2) / TK)) {
-        CUtensorMap h1, h2;
-        if (!act_map_halo(&h1, x1, c1, n, h, w)) return 0;
-        if (c2 > 0) {
-            if (!act_map_halo(&h2, x2, c2, n, h, w)) return 0;
-        } else {
-            h2 = h1;
-        }
-        if ((relu ? conv_halo_smem_attr<0, 1>() : conv_halo_smem_attr<0, 0>()) != cudaSuccess) return 0;
-        const int nmt = (int)(P / TM), NT = cout / TN, smem = halo_smem_bytes((c1 + c2) / TK);
-        if (relu)
-            k_conv_tma_halo<0, 1><<<halo_grid<0, 1>(NT, nmt, smem), P_THREADS, smem, s>>>(
-                h1, h2, tb, bias, (bf16*)y, cout, nullptr, 0, c1, c2, h, w, nmt, NT, err);
-        else
-            k_conv_tma_halo<0, 0><<<halo_grid<0, 0>(NT, nmt, smem), P_THREADS, smem, s>>>(
-                h1, h2, tb, bias, (bf16*)y, cout, nullptr, 0, c1, c2, h, w, nmt, NT, err);
-        return 1;
-    }
-    if (g_conv_tma == 2 && 9 * ((c1 + c2) / TK) <= BR_MAX_CHUNKS) {
-        if ((relu ? conv_bres_smem_attr<0, 1>() : conv_bres_smem_attr<0, 0>()) != cudaSuccess) return 0;
-        const int nmt = (int)(P / TM), NT = cout / TN, smem = br_smem_bytes(9 * ((c1 + c2) / TK));
-        if (relu)
-            k_conv_tma_bres<0, 1><<<bres_grid<0, 1>(NT, nmt, smem), P_THREADS, smem, s>>>(
-                t1, t2, tb, bias, (bf16*)y, cout, nullptr, 0, c1, c2, h, w, nmt, NT, err);
-        else
-            k_conv_tma_bres<0, 0><<<bres_grid<0, 0>(NT, nmt, smem), P_THREADS, smem, s>>>(
-                t1, t2, tb, bias, (bf16*)y, cout, nullptr, 0, c1, c2, h, w, nmt, NT, err);
-        return 1;
-    }
     if (g_conv_tma == 2) {
         if ((relu ? conv_persist_smem_attr<0, 1>() : conv_persist_smem_attr<0, 0>()) != cudaSuccess) return 0;
         const int nmt = (int)(P / TM), ntiles = nmt * (cout / TN);
@@ -1540,6 +925,13 @@ static int conv_tc_args_ok(int c1, int c2, int n, int h, int w, int cout) {
            (long long)n * h * w < (1LL << 31);
 }
 
+// nn_tile.cu: 8 x 16-pixel tiles, any image and channel counts (1 launched, 0 not taken)
+int glnn_tile_fwd(const void* x1, int c1, const void* x2, int c2, const void* wb, const float* bias, void* y, int n, int h,
+                  int w, int cout, int relu, int* err, cudaStream_t s);
+int glnn_tile_bwd_data(const void* dy, const void* wt, void* dx1, int c1, void* dx2, int c2, int n, int h, int w, int cout,
+                       int* err, cudaStream_t s);
+bool glnn_tc_tiles() { return g_conv_tma == 2; }
+
 extern "C" {
 
 int glnn_set_conv_tma(int32_t enable) {
@@ -1555,7 +947,8 @@ int glnn_conv3x3_fwd(const void* x1, int32_t c1, const void* x2, int32_t c2, con
     const long long P = (long long)n * h * w;
     dim3 grid((unsigned)((P + TM - 1) / TM), (unsigned)((cout + TN - 1) / TN));
     cudaStream_t s = (cudaStream_t)stream;
-    if (conv_fwd_tma(x1, c1, x2, c2, wb, bias, y, n, h, w, cout, relu, err, s))
+    if (conv_fwd_tma(x1, c1, x2, c2, wb, bias, y, n, h, w, cout, relu, err, s) ||
+        (g_conv_tma == 2 && glnn_tile_fwd(x1, c1, x2, c2, wb, bias, y, n, h, w, cout, relu, err, s)))
         return cudaGetLastError() == cudaSuccess ? GLGPU_OK : GLGPU_E_CUDA;
     if ((relu ? conv_tc_smem_attr<0, 1>() : conv_tc_smem_attr<0, 0>()) != cudaSuccess) return GLGPU_E_CUDA;
     if (relu)
@@ -1587,7 +980,8 @@ int glnn_conv3x3_bwd_data(const void* dy, const void* y, int32_t relu, const voi
     const long long P = (long long)n * h * w;
     dim3 grid((unsigned)((P + TM - 1) / TM), (unsigned)((c1 + c2 + TN - 1) / TN));
     cudaStream_t s = (cudaStream_t)stream;
-    if (!relu && conv_bwd_data_tma(dy, wt, dx1, c1, dx2, c2, n, h, w, cout, err, s))
+    if (!relu && (conv_bwd_data_tma(dy, wt, dx1, c1, dx2, c2, n, h, w, cout, err, s) ||
+                  (g_conv_tma == 2 && glnn_tile_bwd_data(dy, wt, dx1, c1, dx2, c2, n, h, w, cout, err, s))))
         return cudaGetLastError() == cudaSuccess ? GLGPU_OK : GLGPU_E_CUDA;
     if ((relu ? conv_tc_smem_attr<1, 1>() : conv_tc_smem_attr<1, 0>()) != cudaSuccess) return GLGPU_E_CUDA;
     if (relu)
