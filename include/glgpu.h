@@ -72,7 +72,7 @@ typedef struct {
     uint32_t rand_t;        /* Langevin seed after the call */
     int32_t used_graph;     /* 1: device-side loop (CUDA graph or one resident launch), 0: host-driven loop */
     int64_t sweep_launches; /* Jacobi sweep kernel launches (psi and A); 1 where the whole call is one
-                             * launch (domains that fit on chip) */
+                             * launch (domains that fit on chip), else 1 per FP64 psi loop */
 } glgpu_td_stats;
 
 /* --- lifetime: GLSolver construction / destruction (svirl/__init__.py:30-179,
@@ -81,20 +81,21 @@ int glgpu_create(const glgpu_grid* grid, int32_t device, glgpu_handle** out);
 int glgpu_destroy(glgpu_handle* h);
 const char* glgpu_last_error(const glgpu_handle* h);   /* h may be NULL: last create error */
 int glgpu_version(void);
-/* Jacobi sweeps of the psi step done by one launch of the psi sweep kernel
- * (temporal blocking; every sweep is still written, so the loop stops exactly
- * where the reference's one-sweep-per-launch loop stops). */
+/* Jacobi sweeps of the psi step that glgpu_time_sweeps times and that
+ * glgpu_set_loop_guard counts as one launch; also what one launch of the FP32 psi
+ * sweep kernel does (temporal blocking; every sweep is still written, so the loop
+ * stops exactly where the reference's one-sweep-per-launch loop stops). */
 int glgpu_psi_sweeps_per_launch(void);
 /* Rows per warp strip of the psi sweep chosen for this handle (from the compiled
  * strip heights, by the item-count model of the persistent sweep); 0 if h is NULL. */
 int glgpu_psi_strip_rows(const glgpu_handle* h);
 /* Force the strip height (one of the compiled heights; 0 = the model's choice).
- * Results do not depend on it: every node gets the same arithmetic. */
+ * Results do not depend on it: every node gets the same arithmetic.  FP64 sweeps
+ * have no strips: there it is only stored. */
 int glgpu_set_psi_strip_rows(glgpu_handle* h, int32_t rows);
-/* The FP32 psi sweep kernel: 0 (default) = the register-strip kernel (the FP64
- * build always uses it); 1 = inputs staged in shared memory by bulk copies
- * (TMA), four strips per CTA, measured slower on GB300 (172 against 89 us per
- * launch on the 2049^2 workload).  Both compute the same values bitwise. */
+/* The FP32 psi sweep kernel: 0 (default) = the register-strip kernel; 1 = inputs
+ * staged in shared memory by bulk copies (TMA), four strips per CTA, measured slower
+ * on GB300 (172 against 89 us per launch on the 2049^2 workload).  Both compute the same values bitwise. */
 int glgpu_set_psi_sweep_kernel(glgpu_handle* h, int32_t select);
 /* Time stepping of the order parameter: 0 (default) = backward Euler, the
  * reference's scheme (svirl/cuda/td.h:4-133); 1 = Crank-Nicolson of the

@@ -1,7 +1,8 @@
 """Measured choice of the psi sweep's launch shape, persisted per problem.
 
-The psi sweep kernel is compiled for the strip heights in ``STRIP_ROWS`` and,
-in FP32, as two kernels (register strip, bulk-copy ring).  By default a handle
+The FP32 psi sweep kernel is compiled for the strip heights in ``STRIP_ROWS`` and
+as two kernels (register strip, bulk-copy ring); FP64 has no strips, and there every
+height measures the same.  By default a handle
 takes the height an item-count model picks.  ``tune(handle)`` measures instead:
 it times one sweep launch (``glgpu_time_sweeps``: CUDA events, L2 flushed
 before each launch) for every (kernel, height) pair, applies the fastest, and

@@ -111,11 +111,15 @@ struct LoopState {
     int ninst;
     long long total_launches;  // sweep kernel launches (psi and A) in the current call
     int guard;                // launches after which a Jacobi loop is stopped with kErrLoopGuard
+    unsigned arrived, round;  // cooperative Jacobi loop (grid_round): CTAs arrived; 2 x finished sweeps + go on
 };
 
 constexpr int kErrLoopGuard = 1;
 constexpr int kErrCopyWait = 2;  // a wait for a bulk copy into shared memory ran out (psi sweep)
 constexpr int kErrBarrier = 4;   // a wait at an instance's barrier ran out (resident time loop)
+
+// Polls of a barrier between CTAs before one gives up (about a microsecond each: seconds).
+constexpr unsigned kBarrierSpins = 1u << 22;
 
 // Resident time loop (tdr.cu).  An instance's barrier: CTAs arrived so far in the
 // call, and the residual maxima and NaN bits of the last three rounds.
@@ -324,10 +328,9 @@ size_t real_size(const glgpu_handle* h);
 int td_run(glgpu_handle* h, double dt, int Nt, int eqn, glgpu_td_stats* stats, double* elapsed_ms);
 int time_sweeps(glgpu_handle* h, int which, int nrep, double* avg_ms);
 int choose_strip_rows(int dtype, const Geo* const* geos, int n);
-// psi sweep kernel of a dtype and a selection (0: register strip, the default;
-// 1: FP32 bulk-copy ring): 8 = FP64 register strip, 4 = FP32 register strip,
-// 5 = FP32 bulk-copy ring
-inline int psi_kind(int dtype, int select) { return dtype == 8 ? 8 : (select == 1 ? 5 : 4); }
+// FP32 psi sweep kernel of a selection: 4 = register strip (0, the default), 5 =
+// bulk-copy ring (1).  FP64 runs its Jacobi loop without strips (k_psi_loop_one).
+inline int psi_kind(int dtype, int select) { return dtype == 4 && select == 1 ? 5 : 4; }
 int psi_sweep_grid(int kind, int rows, int nitems);
 std::vector<Item> make_items(const Geo& g, int inst, int rows);
 // tdr.cu

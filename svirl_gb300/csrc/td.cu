@@ -75,7 +75,9 @@ __device__ void finish_instance_A(const Inst& I, LoopState* loop, int k) {
 // Buffer of psi^(s) in a psi Jacobi loop whose right-hand side psi^(0) is in
 // buffer R: the kFuse + 1 other buffers rotate, so the input of a launch and its
 // kFuse outputs are always distinct.
-__device__ __forceinline__ int pbuf(int R, int s) { return s == 0 ? R : (R + 1 + (s - 1) % (kFuse + 1)) % kPsiBufs; }
+// A launch of K sweeps needs K + 1 of them.
+template <int K = kFuse>
+__device__ __forceinline__ int pbuf(int R, int s) { return s == 0 ? R : (R + 1 + (s - 1) % (K + 1)) % kPsiBufs; }
 
 // Called by the warp that finishes the last strip of an instance in a psi
 // launch that did sweeps k+1 .. k+kFuse: the loop stops after the first of them
@@ -403,6 +405,200 @@ k_psi_sweep(const Inst* __restrict__ insts, const Item* __restrict__ items, int 
         __threadfence();
         unsigned gdone = atomicAdd(&loop->blocks_done, 1u);
         if (gdone == gridDim.x - 1u) finish_launch(loop, cond, use_cond);
+    }
+}
+
+// The Jacobi loop of the psi step in one cooperative launch, one sweep per round and a
+// node per thread, for FP64 domains that fill the chip: the same node arithmetic as
+// k_psi_sweep, bitwise the same values and the same sweep counts.  The FP64 pipe bounds
+// it (20 FP64 instructions a node; a warp instruction takes 64 cycles of its scheduler),
+// so nothing is recomputed, while the strips of k_psi_sweep compute 32 columns for 26
+// and RR + 2 rows for RR; the five psi values and the link factors of a node come from
+// L1/L2, which are far from their limits.  A CTA's threads stride over the tiles (256
+// consecutive nodes).  All instances are at the same sweep of their loops, so a round's
+// buffers follow from its number, and of the loop state only `done` is read again.
+// Only whether a residual meets the stop rule counts, so where a CTA already holds one
+// that does not, the differences (two of the FP64 instructions) are left out.
+// Sweep at 1025 x 1025: 45 us, 38 of them FP64 pipe, against 72 for a third of a strip
+// launch of three sweeps inside a conditional graph node (513^2: 19 against 23, 65^2: 7.4
+// against 15; as a launch per sweep in the conditional node 61, 26 and 14).
+template <typename T>
+__device__ __forceinline__ void one_flush(const Inst& I, unsigned long long rmax, bool nan, unsigned long long* s_max) {
+    const int lane = threadIdx.x & 31;
+    const unsigned hi = __reduce_max_sync(0xffffffffu, (unsigned)(rmax >> 32));
+    const unsigned lo = __reduce_max_sync(0xffffffffu, (unsigned)(rmax >> 32) == hi ? (unsigned)rmax : 0u);
+    const bool any_nan = __any_sync(0xffffffffu, nan);
+    if (lane == 0) {
+        s_max[threadIdx.x >> 5] = (unsigned long long)hi << 32 | lo;
+        if (any_nan) atomicOr(&I.st->nanlv, 1);
+    }
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        unsigned long long v = s_max[0];
+        for (int q = 1; q < kWarps; ++q) v = v > s_max[q] ? v : s_max[q];
+        atomicMax(&I.st->resp[0], v);
+    }
+    __syncthreads();
+}
+
+// End of round `round`: the CTA that arrives last closes the sweep for every instance
+// whose loop still runs (finish_instance_psi), decides whether one is left, and publishes
+// round and decision in one word.  What the CTAs wrote in the sweep is visible after it.
+// false: leave the loop (finished, or a wait ran out).  The word of a round stays until
+// this CTA has arrived at the next one, so nobody misses it.
+__device__ __forceinline__ bool one_round(const Inst* insts, int ninst, LoopState* loop, int first, int round, int& s_word) {
+    const int seq = round - first + 1;  // rounds of this launch
+    if (threadIdx.x == 0) {
+        __threadfence();
+        s_word = atomicAdd(&loop->arrived, 1u) + 1u == (unsigned)seq * gridDim.x ? -1 : 0;
+    }
+    __syncthreads();
+    const bool last = s_word < 0;
+    if (last) {
+        int left = 0;
+        __threadfence();
+        for (int q = threadIdx.x; q < ninst; q += kThreads) {
+            const Inst& I = insts[q];
+            InstState* st = I.st;
+            if (*(volatile const int*)&st->done) continue;
+            const bool stop = atomicExch(&st->resp[0], 0ull) <= I.thr_psi || round + 1 >= kMaxSweeps;
+            if (atomicExch(&st->nanlv, 0)) st->nan_seen = 1;
+            if (stop) {
+                const int s = round + 1;
+                st->sweep = s;
+                st->done = 1;
+                st->rhs = pbuf<1>(st->rhs, s);
+                st->last_sweeps_psi = s;
+                st->total_sweeps_psi += s;
+                if (s > st->max_sweeps_psi) st->max_sweeps_psi = s;
+            } else {
+                left = 1;
+            }
+            __threadfence();
+        }
+        left = __syncthreads_or(left);
+        if (threadIdx.x == 0) {
+            if (seq == 1) loop->total_launches += 1;
+            if (!left) loop->active = 0;
+            if (left && seq >= kFuse * min(loop->guard, kMaxSweeps)) {  // the guard counts launches of kFuse sweeps
+                left = 0;
+                loop->err |= kErrLoopGuard;
+            }
+            loop->cont = left;
+            s_word = 2 * seq + left;
+            __threadfence();
+            asm volatile("st.release.gpu.global.u32 [%0], %1;" ::"l"(&loop->round), "r"(s_word) : "memory");
+        }
+    } else if (threadIdx.x == 0) {
+        unsigned word, it = 0;
+        for (;;) {
+            asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(word) : "l"(&loop->round) : "memory");
+            if (word >> 1 == (unsigned)seq) break;
+            if (++it >= kBarrierSpins || ((it & 1023u) == 0u && (*(volatile int*)&loop->err & kErrBarrier))) {
+                atomicOr(&loop->err, kErrBarrier);
+                word = 0u;
+                break;
+            }
+        }
+        __threadfence();
+        s_word = (int)word;
+    }
+    __syncthreads();
+    return s_word & 1;
+}
+
+template <typename T>
+__global__ void __launch_bounds__(kThreads)
+k_psi_loop_one(const Inst* __restrict__ insts, int ninst, const Tile* __restrict__ tiles, int ntiles, LoopState* loop,
+               int first) {
+    __shared__ int s_word, s_big;
+    __shared__ unsigned long long s_max[kWarps];
+    __shared__ C2<T>* s_psi[kPsiBufs];
+    int cur_inst = -1, R = 0, done = 1;
+    uint32_t rt = 0;
+    for (int round = first;; ++round) {
+        const C2<T>* cur = nullptr;
+        const C2<T>* rhs = nullptr;
+        C2<T>* nxt = nullptr;
+        unsigned long long rmax = 0ull, thr = 0ull;
+        bool rnan = false, fresh = true;
+        for (int it = blockIdx.x; it < ntiles; it += gridDim.x) {
+            const Tile t = tiles[it];
+            if (fresh || t.inst != cur_inst) {
+                if (!fresh && !done) one_flush<T>(insts[cur_inst], rmax, rnan, s_max);
+                // an instance's `done` changes only at the end of a round
+                const InstState* st = insts[t.inst].st;
+                if (t.inst != cur_inst || ninst > 1) {
+                    const Inst& I = insts[t.inst];
+                    done = *(volatile const int*)&st->done;
+                    R = *(volatile const int*)&st->rhs;
+                    rt = *(volatile const uint32_t*)&st->rand_t;
+                    if (threadIdx.x < kPsiBufs) s_psi[threadIdx.x] = (C2<T>*)I.psi[threadIdx.x];
+                }
+                if (threadIdx.x == 0) s_big = 0;
+                cur_inst = t.inst;
+                fresh = false;
+                __syncthreads();
+                cur = s_psi[pbuf<1>(R, round)];
+                rhs = s_psi[R];
+                nxt = s_psi[pbuf<1>(R, round + 1)];
+                thr = insts[cur_inst].thr_psi;
+                rmax = 0ull;
+                rnan = false;
+            }
+            const int n = t.n0 + (int)threadIdx.x;
+            const Inst& I = insts[cur_inst];
+            const Geo& g = I.g;
+            if (done || n >= g.N) continue;
+            const int Nx = g.Nx, j = n / Nx, i = n - j * Nx;
+            const C2<T>* __restrict__ U = (const C2<T>*)I.U;
+            const C2<T> z = cmk<T>(T(0), T(0));
+            const bool lt = i > 0, rg = i + 1 < Nx, dn = j > 0, up = j + 1 < g.Ny;
+            // psi was written by other SMs in the round before: no read-only loads
+            const C2<T> pc = cur[n];
+            const C2<T> pl = lt ? cur[n - 1] : z, pr = rg ? cur[n + 1] : z;
+            const C2<T> pd = dn ? cur[n - Nx] : z, pu = up ? cur[n + Nx] : z;
+            const C2<T> ua = __ldg(&U[2 * n]), ub = __ldg(&U[2 * n + 1]);
+            const C2<T> ual = lt ? __ldg(&U[2 * n - 2]) : z, ubd = dn ? __ldg(&U[2 * (n - Nx) + 1]) : z;
+            const unsigned cd = (unsigned)__ldg(&I.code[n]);
+            C2<T> rq = rhs[n];
+            if (I.lang_psi_on) {
+                const T lc = gsel<T>(I.lang_psi, I.flang_psi);
+                rq.x = add_noise<T>(rq.x, lc, rand_1<T>((uint32_t)n, rt));
+                rq.y = add_noise<T>(rq.y, lc, rand_2<T>((uint32_t)n, rt));
+            }
+            // the first sweep of a step stores the diagonal's reciprocal for the others
+            T* dinv = (T*)I.dinv;
+            T inv;
+            if (round > 0) {
+                inv = dinv[n];
+            } else {
+                const T* eps_sp = (const T*)I.eps_sp;
+                const T eps = eps_sp ? __ldg(&eps_sp[n]) : gsel<T>(I.epsilon, I.fepsilon);
+                inv = (cd & 3u) ? psi_diag_inv<T>(rq, eps, cd, gsel<T>(I.dt, I.fdt), GT(g, idx2), GT(g, idy2)) : T(0);
+                dinv[n] = inv;
+            }
+            const C2<T> out = psi_node<T>(pl, pr, pd, pu, ual, ua, ubd, ub, rq, inv, cd);
+            nxt[n] = out;
+            // a NaN component counts as 0 (the reference's int conversion); magnitudes are
+            // compared as integers, off the FP64 pipe.  A difference that overflows or is
+            // NaN needs an operand beyond 2^1022.
+            const unsigned big = max(max((unsigned)__double2hiint(out.x) & 0x7fffffffu, (unsigned)__double2hiint(out.y) & 0x7fffffffu),
+                                     max((unsigned)__double2hiint(pc.x) & 0x7fffffffu, (unsigned)__double2hiint(pc.y) & 0x7fffffffu));
+            if (__any_sync(__activemask(), *(volatile int*)&s_big == 0 || big >= 0x7fd00000u)) {
+                const unsigned long long kAbs = 0x7fffffffffffffffull, kInf = 0x7ff0000000000000ull;
+                unsigned long long bx = (unsigned long long)__double_as_longlong(out.x - pc.x) & kAbs;
+                unsigned long long by = (unsigned long long)__double_as_longlong(out.y - pc.y) & kAbs;
+                if ((bx > kInf) | (by > kInf)) rnan = true;
+                bx = bx > kInf ? 0ull : bx;
+                by = by > kInf ? 0ull : by;
+                const unsigned long long m = bx > by ? bx : by;
+                rmax = rmax > m ? rmax : m;
+                if (rmax > thr) *(volatile int*)&s_big = 1;
+            }
+        }
+        if (!fresh && !done) one_flush<T>(insts[cur_inst], rmax, rnan, s_max);
+        if (!one_round(insts, ninst, loop, first, round, s_word)) break;
     }
 }
 
@@ -1206,6 +1402,8 @@ __global__ void k_loop_begin(const Inst* __restrict__ insts, int ninst, LoopStat
         loop->active = active;
         loop->launches = 0;
         loop->blocks_done = 0u;
+        loop->arrived = 0u;
+        loop->round = 0u;
         loop->cont = active > 0 ? 1 : 0;
         if (use_cond) cudaGraphSetConditional(cond, active > 0 ? 1u : 0u);
     }
@@ -1342,22 +1540,22 @@ struct TDLaunch {
     bool any_solveA;
     bool any_fv;  // an instance has fixed vortices (irregular potential or phase lock)
     const ResState* res;  // the resident loop (tdr.cu), or null: a launch per sweep
+    int one_grid;     // CTAs of the FP64 psi loop (psi_one_grid), 0: a launch per kFuse sweeps
 };
 
 static void* fv_psi_pre_fn(int dt) { return dt == 8 ? (void*)k_fv_psi_pre<double> : (void*)k_fv_psi_pre<float>; }
 static void* fv_psi_post_fn(int dt) { return dt == 8 ? (void*)k_fv_psi_post<double> : (void*)k_fv_psi_post<float>; }
 static void* fv_A_fn(int dt) { return dt == 8 ? (void*)k_fv_A<double> : (void*)k_fv_A<float>; }
 
-// The psi sweep kernel of a kind (psi_kind): FP64 and FP32 register strip (the
-// default), FP32 bulk-copy ring (selected per handle).
+// The FP32 psi sweep kernel of a kind (psi_kind): register strip (the default) or
+// bulk-copy ring (selected per handle).
 static bool psi_bulk(int kind) { return kind == 5; }
 template <int V>
 static void* psi_sweep_fn_v(int kind, int rows) {
     if constexpr (V < kNumStripRows) {
         constexpr int R = kStripRowsSet[V];
         if (rows == R)
-            return kind == 8 ? (void*)k_psi_sweep<double, R>
-                             : (kind == 5 ? (void*)k_psi_sweep_bulk<R> : (void*)k_psi_sweep<float, R>);
+            return kind == 5 ? (void*)k_psi_sweep_bulk<R> : (void*)k_psi_sweep<float, R>;
         return psi_sweep_fn_v<V + 1>(kind, rows);
     } else {
         return nullptr;
@@ -1374,6 +1572,17 @@ static cudaError_t launch_psi_sweep(int kind, int rows, int grid, cudaStream_t s
     void* a[] = {&insts, &items, &nitems, &loop, &none, &zero};
     return cudaLaunchKernel(psi_sweep_fn(kind, rows), dim3(grid), dim3(psi_threads(kind)), a, 0, s);
 }
+// CTAs of the FP64 Jacobi loop over `ntiles` tiles (all of them are resident).
+static int psi_one_grid(int ntiles) {
+    int dev = 0, sms = 1, per_sm = 1;
+    cudaGetDevice(&dev);
+    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, (const void*)k_psi_loop_one<double>, kThreads, 0) != cudaSuccess ||
+        per_sm < 1)
+        per_sm = 1;
+    return ntiles < sms * per_sm ? ntiles : sms * per_sm;
+}
+
 static void* A_sweep_fn(int dtype) {
     return dtype == 8 ? (void*)k_A_sweep<double> : (void*)k_A_sweep<float>;
 }
@@ -1409,7 +1618,21 @@ cudaError_t add_while(cudaGraph_t g, cudaGraphNode_t* node, const cudaGraphNode_
     return e;
 }
 
+// Marks a graph's kernel node as a cooperative launch (its CTAs wait for one another).
+static cudaError_t set_cooperative(cudaGraphNode_t node) {
+    cudaLaunchAttributeValue v;
+    memset(&v, 0, sizeof(v));
+    v.cooperative = 1;
+    return cudaGraphKernelNodeSetAttribute(node, cudaLaunchAttributeCooperative, &v);
+}
+
 #define GCHK(x) do { cudaError_t e_ = (x); if (e_ != cudaSuccess) { err = e_; goto fail; } } while (0)
+
+static cudaError_t launch_psi_loop_one(int grid, cudaStream_t s, const Inst* insts, int ninst, const Tile* tiles, int ntiles,
+                                       LoopState* loop, int first) {
+    void* a[] = {&insts, &ninst, &tiles, &ntiles, &loop, &first};
+    return cudaLaunchCooperativeKernel((const void*)k_psi_loop_one<double>, dim3(grid), dim3(kThreads), a, 0, s);
+}
 
 // Build the whole TD run of all instances as one graph:
 //   [fixed vortices: A += A_irr, psi-only mode] -> [tables, all instances] -> WHILE(step < Nt) {
@@ -1454,7 +1677,8 @@ static cudaError_t build_td_graph(const TDLaunch& L, int eqn, cudaGraphExec_t* e
     GCHK(add_while(top, &n_out, prev ? &prev : nullptr, prev ? 1 : 0, hout, &obody));
     prev = nullptr;
     if (do_psi) {
-        GCHK(cudaGraphConditionalHandleCreate(&hpsi, obody, 1, cudaGraphCondAssignDefault));
+        int cond = L.one_grid == 0 ? 1 : 0;
+        if (cond) GCHK(cudaGraphConditionalHandleCreate(&hpsi, obody, 1, cudaGraphCondAssignDefault));
         if (eqn == 0 && L.any_fv) {
             void* a[] = {&insts, &tiles};
             GCHK(chain(obody, fv_psi_pre_fn(L.dtype), gt, bt, a));
@@ -1464,12 +1688,16 @@ static cudaError_t build_td_graph(const TDLaunch& L, int eqn, cudaGraphExec_t* e
             GCHK(chain(obody, link_fn(L.dtype), dim3(call_grid(ntiles)), bt, a));
         }
         {
-            void* a[] = {&insts, &ninst, &loop, &hpsi, &one, &zero};
+            void* a[] = {&insts, &ninst, &loop, &hpsi, &cond, &zero};
             GCHK(chain(obody, (void*)k_loop_begin, g1, b1, a));
         }
-        GCHK(add_while(obody, &nd, &prev, 1, hpsi, &pbody));
-        prev = nd;
-        {
+        if (L.one_grid > 0) {
+            void* a[] = {&insts, &ninst, &tiles, &ntiles, &loop, &zero};
+            GCHK(chain(obody, (void*)k_psi_loop_one<double>, dim3(L.one_grid), bt, a));
+            GCHK(set_cooperative(prev));
+        } else {
+            GCHK(add_while(obody, &nd, &prev, 1, hpsi, &pbody));
+            prev = nd;
             cudaGraphNode_t sw;
             if (L.psi_cn) {
                 int aw = L.psi_cn == 2 ? 1 : 0;
@@ -1576,7 +1804,11 @@ static cudaError_t run_host_loop(const TDLaunch& L, int eqn, int Nt, cudaStream_
             if (part == 0 && (L.any_solveA || L.any_fv)) launch_link_U(L, 1, s);
             if (part == 1 && L.any_fv) fv_A(0);
             k_loop_begin<<<1, 32, 0, s>>>(L.insts, L.ninst, L.loop, none, 0, part);
-            for (;;) {
+            if (part == 0 && L.one_grid > 0) {
+                const cudaError_t e = launch_psi_loop_one(L.one_grid, s, L.insts, L.ninst, L.tiles, L.ntiles, L.loop, 0);
+                if (e != cudaSuccess) return e;
+            }
+            for (; part == 1 || L.one_grid == 0;) {
                 for (int c = 0; c < chunk; ++c) {
                     if (part == 0 && L.psi_cn) {
                         const int aw = L.psi_cn == 2 ? 1 : 0;
@@ -1630,6 +1862,9 @@ __global__ void k_bench_prep(const Inst* __restrict__ insts, int ninst, LoopStat
         loop->active = ninst;
         loop->launches = 0;
         loop->blocks_done = 0u;
+        loop->arrived = 0u;
+        loop->round = 0u;
+        loop->guard = 1;
         loop->cont = 1;
     }
 }
@@ -1685,7 +1920,9 @@ int time_sweeps(glgpu_handle* h, int which, int nrep, double* avg_ms) {
         for (int q = 0; q < per_rep && e == cudaSuccess; ++q) {
             k_bench_prep<<<1, 32, 0, h->stream>>>(h->inst, 1, h->loop, which == 0 ? 1 : q);
             cudaEventRecord(e0, h->stream);
-            if (which == 0) {
+            if (which == 0 && h->dtype == 8) {
+                e = launch_psi_loop_one(psi_one_grid(h->ntiles), h->stream, h->inst, 1, h->tiles, h->ntiles, h->loop, 1);
+            } else if (which == 0) {
                 launch_psi_sweep(psi_kind(h->dtype, h->psi_select), h->strip_rows, h->psi_grid, h->stream, h->inst, h->items,
                                  h->nitems, h->loop);
             } else {
@@ -1693,7 +1930,7 @@ int time_sweeps(glgpu_handle* h, int which, int nrep, double* avg_ms) {
                 else k_A_sweep<float><<<h->natiles, kThreads, 0, h->stream>>>(h->inst, h->atiles, h->loop, none, 0);
             }
             cudaEventRecord(e1, h->stream);
-            e = cudaEventSynchronize(e1);
+            if (e == cudaSuccess) e = cudaEventSynchronize(e1);
             float ms = 0.f;
             if (e == cudaSuccess) e = cudaEventElapsedTime(&ms, e0, e1);
             total += ms;
@@ -1884,6 +2121,7 @@ int td_run(glgpu_handle* h, double dt, int Nt, int eqn, glgpu_td_stats* stats, d
     L.any_solveA = h->inst_h.solveA != 0;
     L.any_fv = h->vpi != nullptr || h->lock_n > 0;
     L.res = resident ? &h->res : nullptr;
+    L.one_grid = resident || h->psi_scheme != 0 || h->dtype != 8 ? 0 : psi_one_grid(h->ntiles);
     TDOutcome o = td_core(h->stream, L, Nt, eqn, h->td_exec, &h->td_graph_failed, h->use_graphs, h->loop_guard,
                           elapsed_ms != nullptr,
                           h->st_gather, &ps->st, &ps->loop);
@@ -1933,6 +2171,7 @@ int batch_td(glgpu_batch* b, double dt, int Nt, int eqn, glgpu_td_stats* stats, 
     L.any_solveA = any_solveA;
     L.any_fv = any_fv;
     L.res = resident ? &b->res : nullptr;
+    L.one_grid = resident || b->dtype != 8 ? 0 : psi_one_grid(b->ntiles);
     TDOutcome o = td_core(b->stream, L, Nt, eqn, b->td_exec, &b->td_graph_failed, b->use_graphs, b->loop_guard,
                           elapsed_ms != nullptr,
                           b->gather, b->gather_pin, b->loop_pin);

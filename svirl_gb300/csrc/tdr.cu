@@ -60,9 +60,6 @@ template <int BX, int BY, int R, int K, int KA> struct ResShape {
     static_assert(K <= kResSweeps && 4 * R <= 32 && IW >= K && IH >= K, "residual words, link-weight bits, halo within one tile");
 };
 
-// Polls of a barrier before a CTA gives up (about a microsecond each: seconds).
-constexpr unsigned kResSpins = 1u << 22;
-
 // One round of the instance's barrier: everything this CTA wrote is visible to the
 // CTAs that pass it.  false: the wait ran out (or another CTA's did).
 __device__ __forceinline__ bool res_barrier(ResGroup* g, unsigned& target, unsigned ncta, LoopState* loop, int& s_broken) {
@@ -75,7 +72,7 @@ __device__ __forceinline__ bool res_barrier(ResGroup* g, unsigned& target, unsig
         for (;;) {
             asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(seen) : "l"(&g->arrived) : "memory");
             if ((int)(seen - target) >= 0) break;
-            if (++it >= kResSpins || ((it & 1023u) == 0u && (*(volatile int*)&loop->err & kErrBarrier))) {
+            if (++it >= kBarrierSpins || ((it & 1023u) == 0u && (*(volatile int*)&loop->err & kErrBarrier))) {
                 atomicOr(&loop->err, kErrBarrier);
                 s_broken = 1;
                 break;
