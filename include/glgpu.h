@@ -72,7 +72,7 @@ typedef struct {
     uint32_t rand_t;        /* Langevin seed after the call */
     int32_t used_graph;     /* 1: device-side loop (CUDA graph or one resident launch), 0: host-driven loop */
     int64_t sweep_launches; /* Jacobi sweep kernel launches (psi and A); 1 where the whole call is one
-                             * launch (domains that fit on chip), else 1 per FP64 psi loop */
+                             * launch (domains that fit on chip), else 1 per psi loop and per A sweep */
 } glgpu_td_stats;
 
 /* --- lifetime: GLSolver construction / destruction (svirl/__init__.py:30-179,
@@ -82,20 +82,23 @@ int glgpu_destroy(glgpu_handle* h);
 const char* glgpu_last_error(const glgpu_handle* h);   /* h may be NULL: last create error */
 int glgpu_version(void);
 /* Jacobi sweeps of the psi step that glgpu_time_sweeps times and that
- * glgpu_set_loop_guard counts as one launch; also what one launch of the FP32 psi
- * sweep kernel does (temporal blocking; every sweep is still written, so the loop
- * stops exactly where the reference's one-sweep-per-launch loop stops). */
+ * glgpu_set_loop_guard counts as one launch; FP32 does them in one pass over the
+ * state (temporal blocking).  The loop stops exactly where the reference's
+ * one-sweep-per-launch loop stops. */
 int glgpu_psi_sweeps_per_launch(void);
-/* Rows per warp strip of the psi sweep chosen for this handle (from the compiled
- * strip heights, by the item-count model of the persistent sweep); 0 if h is NULL. */
+/* Rows per warp strip of the bulk-copy psi sweep chosen for this handle (from the
+ * compiled strip heights, by the item-count model of the persistent sweep), or what
+ * glgpu_set_psi_strip_rows set; 0 if h is NULL. */
 int glgpu_psi_strip_rows(const glgpu_handle* h);
-/* Force the strip height (one of the compiled heights; 0 = the model's choice).
+/* Force the strip height of both FP32 psi sweeps (one of the compiled heights; 0 = the
+ * models' choices, which for the default sweep may be other heights).
  * Results do not depend on it: every node gets the same arithmetic.  FP64 sweeps
  * have no strips: there it is only stored. */
 int glgpu_set_psi_strip_rows(glgpu_handle* h, int32_t rows);
-/* The FP32 psi sweep kernel: 0 (default) = the register-strip kernel; 1 = inputs
- * staged in shared memory by bulk copies (TMA), four strips per CTA, measured slower
- * on GB300 (172 against 89 us per launch on the 2049^2 workload).  Both compute the same values bitwise. */
+/* The FP32 psi sweep kernel: 0 (default) = the whole Jacobi loop as one cooperative
+ * launch; 1 = a launch per three sweeps, inputs staged in shared memory by bulk copies
+ * (TMA), four strips per CTA, measured slower on GB300 (172 us per launch against 59 for
+ * three sweeps on the 2049^2 workload).  Both compute the same values bitwise. */
 int glgpu_set_psi_sweep_kernel(glgpu_handle* h, int32_t select);
 /* Time stepping of the order parameter: 0 (default) = backward Euler, the
  * reference's scheme (svirl/cuda/td.h:4-133); 1 = Crank-Nicolson of the

@@ -1,8 +1,8 @@
 """Measured choice of the psi sweep's launch shape, persisted per problem.
 
-The FP32 psi sweep kernel is compiled for the strip heights in ``STRIP_ROWS`` and
-as two kernels (register strip, bulk-copy ring); FP64 has no strips, and there every
-height measures the same.  By default a handle
+The FP32 psi sweep takes the strip heights in ``STRIP_ROWS`` in two kernels (the
+cooperative loop, the bulk-copy ring); FP64 has no strips, and there every height
+measures the same.  By default a handle
 takes the height an item-count model picks.  ``tune(handle)`` measures instead:
 it times one sweep launch (``glgpu_time_sweeps``: CUDA events, L2 flushed
 before each launch) for every (kernel, height) pair, applies the fastest, and
@@ -21,7 +21,7 @@ import os
 import numpy as np
 
 STRIP_ROWS = (8, 12, 17)  # the heights libglgpu compiles the sweep for
-KERNELS_FP32 = (0, 1)     # 0 register strip, 1 bulk-copy ring (glgpu_set_psi_sweep_kernel)
+KERNELS_FP32 = (0, 1)     # 0 cooperative loop, 1 bulk-copy ring (glgpu_set_psi_sweep_kernel)
 
 
 def cache_path():

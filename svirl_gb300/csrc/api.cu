@@ -116,7 +116,7 @@ static void free_all(glgpu_handle* h) {
         if (h->dir_psi[q]) cudaFree(h->dir_psi[q]);
         if (h->dir_A[q]) cudaFree(h->dir_A[q]);
     }
-    void* ptrs[] = {h->abei, h->mt, h->eps_sp, h->U, h->code, h->dinv, h->st, h->inst, h->tiles, h->atiles, h->items, h->loop, h->partials, h->counter,
+    void* ptrs[] = {h->abei, h->mt, h->eps_sp, h->U, h->code, h->dinv, h->st, h->inst, h->tiles, h->atiles, h->items, h->litems, h->loop, h->partials, h->counter,
                     h->dscal, h->out, h->vort, h->vort_n, h->flush};
     for (void* p : ptrs)
         if (p) cudaFree(p);
@@ -168,19 +168,24 @@ int glgpu_create(const glgpu_grid* grid, int32_t device, glgpu_handle** out) {
     // link factors: Nab complex for the CG, one (x link, y link) pair per node for the TD step
     ok = ok && cudaMalloc(&h->U, std::max((size_t)h->g.Nab * 2, (size_t)h->g.N * 4) * rs) == cudaSuccess;
     ok = ok && cudaMalloc(&h->code, (size_t)h->g.N + 64) == cudaSuccess;
-    if (h->dtype == 8) ok = ok && cudaMalloc(&h->dinv, (size_t)h->g.N * rs) == cudaSuccess;
+    ok = ok && cudaMalloc(&h->dinv, (size_t)h->g.N * rs) == cudaSuccess;
     ok = ok && cudaMalloc(&h->st, sizeof(InstState)) == cudaSuccess;
     ok = ok && cudaMalloc(&h->st_gather, sizeof(InstState)) == cudaSuccess;
     ok = ok && cudaMalloc(&h->inst, sizeof(Inst)) == cudaSuccess;
     ok = ok && cudaMalloc(&h->tiles, sizeof(Tile) * (size_t)h->ntiles) == cudaSuccess;
     h->natiles = atiles_of(h->g.Nx, h->g.Ny);
     ok = ok && cudaMalloc(&h->atiles, sizeof(ATile) * (size_t)h->natiles) == cudaSuccess;
-    {
-        const Geo* gp = &h->g;
-        h->strip_rows = choose_strip_rows(h->dtype, &gp, 1);
-    }
+    h->strip_rows = choose_strip_rows(h->g);
     h->nitems = strip_table_len(h->g.Nx, h->g.Ny, h->strip_rows);
     ok = ok && cudaMalloc(&h->items, sizeof(Item) * (size_t)h->nitems) == cudaSuccess;
+    std::vector<Item> litems;
+    if (h->dtype == 4) {
+        const Geo* gp = &h->g;
+        h->loop_rows = choose_loop_rows(&gp, 1);
+        add_loop_items(litems, h->g, 0, h->loop_rows);
+        h->nlitems = (int)litems.size();
+        ok = ok && cudaMalloc(&h->litems, sizeof(Item) * litems.size()) == cudaSuccess;
+    }
     ok = ok && cudaMalloc(&h->loop, sizeof(LoopState)) == cudaSuccess;
     ok = ok && cudaMalloc(&h->partials, sizeof(double) * 17 * (size_t)nblk) == cudaSuccess;
     ok = ok && cudaMalloc(&h->counter, sizeof(unsigned) * 4) == cudaSuccess;
@@ -198,7 +203,7 @@ int glgpu_create(const glgpu_grid* grid, int32_t device, glgpu_handle** out) {
     std::vector<Tile> tiles(h->ntiles);
     for (int k = 0; k < h->ntiles; ++k) tiles[k] = Tile{0, k * kThreads};
     const std::vector<Item> items = make_items(h->g, 0, h->strip_rows);
-    h->psi_grid = psi_sweep_grid(psi_kind(h->dtype, h->psi_select), h->strip_rows, h->nitems);
+    h->psi_grid = bulk_sweep_grid(h->strip_rows, h->nitems);
     InstState st;
     memset(&st, 0, sizeof(st));
     st.rand_t = h->p.rand_t;
@@ -208,6 +213,8 @@ int glgpu_create(const glgpu_grid* grid, int32_t device, glgpu_handle** out) {
     e = cudaMemcpyAsync(h->tiles, tiles.data(), sizeof(Tile) * tiles.size(), cudaMemcpyHostToDevice, h->stream);
     if (e == cudaSuccess)
         e = cudaMemcpyAsync(h->atiles, atiles.data(), sizeof(ATile) * atiles.size(), cudaMemcpyHostToDevice, h->stream);
+    if (e == cudaSuccess && h->litems)
+        e = cudaMemcpyAsync(h->litems, litems.data(), sizeof(Item) * litems.size(), cudaMemcpyHostToDevice, h->stream);
     if (e == cudaSuccess) e = cudaMemcpyAsync(h->items, items.data(), sizeof(Item) * items.size(), cudaMemcpyHostToDevice, h->stream);
     if (e == cudaSuccess) e = cudaMemcpyAsync(h->st, &st, sizeof(st), cudaMemcpyHostToDevice, h->stream);
     if (e == cudaSuccess) e = cudaMemsetAsync(h->counter, 0, sizeof(unsigned) * 4, h->stream);
@@ -367,7 +374,6 @@ int glgpu_set_psi_sweep_kernel(glgpu_handle* h, int32_t select) {
     cudaError_t e = cudaStreamSynchronize(h->stream);
     if (e != cudaSuccess) return cuda_check(h, e, "set_psi_sweep_kernel");
     h->psi_select = select;
-    h->psi_grid = psi_sweep_grid(psi_kind(h->dtype, h->psi_select), h->strip_rows, h->nitems);
     drop_td_graphs(h);  // the TD graphs hold the kernel and its grid
     return GLGPU_OK;
 }
@@ -375,28 +381,36 @@ int glgpu_set_psi_sweep_kernel(glgpu_handle* h, int32_t select) {
 int glgpu_set_psi_strip_rows(glgpu_handle* h, int32_t rows) {
     if (check_handle(h)) return GLGPU_E_ARG;
     cudaSetDevice(h->device);
-    if (rows == 0) {
-        const Geo* gp = &h->g;
-        rows = choose_strip_rows(h->dtype, &gp, 1);
-    }
+    const Geo* gp = &h->g;
+    int loop_rows = h->dtype == 4 ? (rows == 0 ? choose_loop_rows(&gp, 1) : rows) : 0;
+    if (rows == 0) rows = choose_strip_rows(h->g);
     bool known = false;
     for (int v = 0; v < kNumStripRows; ++v) known = known || kStripRowsSet[v] == rows;
     if (!known) return set_error(h, GLGPU_E_ARG, "set_psi_strip_rows: strip height not compiled in");
-    if (rows == h->strip_rows) return GLGPU_OK;
+    if (rows == h->strip_rows && loop_rows == h->loop_rows) return GLGPU_OK;
     const std::vector<Item> items = make_items(h->g, 0, rows);
-    Item* buf = nullptr;
+    std::vector<Item> litems;
+    if (loop_rows) add_loop_items(litems, h->g, 0, loop_rows);
+    Item *buf = nullptr, *lbuf = nullptr;
     cudaError_t e = cudaStreamSynchronize(h->stream);
     if (e == cudaSuccess) e = cudaMalloc(&buf, sizeof(Item) * items.size());
     if (e == cudaSuccess) e = cudaMemcpy(buf, items.data(), sizeof(Item) * items.size(), cudaMemcpyHostToDevice);
+    if (e == cudaSuccess && loop_rows) e = cudaMalloc(&lbuf, sizeof(Item) * litems.size());
+    if (e == cudaSuccess && loop_rows) e = cudaMemcpy(lbuf, litems.data(), sizeof(Item) * litems.size(), cudaMemcpyHostToDevice);
     if (e != cudaSuccess) {
         if (buf) cudaFree(buf);
+        if (lbuf) cudaFree(lbuf);
         return cuda_check(h, e, "set_psi_strip_rows");
     }
     cudaFree(h->items);
     h->items = buf;
+    if (h->litems) cudaFree(h->litems);
+    h->litems = lbuf;
+    h->nlitems = (int)litems.size();
+    h->loop_rows = loop_rows;
     h->strip_rows = rows;
     h->nitems = (int)items.size();
-    h->psi_grid = psi_sweep_grid(psi_kind(h->dtype, h->psi_select), rows, h->nitems);
+    h->psi_grid = bulk_sweep_grid(rows, h->nitems);
     drop_td_graphs(h);  // the TD graphs hold the old kernel, grid and table
     upload_inst(h);
     return cuda_check(h, cudaStreamSynchronize(h->stream), "set_psi_strip_rows");
@@ -556,30 +570,28 @@ int glgpu_batch_create(glgpu_handle* const* handles, int32_t n, glgpu_batch** ou
     cudaSetDevice(b->device);
     std::vector<Tile> tiles;
     std::vector<ATile> atiles;
-    std::vector<Item> items;
     std::vector<const Geo*> geos(n);
     for (int q = 0; q < n; ++q) geos[q] = &handles[q]->g;
-    b->strip_rows = choose_strip_rows(b->dtype, geos.data(), n);
-    b->inst_items.resize(n);
     for (int q = 0; q < n; ++q) {
         for (int k = 0; k < handles[q]->ntiles; ++k) tiles.push_back(Tile{q, k * kThreads});
         for (int j0 = 0; j0 < handles[q]->g.Ny; j0 += kATY)
             for (int i0 = 0; i0 < handles[q]->g.Nx; i0 += kATX) atiles.push_back(ATile{q, i0, j0, 0});
-        const std::vector<Item> it = make_items(handles[q]->g, q, b->strip_rows);
-        b->inst_items[q] = strip_items(handles[q]->g.Nx, handles[q]->g.Ny, b->strip_rows);
-        items.insert(items.end(), it.begin(), it.end());
     }
     b->ntiles = (int)tiles.size();
     b->natiles = (int)atiles.size();
-    b->nitems = (int)items.size();
-    b->psi_grid = psi_sweep_grid(psi_kind(b->dtype, 0), b->strip_rows, b->nitems);
+    std::vector<Item> litems;
+    if (b->dtype == 4) {
+        b->loop_rows = choose_loop_rows(geos.data(), n);
+        for (int q = 0; q < n; ++q) add_loop_items(litems, handles[q]->g, q, b->loop_rows);
+        b->nlitems = (int)litems.size();
+    }
     b->gather_h.resize(n);
     bool ok = cudaStreamCreateWithFlags(&b->stream, cudaStreamNonBlocking) == cudaSuccess;
     ok = ok && cudaMalloc(&b->insts, sizeof(Inst) * (size_t)n) == cudaSuccess;
     ok = ok && cudaMalloc(&b->gather, sizeof(InstState) * (size_t)n) == cudaSuccess;
     ok = ok && cudaMalloc(&b->tiles, sizeof(Tile) * tiles.size()) == cudaSuccess;
     ok = ok && cudaMalloc(&b->atiles, sizeof(ATile) * atiles.size()) == cudaSuccess;
-    ok = ok && cudaMalloc(&b->items, sizeof(Item) * items.size()) == cudaSuccess;
+    if (b->nlitems > 0) ok = ok && cudaMalloc(&b->litems, sizeof(Item) * litems.size()) == cudaSuccess;
     ok = ok && cudaMalloc(&b->loop, sizeof(LoopState)) == cudaSuccess;
     ok = ok && cudaMallocHost(&b->gather_pin, sizeof(InstState) * (size_t)n) == cudaSuccess;
     ok = ok && cudaMallocHost(&b->loop_pin, sizeof(LoopState)) == cudaSuccess;
@@ -588,7 +600,8 @@ int glgpu_batch_create(glgpu_handle* const* handles, int32_t n, glgpu_batch** ou
     if (e == cudaSuccess) e = cudaMemcpyAsync(b->tiles, tiles.data(), sizeof(Tile) * tiles.size(), cudaMemcpyHostToDevice, b->stream);
     if (e == cudaSuccess)
         e = cudaMemcpyAsync(b->atiles, atiles.data(), sizeof(ATile) * atiles.size(), cudaMemcpyHostToDevice, b->stream);
-    if (e == cudaSuccess) e = cudaMemcpyAsync(b->items, items.data(), sizeof(Item) * items.size(), cudaMemcpyHostToDevice, b->stream);
+    if (e == cudaSuccess && b->nlitems > 0)
+        e = cudaMemcpyAsync(b->litems, litems.data(), sizeof(Item) * litems.size(), cudaMemcpyHostToDevice, b->stream);
     if (e == cudaSuccess) e = cudaStreamSynchronize(b->stream);
     if (e != cudaSuccess) {
         glgpu_batch_destroy(b);
@@ -607,7 +620,7 @@ int glgpu_batch_destroy(glgpu_batch* b) {
         if (b->td_exec[q]) cudaGraphExecDestroy(b->td_exec[q]);
     if (b->cg_exec) cudaGraphExecDestroy(b->cg_exec);
     res_free(&b->res);
-    void* ptrs[] = {b->insts, b->gather, b->tiles, b->atiles, b->items, b->loop, b->cg_partials, b->cg_loop, b->cg_tiles};
+    void* ptrs[] = {b->insts, b->gather, b->tiles, b->atiles, b->litems, b->loop, b->cg_partials, b->cg_loop, b->cg_tiles};
     for (void* p : ptrs)
         if (p) cudaFree(p);
     void* pins[] = {b->gather_pin, b->loop_pin, b->insts_pin};

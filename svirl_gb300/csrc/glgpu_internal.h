@@ -43,6 +43,8 @@ struct InstState {
     int last_sweeps_psi, last_sweeps_A, max_sweeps_psi, max_sweeps_A;
     long long total_sweeps_psi, total_sweeps_A;
     int steps;                // time steps done in the current call
+    int redo, keep;           // cooperative psi loop (tdl.cu): the sweep of the last round that the next one
+                              // repeats up to (0: none), the round keeps every sweep
     int commitA;              // FP32 A loop: 1 + the buffer of A^(0) to add to the final offsets (0: none)
 };
 
@@ -79,7 +81,7 @@ struct Inst {
     void* U;                  // link factors of the psi loop (Nab complex); during the A loop the
                               // fixed parts of the link updates (k_A_sweep), 2 Nab reals
     uint8_t* code;            // per-node link-weight bits of the psi loop, N bytes
-    void* dinv;               // FP64: per-node reciprocal of the psi step's diagonal, N reals (NULL for FP32)
+    void* dinv;               // per-node reciprocal of the psi step's diagonal, N reals (FP32: bits ^ kDead, tdl.cu)
     uint8_t* cbits;           // per-node cell bits (cell_bits) for the batched CG, N bytes (NULL until CG)
     void* vpi;                // irregular vector potential of fixed vortices, Nab, or NULL
     const int32_t* lock;      // phase-lock node list or NULL
@@ -175,11 +177,10 @@ struct ATile {
 };
 inline int atiles_of(int Nx, int Ny) { return ((Nx + kATX - 1) / kATX) * ((Ny + kATY - 1) / kATY); }
 
-// Work item of the warp-strip psi sweep: kStripCols output columns (x0..) by
-// `rows` rows (j0..) of one instance, processed by one warp whose 32 lanes also
-// cover kFuse halo columns on each side.  The sweep kernel is compiled for the
-// strip heights of kStripRowsSet; a handle or batch uses the one that
-// choose_strip_rows (td.cu) picks for its item count.
+// Work item of a warp in a psi sweep: a strip of columns (x0..) by rows (j0..) of one
+// instance.  Bulk-copy sweep: kStripCols columns and one of the heights of kStripRowsSet
+// (chosen by choose_strip_rows, td.cu), the warp's 32 lanes also covering kFuse halo
+// columns on each side.  Loop of tdl.cu: kWideCols columns and `pad` rows.
 #ifdef GLGPU_STRIP_ROWS
 constexpr int kStripRowsSet[] = {GLGPU_STRIP_ROWS};
 #else
@@ -190,7 +191,7 @@ constexpr int kStripCols = 32 - 2 * kFuse;
 inline int strip_items(int Nx, int Ny, int rows) {
     return ((Nx + kStripCols - 1) / kStripCols) * ((Ny + rows - 1) / rows);
 }
-// The FP32 sweep runs kPsiGroup adjacent strips of one row band per CTA (they
+// The bulk-copy sweep runs kPsiGroup adjacent strips of one row band per CTA (they
 // share one ring of rows in shared memory), so the item table lists each band's
 // strips in groups of kPsiGroup, the last group of a band padded with empty
 // items (inst = -1).  strip_table_len: entries of one instance's table.
@@ -200,7 +201,7 @@ inline int strip_table_len(int Nx, int Ny, int rows) {
     return (nstrips + kPsiGroup - 1) / kPsiGroup * kPsiGroup * ((Ny + rows - 1) / rows);
 }
 struct Item {
-    int inst, x0, j0, pad;  // inst = -1: an empty item (group padding)
+    int inst, x0, j0, pad;  // inst = -1: an empty item (group padding of the bulk-copy sweep)
 };
 
 }  // namespace glgpu
@@ -230,6 +231,8 @@ struct glgpu_handle {
     glgpu::Item* items = nullptr;
     int nitems = 0;
     int strip_rows = 0;                 // strip height of the psi sweep items
+    glgpu::Item* litems = nullptr;      // FP32: items of the cooperative psi loop and their height
+    int nlitems = 0, loop_rows = 0;
     int psi_grid = 0;                   // CTAs of the persistent psi sweep
     glgpu::LoopState* loop = nullptr;
     int ntiles = 0;
@@ -258,7 +261,7 @@ struct glgpu_handle {
     bool td_graph_failed = false;
     bool use_graphs = true;
     int loop_guard = 0;                 // Jacobi loop guard in sweep launches (0: kLoopGuard)
-    int psi_select = 0;                 // psi sweep kernel (psi_kind)
+    int psi_select = 0;                 // psi sweep kernel (bulk_selected)
     int psi_scheme = 0;                 // psi time stepping: 0 backward Euler, 1 Crank-Nicolson, 2 as written
     std::string last_error;
     void* flush = nullptr;              // L2 flush buffer for kernel timing
@@ -288,15 +291,15 @@ struct glgpu_batch {
     glgpu::Tile* tiles = nullptr;
     glgpu::ATile* atiles = nullptr;     // A-sweep tiles
     int natiles = 0;
-    glgpu::Item* items = nullptr;
     glgpu::LoopState* loop = nullptr;
     glgpu::InstState* gather = nullptr;
     std::vector<glgpu::InstState> gather_h;
     glgpu::InstState* gather_pin = nullptr;  // pinned host copies of the per-call transfers
     glgpu::LoopState* loop_pin = nullptr;
     glgpu::Inst* insts_pin = nullptr;
-    int ntiles = 0, nitems = 0, psi_grid = 0, strip_rows = 0;
-    std::vector<int> inst_items;         // psi sweep items of each instance (at strip_rows)
+    int ntiles = 0;
+    glgpu::Item* litems = nullptr;       // FP32: items of the cooperative psi loop and their height
+    int nlitems = 0, loop_rows = 0;
     cudaGraphExec_t td_exec[glgpu::kTDGraphs] = {};
     bool td_graph_failed = false, use_graphs = true;
     int loop_guard = 0;                  // Jacobi loop guard in sweep launches (0: kLoopGuard)
@@ -327,12 +330,18 @@ size_t real_size(const glgpu_handle* h);
 // td.cu
 int td_run(glgpu_handle* h, double dt, int Nt, int eqn, glgpu_td_stats* stats, double* elapsed_ms);
 int time_sweeps(glgpu_handle* h, int which, int nrep, double* avg_ms);
-int choose_strip_rows(int dtype, const Geo* const* geos, int n);
-// FP32 psi sweep kernel of a selection: 4 = register strip (0, the default), 5 =
-// bulk-copy ring (1).  FP64 runs its Jacobi loop without strips (k_psi_loop_one).
-inline int psi_kind(int dtype, int select) { return dtype == 4 && select == 1 ? 5 : 4; }
-int psi_sweep_grid(int kind, int rows, int nitems);
+int choose_strip_rows(const Geo& g);
+// the FP32 bulk-copy psi sweep is selected (glgpu_set_psi_sweep_kernel)
+inline bool bulk_selected(const glgpu_handle* h) { return h->dtype == 4 && h->psi_select == 1; }
+int bulk_sweep_grid(int rows, int nitems);
 std::vector<Item> make_items(const Geo& g, int inst, int rows);
+// tdl.cu: the cooperative psi loop's kernel, its CTA size, its CTAs over n tiles (FP64) or items (FP32)
+const void* psi_loop_fn(int dtype);
+int psi_loop_threads(int dtype);
+int psi_loop_grid(int dtype, int n);
+constexpr int kWideCols = 56;  // output columns of an FP32 item of the loop
+int choose_loop_rows(const Geo* const* geos, int n);
+void add_loop_items(std::vector<Item>& items, const Geo& g, int inst, int rows);
 // tdr.cu
 bool res_prepare(ResState* r, glgpu_handle* const* hs, int n);
 void res_free(ResState* r);

@@ -179,434 +179,10 @@ template <typename T> struct PsiRow {
     unsigned cd;
 };
 
-// kFuse Jacobi sweeps of the psi step (svirl/cuda/td.h:4-133) over every active
-// instance in one launch, reading the per-step tables of k_link_U (link factors
-// U and link-weight codes), so the sweep does no transcendental math and no mask
-// logic.  A warp owns a strip of kStripCols output columns and RR rows;
-// its 32 lanes hold the columns x0-kFuse .. x0+31-kFuse, and sweep l (1..kFuse)
-// is valid on lanes l..31-l, so the halo columns are recomputed in registers
-// instead of being exchanged.  The warp walks down the rows: at step s it loads
-// row j0-kFuse+s of psi^(k) and the per-row inputs one row behind, and sweep l
-// produces row j0-kFuse+s-l from the three newest rows of sweep l-1 (each level
-// lags the previous one by a row).  x neighbours come from the adjacent lanes.
-// Every sweep's values on the strip are stored, and its residual kept, so the
-// loop can stop after any of the fused sweeps.  The row walk is unrolled with
-// every load issued one step ahead of its use.  Persistent grid: warps stride
-// over the item table.
-// CTAs of the psi sweep are small: its warps are independent, and registers are
-// allocated per CTA, so small CTAs fill an SM with more warps.
-#ifndef GLGPU_PSI_THREADS
-#define GLGPU_PSI_THREADS 64
-#endif
-// CTAs per SM the register allocation must allow: FP32 at 8 (128 registers a
-// thread, 16 warps per SM), FP64 at 1 (its sweep needs about 190 registers)
-#ifndef GLGPU_PSI_MIN_CTAS_F32
-#define GLGPU_PSI_MIN_CTAS_F32 8
-#endif
-#ifndef GLGPU_PSI_MIN_CTAS_F64
-#define GLGPU_PSI_MIN_CTAS_F64 1
-#endif
-// Row steps of the strip walk unrolled together (0: the whole walk).
-#ifndef GLGPU_PSI_ROW_UNROLL
-#define GLGPU_PSI_ROW_UNROLL 0
-#endif
-
-// Rows of inputs loaded ahead of their use in the register-strip sweep: FP32 2
-// (measured on 2049^2: 75 us per launch against 88 with 1 row; 3 rows: 76-77 us),
-// FP64 1 (register bound).
-#ifndef GLGPU_PSI_PREFETCH_F32
-#define GLGPU_PSI_PREFETCH_F32 2
-#endif
-template <typename T> constexpr int kPFof = sizeof(T) == 4 ? GLGPU_PSI_PREFETCH_F32 : 1;
-constexpr int kPsiThreads = GLGPU_PSI_THREADS, kPsiWarps = kPsiThreads / 32;
-template <typename T> constexpr bool kStoreInv = sizeof(T) == 8;
-template <typename T, int RR>
-__global__ void __launch_bounds__(kPsiThreads, sizeof(T) == 4 ? GLGPU_PSI_MIN_CTAS_F32 : GLGPU_PSI_MIN_CTAS_F64)
-k_psi_sweep(const Inst* __restrict__ insts, const Item* __restrict__ items, int nitems, LoopState* loop,
-            cudaGraphConditionalHandle cond, int use_cond) {
-    constexpr int K = kFuse, S = RR + 2 * kFuse, kPF = kPFof<T>;
-    constexpr int kRowUnroll = GLGPU_PSI_ROW_UNROLL > 0 ? GLGPU_PSI_ROW_UNROLL : S;
-    const int lane = threadIdx.x & 31;
-    const int gw = blockIdx.x * kPsiWarps + (threadIdx.x >> 5), nw = gridDim.x * kPsiWarps;
-    int cur_inst = -1, k = 0, count = 0, done = 1;
-    T wmax[K];
-    bool wnan[K];
-#pragma unroll
-    for (int l = 0; l < K; ++l) {
-        wmax[l] = T(0);
-        wnan[l] = false;
-    }
-    // per-instance values, refreshed when the warp moves to another instance
-    const C2<T>* cur = nullptr;
-    const C2<T>* rhs = nullptr;
-    C2<T>* outb[K];
-    const C2<T>* U = nullptr;
-    const uint8_t* code = nullptr;
-    T* dinv = nullptr;
-    uint32_t rt = 0;
-    for (int it = gw; it < nitems; it += nw) {
-        const Item w = items[it];
-        if (w.inst < 0) continue;  // group padding
-        if (w.inst != cur_inst) {
-            if (cur_inst >= 0 && !done) warp_flush<T>(insts, cur_inst, k, wmax, wnan, count, loop);
-            cur_inst = w.inst;
-            const InstState* st = insts[cur_inst].st;
-            done = *(volatile const int*)&st->done;
-            k = *(volatile const int*)&st->sweep;
-            const int R = *(volatile const int*)&st->rhs;
-            rt = *(volatile const uint32_t*)&st->rand_t;
-            const Inst& I = insts[cur_inst];
-            cur = (const C2<T>*)I.psi[pbuf(R, k)];
-            rhs = (const C2<T>*)I.psi[R];
-#pragma unroll
-            for (int l = 0; l < K; ++l) {
-                outb[l] = (C2<T>*)I.psi[pbuf(R, k + 1 + l)];
-                wmax[l] = T(0);
-                wnan[l] = false;
-            }
-            U = (const C2<T>*)I.U;
-            code = I.code;
-            dinv = (T*)I.dinv;
-            count = 0;
-        }
-        if (done) continue;
-        const Inst& I = insts[cur_inst];
-        const Geo g = I.g;
-        const T* eps_sp = (const T*)I.eps_sp;
-        const T dt = gsel<T>(I.dt, I.fdt), eps0 = gsel<T>(I.epsilon, I.fepsilon);
-        const T idx2 = GT(g, idx2), idy2 = GT(g, idy2);
-        const bool lang = I.lang_psi_on != 0;
-        const T lc = gsel<T>(I.lang_psi, I.flang_psi);
-        const int Nx = g.Nx, Ny = g.Ny;
-        const int i = w.x0 - K + lane;
-        const bool in_x = i >= 0 && i < Nx;
-        const bool calc_lane = in_x && lane >= 1 && lane <= 30;        // lanes any sweep computes
-        const bool own_lane = in_x && lane >= K && lane <= 31 - K;     // the strip's own columns
-        const int j0 = w.j0;
-        // FP64: the first launch of a step stores the diagonal reciprocals of the
-        // strip's own nodes, later launches of the step load them (the diagonal is
-        // fixed during the Jacobi loop; the FP64 pipe binds this build)
-        const bool load_inv = kStoreInv<T> && k > 0, store_inv = kStoreInv<T> && k == 0;
-        const C2<T> z = cmk<T>(T(0), T(0));
-        auto load_psi = [&](int y) -> C2<T> { return (in_x && y >= 0 && y < Ny) ? __ldg(&cur[i + Nx * y]) : z; };
-        auto load_side = [&](int y) -> PsiSide<T> {
-            PsiSide<T> q;
-            const bool row = y >= 0 && y < Ny;
-            const int n = i + Nx * y;
-            const bool ld = in_x && row, ldc = calc_lane && row;
-            if constexpr (sizeof(T) == 4) {
-                const float4 v = ld ? __ldg((const float4*)U + n) : make_float4(0.f, 0.f, 0.f, 0.f);
-                q.ua = cmk<T>(v.x, v.y);
-                q.ub = cmk<T>(v.z, v.w);
-            } else {
-                q.ua = ld ? __ldg(&U[2 * n]) : z;
-                q.ub = ld ? __ldg(&U[2 * n + 1]) : z;
-            }
-            q.cd = ldc ? (unsigned)__ldg(&code[n]) : 0u;
-            q.rr = ldc ? __ldg(&rhs[n]) : z;
-            if (load_inv) q.eps = ldc ? __ldg(&dinv[n]) : T(0);  // the stored reciprocal
-            else q.eps = (ldc && eps_sp) ? __ldg(&eps_sp[n]) : eps0;
-            return q;
-        };
-        // window of sweep l-1 (l = 1..K) as seen by sweep l: rows y-1 and y
-        C2<T> wp[K], wc[K];
-        PsiRow<T> D[K + 1];  // D[m]: per-row inputs of row (j0 - K + s - 1) - m
-#pragma unroll
-        for (int l = 0; l < K; ++l) wp[l] = wc[l] = z;
-#pragma unroll
-        for (int m = 0; m <= K; ++m) D[m] = PsiRow<T>{z, z, z, T(0), 0u};
-        // loaded inputs of row y -> sweep inputs (done one step after the loads were issued)
-        auto finish_side = [&](const PsiSide<T>& q, int y) -> PsiRow<T> {
-            PsiRow<T> r;
-            r.ua = q.ua;
-            r.ub = q.ub;
-            r.cd = q.cd;
-            r.rq = q.rr;
-            if (lang && calc_lane && y >= 0 && y < Ny) {
-                const uint32_t n = (uint32_t)(i + Nx * y);
-                r.rq.x = add_noise<T>(r.rq.x, lc, rand_1<T>(n, rt));
-                r.rq.y = add_noise<T>(r.rq.y, lc, rand_2<T>(n, rt));
-            }
-            if (load_inv) {
-                r.inv = q.eps;
-            } else {
-                r.inv = (q.cd & 3u) ? psi_diag_inv<T>(r.rq, q.eps, q.cd, dt, idx2, idy2) : T(0);
-                if (store_inv && own_lane && y >= j0 && y < j0 + RR && y < Ny) dinv[i + Nx * y] = r.inv;
-            }
-            return r;
-        };
-        // the rows' loads are issued kPF row steps ahead of their use (a ring of
-        // kPF rows in registers; the walk is unrolled, so the indexing is static)
-        C2<T> nx_p[kPF];
-        PsiSide<T> nx_s[kPF];
-#pragma unroll
-        for (int a = 0; a < kPF; ++a) {
-            nx_p[a] = load_psi(j0 - K + a);
-            nx_s[a] = load_side(j0 - K - 1 + a);
-        }
-#pragma unroll kRowUnroll
-        for (int s = 0; s < S; ++s) {
-            C2<T> newrow = nx_p[s % kPF];  // psi^(k) on row j0 - K + s
-#pragma unroll
-            for (int m = K; m >= 1; --m) D[m] = D[m - 1];
-            D[0] = finish_side(nx_s[s % kPF], j0 - K + s - 1);
-            if (s + kPF < S) {
-                nx_p[s % kPF] = load_psi(j0 - K + s + kPF);
-                nx_s[s % kPF] = load_side(j0 - K - 1 + s + kPF);
-            }
-#pragma unroll
-            for (int l = 1; l <= K; ++l) {
-                C2<T> out = z;
-                if (s >= 2 * l) {  // earlier rows of sweep l are above the strip's halo
-                    const int y = j0 - K + s - l;
-                    const C2<T> pc = wc[l - 1];
-                    const C2<T> pl = shfl_up_c<T>(pc, 1), pr = shfl_down_c<T>(pc, 1);
-                    const PsiRow<T>& d = D[l - 1];
-                    const C2<T> ual = shfl_up_c<T>(d.ua, 1);
-                    // every lane computes: outside the domain and on the edge lanes the
-                    // loaded inputs are zero with code 0, and psi_node returns 0 there
-                    {
-                        out = psi_node<T>(pl, pr, wp[l - 1], newrow, ual, d.ua, D[l].ub, d.ub, d.rq, d.inv, d.cd);
-                        if (own_lane && y >= j0 && y < j0 + RR && y < Ny) {
-                            outb[l - 1][i + Nx * y] = out;
-                            // max(|d re|, |d im|); a NaN component counts as 0 (the reference's
-                            // int conversion).  FP64 compares the bit patterns (non-negative
-                            // doubles order as integers), off the FP64 pipe; FP32 uses fmax,
-                            // which drops NaN operands.
-                            if constexpr (sizeof(T) == 8) {
-                                const unsigned long long kAbs = 0x7fffffffffffffffull, kInf = 0x7ff0000000000000ull;
-                                unsigned long long bx = (unsigned long long)__double_as_longlong(out.x - pc.x) & kAbs;
-                                unsigned long long by = (unsigned long long)__double_as_longlong(out.y - pc.y) & kAbs;
-                                if ((bx > kInf) | (by > kInf)) wnan[l - 1] = true;
-                                bx = bx > kInf ? 0ull : bx;
-                                by = by > kInf ? 0ull : by;
-                                const unsigned long long m = bx > by ? bx : by;
-                                const unsigned long long w = (unsigned long long)__double_as_longlong(wmax[l - 1]);
-                                wmax[l - 1] = __longlong_as_double((long long)(w > m ? w : m));
-                            } else {
-                                const T dr = fabs(out.x - pc.x), di = fabs(out.y - pc.y);
-                                if (isnan(dr) | isnan(di)) wnan[l - 1] = true;
-                                wmax[l - 1] = fmax(wmax[l - 1], fmax(dr, di));
-                            }
-                        }
-                    }
-                }
-                // sweep l has used the window of sweep l-1: advance it by one row
-                wp[l - 1] = wc[l - 1];
-                wc[l - 1] = newrow;
-                newrow = out;
-            }
-        }
-        ++count;
-    }
-    if (cur_inst >= 0 && !done) warp_flush<T>(insts, cur_inst, k, wmax, wnan, count, loop);
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        __threadfence();
-        unsigned gdone = atomicAdd(&loop->blocks_done, 1u);
-        if (gdone == gridDim.x - 1u) finish_launch(loop, cond, use_cond);
-    }
-}
-
-// The Jacobi loop of the psi step in one cooperative launch, one sweep per round and a
-// node per thread, for FP64 domains that fill the chip: the same node arithmetic as
-// k_psi_sweep, bitwise the same values and the same sweep counts.  The FP64 pipe bounds
-// it (20 FP64 instructions a node; a warp instruction takes 64 cycles of its scheduler),
-// so nothing is recomputed, while the strips of k_psi_sweep compute 32 columns for 26
-// and RR + 2 rows for RR; the five psi values and the link factors of a node come from
-// L1/L2, which are far from their limits.  A CTA's threads stride over the tiles (256
-// consecutive nodes).  All instances are at the same sweep of their loops, so a round's
-// buffers follow from its number, and of the loop state only `done` is read again.
-// Only whether a residual meets the stop rule counts, so where a CTA already holds one
-// that does not, the differences (two of the FP64 instructions) are left out.
-// Sweep at 1025 x 1025: 45 us, 38 of them FP64 pipe, against 72 for a third of a strip
-// launch of three sweeps inside a conditional graph node (513^2: 19 against 23, 65^2: 7.4
-// against 15; as a launch per sweep in the conditional node 61, 26 and 14).
-template <typename T>
-__device__ __forceinline__ void one_flush(const Inst& I, unsigned long long rmax, bool nan, unsigned long long* s_max) {
-    const int lane = threadIdx.x & 31;
-    const unsigned hi = __reduce_max_sync(0xffffffffu, (unsigned)(rmax >> 32));
-    const unsigned lo = __reduce_max_sync(0xffffffffu, (unsigned)(rmax >> 32) == hi ? (unsigned)rmax : 0u);
-    const bool any_nan = __any_sync(0xffffffffu, nan);
-    if (lane == 0) {
-        s_max[threadIdx.x >> 5] = (unsigned long long)hi << 32 | lo;
-        if (any_nan) atomicOr(&I.st->nanlv, 1);
-    }
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        unsigned long long v = s_max[0];
-        for (int q = 1; q < kWarps; ++q) v = v > s_max[q] ? v : s_max[q];
-        atomicMax(&I.st->resp[0], v);
-    }
-    __syncthreads();
-}
-
-// End of round `round`: the CTA that arrives last closes the sweep for every instance
-// whose loop still runs (finish_instance_psi), decides whether one is left, and publishes
-// round and decision in one word.  What the CTAs wrote in the sweep is visible after it.
-// false: leave the loop (finished, or a wait ran out).  The word of a round stays until
-// this CTA has arrived at the next one, so nobody misses it.
-__device__ __forceinline__ bool one_round(const Inst* insts, int ninst, LoopState* loop, int first, int round, int& s_word) {
-    const int seq = round - first + 1;  // rounds of this launch
-    if (threadIdx.x == 0) {
-        __threadfence();
-        s_word = atomicAdd(&loop->arrived, 1u) + 1u == (unsigned)seq * gridDim.x ? -1 : 0;
-    }
-    __syncthreads();
-    const bool last = s_word < 0;
-    if (last) {
-        int left = 0;
-        __threadfence();
-        for (int q = threadIdx.x; q < ninst; q += kThreads) {
-            const Inst& I = insts[q];
-            InstState* st = I.st;
-            if (*(volatile const int*)&st->done) continue;
-            const bool stop = atomicExch(&st->resp[0], 0ull) <= I.thr_psi || round + 1 >= kMaxSweeps;
-            if (atomicExch(&st->nanlv, 0)) st->nan_seen = 1;
-            if (stop) {
-                const int s = round + 1;
-                st->sweep = s;
-                st->done = 1;
-                st->rhs = pbuf<1>(st->rhs, s);
-                st->last_sweeps_psi = s;
-                st->total_sweeps_psi += s;
-                if (s > st->max_sweeps_psi) st->max_sweeps_psi = s;
-            } else {
-                left = 1;
-            }
-            __threadfence();
-        }
-        left = __syncthreads_or(left);
-        if (threadIdx.x == 0) {
-            if (seq == 1) loop->total_launches += 1;
-            if (!left) loop->active = 0;
-            if (left && seq >= kFuse * min(loop->guard, kMaxSweeps)) {  // the guard counts launches of kFuse sweeps
-                left = 0;
-                loop->err |= kErrLoopGuard;
-            }
-            loop->cont = left;
-            s_word = 2 * seq + left;
-            __threadfence();
-            asm volatile("st.release.gpu.global.u32 [%0], %1;" ::"l"(&loop->round), "r"(s_word) : "memory");
-        }
-    } else if (threadIdx.x == 0) {
-        unsigned word, it = 0;
-        for (;;) {
-            asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(word) : "l"(&loop->round) : "memory");
-            if (word >> 1 == (unsigned)seq) break;
-            if (++it >= kBarrierSpins || ((it & 1023u) == 0u && (*(volatile int*)&loop->err & kErrBarrier))) {
-                atomicOr(&loop->err, kErrBarrier);
-                word = 0u;
-                break;
-            }
-        }
-        __threadfence();
-        s_word = (int)word;
-    }
-    __syncthreads();
-    return s_word & 1;
-}
-
-template <typename T>
-__global__ void __launch_bounds__(kThreads)
-k_psi_loop_one(const Inst* __restrict__ insts, int ninst, const Tile* __restrict__ tiles, int ntiles, LoopState* loop,
-               int first) {
-    __shared__ int s_word, s_big;
-    __shared__ unsigned long long s_max[kWarps];
-    __shared__ C2<T>* s_psi[kPsiBufs];
-    int cur_inst = -1, R = 0, done = 1;
-    uint32_t rt = 0;
-    for (int round = first;; ++round) {
-        const C2<T>* cur = nullptr;
-        const C2<T>* rhs = nullptr;
-        C2<T>* nxt = nullptr;
-        unsigned long long rmax = 0ull, thr = 0ull;
-        bool rnan = false, fresh = true;
-        for (int it = blockIdx.x; it < ntiles; it += gridDim.x) {
-            const Tile t = tiles[it];
-            if (fresh || t.inst != cur_inst) {
-                if (!fresh && !done) one_flush<T>(insts[cur_inst], rmax, rnan, s_max);
-                // an instance's `done` changes only at the end of a round
-                const InstState* st = insts[t.inst].st;
-                if (t.inst != cur_inst || ninst > 1) {
-                    const Inst& I = insts[t.inst];
-                    done = *(volatile const int*)&st->done;
-                    R = *(volatile const int*)&st->rhs;
-                    rt = *(volatile const uint32_t*)&st->rand_t;
-                    if (threadIdx.x < kPsiBufs) s_psi[threadIdx.x] = (C2<T>*)I.psi[threadIdx.x];
-                }
-                if (threadIdx.x == 0) s_big = 0;
-                cur_inst = t.inst;
-                fresh = false;
-                __syncthreads();
-                cur = s_psi[pbuf<1>(R, round)];
-                rhs = s_psi[R];
-                nxt = s_psi[pbuf<1>(R, round + 1)];
-                thr = insts[cur_inst].thr_psi;
-                rmax = 0ull;
-                rnan = false;
-            }
-            const int n = t.n0 + (int)threadIdx.x;
-            const Inst& I = insts[cur_inst];
-            const Geo& g = I.g;
-            if (done || n >= g.N) continue;
-            const int Nx = g.Nx, j = n / Nx, i = n - j * Nx;
-            const C2<T>* __restrict__ U = (const C2<T>*)I.U;
-            const C2<T> z = cmk<T>(T(0), T(0));
-            const bool lt = i > 0, rg = i + 1 < Nx, dn = j > 0, up = j + 1 < g.Ny;
-            // psi was written by other SMs in the round before: no read-only loads
-            const C2<T> pc = cur[n];
-            const C2<T> pl = lt ? cur[n - 1] : z, pr = rg ? cur[n + 1] : z;
-            const C2<T> pd = dn ? cur[n - Nx] : z, pu = up ? cur[n + Nx] : z;
-            const C2<T> ua = __ldg(&U[2 * n]), ub = __ldg(&U[2 * n + 1]);
-            const C2<T> ual = lt ? __ldg(&U[2 * n - 2]) : z, ubd = dn ? __ldg(&U[2 * (n - Nx) + 1]) : z;
-            const unsigned cd = (unsigned)__ldg(&I.code[n]);
-            C2<T> rq = rhs[n];
-            if (I.lang_psi_on) {
-                const T lc = gsel<T>(I.lang_psi, I.flang_psi);
-                rq.x = add_noise<T>(rq.x, lc, rand_1<T>((uint32_t)n, rt));
-                rq.y = add_noise<T>(rq.y, lc, rand_2<T>((uint32_t)n, rt));
-            }
-            // the first sweep of a step stores the diagonal's reciprocal for the others
-            T* dinv = (T*)I.dinv;
-            T inv;
-            if (round > 0) {
-                inv = dinv[n];
-            } else {
-                const T* eps_sp = (const T*)I.eps_sp;
-                const T eps = eps_sp ? __ldg(&eps_sp[n]) : gsel<T>(I.epsilon, I.fepsilon);
-                inv = (cd & 3u) ? psi_diag_inv<T>(rq, eps, cd, gsel<T>(I.dt, I.fdt), GT(g, idx2), GT(g, idy2)) : T(0);
-                dinv[n] = inv;
-            }
-            const C2<T> out = psi_node<T>(pl, pr, pd, pu, ual, ua, ubd, ub, rq, inv, cd);
-            nxt[n] = out;
-            // a NaN component counts as 0 (the reference's int conversion); magnitudes are
-            // compared as integers, off the FP64 pipe.  A difference that overflows or is
-            // NaN needs an operand beyond 2^1022.
-            const unsigned big = max(max((unsigned)__double2hiint(out.x) & 0x7fffffffu, (unsigned)__double2hiint(out.y) & 0x7fffffffu),
-                                     max((unsigned)__double2hiint(pc.x) & 0x7fffffffu, (unsigned)__double2hiint(pc.y) & 0x7fffffffu));
-            if (__any_sync(__activemask(), *(volatile int*)&s_big == 0 || big >= 0x7fd00000u)) {
-                const unsigned long long kAbs = 0x7fffffffffffffffull, kInf = 0x7ff0000000000000ull;
-                unsigned long long bx = (unsigned long long)__double_as_longlong(out.x - pc.x) & kAbs;
-                unsigned long long by = (unsigned long long)__double_as_longlong(out.y - pc.y) & kAbs;
-                if ((bx > kInf) | (by > kInf)) rnan = true;
-                bx = bx > kInf ? 0ull : bx;
-                by = by > kInf ? 0ull : by;
-                const unsigned long long m = bx > by ? bx : by;
-                rmax = rmax > m ? rmax : m;
-                if (rmax > thr) *(volatile int*)&s_big = 1;
-            }
-        }
-        if (!fresh && !done) one_flush<T>(insts[cur_inst], rmax, rnan, s_max);
-        if (!one_round(insts, ninst, loop, first, round, s_word)) break;
-    }
-}
-
-// FP32 psi sweep with the inputs staged by bulk copies (TMA).  The same three
-// fused Jacobi sweeps per launch and the same register walk down a strip as
-// k_psi_sweep, bitwise the same values, but the rows a warp reads come from a
-// ring of shared-memory stages filled by the copy engine several rows ahead,
-// so the warps do not wait on global-memory latency.  A CTA runs kPsiGroup
+// FP32 psi sweep with the inputs staged by bulk copies (TMA): three fused Jacobi
+// sweeps per launch by the register walk of k_psi_loop_f32 (tdl.cu) on strips of 32
+// columns, bitwise the same values, but the rows a warp reads come from a ring of
+// shared-memory stages filled by the copy engine several rows ahead.  A CTA runs kPsiGroup
 // adjacent strips of one row band (one group of the item table); one thread
 // (thread 0) copies, per row of the band, the group's columns x0 - 3 ..
 // x0_last + 28 of psi^(k), of the right-hand side, of the link table and of the
@@ -1395,6 +971,10 @@ __global__ void k_loop_begin(const Inst* __restrict__ insts, int ninst, LoopStat
         st->res = 0ull;
         for (int l = 0; l < 4; ++l) st->resp[l] = 0ull;
         st->nanlv = 0;
+        if (which == 0) {
+            st->redo = 0;
+            st->keep = st->last_sweeps_psi < kFuse;
+        }
         active += part ? 1 : 0;
     }
     for (int o = 16; o > 0; o >>= 1) active += __shfl_down_sync(0xffffffffu, active, o);
@@ -1535,54 +1115,37 @@ struct TDLaunch {
     int natiles;
     const Item* items;
     LoopState* loop;
-    int ninst, ntiles, nitems, psi_grid, dtype, strip_rows, psi_kind;
+    int ninst, ntiles, nitems, psi_grid, dtype, strip_rows;
     int psi_cn;       // psi time stepping: 0 backward Euler, 1 Crank-Nicolson, 2 its kernel as written
     bool any_solveA;
     bool any_fv;  // an instance has fixed vortices (irregular potential or phase lock)
     const ResState* res;  // the resident loop (tdr.cu), or null: a launch per sweep
-    int one_grid;     // CTAs of the FP64 psi loop (psi_one_grid), 0: a launch per kFuse sweeps
+    const void* work;  // tiles or items of the cooperative psi loop (tdl.cu) and its CTAs; 0 CTAs: a launch per sweep or kFuse sweeps
+    int nwork, loop_grid;
 };
 
 static void* fv_psi_pre_fn(int dt) { return dt == 8 ? (void*)k_fv_psi_pre<double> : (void*)k_fv_psi_pre<float>; }
 static void* fv_psi_post_fn(int dt) { return dt == 8 ? (void*)k_fv_psi_post<double> : (void*)k_fv_psi_post<float>; }
 static void* fv_A_fn(int dt) { return dt == 8 ? (void*)k_fv_A<double> : (void*)k_fv_A<float>; }
 
-// The FP32 psi sweep kernel of a kind (psi_kind): register strip (the default) or
-// bulk-copy ring (selected per handle).
-static bool psi_bulk(int kind) { return kind == 5; }
-template <int V>
-static void* psi_sweep_fn_v(int kind, int rows) {
+// The bulk-copy psi sweep for strips of `rows` rows (one of kStripRowsSet): FP32, selected
+// per handle; the default is the loop of tdl.cu.
+template <int V = 0>
+static void* bulk_fn(int rows) {
     if constexpr (V < kNumStripRows) {
-        constexpr int R = kStripRowsSet[V];
-        if (rows == R)
-            return kind == 5 ? (void*)k_psi_sweep_bulk<R> : (void*)k_psi_sweep<float, R>;
-        return psi_sweep_fn_v<V + 1>(kind, rows);
+        return rows == kStripRowsSet[V] ? (void*)k_psi_sweep_bulk<kStripRowsSet[V]> : bulk_fn<V + 1>(rows);
     } else {
         return nullptr;
     }
 }
-// the sweep kernel compiled for strip height `rows` (one of kStripRowsSet), and its CTA size
-static void* psi_sweep_fn(int kind, int rows) { return psi_sweep_fn_v<0>(kind, rows); }
-static int psi_threads(int kind) { return psi_bulk(kind) ? kBulkThreads : kPsiThreads; }
 
-static cudaError_t launch_psi_sweep(int kind, int rows, int grid, cudaStream_t s, const Inst* insts, const Item* items,
-                                    int nitems, LoopState* loop) {
+static cudaError_t launch_bulk_sweep(int rows, int grid, cudaStream_t s, const Inst* insts, const Item* items, int nitems,
+                                     LoopState* loop) {
     cudaGraphConditionalHandle none = 0;
     int zero = 0;
     void* a[] = {&insts, &items, &nitems, &loop, &none, &zero};
-    return cudaLaunchKernel(psi_sweep_fn(kind, rows), dim3(grid), dim3(psi_threads(kind)), a, 0, s);
+    return cudaLaunchKernel(bulk_fn(rows), dim3(grid), dim3(kBulkThreads), a, 0, s);
 }
-// CTAs of the FP64 Jacobi loop over `ntiles` tiles (all of them are resident).
-static int psi_one_grid(int ntiles) {
-    int dev = 0, sms = 1, per_sm = 1;
-    cudaGetDevice(&dev);
-    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, (const void*)k_psi_loop_one<double>, kThreads, 0) != cudaSuccess ||
-        per_sm < 1)
-        per_sm = 1;
-    return ntiles < sms * per_sm ? ntiles : sms * per_sm;
-}
-
 static void* A_sweep_fn(int dtype) {
     return dtype == 8 ? (void*)k_A_sweep<double> : (void*)k_A_sweep<float>;
 }
@@ -1628,10 +1191,11 @@ static cudaError_t set_cooperative(cudaGraphNode_t node) {
 
 #define GCHK(x) do { cudaError_t e_ = (x); if (e_ != cudaSuccess) { err = e_; goto fail; } } while (0)
 
-static cudaError_t launch_psi_loop_one(int grid, cudaStream_t s, const Inst* insts, int ninst, const Tile* tiles, int ntiles,
-                                       LoopState* loop, int first) {
-    void* a[] = {&insts, &ninst, &tiles, &ntiles, &loop, &first};
-    return cudaLaunchCooperativeKernel((const void*)k_psi_loop_one<double>, dim3(grid), dim3(kThreads), a, 0, s);
+// The cooperative psi loop (tdl.cu) from sweep round `first` on.
+static cudaError_t launch_psi_loop(int dtype, int grid, cudaStream_t s, const Inst* insts, int ninst,
+                                   const void* work, int nwork, LoopState* loop, int first) {
+    void* a[] = {&insts, &ninst, &work, &nwork, &loop, &first};
+    return cudaLaunchCooperativeKernel(psi_loop_fn(dtype), dim3(grid), dim3(psi_loop_threads(dtype)), a, 0, s);
 }
 
 // Build the whole TD run of all instances as one graph:
@@ -1677,7 +1241,7 @@ static cudaError_t build_td_graph(const TDLaunch& L, int eqn, cudaGraphExec_t* e
     GCHK(add_while(top, &n_out, prev ? &prev : nullptr, prev ? 1 : 0, hout, &obody));
     prev = nullptr;
     if (do_psi) {
-        int cond = L.one_grid == 0 ? 1 : 0;
+        int cond = L.loop_grid == 0 ? 1 : 0;
         if (cond) GCHK(cudaGraphConditionalHandleCreate(&hpsi, obody, 1, cudaGraphCondAssignDefault));
         if (eqn == 0 && L.any_fv) {
             void* a[] = {&insts, &tiles};
@@ -1691,9 +1255,11 @@ static cudaError_t build_td_graph(const TDLaunch& L, int eqn, cudaGraphExec_t* e
             void* a[] = {&insts, &ninst, &loop, &hpsi, &cond, &zero};
             GCHK(chain(obody, (void*)k_loop_begin, g1, b1, a));
         }
-        if (L.one_grid > 0) {
-            void* a[] = {&insts, &ninst, &tiles, &ntiles, &loop, &zero};
-            GCHK(chain(obody, (void*)k_psi_loop_one<double>, dim3(L.one_grid), bt, a));
+        if (L.loop_grid > 0) {
+            const void* work = L.work;
+            int nwork = L.nwork;
+            void* a[] = {&insts, &ninst, &work, &nwork, &loop, &zero};
+            GCHK(chain(obody, (void*)psi_loop_fn(L.dtype), dim3(L.loop_grid), dim3(psi_loop_threads(L.dtype)), a));
             GCHK(set_cooperative(prev));
         } else {
             GCHK(add_while(obody, &nd, &prev, 1, hpsi, &pbody));
@@ -1705,8 +1271,8 @@ static cudaError_t build_td_graph(const TDLaunch& L, int eqn, cudaGraphExec_t* e
                 GCHK(add_kernel(pbody, &sw, nullptr, 0, cn_fn(L.dtype), gt, bt, a));
             } else {
                 void* a[] = {&insts, &items, &nitems, &loop, &hpsi, &one};
-                GCHK(add_kernel(pbody, &sw, nullptr, 0, psi_sweep_fn(L.psi_kind, L.strip_rows), dim3(L.psi_grid),
-                                dim3(psi_threads(L.psi_kind)), a));
+                GCHK(add_kernel(pbody, &sw, nullptr, 0, bulk_fn(L.strip_rows), dim3(L.psi_grid),
+                                dim3(kBulkThreads), a));
             }
         }
         {
@@ -1804,11 +1370,11 @@ static cudaError_t run_host_loop(const TDLaunch& L, int eqn, int Nt, cudaStream_
             if (part == 0 && (L.any_solveA || L.any_fv)) launch_link_U(L, 1, s);
             if (part == 1 && L.any_fv) fv_A(0);
             k_loop_begin<<<1, 32, 0, s>>>(L.insts, L.ninst, L.loop, none, 0, part);
-            if (part == 0 && L.one_grid > 0) {
-                const cudaError_t e = launch_psi_loop_one(L.one_grid, s, L.insts, L.ninst, L.tiles, L.ntiles, L.loop, 0);
+            if (part == 0 && L.loop_grid > 0) {
+                const cudaError_t e = launch_psi_loop(L.dtype, L.loop_grid, s, L.insts, L.ninst, L.work, L.nwork, L.loop, 0);
                 if (e != cudaSuccess) return e;
             }
-            for (; part == 1 || L.one_grid == 0;) {
+            for (; part == 1 || L.loop_grid == 0;) {
                 for (int c = 0; c < chunk; ++c) {
                     if (part == 0 && L.psi_cn) {
                         const int aw = L.psi_cn == 2 ? 1 : 0;
@@ -1817,7 +1383,7 @@ static cudaError_t run_host_loop(const TDLaunch& L, int eqn, int Nt, cudaStream_
                         else
                             k_psi_sweep_cn<float><<<L.ntiles, kThreads, 0, s>>>(L.insts, L.tiles, L.loop, none, 0, aw);
                     } else if (part == 0) {
-                        launch_psi_sweep(L.psi_kind, L.strip_rows, L.psi_grid, s, L.insts, L.items, L.nitems, L.loop);
+                        launch_bulk_sweep(L.strip_rows, L.psi_grid, s, L.insts, L.items, L.nitems, L.loop);
                     } else {
                         if (L.dtype == 8) k_A_sweep<double><<<L.natiles, kThreads, 0, s>>>(L.insts, L.atiles, L.loop, none, 0);
                         else k_A_sweep<float><<<L.natiles, kThreads, 0, s>>>(L.insts, L.atiles, L.loop, none, 0);
@@ -1857,6 +1423,7 @@ __global__ void k_bench_prep(const Inst* __restrict__ insts, int ninst, LoopStat
         st->res = 0ull;
         for (int l = 0; l < 4; ++l) st->resp[l] = 0ull;
         st->nanlv = 0;
+        st->redo = st->keep = 0;
     }
     if (threadIdx.x == 0) {
         loop->active = ninst;
@@ -1920,10 +1487,13 @@ int time_sweeps(glgpu_handle* h, int which, int nrep, double* avg_ms) {
         for (int q = 0; q < per_rep && e == cudaSuccess; ++q) {
             k_bench_prep<<<1, 32, 0, h->stream>>>(h->inst, 1, h->loop, which == 0 ? 1 : q);
             cudaEventRecord(e0, h->stream);
-            if (which == 0 && h->dtype == 8) {
-                e = launch_psi_loop_one(psi_one_grid(h->ntiles), h->stream, h->inst, 1, h->tiles, h->ntiles, h->loop, 1);
+            if (which == 0 && !bulk_selected(h)) {
+                const void* work = h->dtype == 8 ? (const void*)h->tiles : h->litems;
+                const int n = h->dtype == 8 ? h->ntiles : h->nlitems;
+                e = launch_psi_loop(h->dtype, psi_loop_grid(h->dtype, n), h->stream, h->inst, 1,
+                                    work, n, h->loop, 1);
             } else if (which == 0) {
-                launch_psi_sweep(psi_kind(h->dtype, h->psi_select), h->strip_rows, h->psi_grid, h->stream, h->inst, h->items,
+                launch_bulk_sweep(h->strip_rows, h->psi_grid, h->stream, h->inst, h->items,
                                  h->nitems, h->loop);
             } else {
                 if (h->dtype == 8) k_A_sweep<double><<<h->natiles, kThreads, 0, h->stream>>>(h->inst, h->atiles, h->loop, none, 0);
@@ -1950,40 +1520,29 @@ int time_sweeps(glgpu_handle* h, int which, int nrep, double* avg_ms) {
     return GLGPU_OK;
 }
 
-// CTAs of the persistent psi sweep (nitems: length of the item table): one warp
-// per item (register-strip kernel) or one CTA per group of kPsiGroup items
-// (bulk-copy kernel), up to all SMs at full occupancy.
-int psi_sweep_grid(int kind, int rows, int nitems) {
+// CTAs of the persistent bulk-copy sweep (nitems: length of the item table): one per group
+// of kPsiGroup items, up to all SMs at full occupancy.
+int bulk_sweep_grid(int rows, int nitems) {
     int dev = 0, sms = 1, per_sm = 1;
     cudaGetDevice(&dev);
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-    void* fn = psi_sweep_fn(kind, rows);
-    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, fn, psi_threads(kind), 0) != cudaSuccess || per_sm < 1)
+    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, bulk_fn(rows), kBulkThreads, 0) != cudaSuccess || per_sm < 1)
         per_sm = 1;
-    const int need = psi_bulk(kind) ? nitems / kPsiGroup : (nitems + kPsiWarps - 1) / kPsiWarps;
-    const int full = sms * per_sm;
+    const int need = nitems / kPsiGroup, full = sms * per_sm;
     return need < full ? (need > 0 ? need : 1) : full;
 }
 
-// Strip height for a set of instances (a handle or a batch), from a model of
-// the persistent sweep: warps take items round-robin, so a launch lasts as long
-// as the warp with the most items, ceil(items / warps), and an item of R rows
-// costs about 3R + 6 row-sweeps (sweep l of the kFuse = 3 fused sweeps covers
-// R + 2(3 - l) rows).  Measured on 2049^2 (FP32, us per node-sweep): R = 8: 38.1,
-// 12: 34.7, 14: 33.5, 17: 32.2, 18: 32.7; the model ranks them the same way.
-int choose_strip_rows(int dtype, const Geo* const* geos, int n) {
+// Strip height of the bulk-copy sweep for a domain, from a model of the persistent sweep:
+// CTAs take groups round-robin, so a launch lasts as long as the CTA with the most,
+// ceil(groups / CTAs), and a strip of R rows costs about 3R + 6 row-sweeps (sweep l of the
+// kFuse = 3 fused sweeps covers R + 2(3 - l) rows).
+int choose_strip_rows(const Geo& g) {
     int best = kStripRowsSet[0];
     long long best_cost = -1;
-    for (int v = 0; v < kNumStripRows; ++v) {
-        const int R = kStripRowsSet[v];
-        long long table = 0;
-        for (int q = 0; q < n; ++q) table += strip_table_len(geos[q]->Nx, geos[q]->Ny, R);
-        // work units: groups of kPsiGroup items per CTA (bulk-copy kernel) or items per warp
-        const int kind = psi_kind(dtype, 0);
-        const bool bulk = psi_bulk(kind);
-        const long long units = bulk ? table / kPsiGroup : table;
-        const long long slots = (long long)psi_sweep_grid(kind, R, (int)table) * (bulk ? 1 : kPsiWarps);
-        const long long cost = (units + slots - 1) / slots * (3LL * R + 2LL * kFuse);
+    for (int R : kStripRowsSet) {
+        const long long table = strip_table_len(g.Nx, g.Ny, R), groups = table / kPsiGroup;
+        const long long slots = bulk_sweep_grid(R, (int)table);
+        const long long cost = (groups + slots - 1) / slots * (3LL * R + 2LL * kFuse);
         if (best_cost < 0 || cost < best_cost) {
             best_cost = cost;
             best = R;
@@ -2116,12 +1675,13 @@ int td_run(glgpu_handle* h, double dt, int Nt, int eqn, glgpu_td_stats* stats, d
     L.atiles = h->atiles; L.natiles = h->natiles;
     L.ninst = 1; L.ntiles = h->ntiles; L.nitems = h->nitems; L.psi_grid = h->psi_grid; L.dtype = h->dtype;
     L.strip_rows = h->strip_rows;
-    L.psi_kind = psi_kind(h->dtype, h->psi_select);
     L.psi_cn = h->psi_scheme;
     L.any_solveA = h->inst_h.solveA != 0;
     L.any_fv = h->vpi != nullptr || h->lock_n > 0;
     L.res = resident ? &h->res : nullptr;
-    L.one_grid = resident || h->psi_scheme != 0 || h->dtype != 8 ? 0 : psi_one_grid(h->ntiles);
+    L.work = h->dtype == 8 ? (const void*)h->tiles : h->litems;
+    L.nwork = h->dtype == 8 ? h->ntiles : h->nlitems;
+    L.loop_grid = resident || h->psi_scheme != 0 || bulk_selected(h) ? 0 : psi_loop_grid(h->dtype, L.nwork);
     TDOutcome o = td_core(h->stream, L, Nt, eqn, h->td_exec, &h->td_graph_failed, h->use_graphs, h->loop_guard,
                           elapsed_ms != nullptr,
                           h->st_gather, &ps->st, &ps->loop);
@@ -2154,7 +1714,6 @@ int batch_td(glgpu_batch* b, double dt, int Nt, int eqn, glgpu_td_stats* stats, 
         h->inst_h.dt = dt;
         h->inst_h.fdt = (float)dt;
         insts[q] = h->inst_h;
-        insts[q].nitems = b->inst_items[q];  // at the batch's strip height
         any_solveA = any_solveA || h->inst_h.solveA != 0;
         any_fv = any_fv || h->vpi != nullptr || h->lock_n > 0;
     }
@@ -2162,16 +1721,16 @@ int batch_td(glgpu_batch* b, double dt, int Nt, int eqn, glgpu_td_stats* stats, 
     cudaError_t e = cudaMemcpyAsync(b->insts, b->insts_pin, sizeof(Inst) * insts.size(), cudaMemcpyHostToDevice, b->stream);
     if (e != cudaSuccess) return batch_error(b, GLGPU_E_CUDA, std::string("batch_td: ") + cudaGetErrorString(e));
     TDLaunch L;
-    L.insts = b->insts; L.tiles = b->tiles; L.items = b->items; L.loop = b->loop;
+    L.insts = b->insts; L.tiles = b->tiles; L.items = nullptr; L.loop = b->loop;
     L.atiles = b->atiles; L.natiles = b->natiles;
-    L.ninst = b->ninst; L.ntiles = b->ntiles; L.nitems = b->nitems; L.psi_grid = b->psi_grid; L.dtype = b->dtype;
-    L.strip_rows = b->strip_rows;
-    L.psi_kind = psi_kind(b->dtype, 0);
+    L.ninst = b->ninst; L.ntiles = b->ntiles; L.nitems = L.psi_grid = L.strip_rows = 0; L.dtype = b->dtype;
     L.psi_cn = 0;
     L.any_solveA = any_solveA;
     L.any_fv = any_fv;
     L.res = resident ? &b->res : nullptr;
-    L.one_grid = resident || b->dtype != 8 ? 0 : psi_one_grid(b->ntiles);
+    L.work = b->dtype == 8 ? (const void*)b->tiles : b->litems;
+    L.nwork = b->dtype == 8 ? b->ntiles : b->nlitems;
+    L.loop_grid = resident ? 0 : psi_loop_grid(b->dtype, L.nwork);
     TDOutcome o = td_core(b->stream, L, Nt, eqn, b->td_exec, &b->td_graph_failed, b->use_graphs, b->loop_guard,
                           elapsed_ms != nullptr,
                           b->gather, b->gather_pin, b->loop_pin);
