@@ -32,7 +32,7 @@ namespace glgpu {
 constexpr int kPart = 17;  // doubles of per-tile partials
 // The CG kernels walk tiles of rep x 256 nodes of one instance: each thread
 // accumulates rep nodes in registers before the block reduction, so the
-// reduction's cost is shared by rep nodes.  rep (2, 4 or 8) is a property of the
+// reduction's cost is shared by rep nodes.  rep (1, 2, 4 or 8) is a property of the
 // instance alone (cg_rep_of), so an instance's arithmetic, and with it its CG
 // run, does not depend on the batch it is in.
 constexpr int kCGRepMax = 8;
@@ -44,12 +44,16 @@ struct CGTile {
 // it into at least kCGMinTiles tiles (so that an instance run alone spreads over
 // a quarter of the SMs), else 2.  Deeper tiles share each block reduction among
 // more nodes: 64 instances, 7.19M nodes: 0.77 ms per iteration with depth 4 for
-// all, 0.70 with 8 for all.
+// all, 0.70 with 8 for all.  FP64 (last depth 1): a tile for each of two CTAs per SM, as a
+// node there takes longer than the reduction; 8 instances of 97^2 .. 193^2: 226 us per
+// iteration with depth 1, 241 with 2.
 constexpr int kCGMinTiles = 38;
-static int cg_rep_of(int N) {
-    for (int r = kCGRepMax; r > 2; r /= 2)
-        if ((N + kThreads * r - 1) / (kThreads * r) >= kCGMinTiles) return r;
-    return 2;
+constexpr int kCGMinTiles64 = 304;
+static int cg_rep_of(int N, int dtype) {
+    const int last = dtype == 8 ? 1 : 2, tiles = dtype == 8 ? kCGMinTiles64 : kCGMinTiles;
+    for (int r = kCGRepMax; r > last; r /= 2)
+        if ((N + kThreads * r - 1) / (kThreads * r) >= tiles) return r;
+    return last;
 }
 // Resident CTAs per SM asked of the compiler for the FP32 CG kernels (caps their
 // registers at 65536 / (kThreads * minimum CTAs)), per kernel.  Measured on the
@@ -61,6 +65,10 @@ static int cg_rep_of(int N) {
 #ifndef GLGPU_CG_MINB
 #define GLGPU_CG_MINB 4
 #endif
+// FP64: two CTAs per SM for the gradient and coefficient kernels (128 registers; one CTA,
+// with 190 and 166, leaves the FP64 pipe idle at a tile's start and end).  8 instances of
+// 97^2 .. 193^2, us per iteration at depth 1: 226 with 2, 230 with 3 (spills), 252 with 1.
+constexpr int kCGMinB64 = 2;
 #ifndef GLGPU_CG_MINB_GRAD
 #define GLGPU_CG_MINB_GRAD 5
 #endif
@@ -90,6 +98,89 @@ struct CGLoop {
 template <typename T>
 __device__ __forceinline__ void store_partials(const double* v, int nv, double* out) {
     for (int k = 0; k < nv; ++k) out[k] = v[k];
+}
+
+// Sums of P per-thread values over the CTA into out[0 .. NV - 1], by the threads that hold
+// them.  A warp halves the number of values that a lane carries at each exchange: the
+// lanes of one half keep the first half of the values and hand over the rest, and so on,
+// so P values take P - 1 + log2(32 / P) additions per lane where P separate trees take
+// 5 P (an FP64 addition takes 64 cycles of its scheduler; FP32 carries hi + lo pairs, see
+// block_sum, at a dozen instructions an addition).  Fixed order: deterministic.
+template <int P, int NV = P> __device__ __forceinline__ void fold_sum(double (&v)[P], double* out) {
+    __shared__ double sm[kWarps][P];
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    int comp = 0;
+#pragma unroll
+    for (int o = 16, m = P; o > 0; o >>= 1) {
+        if (m > 1) {
+            m /= 2;
+            const bool upper = (lane & o) != 0;
+#pragma unroll
+            for (int k = 0; k < m; ++k) {
+                const double keep = upper ? v[k + m] : v[k], give = upper ? v[k] : v[k + m];
+                v[k] = keep + __shfl_xor_sync(0xffffffffu, give, o);
+            }
+            if (upper) comp += m;
+        } else {
+            v[0] += __shfl_xor_sync(0xffffffffu, v[0], o);
+        }
+    }
+    __syncthreads();
+    if ((lane & (32 / P - 1)) == 0) sm[w][comp] = v[0];
+    __syncthreads();
+    if (threadIdx.x < NV) {
+        double s = sm[0][threadIdx.x];
+#pragma unroll
+        for (int q = 1; q < kWarps; ++q) s += sm[q][threadIdx.x];
+        out[threadIdx.x] = s;
+    }
+    __threadfence();
+    __syncthreads();
+}
+template <int P, int NV = P> __device__ __forceinline__ void fold_sum(float (&v)[P], double* out) {
+    __shared__ float sh[kWarps][P], sl[kWarps][P];
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    float lo[P];
+#pragma unroll
+    for (int k = 0; k < P; ++k) lo[k] = 0.f;
+    int comp = 0;
+#pragma unroll
+    for (int o = 16, m = P; o > 0; o >>= 1) {
+        const bool split = m > 1;
+        if (split) m /= 2;
+        const bool upper = split && (lane & o) != 0;
+#pragma unroll
+        for (int k = 0; k < m; ++k) {
+            const int k2 = split ? k + m : k;
+            const float hi = upper ? v[k2] : v[k], gh = upper ? v[k] : v[k2];
+            const float hl = upper ? lo[k2] : lo[k], gl = upper ? lo[k] : lo[k2];
+            const float oh = __shfl_xor_sync(0xffffffffu, gh, o), ol = o == 16 ? 0.f : __shfl_xor_sync(0xffffffffu, gl, o);
+            float sum, err;
+            two_sum(hi, oh, sum, err);
+            v[k] = sum;
+            lo[k] = hl + (ol + err);
+        }
+        if (upper) comp += m;
+    }
+    __syncthreads();
+    if ((lane & (32 / P - 1)) == 0) {
+        sh[w][comp] = v[0];
+        sl[w][comp] = lo[0];
+    }
+    __syncthreads();
+    if (threadIdx.x < NV) {
+        float hi = sh[0][threadIdx.x], l = sl[0][threadIdx.x];
+#pragma unroll
+        for (int q = 1; q < kWarps; ++q) {
+            float sum, err;
+            two_sum(hi, sh[q][threadIdx.x], sum, err);
+            hi = sum;
+            l = l + (sl[q][threadIdx.x] + err);
+        }
+        out[threadIdx.x] = (double)hi + (double)l;
+    }
+    __threadfence();
+    __syncthreads();
 }
 
 // Components 0..NV-1 of the partials of one instance's tiles summed by one
@@ -360,7 +451,7 @@ __device__ __forceinline__ void grad_tile(const Inst& I, int n0, int rep, const 
 }
 
 template <typename T>
-__global__ void __launch_bounds__(kThreads, sizeof(T) == 4 ? GLGPU_CG_MINB_GRAD : 1)
+__global__ void __launch_bounds__(kThreads, sizeof(T) == 4 ? GLGPU_CG_MINB_GRAD : kCGMinB64)
 kb_grad(const Inst* __restrict__ insts, const CGTile* __restrict__ tiles, double* __restrict__ partials, CGLoop* loop) {
     const CGTile t = tiles[blockIdx.x];
     const Inst& I = insts[t.inst];
@@ -375,9 +466,8 @@ kb_grad(const Inst* __restrict__ insts, const CGTile* __restrict__ tiles, double
     };
     if (I.solveA) run(std::true_type{});
     else run(std::false_type{});
-    double vs[5];
-    block_sum<5>(v, vs);
-    if (threadIdx.x == 0) store_partials<T>(vs, 5, partials + (size_t)blockIdx.x * kPart);
+    T v8[8] = {v[0], v[1], v[2], v[3], v[4], T(0), T(0), T(0)};
+    fold_sum<8, 5>(v8, partials + (size_t)blockIdx.x * kPart);
     if (last_cta_of_instance(cs, I.ntiles)) inst_beta(I, cs, partials, loop);
 }
 
@@ -621,13 +711,13 @@ __device__ __forceinline__ void dir_coef_tile(const Inst& I, int n0, int rep, T 
             const int i = n % g.Nx, j = n / g.Nx;
             const unsigned cb = I.cbits[n];
             if (SA) {
-                coef_node<T, 17>(g, gsel<T>(I.kappa2, I.fkappa2), eps0, (const T*)I.eps_sp, H, psi_at, phase, ab, lk,
+                coef_node<T, 17, false>(g, gsel<T>(I.kappa2, I.fkappa2), eps0, (const T*)I.eps_sp, H, psi_at, phase, ab, lk,
                                  n, i, j, cb, dpsi, dA, c);
             } else {
                 T c5[5] = {T(0), T(0), T(0), T(0), T(0)};
-                coef_node<T, 5>(g, T(-1), eps0, (const T*)I.eps_sp, H, psi_at, phase, ab, lk, n, i, j, cb, dpsi, dA,
+                coef_node<T, 5, false>(g, T(-1), eps0, (const T*)I.eps_sp, H, psi_at, phase, ab, lk, n, i, j, cb, dpsi, dA,
                                 c5);
-                c[0] += c5[0]; c[5] += c5[1]; c[10] += c5[2]; c[15] += c5[3]; c[16] += c5[4];
+                c[5] += c5[1]; c[10] += c5[2]; c[15] += c5[3]; c[16] += c5[4];
             }
             dN[n] = dpsi(n);
             if (SA) {
@@ -639,7 +729,7 @@ __device__ __forceinline__ void dir_coef_tile(const Inst& I, int n0, int rep, T 
 }
 
 template <typename T>
-__global__ void __launch_bounds__(kThreads, sizeof(T) == 4 ? GLGPU_CG_MINB_COEF : 1)
+__global__ void __launch_bounds__(kThreads, sizeof(T) == 4 ? GLGPU_CG_MINB_COEF : kCGMinB64)
 kb_dir_coef(const Inst* __restrict__ insts, const CGTile* __restrict__ tiles, double* __restrict__ partials,
             CGLoop* loop) {
     const CGTile t = tiles[blockIdx.x];
@@ -658,9 +748,12 @@ kb_dir_coef(const Inst* __restrict__ insts, const CGTile* __restrict__ tiles, do
     };
     if (I.solveA) run(std::true_type{});
     else run(std::false_type{});
-    double cs17[17];
-    block_sum<17>(c, cs17);
-    if (threadIdx.x == 0) store_partials<T>(cs17, 17, partials + (size_t)blockIdx.x * kPart);
+    // c00 is not needed (0 in the partials)
+    T c16[16];
+#pragma unroll
+    for (int k = 0; k < 16; ++k) c16[k] = c[k + 1];
+    fold_sum<16>(c16, partials + (size_t)blockIdx.x * kPart + 1);
+    if (threadIdx.x == 0) partials[(size_t)blockIdx.x * kPart] = 0.0;
     if (last_cta_of_instance(cs, I.ntiles)) inst_alpha<sizeof(T) == 8>(I, cs, partials, loop);
 }
 
@@ -1084,7 +1177,7 @@ int batch_cg(glgpu_batch* b, int n_iter, double rtol, double gtol, int flags, in
         insts[q] = h->inst_h;
         // this copy of the descriptors indexes the CG tile table (rep x 256 nodes per tile)
         insts[q].tile0 = (int)cgtiles.size();
-        const int rep = cg_rep_of(h->g.N);
+        const int rep = cg_rep_of(h->g.N, h->dtype);
         for (int n0 = 0; n0 < h->g.N; n0 += kThreads * rep) cgtiles.push_back(CGTile{q, n0, rep, 0});
         insts[q].ntiles = (int)cgtiles.size() - insts[q].tile0;
         insts[q].cg_exact = (flags & GLGPU_CG_EXACT_BOUNDARY) ? 1 : 0;

@@ -16,14 +16,26 @@ template <typename T> struct DuW {
 };
 template <typename T> __device__ __forceinline__ DuW<T> du_weights(unsigned cb) {
     DuW<T> w;
-    const T mm = GL_MM(cb) ? T(1) : T(0), mp = GL_MP(cb) ? T(1) : T(0);
-    const T pm = GL_PM(cb) ? T(1) : T(0), pp = GL_PP(cb) ? T(1) : T(0);
-    w.r_m0 = T(0.5) * (mm + mp);
-    w.r_p0 = T(0.5) * (pm + pp);
-    w.r_0m = T(0.5) * (mm + pm);
-    w.r_0p = T(0.5) * (mp + pp);
-    w.g = T(0.25) * (w.r_m0 + w.r_p0 + w.r_0m + w.r_0p);
+    const unsigned mm = GL_MM(cb) ? 1u : 0u, mp = GL_MP(cb) ? 1u : 0u, pm = GL_PM(cb) ? 1u : 0u, pp = GL_PP(cb) ? 1u : 0u;
+    // by selects: an FP64 addition or conversion takes 64 cycles of its scheduler
+    auto half = [](unsigned k) -> T { return k == 0u ? T(0) : (k == 1u ? T(0.5) : T(1)); };
+    w.r_m0 = half(mm + mp);
+    w.r_p0 = half(pm + pp);
+    w.r_0m = half(mm + pm);
+    w.r_0p = half(mp + pp);
+    const unsigned k = mm + mp + pm + pp;
+    w.g = k < 2u ? (k == 0u ? T(0) : T(0.25)) : (k == 2u ? T(0.5) : (k == 3u ? T(0.75) : T(1)));
     return w;
+}
+
+// w times the Du weight of a link between two cells, at least one of them there: w, or
+// w / 2 if one is missing.
+template <typename T> __device__ __forceinline__ T du_times(bool both, T w, T half) { return both ? w : half; }
+
+// p0 - p1 U(ph), (s, c) = sincos(ph): the difference along a link, two fused operations
+// per component.
+template <typename T> __device__ __forceinline__ C2<T> link_diff(C2<T> p0, T s, T c, C2<T> p1) {
+    return cmk<T>(fma(-s, p1.y, fma(-c, p1.x, p0.x)), fma(s, p1.x, fma(-c, p1.y, p0.y)));
 }
 
 // abei + ab on one link, each term present when its pointer is non-NULL.
@@ -187,12 +199,8 @@ __device__ __forceinline__ T curlcurl_link_exact(const Geo& g, const T* abei, co
     return curlcurl_link<T>(g, abei, ab, H, i, j, xdir);
 }
 
-// 2 (psi0 - psi1 U(ph)) with (s, c) = sincos(ph) (svirl/cuda/cg.h:4-12)
-template <typename T> __device__ __forceinline__ C2<T> gjac_sc(C2<T> p0, T s, T c, C2<T> p1) {
-    return cmk<T>(T(2) * (p0.x - (p1.x * c + p1.y * s)), T(2) * (p0.y - (p1.y * c - p1.x * s)));
-}
-
-// dF/d(Re psi) + i dF/d(Im psi) at node n (svirl/cuda/cg.h:15-121), dx*dy included.
+// dF/d(Re psi) + i dF/d(Im psi) at node n (svirl/cuda/cg.h:15-121), dx*dy included;
+// a link adds 2 w (psi0 - psi1 U(ph)) (cg.h:4-12).
 template <typename T, typename LK>
 __device__ __forceinline__ C2<T> grad_psi_node(const Geo& g, T eps0, const T* eps_sp, const C2<T>* psi, const LK& lk,
                                                int n, int i, int j, unsigned cb) {
@@ -203,23 +211,28 @@ __device__ __forceinline__ C2<T> grad_psi_node(const Geo& g, T eps0, const T* ep
         const C2<T> p0 = psi[n];
         const T eps = eps_sp ? eps_sp[n] : eps0;
         const T p = p0.x * p0.x + p0.y * p0.y - eps;
-        gj = cadd(gj, cscale(T(2) * w.g * p, p0));
+        const T k = T(2) * w.g * p;
+        gj = cmk<T>(k * p0.x, k * p0.y);
+        auto add = [&gj, p0](T w2, T sn, T cs, C2<T> p1) {
+            const C2<T> d = link_diff<T>(p0, sn, cs, p1);
+            gj = cmk<T>(fma(w2, d.x, gj.x), fma(w2, d.y, gj.y));
+        };
         T sn, cs;  // the links below and left of the node enter with the opposite phase: sin(-x) = -sin(x)
         if (GL_MM(cb) || GL_MP(cb)) {
             lk.sc_sum((i - 1) + (g.Nx - 1) * j, dx, sn, cs);
-            gj = cadd(gj, cscale(w.r_m0 * idx2, gjac_sc<T>(p0, -sn, cs, psi[n - 1])));
+            add(du_times(GL_MM(cb) && GL_MP(cb), T(2) * idx2, idx2), -sn, cs, psi[n - 1]);
         }
         if (GL_PM(cb) || GL_PP(cb)) {
             lk.sc_sum(i + (g.Nx - 1) * j, dx, sn, cs);
-            gj = cadd(gj, cscale(w.r_p0 * idx2, gjac_sc<T>(p0, sn, cs, psi[n + 1])));
+            add(du_times(GL_PM(cb) && GL_PP(cb), T(2) * idx2, idx2), sn, cs, psi[n + 1]);
         }
         if (GL_MM(cb) || GL_PM(cb)) {
             lk.sc_sum(g.Na + i + g.Nx * (j - 1), dy, sn, cs);
-            gj = cadd(gj, cscale(w.r_0m * idy2, gjac_sc<T>(p0, -sn, cs, psi[n - g.Nx])));
+            add(du_times(GL_MM(cb) && GL_PM(cb), T(2) * idy2, idy2), -sn, cs, psi[n - g.Nx]);
         }
         if (GL_MP(cb) || GL_PP(cb)) {
             lk.sc_sum(g.Na + i + g.Nx * j, dy, sn, cs);
-            gj = cadd(gj, cscale(w.r_0p * idy2, gjac_sc<T>(p0, sn, cs, psi[n + g.Nx])));
+            add(du_times(GL_MP(cb) && GL_PP(cb), T(2) * idy2, idy2), sn, cs, psi[n + g.Nx]);
         }
     }
     return cscale(GT(g, dxdy), gj);
@@ -259,8 +272,11 @@ __device__ __forceinline__ T grad_A_link(const Geo& g, T kappa2, T H, const C2<T
 // psi(m) gives the order parameter at node m, phase(l) the phase A_ei + A of link l
 // (link_phase), ab5 the vector potential alone (read by the NV = 5 magnetic term
 // only, which the kappa = inf callers never reach); lk the link factors of the
-// node's own links.
-template <typename T, int NV, typename PS, typename PH, typename FD, typename FA, typename LK>
+// node's own links.  WITH0: c00 too (the search itself does not need it).  A link's part
+// is written with the neighbour's values turned into the node's frame, q = U(ph) psi1 and
+// e = U(ph) d1, from which all its products follow, and with the powers of dA's phase
+// made once: 56 FP64 instructions where the separate products took 85.
+template <typename T, int NV, bool WITH0 = true, typename PS, typename PH, typename FD, typename FA, typename LK>
 __device__ __forceinline__ void coef_node(const Geo& g, T kappa2, T eps0, const T* eps_sp, T H, const PS& psi,
                                           const PH& phase, const T* ab5, const LK& lk, int n, int i, int j,
                                           unsigned cb, const FD& dpsi, const FA& dA, T (&c)[NV]) {
@@ -273,15 +289,17 @@ __device__ __forceinline__ void coef_node(const Geo& g, T kappa2, T eps0, const 
         const T eps = eps_sp ? eps_sp[n] : eps0;
         const T p2 = cabs2(p0), d2 = cabs2(d0);
         const T tw = T(2) * (p0.x * d0.x + p0.y * d0.y);
-        const T k00 = w.g * (T(0.5) * p2 - eps) * p2;
+        const T k00 = WITH0 ? w.g * (T(0.5) * p2 - eps) * p2 : T(0);
         const T k10 = w.g * tw * (p2 - eps);
         const T k20 = w.g * (-eps * d2 + T(0.5) * tw * tw + p2 * d2);
         const T k30 = w.g * tw * d2;
         const T k40 = w.g * T(0.5) * d2 * d2;
         if (NV == 5) {
-            c[0] += k00; c[1] += k10; c[2] += k20; c[3] += k30; c[4] += k40;
+            if (WITH0) c[0] += k00;
+            c[1] += k10; c[2] += k20; c[3] += k30; c[4] += k40;
         } else {
-            c[0] += k00; c[5] += k10; c[10] += k20; c[15] += k30; c[16] += k40;
+            if (WITH0) c[0] += k00;
+            c[5] += k10; c[10] += k20; c[15] += k30; c[16] += k40;
         }
 #pragma unroll
         for (int dir = 0; dir < 2; ++dir) {
@@ -290,37 +308,35 @@ __device__ __forceinline__ void coef_node(const Geo& g, T kappa2, T eps0, const 
             const int nl = dir == 0 ? i + (g.Nx - 1) * j : g.Na + i + g.Nx * j;
             const int m1 = dir == 0 ? n + 1 : n + g.Nx;
             const T d = dir == 0 ? dx : dy;
-            const T wr = (dir == 0 ? w.r_p0 : w.r_0p) * (dir == 0 ? idx2 : idy2);
+            const T full = dir == 0 ? idx2 : idy2;
+            const bool both = GL_PP(cb) && (dir == 0 ? GL_PM(cb) : GL_MP(cb));
+            const T wr = du_times(both, full, T(0.5) * full), wr2 = du_times(both, T(2) * full, full);
             const C2<T> p1 = psi(m1), d1 = dpsi(m1);
             T s, cs;
             lk.sc_split(nl, d, s, cs);
-            const C2<T> gp = grad_c_sc<T>(p0, s, cs, p1), gd = grad_c_sc<T>(d0, s, cs, d1);
-            const T gg_p = gp.x * gp.x + gp.y * gp.y;
-            const T gg_d = gd.x * gd.x + gd.y * gd.y;
-            const T zr = gp.x * gd.x + gp.y * gd.y;  // Re(conj(gp) * gd)
-            if (NV == 5) {
-                c[2] += wr * gg_d;
-                c[1] += wr * T(2) * zr;
-                c[0] += wr * gg_p;
-            } else {
-                c[0] += wr * gg_p;
-                c[5] += wr * T(2) * zr;
-                c[10] += wr * gg_d;
+            const C2<T> gp = link_diff<T>(p0, s, cs, p1), gd = link_diff<T>(d0, s, cs, d1);
+            const T gg_d = fma(gd.x, gd.x, gd.y * gd.y);
+            const T zr = fma(gp.x, gd.x, gp.y * gd.y);  // Re(conj(gp) * gd)
+            constexpr int k1 = NV == 5 ? 1 : 5, k2 = NV == 5 ? 2 : 10;
+            if (WITH0) c[0] = fma(wr, fma(gp.x, gp.x, gp.y * gp.y), c[0]);
+            c[k1] = fma(wr2, zr, c[k1]);
+            c[k2] = fma(wr, gg_d, c[k2]);
+            if constexpr (NV != 5) {
+                const C2<T> q = cmk<T>(p0.x - gp.x, p0.y - gp.y), e = cmk<T>(d0.x - gd.x, d0.y - gd.y);
                 const T dph = d * dA(nl);
-                const T dph2 = dph * dph;
-                const C2<T> Um = cmk<T>(cs, s);  // U(-ph)
-                const C2<T> z1 = cmul(cmul(p0, Um), cconj(p1));
-                const C2<T> z2 = cadd(cmul(cmul(p0, Um), cconj(d1)), cmul(cmul(d0, Um), cconj(p1)));
-                const C2<T> z3 = cmul(cmul(d0, Um), cconj(d1));
-                const C2<T> zz[3] = {z1, z2, z3};
-#pragma unroll
-                for (int q = 0; q < 3; ++q) {
-                    const int b = 1 + 5 * q;
-                    c[b + 0] += wr * T(2) * zz[q].y * dph;
-                    c[b + 1] += wr * zz[q].x * dph2;
-                    c[b + 2] += -wr / T(3) * zz[q].y * dph2 * dph;
-                    c[b + 3] += -wr / T(12) * zz[q].x * dph2 * dph2;
-                }
+                // 2 w dph, w dph^2, -w dph^3 / 3, -w dph^4 / 12
+                const T f1 = wr2 * dph, h = T(0.5) * dph, f2 = f1 * h, f3 = f2 * (T(-1.0 / 3.0) * dph), f4 = f3 * (T(0.5) * h);
+                auto add = [&](int b, T zx, T zy) {
+                    c[b + 0] = fma(zy, f1, c[b + 0]);
+                    c[b + 1] = fma(zx, f2, c[b + 1]);
+                    c[b + 2] = fma(zy, f3, c[b + 2]);
+                    c[b + 3] = fma(zx, f4, c[b + 3]);
+                };
+                // p0 conj(q), p0 conj(e) + d0 conj(q), d0 conj(e)
+                add(1, fma(p0.x, q.x, p0.y * q.y), fma(p0.y, q.x, -(p0.x * q.y)));
+                add(6, fma(p0.x, e.x, fma(p0.y, e.y, fma(d0.x, q.x, d0.y * q.y))),
+                    fma(p0.y, e.x, fma(-p0.x, e.y, fma(d0.y, q.x, -(d0.x * q.y)))));
+                add(11, fma(d0.x, e.x, d0.y * e.y), fma(d0.y, e.x, -(d0.x * e.y)));
             }
         }
     }
@@ -329,15 +345,16 @@ __device__ __forceinline__ void coef_node(const Geo& g, T kappa2, T eps0, const 
         const int ia00 = i + Nxa * j, ia0p = i + Nxa * (j + 1), ib00 = g.Na + i + g.Nx * j, ibp0 = g.Na + i + 1 + g.Nx * j;
         if (NV == 5) {
             const T dB = idx * (ab5[ibp0] - ab5[ib00]) - idy * (ab5[ia0p] - ab5[ia00]) - H;
-            c[0] += kappa2 * dB * dB;
+            if (WITH0) c[0] += kappa2 * dB * dB;
         } else {
             const T a00 = phase(ia00), a0p = phase(ia0p);
             const T b00 = phase(ib00), bp0 = phase(ibp0);
             const T BH = idx * (bp0 - b00) - idy * (a0p - a00) - H;
             const T dB = idx * (dA(ibp0) - dA(ib00)) - idy * (dA(ia0p) - dA(ia00));
-            c[0] += kappa2 * BH * BH;
-            c[1] += kappa2 * T(2) * BH * dB;
-            c[2] += kappa2 * dB * dB;
+            const T kd = kappa2 * dB;
+            if (WITH0) c[0] = fma(kappa2 * BH, BH, c[0]);
+            c[1] = fma(T(2) * kd, BH, c[1]);
+            c[2] = fma(kd, dB, c[2]);
         }
     }
 }
