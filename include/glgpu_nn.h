@@ -38,11 +38,12 @@ int glnn_conv3x3_fwd(const void* x1, int32_t c1, const void* x2, int32_t c2, con
                      void* y, int32_t n, int32_t h, int32_t w, int32_t cout, int32_t relu, int32_t* err, void* stream);
 
 /* Operand loads of glnn_conv3x3_fwd (and of glnn_conv3x3_bwd_data with relu = 0):
- * 2 (default) = by TMA (cp.async.bulk.tensor from 4-D / 2-D / 3-D tensor maps) in a
- * persistent kernel (CTAs loop over output tiles, two tensor-memory accumulators,
- * the epilogue of one tile under the MMAs of the next); 1 = by TMA, one output tile
- * per CTA; both for the shapes they take (c1, c2, cout multiples of 64; w a multiple
- * of 128 or a divisor of 128; h*w a multiple of 128), the thread gather otherwise;
+ * 2 (default) = by TMA (cp.async.bulk.tensor) in persistent kernels: up to 128 input
+ * channels, one box of input per 16 x 8 pixel tile for all nine taps (any image size;
+ * c1 and c2 multiples of 16, or c1 = 8 alone); more input channels, a box per tap with
+ * the epilogue of one tile under the MMAs of the next (c1, c2, cout multiples of 64; w
+ * a multiple of 128 or a divisor of 128; h*w a multiple of 128).  1 = by TMA, one
+ * output tile per CTA, for the latter shapes.  The thread gather otherwise;
  * 0 = always the thread gather.  Every setting computes the same values bitwise.
  * Nonzero also selects the tcgen05 weight gradient (0: the mma.sync one).
  * Process-wide. */
@@ -75,6 +76,18 @@ int glnn_conv3x3_bwd_weight(const void* dy, const void* y, int32_t relu, const v
 /* bfloat16 copies of a float32 weight W[cout][9][cin]: wb (same layout) and
  * wt[9][cin][cout] (for the data gradient); either may be NULL. */
 int glnn_prep_weights(const float* w, void* wb, void* wt, int32_t cout, int32_t cin, void* stream);
+
+/* A layer's calls in one: the bfloat16 copies of w into wpack (wb, then wt: 18 * cout *
+ * cin elements, 16-byte aligned) and the forward; and from that wpack the ReLU mask of
+ * dy, the data gradient (dx1 and dx2 NULL: left out) and the weight gradient, with
+ * glnn_conv3x3_layer_work() bytes of 16-byte aligned scratch. */
+int glnn_conv3x3_layer_fwd(const float* w, void* wpack, const void* x1, int32_t c1, const void* x2, int32_t c2,
+                           const float* bias, void* y, int32_t n, int32_t h, int32_t wd, int32_t cout, int32_t relu,
+                           int32_t* err, void* stream);
+int64_t glnn_conv3x3_layer_work(int32_t n, int32_t h, int32_t w, int32_t cin, int32_t cout, int32_t relu);
+int glnn_conv3x3_layer_bwd(const void* dy, const void* y, int32_t relu, const void* wpack, const void* x1, int32_t c1,
+                           void* dx1, const void* x2, int32_t c2, void* dx2, float* dw, float* db, void* work,
+                           int64_t work_bytes, int32_t n, int32_t h, int32_t w, int32_t cout, int32_t* err, void* stream);
 
 /* 2x2 average pooling (h, w even) and nearest 2x upsampling, with their
  * gradients; h, w are the dimensions of the larger tensor. */

@@ -104,6 +104,11 @@ _SIGNATURES = {
     "glnn_conv3x3_bwd_weight_work": (C.c_int64, [C.c_int32, C.c_int32, C.c_int32, C.c_int32, C.c_int32]),
     "glnn_conv3x3_bwd_weight": (C.c_int, [_P, _P, C.c_int32, _P, C.c_int32, _P, C.c_int32, _P, _P, _P, C.c_int64,
                                           C.c_int32, C.c_int32, C.c_int32, C.c_int32, _P, _P]),
+    "glnn_conv3x3_layer_fwd": (C.c_int, [_P, _P, _P, C.c_int32, _P, C.c_int32, _P, _P, C.c_int32, C.c_int32, C.c_int32,
+                                         C.c_int32, C.c_int32, _P, _P]),
+    "glnn_conv3x3_layer_work": (C.c_int64, [C.c_int32, C.c_int32, C.c_int32, C.c_int32, C.c_int32, C.c_int32]),
+    "glnn_conv3x3_layer_bwd": (C.c_int, [_P, _P, C.c_int32, _P, _P, C.c_int32, _P, _P, C.c_int32, _P, _P, _P, _P, C.c_int64,
+                                         C.c_int32, C.c_int32, C.c_int32, C.c_int32, _P, _P]),
     "glnn_prep_weights": (C.c_int, [_P, _P, _P, C.c_int32, C.c_int32, _P]),
     "glnn_pool2_fwd": (C.c_int, [_P, _P, C.c_int32, C.c_int32, C.c_int32, C.c_int32, _P]),
     "glnn_pool2_bwd": (C.c_int, [_P, _P, C.c_int32, C.c_int32, C.c_int32, C.c_int32, _P]),

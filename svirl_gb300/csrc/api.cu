@@ -62,7 +62,6 @@ void upload_inst(glgpu_handle* h) {
     I.code = h->code;
     I.dinv = h->dinv;
     I.st = h->st;
-    I.cg = h->cgst;
     I.cbits = h->cbits;
     I.vpi = h->vpi;
     I.lock = h->lock;
@@ -106,7 +105,6 @@ static void free_all(glgpu_handle* h) {
     for (int q = 0; q < kTDGraphs; ++q)
         if (h->td_exec[q]) cudaGraphExecDestroy(h->td_exec[q]);
     if (h->st_gather) cudaFree(h->st_gather);
-    if (h->cgst) cudaFree(h->cgst);
     if (h->cbits) cudaFree(h->cbits);
     if (h->vpi) cudaFree(h->vpi);
     if (h->lock) cudaFree(h->lock);
@@ -620,7 +618,7 @@ int glgpu_batch_destroy(glgpu_batch* b) {
         if (b->td_exec[q]) cudaGraphExecDestroy(b->td_exec[q]);
     if (b->cg_exec) cudaGraphExecDestroy(b->cg_exec);
     res_free(&b->res);
-    void* ptrs[] = {b->insts, b->gather, b->tiles, b->atiles, b->litems, b->loop, b->cg_partials, b->cg_loop, b->cg_tiles};
+    void* ptrs[] = {b->insts, b->gather, b->tiles, b->atiles, b->litems, b->loop, b->cg_partials, b->cg_loop, b->cg_tiles, b->cg_states};
     for (void* p : ptrs)
         if (p) cudaFree(p);
     void* pins[] = {b->gather_pin, b->loop_pin, b->insts_pin};

@@ -152,9 +152,8 @@ int cg_ensure(glgpu_handle* h) {
         cudaMemsetAsync(h->dir_A[q], 0, ab, h->stream);
     }
     cudaMemsetAsync(h->dscal + 28, 0, 2 * sizeof(double), h->stream);  // beta = 0
-    if (cudaMalloc(&h->cgst, sizeof(CGState)) != cudaSuccess || cudaMalloc(&h->cbits, (size_t)h->g.N) != cudaSuccess)
+    if (cudaMalloc(&h->cbits, (size_t)h->g.N) != cudaSuccess)
         return set_error(h, GLGPU_E_OOM, "cg: out of device memory");
-    cudaMemsetAsync(h->cgst, 0, sizeof(CGState), h->stream);
     h->cg_g = 0;
     h->cg_dir = 0;
     upload_inst(h);  // the descriptor carries the CG buffers

@@ -1169,6 +1169,7 @@ int batch_cg(glgpu_batch* b, int n_iter, double rtol, double gtol, int flags, in
     if (n_iter < 0 || !(rtol >= 0.0) || !(gtol >= 0.0)) return batch_error(b, GLGPU_E_ARG, "batch_cg: bad n_iter, rtol or gtol");
     std::vector<Inst> insts(b->ninst);
     std::vector<CGTile> cgtiles;
+    int ntiles = 0;
     for (int q = 0; q < b->ninst; ++q) {
         glgpu_handle* h = b->hs[q];
         const int rc = cg_ensure(h);
@@ -1176,10 +1177,12 @@ int batch_cg(glgpu_batch* b, int n_iter, double rtol, double gtol, int flags, in
         cudaStreamSynchronize(h->stream);
         insts[q] = h->inst_h;
         // this copy of the descriptors indexes the CG tile table (rep x 256 nodes per tile)
-        insts[q].tile0 = (int)cgtiles.size();
         const int rep = cg_rep_of(h->g.N, h->dtype);
-        for (int n0 = 0; n0 < h->g.N; n0 += kThreads * rep) cgtiles.push_back(CGTile{q, n0, rep, 0});
-        insts[q].ntiles = (int)cgtiles.size() - insts[q].tile0;
+        insts[q].tile0 = ntiles;
+        insts[q].ntiles = (h->g.N + kThreads * rep - 1) / (kThreads * rep);
+        ntiles += insts[q].ntiles;
+        if (!b->cg_tiles)
+            for (int n0 = 0; n0 < h->g.N; n0 += kThreads * rep) cgtiles.push_back(CGTile{q, n0, rep, 0});
         insts[q].cg_exact = (flags & GLGPU_CG_EXACT_BOUNDARY) ? 1 : 0;
         insts[q].cg_target = b->cg_targets.empty() ? NAN : b->cg_targets[q];
         insts[q].cg_target_tol = b->cg_target_tol;
@@ -1194,6 +1197,10 @@ int batch_cg(glgpu_batch* b, int n_iter, double rtol, double gtol, int flags, in
         return batch_error(b, GLGPU_E_OOM, "batch_cg: out of device memory");
     if (!b->cg_loop && cudaMalloc(&b->cg_loop, sizeof(CGLoop)) != cudaSuccess)
         return batch_error(b, GLGPU_E_OOM, "batch_cg: out of device memory");
+    if (!b->cg_states && cudaMalloc(&b->cg_states, sizeof(CGState) * (size_t)b->ninst) != cudaSuccess)
+        return batch_error(b, GLGPU_E_OOM, "batch_cg: out of device memory");
+    for (int q = 0; q < b->ninst; ++q) insts[q].cg = b->cg_states + q;
+    b->cg_states_h.resize(b->ninst);
     cudaStream_t s = b->stream;
     CGLoop lp;
     memset(&lp, 0, sizeof(lp));
@@ -1243,6 +1250,8 @@ int batch_cg(glgpu_batch* b, int n_iter, double rtol, double gtol, int flags, in
         if (e == cudaSuccess) e = cg_launch_epilogue(L, s);
     }
     if (elapsed_ms) cudaEventRecord(ev1, s);
+    if (e == cudaSuccess)
+        e = cudaMemcpyAsync(b->cg_states_h.data(), b->cg_states, sizeof(CGState) * (size_t)b->ninst, cudaMemcpyDeviceToHost, s);
     if (e == cudaSuccess) e = cudaStreamSynchronize(s);
     if (elapsed_ms) {
         float ms = 0.f;
@@ -1254,9 +1263,7 @@ int batch_cg(glgpu_batch* b, int n_iter, double rtol, double gtol, int flags, in
     if (e != cudaSuccess) return batch_error(b, GLGPU_E_CUDA, std::string("batch_cg: ") + cudaGetErrorString(e));
     int nfail = 0;
     for (int q = 0; q < b->ninst; ++q) {
-        CGState cs;
-        e = cudaMemcpy(&cs, b->hs[q]->cgst, sizeof(cs), cudaMemcpyDeviceToHost);
-        if (e != cudaSuccess) return batch_error(b, GLGPU_E_CUDA, std::string("batch_cg: ") + cudaGetErrorString(e));
+        const CGState& cs = b->cg_states_h[q];
         if (iters) iters[q] = cs.iter;
         if (energies) energies[q] = cs.E;
         if (grad_rel) grad_rel[q] = cs.g2_0 > 0.0 ? std::sqrt(cs.g2 / cs.g2_0) : 0.0;

@@ -87,7 +87,7 @@ struct Inst {
     const int32_t* lock;      // phase-lock node list or NULL
     int lock_n, pad_lock;
     InstState* st;
-    CGState* cg;              // batched device CG state (NULL until used)
+    CGState* cg;              // batched device CG state (set in a batch's descriptors for a CG call)
     void* gpsi[2];            // CG gradient buffers (psi part, A part) and directions
     void* gA[2];
     void* dpsi[2];
@@ -250,7 +250,6 @@ struct glgpu_handle {
     void* dir_psi[2] = {nullptr, nullptr};
     void* dir_A[2] = {nullptr, nullptr};
     int cg_g = 0, cg_dir = 0;           // current index of g / dir
-    glgpu::CGState* cgst = nullptr;     // batched device CG state
     void* vpi = nullptr;                // irregular vector potential (fixed vortices), Nab, or NULL (the TD step's copy)
     int32_t* lock = nullptr;            // phase-lock node list (fixed vortices) or NULL
     int lock_n = 0;
@@ -308,6 +307,8 @@ struct glgpu_batch {
     int cg_ntiles = 0;
     double* cg_partials = nullptr;       // cg_ntiles * 17 doubles
     void* cg_loop = nullptr;             // CGLoop
+    glgpu::CGState* cg_states = nullptr; // one per instance
+    std::vector<glgpu::CGState> cg_states_h;
     cudaGraphExec_t cg_exec = nullptr;
     bool cg_graph_failed = false;
     std::vector<double> cg_targets;      // per-instance energy targets (empty: none)

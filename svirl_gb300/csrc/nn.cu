@@ -584,6 +584,46 @@ int glnn_prep_weights(const float* w, void* wb, void* wt, int32_t cout, int32_t 
     return ret(cudaGetLastError());
 }
 
+int glnn_conv3x3_layer_fwd(const float* w, void* wpack, const void* x1, int32_t c1, const void* x2, int32_t c2,
+                           const float* bias, void* y, int32_t n, int32_t h, int32_t wd, int32_t cout, int32_t relu,
+                           int32_t* err, void* stream) {
+    const int cin = c1 + c2;
+    if (!wpack || cin <= 0 || cout <= 0) return GLGPU_E_ARG;
+    const int rc = glnn_prep_weights(w, wpack, (bf16*)wpack + (size_t)cout * 9 * cin, cout, cin, stream);
+    return rc ? rc : glnn_conv3x3_fwd(x1, c1, x2, c2, wpack, bias, y, n, h, wd, cout, relu, err, stream);
+}
+
+// bytes of the masked output gradient in front of the weight gradient's work space
+static size_t layer_mask_bytes(int n, int h, int w, int cout, int relu) {
+    return relu ? ((size_t)n * h * w * cout * sizeof(bf16) + 255) / 256 * 256 : 0;
+}
+
+int64_t glnn_conv3x3_layer_work(int32_t n, int32_t h, int32_t w, int32_t cin, int32_t cout, int32_t relu) {
+    if (n <= 0 || h <= 0 || w <= 0 || cin <= 0 || cout <= 0) return 0;
+    return (int64_t)(layer_mask_bytes(n, h, w, cout, relu) + (size_t)glnn_conv3x3_bwd_weight_work(n, h, w, cin, cout) * sizeof(float));
+}
+
+int glnn_conv3x3_layer_bwd(const void* dy, const void* y, int32_t relu, const void* wpack, const void* x1, int32_t c1,
+                           void* dx1, const void* x2, int32_t c2, void* dx2, float* dw, float* db, void* work,
+                           int64_t work_bytes, int32_t n, int32_t h, int32_t w, int32_t cout, int32_t* err, void* stream) {
+    const int cin = c1 + c2;
+    if (!dy || !wpack || !work || cin <= 0 || cout <= 0 || work_bytes < glnn_conv3x3_layer_work(n, h, w, cin, cout, relu))
+        return GLGPU_E_ARG;
+    const size_t mask = layer_mask_bytes(n, h, w, cout, relu);
+    if (relu) {
+        const int rc = glnn_relu_mask(dy, y, work, (int64_t)n * h * w * cout, stream);
+        if (rc) return rc;
+        dy = work;
+    }
+    if (dx1 || dx2) {
+        const int rc = glnn_conv3x3_bwd_data(dy, y, 0, (const bf16*)wpack + (size_t)cout * 9 * cin, dx1, c1, dx2, c2, n, h, w, cout,
+                                             err, stream);
+        if (rc) return rc;
+    }
+    return glnn_conv3x3_bwd_weight(dy, y, 0, x1, c1, x2, c2, dw, db, (float*)((char*)work + mask),
+                                   (work_bytes - (int64_t)mask) / (int64_t)sizeof(float), n, h, w, cout, err, stream);
+}
+
 static bool pool_ok(const void* a, const void* b, int n, int h, int w, int c) {
     return a && b && n > 0 && h > 1 && w > 1 && h % 2 == 0 && w % 2 == 0 && c > 0 && c % 8 == 0 && aligned16(a) &&
            aligned16(b);

@@ -60,10 +60,10 @@ _err = {}
 
 def _err_flag(device):
     """Device int the tcgen05 convolutions set when a bounded wait runs out."""
-    key = str(device)
-    if key not in _err:
-        _err[key] = torch.zeros(1, dtype=torch.int32, device=device)
-    return _err[key]
+    t = _err.get(device)
+    if t is None:
+        t = _err[device] = torch.zeros(1, dtype=torch.int32, device=device)
+    return t
 
 
 def check_kernel_errors():
@@ -87,45 +87,38 @@ class Conv3x3(torch.autograd.Function):
         n, h, wd, c1 = x1.shape
         c2 = 0 if x2 is None else x2.shape[3]
         cout = w.shape[0]
-        wb = torch.empty(w.shape, dtype=torch.bfloat16, device=w.device)
-        wt = torch.empty((3, 3, c1 + c2, cout), dtype=torch.bfloat16, device=w.device)
-        s = _stream()
-        _ok(lib.glnn_prep_weights(_ptr(w), _ptr(wb), _ptr(wt), cout, c1 + c2, s), "prep_weights")
+        # the bf16 weights for both directions
+        wp = torch.empty((18 * (c1 + c2) * cout,), dtype=torch.bfloat16, device=w.device)
         y = torch.empty((n, h, wd, cout), dtype=torch.bfloat16, device=x1.device)
-        _ok(lib.glnn_conv3x3_fwd(_ptr(x1), c1, _ptr(x2), c2, _ptr(wb), _ptr(b), _ptr(y), n, h, wd, cout,
-                                 1 if relu else 0, _ptr(_err_flag(x1.device)), s), "conv3x3_fwd")
-        ctx.save_for_backward(x1, x2, wt, y)
+        _ok(lib.glnn_conv3x3_layer_fwd(w.data_ptr(), wp.data_ptr(), x1.data_ptr(), c1, 0 if x2 is None else x2.data_ptr(), c2,
+                                       0 if b is None else b.data_ptr(), y.data_ptr(), n, h, wd, cout, 1 if relu else 0,
+                                       _err_flag(x1.device).data_ptr(), torch.cuda.current_stream().cuda_stream), "conv3x3_fwd")
+        ctx.save_for_backward(x1, x2, wp, y)
         ctx.relu = bool(relu)
         return y
 
     @staticmethod
     def backward(ctx, dy):
         lib = _lib_nn()
-        x1, x2, wt, y = ctx.saved_tensors
+        x1, x2, wp, y = ctx.saved_tensors
         dy = dy.contiguous()
         n, h, wd, c1 = x1.shape
         c2 = 0 if x2 is None else x2.shape[3]
         cout = y.shape[3]
-        s = _stream()
-        relu = 0
-        if ctx.relu:
-            # dy * relu'(y) once, for both gradients (their TMA kernels load it as is)
-            dym = torch.empty_like(dy)
-            _ok(lib.glnn_relu_mask(_ptr(dy), _ptr(y), _ptr(dym), dy.numel(), s), "relu_mask")
-            dy = dym
+        relu = 1 if ctx.relu else 0
         dx1 = dx2 = None
         if ctx.needs_input_grad[0] or ctx.needs_input_grad[1]:
             dx1 = torch.empty_like(x1)
             dx2 = None if x2 is None else torch.empty_like(x2)
-            _ok(lib.glnn_conv3x3_bwd_data(_ptr(dy), _ptr(y), relu, _ptr(wt), _ptr(dx1), c1, _ptr(dx2), c2, n, h, wd,
-                                          cout, _ptr(_err_flag(dy.device)), s), "conv3x3_bwd_data")
         dw = torch.empty((cout, 3, 3, c1 + c2), dtype=torch.float32, device=dy.device)
         db = torch.empty((cout,), dtype=torch.float32, device=dy.device)
-        nwork = int(lib.glnn_conv3x3_bwd_weight_work(n, h, wd, c1 + c2, cout))
-        work = torch.empty((nwork,), dtype=torch.float32, device=dy.device)
-        _ok(lib.glnn_conv3x3_bwd_weight(_ptr(dy), _ptr(y), relu, _ptr(x1), c1, _ptr(x2), c2, _ptr(dw), _ptr(db),
-                                        _ptr(work), nwork, n, h, wd, cout, _ptr(_err_flag(dy.device)), s),
-            "conv3x3_bwd_weight")
+        nbytes = int(lib.glnn_conv3x3_layer_work(n, h, wd, c1 + c2, cout, relu))
+        work = torch.empty((nbytes,), dtype=torch.uint8, device=dy.device)
+        _ok(lib.glnn_conv3x3_layer_bwd(dy.data_ptr(), y.data_ptr(), relu, wp.data_ptr(), x1.data_ptr(), c1,
+                                       0 if dx1 is None else dx1.data_ptr(), 0 if x2 is None else x2.data_ptr(), c2,
+                                       0 if dx2 is None else dx2.data_ptr(), dw.data_ptr(), db.data_ptr(), work.data_ptr(), nbytes,
+                                       n, h, wd, cout, _err_flag(dy.device).data_ptr(),
+                                       torch.cuda.current_stream().cuda_stream), "conv3x3_bwd")
         return dx1, dx2, dw, db, None
 
 
