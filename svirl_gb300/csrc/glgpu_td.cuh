@@ -73,13 +73,18 @@ __device__ __forceinline__ C2<T> psi_node(C2<T> p_left, C2<T> p_right, C2<T> p_p
 // (svirl/cuda/td.h:310-463): values of links outside the domain are passed as 0.
 // x link: the x links below and above, the y links that start below (at this node's
 // column and the next) and at the link; y link: likewise to the left and right.
+// FP32 sums each side by itself: which sweep meets the absolute stop rule hangs on the
+// rounding of these sums (|A| reaches H L, the rule is 1e-6), so their order is part of
+// the results.  FP64 takes the fewest operations on its pipe.
 template <typename T>
 __device__ __forceinline__ T A_nbs_x(T idy2, T idxy, T a_dn, T a_up, T b_dn0, T b_dn1, T b0, T b1) {
-    return fma(idxy, (b_dn1 - b_dn0) + (b0 - b1), mul_rn<T>(idy2, a_dn + a_up));
+    if constexpr (sizeof(T) == 8) return fma(idxy, (b_dn1 - b_dn0) + (b0 - b1), mul_rn<T>(idy2, a_dn + a_up));
+    else return fma(idxy, b_dn1, fma(idy2, a_dn, -mul_rn<T>(idxy, b_dn0))) + fma(-idxy, b1, fma(idy2, a_up, mul_rn<T>(idxy, b0)));
 }
 template <typename T>
 __device__ __forceinline__ T A_nbs_y(T idx2, T idxy, T b_lt, T b_rt, T a_lt0, T a_lt1, T a0, T a1) {
-    return fma(idxy, (a_lt1 - a_lt0) + (a0 - a1), mul_rn<T>(idx2, b_lt + b_rt));
+    if constexpr (sizeof(T) == 8) return fma(idxy, (a_lt1 - a_lt0) + (a0 - a1), mul_rn<T>(idx2, b_lt + b_rt));
+    else return fma(idxy, a_lt1, fma(idx2, b_lt, -mul_rn<T>(idxy, a_lt0))) + fma(-idxy, a1, fma(idx2, b_rt, mul_rn<T>(idxy, a0)));
 }
 // The A^(0) part of an FP32 update (k_A_sweep): dt rho k2 (dd nbs(A^(0)) - 2 d^-2 A^(0)).
 template <typename T> __device__ __forceinline__ T A_base(T dt_rho_k2, T dd, T nbs, T id2, T a0) {
