@@ -592,17 +592,18 @@ k_td_resident(const Inst* __restrict__ insts, const ResTile* __restrict__ tiles,
 // ---------------------------------------------------------------------------
 
 struct ResCfg {
-    int dtype, nt, iw, ih, smem, most;
+    int dtype, nt, iw, ih, nodes, K, smem, most;  // nodes: of a tile, with its halo
     bool waves;
     size_t scratch;  // exchange slots of a CTA, bytes
     void* fn;
 };
 template <typename T, class S, int MINB> static ResCfg res_cfg(int most, bool waves) {
-    return ResCfg{(int)sizeof(T), S::NT, S::IW, S::IH, (int)sizeof(ResSmem<T, S>), most, waves,
+    return ResCfg{(int)sizeof(T), S::NT, S::IW, S::IH, S::kBX * S::H, S::kK, (int)sizeof(ResSmem<T, S>), most, waves,
                   sizeof(C2<T>) * S::kSlots * S::SLOT, (void*)k_td_resident<T, S, MINB>};
 }
-// Shapes in the order they are tried.  A single domain takes the first in which it has
-// at most `most` tiles (0: as many as CTAs are resident at once): small tiles with many
+// Shapes in the order they are tried.  A single FP32 domain takes the first in which it
+// has at most `most` tiles (0: as many as CTAs are resident at once), FP64 the one that
+// res_sweep_us finds fastest: small tiles with many
 // sweeps per round, where the barrier and the halo's way through L2 (2.6 us a round)
 // are most of a step, then larger ones.  Batches whose tiles do not all fit run in
 // waves on a shape marked `waves`.  Measured, us per time step (22 psi sweeps), by the
@@ -610,7 +611,7 @@ template <typename T, class S, int MINB> static ResCfg res_cfg(int most, bool wa
 //   FP32, kappa = inf:  129^2 145, 16x16 19;  513^2 164, 58x26 52;  700^2 172, 60x60 72
 //   FP32, kappa = 4:    257^2 22x22 39 (16x16 42);  385^2 250, 24x24 53 (58x26 72)
 //   FP64, kappa = inf:  129^2 315, 12x12 63 (28x12 93);  257^2 321, 28x12 150 (28x28 162);
-//                       385^2 378, 62x30 325
+//                       385^2 378, 62x14 306 (62x30 323)
 //   32 films of 64^2 .. 512^2, 20 steps, FP32: 18.8 ms, in waves of 58x26 tiles 14.0
 //   (60x60: 16.0)
 static const ResCfg* res_cfgs(int* n) {
@@ -623,10 +624,20 @@ static const ResCfg* res_cfgs(int* n) {
         res_cfg<double, ResShape<16, 16, 1, 2, 1>, 2>(230, false),  // 12 x 12
         res_cfg<double, ResShape<32, 8, 2, 2, 1>, 2>(0, false),     // 28 x 12
         res_cfg<double, ResShape<32, 16, 2, 2, 1>, 1>(0, false),    // 28 x 28
+        res_cfg<double, ResShape<64, 4, 4, 1, 1>, 2>(0, false),     // 62 x 14
         res_cfg<double, ResShape<64, 8, 4, 1, 1>, 1>(0, false),     // 62 x 30
     };
     *n = (int)(sizeof(c) / sizeof(c[0]));
     return c;
+}
+
+// FP64: a sweep's time by a model, us: the FP64 pipe for the tiles of the SM that has the
+// most (20 instructions a node, 64 cycles of a scheduler each for 32 nodes) and a barrier
+// round for every K sweeps.  It follows the measured times above within 8 %: 257^2 28x12
+// 157, 28x28 157; 385^2 62x30 318.  Sizes between the steps: 470 x 230 took 62 x 30 tiles
+// on 64 SMs and 323 us per step, 62 x 14 tiles on 136 SMs take 188.
+static double res_sweep_us(const ResCfg& c, long long tiles, int sms) {
+    return (double)((tiles + sms - 1) / sms) * c.nodes * 0.0052 + 3.6 / c.K;
 }
 
 static int res_tiles_of(const ResCfg& c, const Geo& g) {
@@ -647,6 +658,7 @@ static bool res_schedule(int dtype, glgpu_handle* const* hs, int n, ResPlan* pla
     cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, dev);
     if (!coop) return false;
     int best = -1, best_cap = 0;
+    double best_us = 0.0;
     for (int c = 0; c < nc; ++c) {
         if (cs[c].dtype != dtype) continue;
         int per = 0;
@@ -663,9 +675,12 @@ static bool res_schedule(int dtype, glgpu_handle* const* hs, int n, ResPlan* pla
         }
         const bool fits = all <= (cs[c].most > 0 ? std::min(cs[c].most, cap) : cap);
         if (!fits && !(n > 1 && cs[c].waves && largest <= cap)) continue;
+        const double us = res_sweep_us(cs[c], all, sms);
+        if (best >= 0 && us >= best_us) continue;
         best = c;
         best_cap = cap;
-        break;
+        best_us = us;
+        if (dtype == 4) break;  // in order
     }
     if (best < 0) return false;
     const ResCfg& c = cs[best];
