@@ -72,7 +72,8 @@ typedef struct {
     uint32_t rand_t;        /* Langevin seed after the call */
     int32_t used_graph;     /* 1: device-side loop (CUDA graph or one resident launch), 0: host-driven loop */
     int64_t sweep_launches; /* Jacobi sweep kernel launches (psi and A); 1 where the whole call is one
-                             * launch (domains that fit on chip), else 1 per psi loop and per A sweep */
+                             * launch (domains that fit on chip), else 1 per psi loop and per A loop
+                             * (FP64: per A sweep) */
 } glgpu_td_stats;
 
 /* --- lifetime: GLSolver construction / destruction (svirl/__init__.py:30-179,

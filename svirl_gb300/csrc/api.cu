@@ -114,7 +114,7 @@ static void free_all(glgpu_handle* h) {
         if (h->dir_psi[q]) cudaFree(h->dir_psi[q]);
         if (h->dir_A[q]) cudaFree(h->dir_A[q]);
     }
-    void* ptrs[] = {h->abei, h->mt, h->eps_sp, h->U, h->code, h->dinv, h->st, h->inst, h->tiles, h->atiles, h->items, h->litems, h->loop, h->partials, h->counter,
+    void* ptrs[] = {h->abei, h->mt, h->eps_sp, h->U, h->code, h->dinv, h->st, h->inst, h->tiles, h->atiles, h->items, h->litems, h->aitems, h->loop, h->partials, h->counter,
                     h->dscal, h->out, h->vort, h->vort_n, h->flush};
     for (void* p : ptrs)
         if (p) cudaFree(p);
@@ -176,13 +176,16 @@ int glgpu_create(const glgpu_grid* grid, int32_t device, glgpu_handle** out) {
     h->strip_rows = choose_strip_rows(h->g);
     h->nitems = strip_table_len(h->g.Nx, h->g.Ny, h->strip_rows);
     ok = ok && cudaMalloc(&h->items, sizeof(Item) * (size_t)h->nitems) == cudaSuccess;
-    std::vector<Item> litems;
+    std::vector<Item> litems, aitems;
     if (h->dtype == 4) {
         const Geo* gp = &h->g;
         h->loop_rows = choose_loop_rows(&gp, 1);
-        add_loop_items(litems, h->g, 0, h->loop_rows);
+        add_loop_items(litems, h->g, 0, h->loop_rows, kWideCols);
+        add_loop_items(aitems, h->g, 0, choose_A_rows(&gp, 1), kACols);
         h->nlitems = (int)litems.size();
+        h->naitems = (int)aitems.size();
         ok = ok && cudaMalloc(&h->litems, sizeof(Item) * litems.size()) == cudaSuccess;
+        ok = ok && cudaMalloc(&h->aitems, sizeof(Item) * aitems.size()) == cudaSuccess;
     }
     ok = ok && cudaMalloc(&h->loop, sizeof(LoopState)) == cudaSuccess;
     ok = ok && cudaMalloc(&h->partials, sizeof(double) * 17 * (size_t)nblk) == cudaSuccess;
@@ -213,6 +216,8 @@ int glgpu_create(const glgpu_grid* grid, int32_t device, glgpu_handle** out) {
         e = cudaMemcpyAsync(h->atiles, atiles.data(), sizeof(ATile) * atiles.size(), cudaMemcpyHostToDevice, h->stream);
     if (e == cudaSuccess && h->litems)
         e = cudaMemcpyAsync(h->litems, litems.data(), sizeof(Item) * litems.size(), cudaMemcpyHostToDevice, h->stream);
+    if (e == cudaSuccess && h->aitems)
+        e = cudaMemcpyAsync(h->aitems, aitems.data(), sizeof(Item) * aitems.size(), cudaMemcpyHostToDevice, h->stream);
     if (e == cudaSuccess) e = cudaMemcpyAsync(h->items, items.data(), sizeof(Item) * items.size(), cudaMemcpyHostToDevice, h->stream);
     if (e == cudaSuccess) e = cudaMemcpyAsync(h->st, &st, sizeof(st), cudaMemcpyHostToDevice, h->stream);
     if (e == cudaSuccess) e = cudaMemsetAsync(h->counter, 0, sizeof(unsigned) * 4, h->stream);
@@ -388,7 +393,7 @@ int glgpu_set_psi_strip_rows(glgpu_handle* h, int32_t rows) {
     if (rows == h->strip_rows && loop_rows == h->loop_rows) return GLGPU_OK;
     const std::vector<Item> items = make_items(h->g, 0, rows);
     std::vector<Item> litems;
-    if (loop_rows) add_loop_items(litems, h->g, 0, loop_rows);
+    if (loop_rows) add_loop_items(litems, h->g, 0, loop_rows, kWideCols);
     Item *buf = nullptr, *lbuf = nullptr;
     cudaError_t e = cudaStreamSynchronize(h->stream);
     if (e == cudaSuccess) e = cudaMalloc(&buf, sizeof(Item) * items.size());
@@ -577,11 +582,16 @@ int glgpu_batch_create(glgpu_handle* const* handles, int32_t n, glgpu_batch** ou
     }
     b->ntiles = (int)tiles.size();
     b->natiles = (int)atiles.size();
-    std::vector<Item> litems;
+    std::vector<Item> litems, aitems;
     if (b->dtype == 4) {
         b->loop_rows = choose_loop_rows(geos.data(), n);
-        for (int q = 0; q < n; ++q) add_loop_items(litems, handles[q]->g, q, b->loop_rows);
+        const int arows = choose_A_rows(geos.data(), n);
+        for (int q = 0; q < n; ++q) {
+            add_loop_items(litems, handles[q]->g, q, b->loop_rows, kWideCols);
+            add_loop_items(aitems, handles[q]->g, q, arows, kACols);
+        }
         b->nlitems = (int)litems.size();
+        b->naitems = (int)aitems.size();
     }
     b->gather_h.resize(n);
     bool ok = cudaStreamCreateWithFlags(&b->stream, cudaStreamNonBlocking) == cudaSuccess;
@@ -590,6 +600,7 @@ int glgpu_batch_create(glgpu_handle* const* handles, int32_t n, glgpu_batch** ou
     ok = ok && cudaMalloc(&b->tiles, sizeof(Tile) * tiles.size()) == cudaSuccess;
     ok = ok && cudaMalloc(&b->atiles, sizeof(ATile) * atiles.size()) == cudaSuccess;
     if (b->nlitems > 0) ok = ok && cudaMalloc(&b->litems, sizeof(Item) * litems.size()) == cudaSuccess;
+    if (b->naitems > 0) ok = ok && cudaMalloc(&b->aitems, sizeof(Item) * aitems.size()) == cudaSuccess;
     ok = ok && cudaMalloc(&b->loop, sizeof(LoopState)) == cudaSuccess;
     ok = ok && cudaMallocHost(&b->gather_pin, sizeof(InstState) * (size_t)n) == cudaSuccess;
     ok = ok && cudaMallocHost(&b->loop_pin, sizeof(LoopState)) == cudaSuccess;
@@ -600,6 +611,8 @@ int glgpu_batch_create(glgpu_handle* const* handles, int32_t n, glgpu_batch** ou
         e = cudaMemcpyAsync(b->atiles, atiles.data(), sizeof(ATile) * atiles.size(), cudaMemcpyHostToDevice, b->stream);
     if (e == cudaSuccess && b->nlitems > 0)
         e = cudaMemcpyAsync(b->litems, litems.data(), sizeof(Item) * litems.size(), cudaMemcpyHostToDevice, b->stream);
+    if (e == cudaSuccess && b->naitems > 0)
+        e = cudaMemcpyAsync(b->aitems, aitems.data(), sizeof(Item) * aitems.size(), cudaMemcpyHostToDevice, b->stream);
     if (e == cudaSuccess) e = cudaStreamSynchronize(b->stream);
     if (e != cudaSuccess) {
         glgpu_batch_destroy(b);
@@ -618,7 +631,7 @@ int glgpu_batch_destroy(glgpu_batch* b) {
         if (b->td_exec[q]) cudaGraphExecDestroy(b->td_exec[q]);
     if (b->cg_exec) cudaGraphExecDestroy(b->cg_exec);
     res_free(&b->res);
-    void* ptrs[] = {b->insts, b->gather, b->tiles, b->atiles, b->litems, b->loop, b->cg_partials, b->cg_loop, b->cg_tiles, b->cg_states};
+    void* ptrs[] = {b->insts, b->gather, b->tiles, b->atiles, b->litems, b->aitems, b->loop, b->cg_partials, b->cg_loop, b->cg_tiles, b->cg_states};
     for (void* p : ptrs)
         if (p) cudaFree(p);
     void* pins[] = {b->gather_pin, b->loop_pin, b->insts_pin};

@@ -43,8 +43,8 @@ struct InstState {
     int last_sweeps_psi, last_sweeps_A, max_sweeps_psi, max_sweeps_A;
     long long total_sweeps_psi, total_sweeps_A;
     int steps;                // time steps done in the current call
-    int redo, keep;           // cooperative psi loop (tdl.cu): the sweep of the last round that the next one
-                              // repeats up to (0: none), the round keeps every sweep
+    int redo, keep;           // cooperative loops (tdl.cu): what the next round repeats the last one for (0: it
+                              // does not), which sweeps the round keeps
     int commitA;              // FP32 A loop: 1 + the buffer of A^(0) to add to the final offsets (0: none)
 };
 
@@ -79,7 +79,7 @@ struct Inst {
     const uint8_t* mt;        // material tiling (cells) or NULL
     const void* eps_sp;       // spatial linear coefficient (nodes) or NULL
     void* U;                  // link factors of the psi loop (Nab complex); during the A loop the
-                              // fixed parts of the link updates (k_A_sweep), 2 Nab reals
+                              // fixed parts of the FP64 link updates (k_A_sweep), Nab reals
     uint8_t* code;            // per-node link-weight bits of the psi loop, N bytes
     void* dinv;               // per-node reciprocal of the psi step's diagonal, N reals (FP32: bits ^ kDead, tdl.cu)
     uint8_t* cbits;           // per-node cell bits (cell_bits) for the batched CG, N bytes (NULL until CG)
@@ -233,6 +233,8 @@ struct glgpu_handle {
     int strip_rows = 0;                 // strip height of the psi sweep items
     glgpu::Item* litems = nullptr;      // FP32: items of the cooperative psi loop and their height
     int nlitems = 0, loop_rows = 0;
+    glgpu::Item* aitems = nullptr;      // FP32: items of the cooperative A loop
+    int naitems = 0;
     int psi_grid = 0;                   // CTAs of the persistent psi sweep
     glgpu::LoopState* loop = nullptr;
     int ntiles = 0;
@@ -299,6 +301,8 @@ struct glgpu_batch {
     int ntiles = 0;
     glgpu::Item* litems = nullptr;       // FP32: items of the cooperative psi loop and their height
     int nlitems = 0, loop_rows = 0;
+    glgpu::Item* aitems = nullptr;      // FP32: items of the cooperative A loop
+    int naitems = 0;
     cudaGraphExec_t td_exec[glgpu::kTDGraphs] = {};
     bool td_graph_failed = false, use_graphs = true;
     int loop_guard = 0;                  // Jacobi loop guard in sweep launches (0: kLoopGuard)
@@ -340,9 +344,12 @@ std::vector<Item> make_items(const Geo& g, int inst, int rows);
 const void* psi_loop_fn(int dtype);
 int psi_loop_threads(int dtype);
 int psi_loop_grid(int dtype, int n);
-constexpr int kWideCols = 56;  // output columns of an FP32 item of the loop
+constexpr int kWideCols = 56, kACols = 60;  // output columns of an FP32 item of the psi loop, of the A loop
 int choose_loop_rows(const Geo* const* geos, int n);
-void add_loop_items(std::vector<Item>& items, const Geo& g, int inst, int rows);
+int choose_A_rows(const Geo* const* geos, int n);
+void add_loop_items(std::vector<Item>& items, const Geo& g, int inst, int rows, int cols);
+const void* A_loop_fn();  // the cooperative A loop (FP32), its CTAs over n items
+int A_loop_grid(int n);
 // tdr.cu
 bool res_prepare(ResState* r, glgpu_handle* const* hs, int n);
 void res_free(ResState* r);

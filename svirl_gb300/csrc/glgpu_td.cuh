@@ -86,7 +86,7 @@ __device__ __forceinline__ T A_nbs_y(T idx2, T idxy, T b_lt, T b_rt, T a_lt0, T 
     if constexpr (sizeof(T) == 8) return fma(idxy, (a_lt1 - a_lt0) + (a0 - a1), mul_rn<T>(idx2, b_lt + b_rt));
     else return fma(idxy, a_lt1, fma(idx2, b_lt, -mul_rn<T>(idxy, a_lt0))) + fma(-idxy, a1, fma(idx2, b_rt, mul_rn<T>(idxy, a0)));
 }
-// The A^(0) part of an FP32 update (k_A_sweep): dt rho k2 (dd nbs(A^(0)) - 2 d^-2 A^(0)).
+// The A^(0) part of an FP32 update (k_A_loop_f32): dt rho k2 (dd nbs(A^(0)) - 2 d^-2 A^(0)).
 template <typename T> __device__ __forceinline__ T A_base(T dt_rho_k2, T dd, T nbs, T id2, T a0) {
     return mul_rn<T>(dt_rho_k2, fma(dd, nbs, -mul_rn<T>(T(2) * id2, a0)));
 }

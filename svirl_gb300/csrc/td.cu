@@ -49,7 +49,7 @@ __device__ void finish_launch(LoopState* loop, cudaGraphConditionalHandle cond, 
     if (use_cond) cudaGraphSetConditional(cond, (unsigned)cont);
 }
 
-// Called by the CTA that finishes the last tile of an instance in an A sweep.
+// Called by the CTA that finishes the last tile of an instance in an FP64 A sweep.
 template <typename T>
 __device__ void finish_instance_A(const Inst& I, LoopState* loop, int k) {
     InstState* st = I.st;
@@ -62,8 +62,6 @@ __device__ void finish_instance_A(const Inst& I, LoopState* loop, int k) {
     st->blocks_done = 0u;
     if (conv || s >= kMaxSweeps) {
         st->done = 1;
-        // FP32: the buffers hold offsets from A^(0) (k_A_sweep); k_A_commit adds A^(0)
-        if (sizeof(T) == 4) st->commitA = 1 + st->rhsA;
         st->rhsA = buf_of(st->rhsA, s);
         st->last_sweeps_A = s;
         st->total_sweeps_A += s;
@@ -562,7 +560,8 @@ k_psi_sweep_cn(const Inst* __restrict__ insts, const Tile* __restrict__ tiles, L
     }
 }
 
-// One Jacobi sweep of the A step (svirl/cuda/td.h:310-463): each thread owns the
+// One Jacobi sweep of the A step (svirl/cuda/td.h:310-463) in FP64 (FP32: k_A_loop_f32,
+// tdl.cu): each thread owns the
 // x link and the y link that start at its node.  A CTA takes a 2-D tile of
 // kATX x kATY nodes (ATile) and first stages the current iterate of the links its
 // nodes read (x links of rows j0-1 .. j0+kATY and columns i0-1 .. i0+kATX-1, y links
@@ -572,14 +571,10 @@ k_psi_sweep_cn(const Inst* __restrict__ insts, const Tile* __restrict__ tiles, L
 // atomics per tile (2,048 nodes; per 256 they made each CTA's life a chain of
 // dependent loads and atomics; that version took 0.202 ms per sweep at 2049^2,
 // 0.125 ms with four 256-node tiles per CTA).  The arithmetic of a link is unchanged.
-// resident CTAs per SM asked of the compiler for the FP32 A sweep (caps its registers)
-#ifndef GLGPU_A_MINB
-#define GLGPU_A_MINB 8
-#endif
-template <typename T>
-__global__ void __launch_bounds__(kThreads, sizeof(T) == 4 ? GLGPU_A_MINB : 1)
+__global__ void __launch_bounds__(kThreads)
 k_A_sweep(const Inst* __restrict__ insts, const ATile* __restrict__ atiles, LoopState* loop,
           cudaGraphConditionalHandle cond, int use_cond) {
+    using T = double;
     const int tid = threadIdx.x;
     __shared__ int s_skip, s_k, s_R, s_P;
     __shared__ uint32_t s_rt;
@@ -599,10 +594,7 @@ k_A_sweep(const Inst* __restrict__ insts, const ATile* __restrict__ atiles, Loop
         __syncthreads();
         if (!s_skip) {
             const int k = s_k, R = s_R;
-            // FP32: the iterates are offsets delta = A - A^(0) from the loop's right-hand
-            // side (see the delta branch below); delta^(0) = 0
-            constexpr bool kDelta = sizeof(T) == 4;
-            const T* cur = (kDelta && k == 0) ? nullptr : (const T*)I.ab[buf_of(R, k)];
+            const T* cur = (const T*)I.ab[buf_of(R, k)];
             const T* rhs = (const T*)I.ab[R];
             // with fixed vortices the supercurrent phases come from the irregular
             // potential buffer, which holds A_irr + A^(0) on its first N elements
@@ -613,7 +605,7 @@ k_A_sweep(const Inst* __restrict__ insts, const ATile* __restrict__ atiles, Loop
             const Geo g = I.g;
             // the current iterate around the tile into shared memory (0 outside the domain;
             // those entries are never read)
-            if (cur) {
+            {
                 for (int e = tid; e < (kATY + 2) * (kATX + 1); e += kThreads) {
                     const int r = e / (kATX + 1), c = e - r * (kATX + 1);
                     const int i = t.i0 - 1 + c, j = t.j0 - 1 + r;
@@ -634,14 +626,11 @@ k_A_sweep(const Inst* __restrict__ insts, const ATile* __restrict__ atiles, Loop
             // through the supercurrent argument A^(2 floor(k/2)) (the fixed-vortex potential
             // with fixed vortices, constant over the loop).  Sweeps that start a pair
             // (`fresh`) compute X and store it; the other sweeps of the pair read it back,
-            // so the sincos, the psi loads and the right-hand side's neighbour loads are paid
-            // once per two sweeps.  X (and in FP32 the A^(0) part G of X, constant over the
-            // loop) live in the link-factor buffer U, which the A loop does not read and
-            // k_link_U rebuilds before the next psi loop.  Both are stored rounded (mul_rn
-            // keeps G out of a fused multiply-add), so a pair's two sweeps use equal values.
+            // so the sincos and the psi loads are paid once per two sweeps.  X lives in the
+            // link-factor buffer U, which the A loop does not read and k_link_U rebuilds
+            // before the next psi loop.
             const bool fresh = k == 0 || (!I.vpi && (k & 1) == 0);
             T* Xc = (T*)I.U;
-            T* Gc = Xc + g.Nab;
             const T c2 = gsel<T>(I.dt, I.fdt) * gsel<T>(I.rho, I.frho) * gsel<T>(I.kappa2, I.fkappa2);
             const T den_a = T(1) + T(2) * c2 * GT(g, idy2), den_b = T(1) + T(2) * c2 * GT(g, idx2);
             const T rden_a = T(1) / den_a, rden_b = T(1) / den_b;
@@ -659,18 +648,6 @@ k_A_sweep(const Inst* __restrict__ insts, const ATile* __restrict__ atiles, Loop
                     T va = T(0), vb = T(0), ca = T(0), cbv = T(0);
                     bool has_a = false, has_b = false;
                     int na = 0, nb = 0;
-                    // FP64 iterates A; FP32 the offset delta.  FP32:
-                    // The same Jacobi iteration as the FP64 branch, written for delta: with
-                    // A^(k) = A^(0) + delta^(k) the update of a link is
-                    //   delta' = (noise + dt rho (js + rh) + dt rho k2 (dd nbs(A^(0)) - 2 d^-2 A^(0))
-                    //            + dt rho k2 dd nbs(delta^(k))) / D,
-                    // and the stop rule's |A^(k+1) - A^(k)| = |delta^(k+1) - delta^(k)|.  In FP32 the
-                    // iterates of A itself differ by whole units in the last place once |A| > 8
-                    // (the Landau gauge reaches H L), which the absolute stop rule of 1e-6
-                    // (svirl/solvers/td.py:53-57) never accepts; delta is small, so the loop
-                    // converges.  The supercurrent phase is that of A^(0) + delta^(2 floor(k/2)).
-                    // The division by a link's constant diagonal is a multiplication by
-                    // its reciprocal here; FP64 divides as the reference does.
                     if (n < g.N) {
                         const int i = ti, j = tj;
                         const int Nxa = g.Nx - 1, Na = g.Na;
@@ -678,20 +655,14 @@ k_A_sweep(const Inst* __restrict__ insts, const ATile* __restrict__ atiles, Loop
                         has_b = j < g.Ny - 1;
                         na = i + Nxa * j;
                         nb = Na + i + g.Nx * j;
-                        auto dlx = [&](int ii, int jj) -> T { return cur ? cx(ii, jj) : T(0); };
-                        auto dly = [&](int ii, int jj) -> T { return cur ? cy(ii, jj) : T(0); };
                         const T idx2 = GT(g, idx2), idy2 = GT(g, idy2), idxy = GT(g, idxy);
                         const T k2 = gsel<T>(I.kappa2, I.fkappa2);
                         const T dt_rho = gsel<T>(I.dt, I.fdt) * gsel<T>(I.rho, I.frho), dt_rho_k2 = dt_rho * k2;
                         const T dda = (j == 0 || j == g.Ny - 1) ? T(2) : T(1), ddb = (i == 0 || i == g.Nx - 1) ? T(2) : T(1);
                         T xa = T(0), xb = T(0);
                         if constexpr (kFresh) {
-                            // read the supercurrent phases before anything is stored (aliasing, see top);
-                            // FP32: A^(0) + delta^(2 floor(k/2))
-                            const T* al = (!kDelta || I.vpi || k < 2) ? nullptr : (const T*)I.ab[(R + 2) % 3];
-                            const bool base = kDelta && !I.vpi;
-                            const T ph_a = has_a ? (base ? rhs[na] + (al ? al[na] : T(0)) : abi[na]) : T(0);
-                            const T ph_b = has_b ? (base ? rhs[nb] + (al ? al[nb] : T(0)) : abi[nb]) : T(0);
+                            // read the supercurrent phases before anything is stored (aliasing, see top)
+                            const T ph_a = has_a ? abi[na] : T(0), ph_b = has_b ? abi[nb] : T(0);
                             const unsigned cb = cell_bits(g, I.mt, i, j);
                             const C2<T> psi0 = psi[n];
                             const T dx = GT(g, dx), dy = GT(g, dy);
@@ -699,10 +670,8 @@ k_A_sweep(const Inst* __restrict__ insts, const ATile* __restrict__ atiles, Loop
                             const T H = gsel<T>(I.H, I.fH);
                             const T lc = gsel<T>(I.lang_A, I.flang_A);
                             const bool lang = I.lang_A_on != 0;
-                            auto rx = [&](int ii, int jj) -> T { return ii >= 0 && ii < Nxa && jj >= 0 && jj < g.Ny ? rhs[ii + Nxa * jj] : T(0); };
-                            auto ry = [&](int ii, int jj) -> T { return ii >= 0 && ii < g.Nx && jj >= 0 && jj < g.Ny - 1 ? rhs[Na + ii + g.Nx * jj] : T(0); };
                             if (has_a) {
-                                T first = kDelta ? T(0) : rhs[na];
+                                T first = rhs[na];
                                 if (lang) first = add_noise<T>(first, lc, rand_1<T>((uint32_t)na, s_rt));
                                 T rh = T(0);
                                 if (j == 0) rh = T(2) * k2 * H * idy;
@@ -710,22 +679,10 @@ k_A_sweep(const Inst* __restrict__ insts, const ATile* __restrict__ atiles, Loop
                                 T jl = T(0);
                                 if (GL_PM(cb) || GL_PP(cb)) jl = mul_rn<T>(idx, js_of<T>(psi0, dx * ph_a, psi[n + 1]));
                                 xa = A_fixed<T>(first, dt_rho, jl, rh);
-                                if constexpr (kDelta) {
-                                    T ga;
-                                    if (k == 0) {
-                                        ga = A_base<T>(dt_rho_k2, dda,
-                                                       A_nbs_x<T>(idy2, idxy, rx(i, j - 1), rx(i, j + 1), ry(i, j - 1), ry(i + 1, j - 1),
-                                                                  ry(i, j), ry(i + 1, j)), idy2, rhs[na]);
-                                        Gc[na] = ga;
-                                    } else {
-                                        ga = Gc[na];
-                                    }
-                                    xa += ga;
-                                }
                                 Xc[na] = xa;
                             }
                             if (has_b) {
-                                T first = kDelta ? T(0) : rhs[nb];
+                                T first = rhs[nb];
                                 if (lang) first = add_noise<T>(first, lc, rand_2<T>((uint32_t)nb, s_rt));
                                 T rh = T(0);
                                 if (i == 0) rh = -T(2) * k2 * H * idx;
@@ -733,18 +690,6 @@ k_A_sweep(const Inst* __restrict__ insts, const ATile* __restrict__ atiles, Loop
                                 T jl = T(0);
                                 if (GL_MP(cb) || GL_PP(cb)) jl = mul_rn<T>(idy, js_of<T>(psi0, dy * ph_b, psi[n + g.Nx]));
                                 xb = A_fixed<T>(first, dt_rho, jl, rh);
-                                if constexpr (kDelta) {
-                                    T gb;
-                                    if (k == 0) {
-                                        gb = A_base<T>(dt_rho_k2, ddb,
-                                                       A_nbs_y<T>(idx2, idxy, ry(i - 1, j), ry(i + 1, j), rx(i - 1, j), rx(i - 1, j + 1),
-                                                                  rx(i, j), rx(i, j + 1)), idx2, rhs[nb]);
-                                        Gc[nb] = gb;
-                                    } else {
-                                        gb = Gc[nb];
-                                    }
-                                    xb += gb;
-                                }
                                 Xc[nb] = xb;
                             }
                         } else {
@@ -752,16 +697,16 @@ k_A_sweep(const Inst* __restrict__ insts, const ATile* __restrict__ atiles, Loop
                             if (has_b) xb = Xc[nb];
                         }
                         if (has_a) {
-                            const T nd = A_nbs_x<T>(idy2, idxy, dlx(i, j - 1), dlx(i, j + 1), dly(i, j - 1), dly(i + 1, j - 1),
-                                                    dly(i, j), dly(i + 1, j));
+                            const T nd = A_nbs_x<T>(idy2, idxy, cx(i, j - 1), cx(i, j + 1), cy(i, j - 1), cy(i + 1, j - 1),
+                                                    cy(i, j), cy(i + 1, j));
                             va = div_by(fma(dt_rho_k2 * dda, nd, xa), den_a, rden_a);
-                            ca = dlx(i, j);
+                            ca = cx(i, j);
                         }
                         if (has_b) {
-                            const T nd = A_nbs_y<T>(idx2, idxy, dly(i - 1, j), dly(i + 1, j), dlx(i - 1, j), dlx(i - 1, j + 1),
-                                                    dlx(i, j), dlx(i, j + 1));
+                            const T nd = A_nbs_y<T>(idx2, idxy, cy(i - 1, j), cy(i + 1, j), cx(i - 1, j), cx(i - 1, j + 1),
+                                                    cx(i, j), cx(i, j + 1));
                             vb = div_by(fma(dt_rho_k2 * ddb, nd, xb), den_b, rden_b);
-                            cbv = dly(i, j);
+                            cbv = cy(i, j);
                         }
                     }
                     if (n < g.N) {
@@ -971,10 +916,8 @@ __global__ void k_loop_begin(const Inst* __restrict__ insts, int ninst, LoopStat
         st->res = 0ull;
         for (int l = 0; l < 4; ++l) st->resp[l] = 0ull;
         st->nanlv = 0;
-        if (which == 0) {
-            st->redo = 0;
-            st->keep = st->last_sweeps_psi < kFuse;
-        }
+        st->redo = 0;
+        st->keep = which == 0 ? st->last_sweeps_psi < kFuse : (st->last_sweeps_A == 1 ? 1 : 2);
         active += part ? 1 : 0;
     }
     for (int o = 16; o > 0; o >>= 1) active += __shfl_down_sync(0xffffffffu, active, o);
@@ -999,7 +942,7 @@ __global__ void k_loop_end(const Inst* __restrict__ insts, int ninst, int which)
 }
 
 // After an FP32 A loop: the state buffer holds the offsets delta = A - A^(0) of
-// the loop's last sweep (k_A_sweep); A = A^(0) + delta, in place.  A loop that
+// the loop's last sweep (k_A_loop_f32, tdl.cu); A = A^(0) + delta, in place.  A loop that
 // stopped on the guard leaves no commit pending and the state at A^(0).
 __global__ void __launch_bounds__(kThreads) k_A_commit(const Inst* __restrict__ insts, const Tile* __restrict__ tiles) {
     const Tile t = tiles[blockIdx.x];
@@ -1122,6 +1065,8 @@ struct TDLaunch {
     const ResState* res;  // the resident loop (tdr.cu), or null: a launch per sweep
     const void* work;  // tiles or items of the cooperative psi loop (tdl.cu) and its CTAs; 0 CTAs: a launch per sweep or kFuse sweeps
     int nwork, loop_grid;
+    const Item* aitems;  // FP32: items of the cooperative A loop and its CTAs; FP64: a launch per sweep
+    int naitems, A_grid;
 };
 
 static void* fv_psi_pre_fn(int dt) { return dt == 8 ? (void*)k_fv_psi_pre<double> : (void*)k_fv_psi_pre<float>; }
@@ -1145,9 +1090,6 @@ static cudaError_t launch_bulk_sweep(int rows, int grid, cudaStream_t s, const I
     int zero = 0;
     void* a[] = {&insts, &items, &nitems, &loop, &none, &zero};
     return cudaLaunchKernel(bulk_fn(rows), dim3(grid), dim3(kBulkThreads), a, 0, s);
-}
-static void* A_sweep_fn(int dtype) {
-    return dtype == 8 ? (void*)k_A_sweep<double> : (void*)k_A_sweep<float>;
 }
 static void* cn_fn(int dtype) {
     return dtype == 8 ? (void*)k_psi_sweep_cn<double> : (void*)k_psi_sweep_cn<float>;
@@ -1198,6 +1140,13 @@ static cudaError_t launch_psi_loop(int dtype, int grid, cudaStream_t s, const In
     return cudaLaunchCooperativeKernel(psi_loop_fn(dtype), dim3(grid), dim3(psi_loop_threads(dtype)), a, 0, s);
 }
 
+static cudaError_t launch_A_loop(int grid, cudaStream_t s, const Inst* insts, int ninst, const Item* items, int nitems,
+                                 LoopState* loop) {
+    int zero = 0;
+    void* a[] = {&insts, &ninst, &items, &nitems, &loop, &zero};
+    return cudaLaunchCooperativeKernel(A_loop_fn(), dim3(grid), dim3(psi_loop_threads(4)), a, 0, s);
+}
+
 // Build the whole TD run of all instances as one graph:
 //   [fixed vortices: A += A_irr, psi-only mode] -> [tables, all instances] -> WHILE(step < Nt) {
 //       [A += A_irr] -> [tables, finite-kappa / fixed-vortex instances]
@@ -1234,7 +1183,7 @@ static cudaError_t build_td_graph(const TDLaunch& L, int eqn, cudaGraphExec_t* e
         void* a[] = {&insts, &tiles};
         GCHK(chain(top, fv_psi_pre_fn(L.dtype), gt, bt, a));
     }
-    if (do_psi) {
+    if (do_psi || L.A_grid > 0) {  // (the FP32 A loop reads the link-weight codes)
         void* a[] = {&insts, &tiles, &ntiles, &zero};
         GCHK(chain(top, link_fn(L.dtype), dim3(call_grid(ntiles)), bt, a));
     }
@@ -1285,22 +1234,29 @@ static cudaError_t build_td_graph(const TDLaunch& L, int eqn, cudaGraphExec_t* e
         }
     }
     if (do_A) {
-        GCHK(cudaGraphConditionalHandleCreate(&hA, obody, 1, cudaGraphCondAssignDefault));
+        int cond = L.A_grid == 0 ? 1 : 0;
+        if (cond) GCHK(cudaGraphConditionalHandleCreate(&hA, obody, 1, cudaGraphCondAssignDefault));
         if (L.any_fv) {
             void* a[] = {&insts, &tiles, &zero};
             GCHK(chain(obody, fv_A_fn(L.dtype), gt, bt, a));
         }
         {
-            void* a[] = {&insts, &ninst, &loop, &hA, &one, &one};
+            void* a[] = {&insts, &ninst, &loop, &hA, &cond, &one};
             GCHK(chain(obody, (void*)k_loop_begin, g1, b1, a));
         }
-        GCHK(add_while(obody, &nd, &prev, 1, hA, &abody));
-        prev = nd;
-        {
+        if (L.A_grid > 0) {
+            const Item* aitems = L.aitems;
+            int naitems = L.naitems;
+            void* a[] = {&insts, &ninst, &aitems, &naitems, &loop, &zero};
+            GCHK(chain(obody, (void*)A_loop_fn(), dim3(L.A_grid), dim3(psi_loop_threads(4)), a));
+            GCHK(set_cooperative(prev));
+        } else {
+            GCHK(add_while(obody, &nd, &prev, 1, hA, &abody));
+            prev = nd;
             cudaGraphNode_t sw;
             ATile const* atiles = L.atiles;
             void* a[] = {&insts, &atiles, &loop, &hA, &one};
-            GCHK(add_kernel(abody, &sw, nullptr, 0, A_sweep_fn(L.dtype), dim3(L.natiles), bt, a));
+            GCHK(add_kernel(abody, &sw, nullptr, 0, (void*)k_A_sweep, dim3(L.natiles), bt, a));
         }
         if (L.dtype == 4) {
             void* a[] = {&insts, &tiles};
@@ -1361,7 +1317,7 @@ static cudaError_t run_host_loop(const TDLaunch& L, int eqn, int Nt, cudaStream_
         else k_fv_A<float><<<L.ntiles, kThreads, 0, s>>>(L.insts, L.tiles, post);
     };
     if (do_psi && eqn == 1 && L.any_fv) fv_psi(false);
-    if (do_psi) launch_link_U(L, 0, s);
+    if (do_psi || L.A_grid > 0) launch_link_U(L, 0, s);
     for (int step = 0; step < Nt; ++step) {
         for (int part = 0; part < 2; ++part) {
             if (part == 0 && !do_psi) continue;
@@ -1374,7 +1330,11 @@ static cudaError_t run_host_loop(const TDLaunch& L, int eqn, int Nt, cudaStream_
                 const cudaError_t e = launch_psi_loop(L.dtype, L.loop_grid, s, L.insts, L.ninst, L.work, L.nwork, L.loop, 0);
                 if (e != cudaSuccess) return e;
             }
-            for (; part == 1 || L.loop_grid == 0;) {
+            if (part == 1 && L.A_grid > 0) {
+                const cudaError_t e = launch_A_loop(L.A_grid, s, L.insts, L.ninst, L.aitems, L.naitems, L.loop);
+                if (e != cudaSuccess) return e;
+            }
+            for (; (part == 0 ? L.loop_grid : L.A_grid) == 0;) {
                 for (int c = 0; c < chunk; ++c) {
                     if (part == 0 && L.psi_cn) {
                         const int aw = L.psi_cn == 2 ? 1 : 0;
@@ -1385,8 +1345,7 @@ static cudaError_t run_host_loop(const TDLaunch& L, int eqn, int Nt, cudaStream_
                     } else if (part == 0) {
                         launch_bulk_sweep(L.strip_rows, L.psi_grid, s, L.insts, L.items, L.nitems, L.loop);
                     } else {
-                        if (L.dtype == 8) k_A_sweep<double><<<L.natiles, kThreads, 0, s>>>(L.insts, L.atiles, L.loop, none, 0);
-                        else k_A_sweep<float><<<L.natiles, kThreads, 0, s>>>(L.insts, L.atiles, L.loop, none, 0);
+                        k_A_sweep<<<L.natiles, kThreads, 0, s>>>(L.insts, L.atiles, L.loop, none, 0);
                     }
                 }
                 cudaError_t e = cudaMemcpyAsync(&cont, &L.loop->cont, sizeof(int), cudaMemcpyDeviceToHost, s);
@@ -1412,7 +1371,7 @@ static cudaError_t run_host_loop(const TDLaunch& L, int eqn, int Nt, cudaStream_
 // distinct from the right-hand side, as in a typical sweep), loop not done, and
 // the right-hand sides at buffer 0 as at rest (a timed launch that meets the stop
 // rule moves them, and the next launch would then write into buffer 0).
-__global__ void k_bench_prep(const Inst* __restrict__ insts, int ninst, LoopState* loop, int k) {
+__global__ void k_bench_prep(const Inst* __restrict__ insts, int ninst, LoopState* loop, int k, int keep) {
     for (int q = threadIdx.x; q < ninst; q += blockDim.x) {
         InstState* st = insts[q].st;
         st->rhs = 0;
@@ -1423,7 +1382,8 @@ __global__ void k_bench_prep(const Inst* __restrict__ insts, int ninst, LoopStat
         st->res = 0ull;
         for (int l = 0; l < 4; ++l) st->resp[l] = 0ull;
         st->nanlv = 0;
-        st->redo = st->keep = 0;
+        st->redo = 0;
+        st->keep = keep;
     }
     if (threadIdx.x == 0) {
         loop->active = ninst;
@@ -1480,12 +1440,13 @@ int time_sweeps(glgpu_handle* h, int which, int nrep, double* avg_ms) {
     else k_link_U<float><<<call_grid(h->ntiles), kThreads, 0, h->stream>>>(h->inst, h->tiles, h->ntiles, 0);
     double total = 0.0;
     // A sweeps come in pairs (sweep 0 computes the links' fixed parts, sweep 1 reuses
-    // them), so an A repetition times both and the average is over sweeps
-    const int per_rep = which == 0 ? 1 : 2;
+    // them), so an A repetition times both (FP32: one round of the loop) and the average
+    // is over sweeps
+    const int per_rep = which == 1 && h->dtype == 8 ? 2 : 1;
     for (int r = 0; r < nrep && e == cudaSuccess; ++r) {
         cudaMemsetAsync(h->flush, r & 0xff, flush_bytes, h->stream);
         for (int q = 0; q < per_rep && e == cudaSuccess; ++q) {
-            k_bench_prep<<<1, 32, 0, h->stream>>>(h->inst, 1, h->loop, which == 0 ? 1 : q);
+            k_bench_prep<<<1, 32, 0, h->stream>>>(h->inst, 1, h->loop, which == 0 ? 1 : q, which == 0 ? 0 : 2);
             cudaEventRecord(e0, h->stream);
             if (which == 0 && !bulk_selected(h)) {
                 const void* work = h->dtype == 8 ? (const void*)h->tiles : h->litems;
@@ -1496,8 +1457,8 @@ int time_sweeps(glgpu_handle* h, int which, int nrep, double* avg_ms) {
                 launch_bulk_sweep(h->strip_rows, h->psi_grid, h->stream, h->inst, h->items,
                                  h->nitems, h->loop);
             } else {
-                if (h->dtype == 8) k_A_sweep<double><<<h->natiles, kThreads, 0, h->stream>>>(h->inst, h->atiles, h->loop, none, 0);
-                else k_A_sweep<float><<<h->natiles, kThreads, 0, h->stream>>>(h->inst, h->atiles, h->loop, none, 0);
+                if (h->dtype == 8) k_A_sweep<<<h->natiles, kThreads, 0, h->stream>>>(h->inst, h->atiles, h->loop, none, 0);
+                else e = launch_A_loop(A_loop_grid(h->naitems), h->stream, h->inst, 1, h->aitems, h->naitems, h->loop);
             }
             cudaEventRecord(e1, h->stream);
             if (e == cudaSuccess) e = cudaEventSynchronize(e1);
@@ -1516,7 +1477,7 @@ int time_sweeps(glgpu_handle* h, int which, int nrep, double* avg_ms) {
     if (e == cudaSuccess) e = cudaStreamSynchronize(h->stream);
     if (e != cudaSuccess) return cuda_check(h, e, "time_sweeps");
     if (hl.err & kErrCopyWait) return set_error(h, GLGPU_E_TIMEOUT, "time_sweeps: psi sweep: a bulk-copy wait ran out");
-    *avg_ms = total / (nrep * per_rep);
+    *avg_ms = total / (nrep * (which == 0 ? 1 : 2));
     return GLGPU_OK;
 }
 
@@ -1679,6 +1640,9 @@ int td_run(glgpu_handle* h, double dt, int Nt, int eqn, glgpu_td_stats* stats, d
     L.any_solveA = h->inst_h.solveA != 0;
     L.any_fv = h->vpi != nullptr || h->lock_n > 0;
     L.res = resident ? &h->res : nullptr;
+    L.aitems = h->aitems;
+    L.naitems = h->naitems;
+    L.A_grid = h->dtype == 4 ? A_loop_grid(h->naitems) : 0;
     L.work = h->dtype == 8 ? (const void*)h->tiles : h->litems;
     L.nwork = h->dtype == 8 ? h->ntiles : h->nlitems;
     L.loop_grid = resident || h->psi_scheme != 0 || bulk_selected(h) ? 0 : psi_loop_grid(h->dtype, L.nwork);
@@ -1728,6 +1692,9 @@ int batch_td(glgpu_batch* b, double dt, int Nt, int eqn, glgpu_td_stats* stats, 
     L.any_solveA = any_solveA;
     L.any_fv = any_fv;
     L.res = resident ? &b->res : nullptr;
+    L.aitems = b->aitems;
+    L.naitems = b->naitems;
+    L.A_grid = b->dtype == 4 ? A_loop_grid(b->naitems) : 0;
     L.work = b->dtype == 8 ? (const void*)b->tiles : b->litems;
     L.nwork = b->dtype == 8 ? b->ntiles : b->nlitems;
     L.loop_grid = resident ? 0 : psi_loop_grid(b->dtype, L.nwork);

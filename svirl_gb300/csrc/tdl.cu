@@ -23,15 +23,14 @@ __device__ __forceinline__ int ring_of(int R, int round) { return round == 0 ? R
 // Buffer of sweep l < K of a round, where it is kept (FP32).
 __device__ __forceinline__ int mid_of(int R, int l) { return (R + 2 + l) % kPsiBufs; }
 
-// End of a round of K sweeps: the CTA that arrives last closes it for every instance
-// whose loop still runs, decides whether one is left, and publishes round and decision in
-// one word.  What the CTAs wrote in the round is visible after it.  false: leave the loop
-// (finished, or a wait ran out).  The word of a round stays until this CTA has arrived at
-// the next one, so nobody misses it.  An instance whose loop stops after a sweep that the
-// round did not keep repeats it up to there in the next round (InstState::redo).
-template <int K>
-__device__ __forceinline__ bool end_round(const Inst* insts, int ninst, LoopState* loop, int first, int round, int& s_word) {
-    const int seq = round - first + 1;  // rounds of this launch
+// End of a round: the CTA that arrives last closes it for every instance whose loop still
+// runs (close(instance, state): bit 0 the loop goes on, bit 1 it has reached the guard),
+// decides whether one is left, and publishes round and decision in one word.  What the CTAs
+// wrote in the round is visible after it.  false: leave the loop (finished, or a wait ran
+// out).  The word of a round stays until this CTA has arrived at the next one, so nobody
+// misses it.
+template <typename Close>
+__device__ __forceinline__ bool end_round(const Inst* insts, int ninst, LoopState* loop, int seq, int& s_word, const Close& close) {
     __syncthreads();
     if (threadIdx.x == 0) {
         __threadfence();
@@ -39,53 +38,16 @@ __device__ __forceinline__ bool end_round(const Inst* insts, int ninst, LoopStat
     }
     __syncthreads();
     if (s_word < 0) {
-        int left = 0, cut = 0;
-        const int guard = kFuse * min(loop->guard, kLoopGuard);  // in launches of kFuse sweeps
+        int flags = 0;
         __threadfence();
         for (int q = threadIdx.x; q < ninst; q += blockDim.x) {
-            const Inst& I = insts[q];
-            InstState* st = I.st;
+            InstState* st = insts[q].st;
             if (*(volatile const int*)&st->done) continue;
-            const int R = *(volatile const int*)&st->rhs, redo = *(volatile const int*)&st->redo;
-            const int k = K * (round - (redo ? 1 : 0)), kg = k - K * first;
-            unsigned long long res[K];
-#pragma unroll
-            for (int l = 0; l < K; ++l) res[l] = atomicExch(&st->resp[l], 0ull);
-            const int nl = atomicExch(&st->nanlv, 0);
-            int stop = redo;
-            if (!redo) {
-#pragma unroll
-                for (int l = K; l >= 1; --l)
-                    if ((res[l - 1] <= I.thr_psi || k + l >= kMaxSweeps) && kg + l <= guard) stop = l;
-                if (nl & ((1 << (stop ? stop : K)) - 1)) st->nan_seen = 1;
-                if (!stop && kg + K >= guard) cut = 1;
-                const int kept = *(volatile const int*)&st->keep;
-                if (stop && stop < K && !kept) {
-                    st->redo = stop;
-                    left = 1;
-                    __threadfence();
-                    continue;
-                }
-            }
-            if (stop) {
-                const int s = k + stop;
-                st->sweep = s;
-                st->done = 1;
-                st->redo = 0;
-                st->rhs = stop == K ? ring_of(R, k / K + 1) : mid_of(R, stop);
-                st->last_sweeps_psi = s;
-                st->total_sweeps_psi += s;
-                if (s > st->max_sweeps_psi) st->max_sweeps_psi = s;
-            } else {
-                // the next round keeps every sweep if the step before stopped within it
-                const int ls = *(volatile const int*)&st->last_sweeps_psi;
-                st->keep = K > 1 && (ls == 0 || (ls > k + K && ls < k + 2 * K));
-                left = 1;
-            }
+            flags |= close(insts[q], st);
             __threadfence();
         }
-        left = __syncthreads_or(left);
-        cut = __syncthreads_or(cut);
+        int left = __syncthreads_or(flags & 1);
+        const int cut = __syncthreads_or(flags & 2);
         if (threadIdx.x == 0) {
             if (seq == 1) loop->total_launches += 1;
             if (!left) loop->active = 0;
@@ -93,6 +55,7 @@ __device__ __forceinline__ bool end_round(const Inst* insts, int ninst, LoopStat
                 left = 0;
                 loop->err |= kErrLoopGuard;
             }
+            left = left ? 1 : 0;
             loop->cont = left;
             s_word = 2 * seq + left;
             __threadfence();
@@ -115,6 +78,49 @@ __device__ __forceinline__ bool end_round(const Inst* insts, int ninst, LoopStat
     __syncthreads();
     return s_word & 1;
 }
+
+// The residual words of an instance's round, read and cleared; the first of its sweeps k + 1
+// .. k + K that meets the stop rule or the sweep cap (0: none), not past `guard` sweeps.
+template <int K>
+__device__ __forceinline__ int stop_level(InstState* st, int k, unsigned long long thr, int guard) {
+    unsigned long long res[K];
+#pragma unroll
+    for (int l = 0; l < K; ++l) res[l] = atomicExch(&st->resp[l], 0ull);
+    const int nl = atomicExch(&st->nanlv, 0);
+    int stop = 0;
+#pragma unroll
+    for (int l = K; l >= 1; --l)
+        if ((res[l - 1] <= thr || k + l >= kMaxSweeps) && k + l <= guard) stop = l;
+    if (nl & ((1 << (stop ? stop : K)) - 1)) st->nan_seen = 1;
+    return stop;
+}
+
+// Closes a psi round of K sweeps.  An instance whose loop stops after a sweep that the round
+// did not keep repeats it up to there in the next round (InstState::redo).
+template <int K> struct ClosePsi {
+    int round, first, guard;  // guard in sweeps
+    __device__ __forceinline__ int operator()(const Inst& I, InstState* st) const {
+        const int R = *(volatile const int*)&st->rhs, redo = *(volatile const int*)&st->redo;
+        const int k = K * (round - (redo ? 1 : 0)), base = K * first;
+        const int stop = redo ? redo : stop_level<K>(st, k, I.thr_psi, guard + base);
+        if (!stop || (!redo && stop < K && !*(volatile const int*)&st->keep)) {
+            st->redo = stop;
+            // the next round keeps every sweep if the step before stopped within it
+            const int ls = *(volatile const int*)&st->last_sweeps_psi;
+            st->keep = !stop && K > 1 && (ls == 0 || (ls > k + K && ls < k + 2 * K));
+            return 1 | (!stop && k + K >= guard + base ? 2 : 0);
+        }
+        const int s = k + stop;
+        st->sweep = s;
+        st->done = 1;
+        st->redo = 0;
+        st->rhs = stop == K ? ring_of(R, k / K + 1) : mid_of(R, stop);
+        st->last_sweeps_psi = s;
+        st->total_sweeps_psi += s;
+        if (s > st->max_sweeps_psi) st->max_sweeps_psi = s;
+        return 0;
+    }
+};
 
 // FP64: one sweep per round, a node per thread.  The FP64 pipe bounds it (20 FP64
 // instructions a node; a warp instruction takes 64 cycles of its scheduler), so nothing
@@ -237,7 +243,8 @@ k_psi_loop_f64(const Inst* __restrict__ insts, int ninst, const Tile* __restrict
             }
         }
         if (!fresh && !done) flush_f64(insts[cur_inst], rmax, rnan, s_max);
-        if (!end_round<1>(insts, ninst, loop, first, round, s_word)) break;
+        if (!end_round(insts, ninst, loop, round - first + 1, s_word, ClosePsi<1>{round, first, kFuse * min(loop->guard, kLoopGuard)}))
+            break;
     }
 }
 
@@ -272,9 +279,10 @@ struct WideRow {
 };
 
 // A warp's residual maxima of a round into the instance's words.
+template <int K = kFuse>
 __device__ __forceinline__ void strip_flush(const Inst& I, const float (&wmax)[kFuse], const float (&wnan)[kFuse]) {
 #pragma unroll
-    for (int l = 0; l < kFuse; ++l) {
+    for (int l = 0; l < K; ++l) {
         const unsigned m = __reduce_max_sync(0xffffffffu, __float_as_uint(wmax[l]));
         const bool nn = __any_sync(0xffffffffu, isnan(wnan[l]));
         if ((threadIdx.x & 31) == 0) {
@@ -490,7 +498,284 @@ k_psi_loop_f32(const Inst* __restrict__ insts, int ninst, const Item* __restrict
                 for (int l = 0; l < K; ++l) wmax[l] = wnan[l] = 0.f;
         }
         if (cur_inst >= 0 && !done) strip_flush(insts[cur_inst], wmax, wnan);
-        if (!end_round<K>(insts, ninst, loop, first, round, s_word)) break;
+        if (!end_round(insts, ninst, loop, round - first + 1, s_word, ClosePsi<K>{round, first, kFuse * min(loop->guard, kLoopGuard)}))
+            break;
+    }
+}
+
+// The Jacobi loop of the A step (svirl/cuda/td.h:310-463) in one cooperative launch, FP32,
+// two sweeps per round.  It iterates the offset delta = A - A^(0) from the loop's
+// right-hand side: with A^(k) = A^(0) + delta^(k) the update of a link is
+//   delta' = (noise + dt rho (js + rh) + dt rho k2 (dd nbs(A^(0)) - 2 d^-2 A^(0))
+//            + dt rho k2 dd nbs(delta^(k))) / D,
+// and the stop rule's |A^(k+1) - A^(k)| = |delta^(k+1) - delta^(k)|.  In FP32 the iterates of
+// A itself differ by whole units in the last place once |A| > 8 (the Landau gauge reaches
+// H L), which the absolute stop rule of 1e-6 (svirl/solvers/td.py:53-57) never accepts;
+// delta is small, so the loop converges.  The division by a link's constant diagonal is a
+// multiplication by its reciprocal.
+// The fixed part X of an update takes the supercurrent phase from delta^(2 floor(k/2)) (the
+// reference's aliasing, td.cu), so a round's two sweeps share it and it stays in
+// registers: one pass over A^(0), delta and psi.
+// Strips as in k_psi_loop_f32: two columns a lane, 64 columns x0 - 2 .. x0 + 61 of which 60
+// are the strip's own, rows through a ring of asynchronous copies.  At a step the row y is
+// new: X and the first sweep of row y - 1, the second sweep of row y - 2.
+// A round stores the sweep after which the loop stopped a step ago, if that is its first,
+// else its second; a loop that stops or goes on elsewhere repeats the round (redo: 1 or 2
+// to stop after that sweep, 3 to go on).
+// Two sweeps at 2049^2, kappa 4, from a flushed L2: 87 us; as a launch per sweep, with X
+// stored and read back and a thread per node that loads its twelve neighbours (531
+// instructions a node in the first of a pair), 158.
+struct AStage {
+    float2 a0[32], b0[32], da[32], db[32];
+    float4 psi[32];
+};
+// A row of link values of a lane's two columns, with the neighbours' left and right of them.
+struct ARow {
+    float a[2], b[2], aL, bL, bR;
+};
+__device__ __forceinline__ void row_sides(ARow& r) {
+    r.aL = __shfl_up_sync(0xffffffffu, r.a[1], 1);
+    r.bL = __shfl_up_sync(0xffffffffu, r.b[1], 1);
+    r.bR = __shfl_down_sync(0xffffffffu, r.b[0], 1);
+}
+__device__ __forceinline__ float row_nbs_x(float idy2, float idxy, const ARow& dn, const ARow& cu, const ARow& up, int c) {
+    return A_nbs_x<float>(idy2, idxy, dn.a[c], up.a[c], dn.b[c], c == 0 ? dn.b[1] : dn.bR, cu.b[c], c == 0 ? cu.b[1] : cu.bR);
+}
+__device__ __forceinline__ float row_nbs_y(float idx2, float idxy, const ARow& cu, const ARow& up, int c) {
+    return A_nbs_y<float>(idx2, idxy, c == 0 ? cu.bL : cu.b[0], c == 0 ? cu.b[1] : cu.bR, c == 0 ? cu.aL : cu.a[0],
+                          c == 0 ? up.aL : up.a[0], cu.a[c], up.a[c]);
+}
+
+// Buffer of delta^(k), k even and positive, of a loop with A^(0) in buffer R.
+__device__ __forceinline__ int delta_of(int R, int k) { return (R + 1 + ((k / 2 - 1) & 1)) % 3; }
+
+struct CloseA {
+    int guard;  // in sweeps
+    __device__ __forceinline__ int operator()(const Inst& I, InstState* st) const {
+        const int R = *(volatile const int*)&st->rhsA, redo = *(volatile const int*)&st->redo, k = *(volatile const int*)&st->sweep;
+        const int stored = *(volatile const int*)&st->keep;  // the sweep that the round stored
+        int stop = redo == 3 ? 0 : redo, go = redo == 3;
+        if (!redo) {
+            stop = stop_level<2>(st, k, I.thr_A, guard);
+            if (!stop && k + 2 >= guard) return 3;
+            if (stop != stored && (stop || stored != 2)) {
+                st->redo = stop ? stop : 3;
+                return 1;
+            }
+            go = !stop;
+        }
+        st->redo = 0;
+        if (go) {
+            st->sweep = k + 2;
+            st->keep = *(volatile const int*)&st->last_sweeps_A == k + 3 ? 1 : 2;
+            return 1;
+        }
+        const int s = k + stop;
+        st->sweep = s;
+        st->done = 1;
+        st->commitA = 1 + R;  // the buffers hold offsets from A^(0); k_A_commit adds it
+        st->rhsA = delta_of(R, k + 2);
+        st->last_sweeps_A = s;
+        st->total_sweeps_A += s;
+        if (s > st->max_sweeps_A) st->max_sweeps_A = s;
+        return 0;
+    }
+};
+
+constexpr int kAMinB = 6;  // CTAs per SM that the registers must allow (7: spills, 56 us a sweep against 43)
+__global__ void __launch_bounds__(kPsiThreads, kAMinB)
+k_A_loop_f32(const Inst* __restrict__ insts, int ninst, const Item* __restrict__ items, int nitems, LoopState* loop, int) {
+    constexpr int NS = kWideStages;
+    __shared__ AStage s_st[kPsiWarps][NS];
+    __shared__ int s_word;
+    const int lane = threadIdx.x & 31;
+    AStage* const st4 = s_st[threadIdx.x >> 5];
+    const int gw = blockIdx.x * kPsiWarps + (threadIdx.x >> 5), nw = gridDim.x * kPsiWarps;
+    for (int seq = 1;; ++seq) {
+        int cur_inst = -1, done = 1, k = 0, R = 0, keep_at = 2;
+        bool quiet = false;  // a repeated round: its residuals are known
+        uint32_t rt = 0;
+        float wmax[kFuse], wnan[kFuse];
+        for (int it = gw; it < nitems; it += nw) {
+            const Item w = items[(seq & 1) ? it : nitems - 1 - it];
+            if (w.inst != cur_inst) {
+                if (cur_inst >= 0 && !done && !quiet) strip_flush<2>(insts[cur_inst], wmax, wnan);
+                cur_inst = w.inst;
+                // an instance's loop state changes only at the end of a round
+                const InstState* st = insts[cur_inst].st;
+                done = *(volatile const int*)&st->done;
+                k = *(volatile const int*)&st->sweep;
+                R = *(volatile const int*)&st->rhsA;
+                const int redo = *(volatile const int*)&st->redo;
+                quiet = redo != 0;
+                keep_at = redo ? (redo == 1 ? 1 : 2) : *(volatile const int*)&st->keep;
+                rt = *(volatile const uint32_t*)&st->rand_t;
+                wmax[0] = wmax[1] = wnan[0] = wnan[1] = 0.f;
+            }
+            if (done) continue;
+            const Inst& I = insts[cur_inst];
+            const int Nx = I.g.Nx, Ny = I.g.Ny, Nxa = Nx - 1, Na = I.g.Na;
+            const float* __restrict__ base = (const float*)I.ab[R];
+            const float* cur = (const float*)I.ab[k == 0 ? R : delta_of(R, k)];  // k = 0: not read
+            const float* vpi = (const float*)I.vpi;
+            float* out = (float*)I.ab[delta_of(R, k + 2)];
+            const float2* __restrict__ psi = (const float2*)I.psi[*(volatile const int*)&I.st->rhs];
+            const float k2 = I.fkappa2, dt_rho = I.fdt * I.frho, dt_rho_k2 = dt_rho * k2, H = I.fH;
+            const float idx = I.g.fidx, idy = I.g.fidy, idx2 = I.g.fidx2, idy2 = I.g.fidy2, idxy = I.g.fidxy, dx = I.g.fdx, dy = I.g.fdy;
+            const float c2 = I.fdt * I.frho * I.fkappa2;
+            const float rden_a = 1.f / (1.f + 2.f * c2 * idy2), rden_b = 1.f / (1.f + 2.f * c2 * idx2);
+            const bool lang = I.lang_A_on != 0;
+            const float lc = I.flang_A;
+            const int i0 = w.x0 - 2 + 2 * lane, j0 = w.j0, rows = w.pad, S = rows + 4;
+            const bool in[2] = {i0 >= 0 && i0 < Nx, i0 + 1 >= 0 && i0 + 1 < Nx};    // node, and its y link's column
+            const bool ina[2] = {i0 >= 0 && i0 < Nxa, i0 + 1 >= 0 && i0 + 1 < Nxa};  // x link's column
+            const bool own = lane >= 1 && lane <= 30;
+            auto issue = [&](int s, AStage& t) {
+                const int y = j0 - 2 + s;
+                const bool row = y >= 0 && y < Ny && s < S, rowb = y >= 0 && y < Ny - 1 && s < S;
+#pragma unroll
+                for (int c = 0; c < 2; ++c) {
+                    const bool ta = row && ina[c], tb = rowb && in[c], tp = row && in[c];
+                    const int la = ta ? i0 + c + Nxa * y : 0, lb = tb ? Na + i0 + c + Nx * y : 0;
+                    copy_async<4>(c ? &t.a0[lane].y : &t.a0[lane].x, base + la, ta);
+                    copy_async<4>(c ? &t.b0[lane].y : &t.b0[lane].x, base + lb, tb);
+                    copy_async<4>(c ? &t.da[lane].y : &t.da[lane].x, cur + la, ta && k > 0);
+                    copy_async<4>(c ? &t.db[lane].y : &t.db[lane].x, cur + lb, tb && k > 0);
+                    copy_async<8>(c ? &t.psi[lane].z : &t.psi[lane].x, psi + (tp ? i0 + c + Nx * y : 0), tp);
+                }
+                copy_async_commit();
+            };
+            // link-weight bits of the row above the new one, fetched with it
+            auto codes = [&](int s) -> unsigned {
+                const int y = j0 - 3 + s;
+                unsigned cd = 0u;
+                if (y >= 0 && y < Ny && s < S) {
+                    if (in[0]) cd = __ldg(&I.code[i0 + Nx * y]);
+                    if (in[1]) cd |= (unsigned)__ldg(&I.code[i0 + 1 + Nx * y]) << 8;
+                }
+                return cd;
+            };
+            const ARow zr = {{0.f, 0.f}, {0.f, 0.f}, 0.f, 0.f, 0.f};
+            // rows y - 1 and y - 2 of A^(0) and delta^(k); y - 2 and y - 3 of the first sweep
+            ARow A1 = zr, A2 = zr, D1 = zr, D2 = zr, F1 = zr, F2 = zr;
+            float2 P1[2] = {make_float2(0.f, 0.f), make_float2(0.f, 0.f)};
+            float xa2[2] = {0.f, 0.f}, xb2[2] = {0.f, 0.f};  // X of row y - 2
+            unsigned cdr[NS];
+#pragma unroll
+            for (int a = 0; a < NS - 1; ++a) {
+                issue(a, st4[a]);
+                cdr[a] = codes(a);
+            }
+            auto step = [&](int s, AStage& t, AStage& tn, unsigned cd) {
+                copy_async_wait<NS - 2>();
+                const int y = j0 - 2 + s;
+                ARow A0, D0;
+                const float2 va = t.a0[lane], vb = t.b0[lane], wa = t.da[lane], wb = t.db[lane];
+                A0.a[0] = va.x; A0.a[1] = va.y; A0.b[0] = vb.x; A0.b[1] = vb.y;
+                D0.a[0] = wa.x; D0.a[1] = wa.y; D0.b[0] = wb.x; D0.b[1] = wb.y;
+                const float4 pv = t.psi[lane];
+                const float2 P0[2] = {make_float2(pv.x, pv.y), make_float2(pv.z, pv.w)};
+                issue(s + NS - 1, tn);  // into the stage that the step before has read
+                row_sides(A0);
+                row_sides(D0);
+                const float2 pr = make_float2(__shfl_down_sync(0xffffffffu, P1[0].x, 1), __shfl_down_sync(0xffffffffu, P1[0].y, 1));
+                // X and the first sweep of row j
+                const int j = y - 1;
+                float xa[2] = {0.f, 0.f}, xb[2] = {0.f, 0.f};
+                ARow F0 = zr;
+                if (j >= 0 && j < Ny) {
+                    const bool edge = j == 0 || j == Ny - 1;
+                    const float dda = edge ? 2.f : 1.f;
+                    const float rha = j == 0 ? 2.f * k2 * H * idy : (j == Ny - 1 ? -2.f * k2 * H * idy : 0.f);
+#pragma unroll
+                    for (int c = 0; c < 2; ++c) {
+                        const int i = i0 + c;
+                        const float ddb = i == 0 || i == Nx - 1 ? 2.f : 1.f;
+                        const float rhb = i == 0 ? -2.f * k2 * H * idx : (i == Nx - 1 ? 2.f * k2 * H * idx : 0.f);
+                        float pa = A1.a[c] + D1.a[c], pb = A1.b[c] + D1.b[c], fa = 0.f, fb = 0.f;
+                        const bool ha = ina[c], hb = in[c] && j < Ny - 1;
+                        if (vpi) {
+                            pa = ha ? vpi[i + Nxa * j] : 0.f;
+                            pb = hb ? vpi[Na + i + Nx * j] : 0.f;
+                        }
+                        if (lang) {
+                            fa = add_noise<float>(0.f, lc, rand_1<float>((uint32_t)(i + Nxa * j), rt));
+                            fb = add_noise<float>(0.f, lc, rand_2<float>((uint32_t)(Na + i + Nx * j), rt));
+                        }
+                        const float ja = mul_rn<float>(idx, js_of<float>(P1[c], dx * pa, c == 0 ? P1[1] : pr));
+                        const float jb = mul_rn<float>(idy, js_of<float>(P1[c], dy * pb, P0[c]));
+                        xa[c] = A_fixed<float>(fa, dt_rho, (cd >> (8 * c)) & 2u ? ja : 0.f, rha) +
+                                A_base<float>(dt_rho_k2, dda, row_nbs_x(idy2, idxy, A2, A1, A0, c), idy2, A1.a[c]);
+                        xb[c] = A_fixed<float>(fb, dt_rho, (cd >> (8 * c)) & 8u ? jb : 0.f, rhb) +
+                                A_base<float>(dt_rho_k2, ddb, row_nbs_y(idx2, idxy, A1, A0, c), idx2, A1.b[c]);
+                        const float na = fma(dt_rho_k2 * dda, row_nbs_x(idy2, idxy, D2, D1, D0, c), xa[c]) * rden_a;
+                        const float nb = fma(dt_rho_k2 * ddb, row_nbs_y(idx2, idxy, D1, D0, c), xb[c]) * rden_b;
+                        F0.a[c] = ha ? na : 0.f;
+                        F0.b[c] = hb ? nb : 0.f;
+                    }
+                }
+                row_sides(F0);
+                // the second sweep of row j - 1
+                float ga[2] = {0.f, 0.f}, gb[2] = {0.f, 0.f};
+                if (j >= 1 && j - 1 < Ny) {
+                    const float dda = j == 1 || j == Ny ? 2.f : 1.f;
+#pragma unroll
+                    for (int c = 0; c < 2; ++c) {
+                        const int i = i0 + c;
+                        const float ddb = i == 0 || i == Nx - 1 ? 2.f : 1.f;
+                        const float na = fma(dt_rho_k2 * dda, row_nbs_x(idy2, idxy, F2, F1, F0, c), xa2[c]) * rden_a;
+                        const float nb = fma(dt_rho_k2 * ddb, row_nbs_y(idx2, idxy, F1, F0, c), xb2[c]) * rden_b;
+                        ga[c] = ina[c] ? na : 0.f;
+                        gb[c] = in[c] && j < Ny ? nb : 0.f;
+                    }
+                }
+                // rows 2 .. rows + 1 of the walk are the strip's own
+                auto tell = [&](int l, float d0, float d1) {
+                    asm("max.abs.f32 %0, %0, %1, %2;" : "+f"(wmax[l]) : "f"(d0), "f"(d1));
+                    asm("max.NaN.abs.f32 %0, %0, %1, %2;" : "+f"(wnan[l]) : "f"(d0), "f"(d1));
+                };
+                auto store = [&](int yy, const float (&va2)[2], const float (&vb2)[2]) {
+#pragma unroll
+                    for (int c = 0; c < 2; ++c) {
+                        if (own && ina[c]) out[i0 + c + Nxa * yy] = va2[c];
+                        if (own && in[c] && yy < Ny - 1) out[Na + i0 + c + Nx * yy] = vb2[c];
+                    }
+                };
+                if (s >= 3 && s < rows + 3) {
+                    tell(0, F0.a[0] - D1.a[0], F0.a[1] - D1.a[1]);
+                    tell(0, F0.b[0] - D1.b[0], F0.b[1] - D1.b[1]);
+                    if (keep_at == 1) store(j, F0.a, F0.b);
+                }
+                if (s >= 4 && s < rows + 4) {
+                    tell(1, ga[0] - F1.a[0], ga[1] - F1.a[1]);
+                    tell(1, gb[0] - F1.b[0], gb[1] - F1.b[1]);
+                    if (keep_at == 2) store(j - 1, ga, gb);
+                }
+                A2 = A1;
+                A1 = A0;
+                D2 = D1;
+                D1 = D0;
+                F2 = F1;
+                F1 = F0;
+#pragma unroll
+                for (int c = 0; c < 2; ++c) {
+                    P1[c] = P0[c];
+                    xa2[c] = xa[c];
+                    xb2[c] = xb[c];
+                }
+            };
+            for (int s = 0; s < S; s += NS) {
+#pragma unroll
+                for (int a = 0; a < NS; ++a) {
+                    cdr[(a + NS - 1) % NS] = codes(s + a + NS - 1);
+                    step(s + a, st4[a], st4[(a + NS - 1) % NS], cdr[a]);
+                }
+            }
+            copy_async_wait<0>();
+            if (!own) wmax[0] = wmax[1] = wnan[0] = wnan[1] = 0.f;  // the halo lanes' columns are other strips'
+        }
+        if (cur_inst >= 0 && !done && !quiet) strip_flush<2>(insts[cur_inst], wmax, wnan);
+        if (!end_round(insts, ninst, loop, seq, s_word, CloseA{min(loop->guard, kLoopGuard)})) break;
     }
 }
 
@@ -498,32 +783,39 @@ k_psi_loop_f32(const Inst* __restrict__ insts, int ninst, const Item* __restrict
 const void* psi_loop_fn(int dtype) { return dtype == 8 ? (const void*)k_psi_loop_f64 : (const void*)k_psi_loop_f32; }
 int psi_loop_threads(int dtype) { return dtype == 8 ? kThreads : kPsiThreads; }
 
-// CTAs of the loop over n tiles or items: all of them are resident.
-int psi_loop_grid(int dtype, int n) {
+const void* A_loop_fn() { return (const void*)k_A_loop_f32; }
+
+// CTAs of a loop kernel that are resident at once.
+static int loop_cap(const void* fn, int threads) {
     int dev = 0, sms = 1, per_sm = 1;
     cudaGetDevice(&dev);
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, psi_loop_fn(dtype), psi_loop_threads(dtype), 0) != cudaSuccess ||
-        per_sm < 1)
-        per_sm = 1;
-    const int need = dtype == 8 ? n : (n + kPsiWarps - 1) / kPsiWarps;
-    return need < sms * per_sm ? need : sms * per_sm;
+    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, fn, threads, 0) != cudaSuccess || per_sm < 1) per_sm = 1;
+    return sms * per_sm;
 }
 
-static int wide_items(const Geo& g, int rows) { return ((g.Nx + kWideCols - 1) / kWideCols) * ((g.Ny + rows - 1) / rows); }
+// CTAs of the loop over n tiles or items.
+int psi_loop_grid(int dtype, int n) {
+    const int need = dtype == 8 ? n : (n + kPsiWarps - 1) / kPsiWarps, cap = loop_cap(psi_loop_fn(dtype), psi_loop_threads(dtype));
+    return need < cap ? need : cap;
+}
+int A_loop_grid(int n) {
+    const int need = (n + kPsiWarps - 1) / kPsiWarps, cap = loop_cap(A_loop_fn(), kPsiThreads);
+    return need < cap ? need : cap;
+}
 
-// Strip height of the FP32 loop for a set of instances: a round lasts as long as the warp
-// with the most items, ceil(items / warps), and an item of R rows costs about 3R + 6
-// row-sweeps (sweep l of the three covers R + 2(3 - l) rows).  R + 6 steps are walked in
-// fours.
-int choose_loop_rows(const Geo* const* geos, int n) {
+// Strip height of an FP32 loop for a set of instances: a round lasts as long as the warp
+// with the most items, ceil(items / warps), and an item of R rows costs about R + halo
+// steps.  R + 2 K steps are walked in fours.
+static int choose_rows(const Geo* const* geos, int n, const void* fn, int cols, int K) {
     int best = 0;
     long long best_cost = -1;
-    for (int R = 6; R <= 62; R += kWideStages) {
+    const long long warps = (long long)loop_cap(fn, kPsiThreads) * kPsiWarps;
+    for (int S = 12; S <= 68; S += kWideStages) {
+        const int R = S - 2 * K;
         long long items = 0;
-        for (int q = 0; q < n; ++q) items += wide_items(*geos[q], R);
-        const long long warps = (long long)psi_loop_grid(4, (int)items) * kPsiWarps;
-        const long long cost = (items + warps - 1) / warps * (3LL * R + 2LL * kFuse);
+        for (int q = 0; q < n; ++q) items += (long long)((geos[q]->Nx + cols - 1) / cols) * ((geos[q]->Ny + R - 1) / R);
+        const long long cost = (items + warps - 1) / warps * (long long)(R + K);
         if (best_cost < 0 || cost < best_cost) {
             best_cost = cost;
             best = R;
@@ -531,12 +823,14 @@ int choose_loop_rows(const Geo* const* geos, int n) {
     }
     return best;
 }
+int choose_loop_rows(const Geo* const* geos, int n) { return choose_rows(geos, n, psi_loop_fn(4), kWideCols, kFuse); }
+int choose_A_rows(const Geo* const* geos, int n) { return choose_rows(geos, n, A_loop_fn(), kACols, 2); }
 
-// Items of an instance for the FP32 loop, band by band (warps that run at the same time
+// Items of an instance for the FP32 loops, band by band (warps that run at the same time
 // share halo rows in L2).
-void add_loop_items(std::vector<Item>& items, const Geo& g, int inst, int rows) {
+void add_loop_items(std::vector<Item>& items, const Geo& g, int inst, int rows, int cols) {
     for (int j0 = 0; j0 < g.Ny; j0 += rows)
-        for (int x0 = 0; x0 < g.Nx; x0 += kWideCols) items.push_back(Item{inst, x0, j0, std::min(rows, g.Ny - j0)});
+        for (int x0 = 0; x0 < g.Nx; x0 += cols) items.push_back(Item{inst, x0, j0, std::min(rows, g.Ny - j0)});
 }
 
 }  // namespace glgpu

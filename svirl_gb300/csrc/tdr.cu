@@ -422,7 +422,7 @@ k_td_resident(const Inst* __restrict__ insts, const ResTile* __restrict__ tiles,
                 for (int r = 0; r < R; ++r) {
                     sp[0][e0 + r + 1][tx + 1] = p[r];
                     sp[1][e0 + r + 1][tx + 1] = cmk<T>(a0[r], b0[r]);
-                    ac[r] = kDelta ? T(0) : a0[r];  // FP32 iterates the offsets from A^(0) (k_A_sweep)
+                    ac[r] = kDelta ? T(0) : a0[r];  // FP32 iterates the offsets from A^(0) (k_A_loop_f32)
                     bc[r] = kDelta ? T(0) : b0[r];
                     xa[r] = xb[r] = T(0);
                 }
