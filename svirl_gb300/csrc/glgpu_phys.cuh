@@ -199,8 +199,15 @@ __device__ __forceinline__ T curlcurl_link_exact(const Geo& g, const T* abei, co
     return curlcurl_link<T>(g, abei, ab, H, i, j, xdir);
 }
 
-// dF/d(Re psi) + i dF/d(Im psi) at node n (svirl/cuda/cg.h:15-121), dx*dy included;
-// a link adds 2 w (psi0 - psi1 U(ph)) (cg.h:4-12).
+// 2 (psi0 - psi1 U(ph)) with (s, c) = sincos(ph) (svirl/cuda/cg.h:4-12)
+template <typename T> __device__ __forceinline__ C2<T> gjac_sc(C2<T> p0, T s, T c, C2<T> p1) {
+    return cmk<T>(T(2) * (p0.x - (p1.x * c + p1.y * s)), T(2) * (p0.y - (p1.y * c - p1.x * s)));
+}
+
+// dF/d(Re psi) + i dF/d(Im psi) at node n (svirl/cuda/cg.h:15-121), dx*dy included.
+// FP64 in the fewest operations on its pipe.  FP32 keeps its own order: a CG run carries
+// the rounding of the gradient and of the line-search sums through its iterations, where
+// a line search can turn 1e-7 into 5e-6 of the state.
 template <typename T, typename LK>
 __device__ __forceinline__ C2<T> grad_psi_node(const Geo& g, T eps0, const T* eps_sp, const C2<T>* psi, const LK& lk,
                                                int n, int i, int j, unsigned cb) {
@@ -212,27 +219,33 @@ __device__ __forceinline__ C2<T> grad_psi_node(const Geo& g, T eps0, const T* ep
         const T eps = eps_sp ? eps_sp[n] : eps0;
         const T p = p0.x * p0.x + p0.y * p0.y - eps;
         const T k = T(2) * w.g * p;
-        gj = cmk<T>(k * p0.x, k * p0.y);
-        auto add = [&gj, p0](T w2, T sn, T cs, C2<T> p1) {
-            const C2<T> d = link_diff<T>(p0, sn, cs, p1);
-            gj = cmk<T>(fma(w2, d.x, gj.x), fma(w2, d.y, gj.y));
+        if constexpr (sizeof(T) == 8) gj = cmk<T>(k * p0.x, k * p0.y);
+        else gj = cadd(gj, cscale(T(2) * w.g * p, p0));
+        auto add = [&gj, p0](T r, bool both, T i2, T sn, T cs, C2<T> p1) {
+            if constexpr (sizeof(T) == 8) {
+                const C2<T> d = link_diff<T>(p0, sn, cs, p1);
+                const T w2 = both ? T(2) * i2 : i2;
+                gj = cmk<T>(fma(w2, d.x, gj.x), fma(w2, d.y, gj.y));
+            } else {
+                gj = cadd(gj, cscale(r * i2, gjac_sc<T>(p0, sn, cs, p1)));
+            }
         };
         T sn, cs;  // the links below and left of the node enter with the opposite phase: sin(-x) = -sin(x)
         if (GL_MM(cb) || GL_MP(cb)) {
             lk.sc_sum((i - 1) + (g.Nx - 1) * j, dx, sn, cs);
-            add(du_times(GL_MM(cb) && GL_MP(cb), T(2) * idx2, idx2), -sn, cs, psi[n - 1]);
+            add(w.r_m0, GL_MM(cb) && GL_MP(cb), idx2, -sn, cs, psi[n - 1]);
         }
         if (GL_PM(cb) || GL_PP(cb)) {
             lk.sc_sum(i + (g.Nx - 1) * j, dx, sn, cs);
-            add(du_times(GL_PM(cb) && GL_PP(cb), T(2) * idx2, idx2), sn, cs, psi[n + 1]);
+            add(w.r_p0, GL_PM(cb) && GL_PP(cb), idx2, sn, cs, psi[n + 1]);
         }
         if (GL_MM(cb) || GL_PM(cb)) {
             lk.sc_sum(g.Na + i + g.Nx * (j - 1), dy, sn, cs);
-            add(du_times(GL_MM(cb) && GL_PM(cb), T(2) * idy2, idy2), -sn, cs, psi[n - g.Nx]);
+            add(w.r_0m, GL_MM(cb) && GL_PM(cb), idy2, -sn, cs, psi[n - g.Nx]);
         }
         if (GL_MP(cb) || GL_PP(cb)) {
             lk.sc_sum(g.Na + i + g.Nx * j, dy, sn, cs);
-            add(du_times(GL_MP(cb) && GL_PP(cb), T(2) * idy2, idy2), sn, cs, psi[n + g.Nx]);
+            add(w.r_0p, GL_MP(cb) && GL_PP(cb), idy2, sn, cs, psi[n + g.Nx]);
         }
     }
     return cscale(GT(g, dxdy), gj);
@@ -308,35 +321,67 @@ __device__ __forceinline__ void coef_node(const Geo& g, T kappa2, T eps0, const 
             const int nl = dir == 0 ? i + (g.Nx - 1) * j : g.Na + i + g.Nx * j;
             const int m1 = dir == 0 ? n + 1 : n + g.Nx;
             const T d = dir == 0 ? dx : dy;
-            const T full = dir == 0 ? idx2 : idy2;
-            const bool both = GL_PP(cb) && (dir == 0 ? GL_PM(cb) : GL_MP(cb));
-            const T wr = du_times(both, full, T(0.5) * full), wr2 = du_times(both, T(2) * full, full);
             const C2<T> p1 = psi(m1), d1 = dpsi(m1);
             T s, cs;
             lk.sc_split(nl, d, s, cs);
-            const C2<T> gp = link_diff<T>(p0, s, cs, p1), gd = link_diff<T>(d0, s, cs, d1);
-            const T gg_d = fma(gd.x, gd.x, gd.y * gd.y);
-            const T zr = fma(gp.x, gd.x, gp.y * gd.y);  // Re(conj(gp) * gd)
-            constexpr int k1 = NV == 5 ? 1 : 5, k2 = NV == 5 ? 2 : 10;
-            if (WITH0) c[0] = fma(wr, fma(gp.x, gp.x, gp.y * gp.y), c[0]);
-            c[k1] = fma(wr2, zr, c[k1]);
-            c[k2] = fma(wr, gg_d, c[k2]);
-            if constexpr (NV != 5) {
-                const C2<T> q = cmk<T>(p0.x - gp.x, p0.y - gp.y), e = cmk<T>(d0.x - gd.x, d0.y - gd.y);
-                const T dph = d * dA(nl);
-                // 2 w dph, w dph^2, -w dph^3 / 3, -w dph^4 / 12
-                const T f1 = wr2 * dph, h = T(0.5) * dph, f2 = f1 * h, f3 = f2 * (T(-1.0 / 3.0) * dph), f4 = f3 * (T(0.5) * h);
-                auto add = [&](int b, T zx, T zy) {
-                    c[b + 0] = fma(zy, f1, c[b + 0]);
-                    c[b + 1] = fma(zx, f2, c[b + 1]);
-                    c[b + 2] = fma(zy, f3, c[b + 2]);
-                    c[b + 3] = fma(zx, f4, c[b + 3]);
-                };
-                // p0 conj(q), p0 conj(e) + d0 conj(q), d0 conj(e)
-                add(1, fma(p0.x, q.x, p0.y * q.y), fma(p0.y, q.x, -(p0.x * q.y)));
-                add(6, fma(p0.x, e.x, fma(p0.y, e.y, fma(d0.x, q.x, d0.y * q.y))),
-                    fma(p0.y, e.x, fma(-p0.x, e.y, fma(d0.y, q.x, -(d0.x * q.y)))));
-                add(11, fma(d0.x, e.x, d0.y * e.y), fma(d0.y, e.x, -(d0.x * e.y)));
+            if constexpr (sizeof(T) == 8) {
+                const T full = dir == 0 ? idx2 : idy2;
+                const bool both = GL_PP(cb) && (dir == 0 ? GL_PM(cb) : GL_MP(cb));
+                const T wr = du_times(both, full, T(0.5) * full), wr2 = du_times(both, T(2) * full, full);
+                const C2<T> gp = link_diff<T>(p0, s, cs, p1), gd = link_diff<T>(d0, s, cs, d1);
+                const T gg_d = fma(gd.x, gd.x, gd.y * gd.y);
+                const T zr = fma(gp.x, gd.x, gp.y * gd.y);  // Re(conj(gp) * gd)
+                constexpr int k1 = NV == 5 ? 1 : 5, k2 = NV == 5 ? 2 : 10;
+                if (WITH0) c[0] = fma(wr, fma(gp.x, gp.x, gp.y * gp.y), c[0]);
+                c[k1] = fma(wr2, zr, c[k1]);
+                c[k2] = fma(wr, gg_d, c[k2]);
+                if constexpr (NV != 5) {
+                    const C2<T> q = cmk<T>(p0.x - gp.x, p0.y - gp.y), e = cmk<T>(d0.x - gd.x, d0.y - gd.y);
+                    const T dph = d * dA(nl);
+                    // 2 w dph, w dph^2, -w dph^3 / 3, -w dph^4 / 12
+                    const T f1 = wr2 * dph, h = T(0.5) * dph, f2 = f1 * h, f3 = f2 * (T(-1.0 / 3.0) * dph), f4 = f3 * (T(0.5) * h);
+                    auto add = [&](int b, T zx, T zy) {
+                        c[b + 0] = fma(zy, f1, c[b + 0]);
+                        c[b + 1] = fma(zx, f2, c[b + 1]);
+                        c[b + 2] = fma(zy, f3, c[b + 2]);
+                        c[b + 3] = fma(zx, f4, c[b + 3]);
+                    };
+                    // p0 conj(q), p0 conj(e) + d0 conj(q), d0 conj(e)
+                    add(1, fma(p0.x, q.x, p0.y * q.y), fma(p0.y, q.x, -(p0.x * q.y)));
+                    add(6, fma(p0.x, e.x, fma(p0.y, e.y, fma(d0.x, q.x, d0.y * q.y))),
+                        fma(p0.y, e.x, fma(-p0.x, e.y, fma(d0.y, q.x, -(d0.x * q.y)))));
+                    add(11, fma(d0.x, e.x, d0.y * e.y), fma(d0.y, e.x, -(d0.x * e.y)));
+                }
+            } else {
+                const T wr = (dir == 0 ? w.r_p0 : w.r_0p) * (dir == 0 ? idx2 : idy2);
+                const C2<T> gp = grad_c_sc<T>(p0, s, cs, p1), gd = grad_c_sc<T>(d0, s, cs, d1);
+                const T gg_p = gp.x * gp.x + gp.y * gp.y;
+                const T gg_d = gd.x * gd.x + gd.y * gd.y;
+                const T zr = gp.x * gd.x + gp.y * gd.y;  // Re(conj(gp) * gd)
+                if (NV == 5) {
+                    c[2] += wr * gg_d;
+                    c[1] += wr * T(2) * zr;
+                    if (WITH0) c[0] += wr * gg_p;
+                } else {
+                    if (WITH0) c[0] += wr * gg_p;
+                    c[5] += wr * T(2) * zr;
+                    c[10] += wr * gg_d;
+                    const T dph = d * dA(nl);
+                    const T dph2 = dph * dph;
+                    const C2<T> Um = cmk<T>(cs, s);  // U(-ph)
+                    const C2<T> z1 = cmul(cmul(p0, Um), cconj(p1));
+                    const C2<T> z2 = cadd(cmul(cmul(p0, Um), cconj(d1)), cmul(cmul(d0, Um), cconj(p1)));
+                    const C2<T> z3 = cmul(cmul(d0, Um), cconj(d1));
+                    const C2<T> zz[3] = {z1, z2, z3};
+#pragma unroll
+                    for (int q = 0; q < 3; ++q) {
+                        const int b = 1 + 5 * q;
+                        c[b + 0] += wr * T(2) * zz[q].y * dph;
+                        c[b + 1] += wr * zz[q].x * dph2;
+                        c[b + 2] += -wr / T(3) * zz[q].y * dph2 * dph;
+                        c[b + 3] += -wr / T(12) * zz[q].x * dph2 * dph2;
+                    }
+                }
             }
         }
     }
@@ -351,10 +396,16 @@ __device__ __forceinline__ void coef_node(const Geo& g, T kappa2, T eps0, const 
             const T b00 = phase(ib00), bp0 = phase(ibp0);
             const T BH = idx * (bp0 - b00) - idy * (a0p - a00) - H;
             const T dB = idx * (dA(ibp0) - dA(ib00)) - idy * (dA(ia0p) - dA(ia00));
-            const T kd = kappa2 * dB;
-            if (WITH0) c[0] = fma(kappa2 * BH, BH, c[0]);
-            c[1] = fma(T(2) * kd, BH, c[1]);
-            c[2] = fma(kd, dB, c[2]);
+            if constexpr (sizeof(T) == 8) {
+                const T kd = kappa2 * dB;
+                if (WITH0) c[0] = fma(kappa2 * BH, BH, c[0]);
+                c[1] = fma(T(2) * kd, BH, c[1]);
+                c[2] = fma(kd, dB, c[2]);
+            } else {
+                if (WITH0) c[0] += kappa2 * BH * BH;
+                c[1] += kappa2 * T(2) * BH * dB;
+                c[2] += kappa2 * dB * dB;
+            }
         }
     }
 }
