@@ -609,7 +609,8 @@ template <typename T, class S, int MINB> static ResCfg res_cfg(int most, bool wa
 // waves on a shape marked `waves`.  Measured, us per time step (22 psi sweeps), by the
 // launch-per-sweep loop and by the shapes here (own nodes per tile):
 //   FP32, kappa = inf:  129^2 145, 16x16 19;  513^2 164, 58x26 52;  700^2 172, 60x60 72
-//   FP32, kappa = 4:    257^2 22x22 39 (16x16 42);  385^2 250, 24x24 53 (58x26 72)
+//   FP32, kappa = 4:    257^2 22x22 39 (16x16 42);  385^2 250, 24x24 53 (58x26 55);
+//                       449^2 58x26 56, two CTAs per SM 73
 //   FP64, kappa = inf:  129^2 315, 12x12 63 (28x12 93);  257^2 321, 28x12 150 (28x28 162);
 //                       385^2 378, 62x14 306 (62x30 323)
 //   32 films of 64^2 .. 512^2, 20 steps, FP32: 18.8 ms, in waves of 58x26 tiles 14.0
@@ -619,7 +620,8 @@ static const ResCfg* res_cfgs(int* n) {
         res_cfg<float, ResShape<32, 16, 2, 8, 4>, 2>(240, false),   // 16 x 16
         res_cfg<float, ResShape<32, 8, 4, 5, 4>, 2>(0, false),      // 22 x 22
         res_cfg<float, ResShape<32, 8, 4, 4, 4>, 2>(0, false),      // 24 x 24
-        res_cfg<float, ResShape<64, 8, 4, 3, 2>, 2>(0, true),       // 58 x 26
+        res_cfg<float, ResShape<64, 8, 4, 3, 2>, 1>(0, false),      // 58 x 26, a CTA per SM (128 registers)
+        res_cfg<float, ResShape<64, 8, 4, 3, 2>, 2>(0, true),       // 58 x 26, two (64 registers, spills)
         res_cfg<float, ResShape<64, 8, 8, 2, 2>, 1>(0, true),       // 60 x 60
         res_cfg<double, ResShape<16, 16, 1, 2, 1>, 2>(230, false),  // 12 x 12
         res_cfg<double, ResShape<32, 8, 2, 2, 1>, 2>(0, false),     // 28 x 12
