@@ -189,21 +189,21 @@ def peaks():
     return 6800.0, "fallback"
 
 
-def ncu_traffic(dtype_name, fuse, rows):
-    """DRAM bytes per psi-sweep launch from the committed ncu summary of the same
-    kernel build (same sweeps per launch and strip height), or None."""
-    p = os.path.join(ROOT, "profiles", "psi_sweep_%s_2049.md" % dtype_name)
+def ncu_traffic(dtype_name, fuse):
+    """DRAM bytes per psi-sweep round from the committed ncu summary of the same
+    kernel build (same sweeps per round), or None."""
+    p = os.path.join(ROOT, "profiles", "psi_loop_%s_2049.md" % dtype_name)
     if not os.path.exists(p):
         return None
     vals = {}
     for line in open(p):
-        if ":" in line and line.split(":", 1)[0] in ("traffic_bytes_per_launch", "sweeps_per_launch", "strip_rows"):
+        if ":" in line and line.split(":", 1)[0] in ("traffic_bytes_per_launch", "sweeps_per_launch"):
             k, v = line.split(":", 1)
             try:
                 vals[k] = float(v.strip())
             except ValueError:
                 return None
-    if int(vals.get("sweeps_per_launch", 1)) != fuse or int(vals.get("strip_rows", 0)) != rows:
+    if int(vals.get("sweeps_per_launch", 1)) != fuse:
         return None
     return vals.get("traffic_bytes_per_launch")
 
@@ -843,7 +843,7 @@ def main():
         a_ms = h.time_sweeps(1, 10)
         a_bytes = (40 if dtype == np.float32 else 80) + 1
         a_gbs = N * a_bytes / (a_ms * 1e-3) / 1e9
-        a_sweep = {"kernel": "k_A_sweep", "launch_ms": a_ms, "bytes_per_node_sweep": a_bytes,
+        a_sweep = {"kernel": "k_A_loop_f32" if dtype == np.float32 else "k_A_sweep", "launch_ms": a_ms, "bytes_per_node_sweep": a_bytes,
                    "achieved_GBps": a_gbs, "frac": a_gbs / peak}
 
     # end to end through the C ABI with pinned host buffers: H2D psi, one TD step, D2H psi
@@ -893,7 +893,7 @@ def main():
                 prec = precision_check(args.size)
             except Exception as e:  # noqa: BLE001
                 prec = {"error": "%s: %s" % (type(e).__name__, e)}
-        # sweep launches counted on the device, plus per step the link table, the
+        # loop and sweep launches counted on the device, plus per step the link table, the
         # loop begin/end and step-end kernels, plus the final copy and reset
         launches = int(st.sweep_launches) + 4 * args.steps + 3
         line = {
@@ -909,13 +909,13 @@ def main():
                              % (N * (3 * (8 if dtype == np.float32 else 16) + (8 if dtype == np.float32 else 16)) / 1e6),
                        "mean_sweeps_per_step": sweeps / args.steps,
                        "mean_A_sweeps_per_step": st.total_sweeps_A / args.steps,
-                       "psi_sweep_shape": {"kernel": ["register strip", "bulk-copy ring"][tuned["kernel"]],
+                       "psi_sweep_shape": {"kernel": ["cooperative loop", "bulk-copy ring"][tuned["kernel"]],
                                            "strip_rows": tuned["rows"], "from_cache": tuned["cached"],
                                            "measured_us": tuned["measured"]}},
             "roofline": {"bound": "hbm", "achieved": achieved, "peak": peak, "unit": "GB/s",
                          "frac": achieved / peak,
-                         "traffic": ncu_traffic(args.dtype, fuse, rows) if tuned["kernel"] == 0 else None,
-                         "kernel": "k_psi_sweep" if tuned["kernel"] == 0 else "k_psi_sweep_bulk",
+                         "traffic": ncu_traffic(args.dtype, fuse) if tuned["kernel"] == 0 else None,
+                         "kernel": ("k_psi_loop_f32" if dtype == np.float32 else "k_psi_loop_f64") if tuned["kernel"] == 0 else "k_psi_sweep_bulk",
                          "sweeps_per_launch": fuse, "strip_rows": rows,
                          "bytes_per_node_sweep": bytes_per_node_sweep, "bytes_per_launch": alg_bytes,
                          "launch_ms": sweep_ms, "peak_kind": peak_kind},

@@ -91,10 +91,9 @@ int glgpu_psi_sweeps_per_launch(void);
  * compiled strip heights, by the item-count model of the persistent sweep), or what
  * glgpu_set_psi_strip_rows set; 0 if h is NULL. */
 int glgpu_psi_strip_rows(const glgpu_handle* h);
-/* Force the strip height of both FP32 psi sweeps (one of the compiled heights; 0 = the
- * models' choices, which for the default sweep may be other heights).
- * Results do not depend on it: every node gets the same arithmetic.  FP64 sweeps
- * have no strips: there it is only stored. */
+/* Force the bulk-copy sweep's strip height (one of the compiled heights; 0 = the model's
+ * choice); the default sweep has heights of its own, chosen by the size.
+ * Results do not depend on it: every node gets the same arithmetic. */
 int glgpu_set_psi_strip_rows(glgpu_handle* h, int32_t rows);
 /* The FP32 psi sweep kernel: 0 (default) = the whole Jacobi loop as one cooperative
  * launch; 1 = a launch per three sweeps, inputs staged in shared memory by bulk copies

@@ -1,9 +1,9 @@
 """Measured choice of the psi sweep's launch shape, persisted per problem.
 
-The FP32 psi sweep takes the strip heights in ``STRIP_ROWS`` in two kernels (the
-cooperative loop, the bulk-copy ring); FP64 has no strips, and there every height
-measures the same.  By default a handle
-takes the height an item-count model picks.  ``tune(handle)`` measures instead:
+The FP32 psi sweep has two kernels: the cooperative loop (the default; its strip
+height follows from the size) and the bulk-copy ring, compiled for the heights in
+``STRIP_ROWS``; FP64 has one without strips.  By default a handle takes the loop, and
+for the ring the height an item-count model picks.  ``tune(handle)`` measures instead:
 it times one sweep launch (``glgpu_time_sweeps``: CUDA events, L2 flushed
 before each launch) for every (kernel, height) pair, applies the fastest, and
 stores it in a JSON cache keyed by (dtype, Nx, Ny, kappa finite), so that later

@@ -179,8 +179,7 @@ int glgpu_create(const glgpu_grid* grid, int32_t device, glgpu_handle** out) {
     std::vector<Item> litems, aitems;
     if (h->dtype == 4) {
         const Geo* gp = &h->g;
-        h->loop_rows = choose_loop_rows(&gp, 1);
-        add_loop_items(litems, h->g, 0, h->loop_rows, kWideCols);
+        add_loop_items(litems, h->g, 0, choose_loop_rows(&gp, 1), kWideCols);
         add_loop_items(aitems, h->g, 0, choose_A_rows(&gp, 1), kACols);
         h->nlitems = (int)litems.size();
         h->naitems = (int)aitems.size();
@@ -384,33 +383,22 @@ int glgpu_set_psi_sweep_kernel(glgpu_handle* h, int32_t select) {
 int glgpu_set_psi_strip_rows(glgpu_handle* h, int32_t rows) {
     if (check_handle(h)) return GLGPU_E_ARG;
     cudaSetDevice(h->device);
-    const Geo* gp = &h->g;
-    int loop_rows = h->dtype == 4 ? (rows == 0 ? choose_loop_rows(&gp, 1) : rows) : 0;
     if (rows == 0) rows = choose_strip_rows(h->g);
     bool known = false;
     for (int v = 0; v < kNumStripRows; ++v) known = known || kStripRowsSet[v] == rows;
     if (!known) return set_error(h, GLGPU_E_ARG, "set_psi_strip_rows: strip height not compiled in");
-    if (rows == h->strip_rows && loop_rows == h->loop_rows) return GLGPU_OK;
+    if (rows == h->strip_rows) return GLGPU_OK;
     const std::vector<Item> items = make_items(h->g, 0, rows);
-    std::vector<Item> litems;
-    if (loop_rows) add_loop_items(litems, h->g, 0, loop_rows, kWideCols);
-    Item *buf = nullptr, *lbuf = nullptr;
+    Item* buf = nullptr;
     cudaError_t e = cudaStreamSynchronize(h->stream);
     if (e == cudaSuccess) e = cudaMalloc(&buf, sizeof(Item) * items.size());
     if (e == cudaSuccess) e = cudaMemcpy(buf, items.data(), sizeof(Item) * items.size(), cudaMemcpyHostToDevice);
-    if (e == cudaSuccess && loop_rows) e = cudaMalloc(&lbuf, sizeof(Item) * litems.size());
-    if (e == cudaSuccess && loop_rows) e = cudaMemcpy(lbuf, litems.data(), sizeof(Item) * litems.size(), cudaMemcpyHostToDevice);
     if (e != cudaSuccess) {
         if (buf) cudaFree(buf);
-        if (lbuf) cudaFree(lbuf);
         return cuda_check(h, e, "set_psi_strip_rows");
     }
     cudaFree(h->items);
     h->items = buf;
-    if (h->litems) cudaFree(h->litems);
-    h->litems = lbuf;
-    h->nlitems = (int)litems.size();
-    h->loop_rows = loop_rows;
     h->strip_rows = rows;
     h->nitems = (int)items.size();
     h->psi_grid = bulk_sweep_grid(rows, h->nitems);
@@ -584,10 +572,9 @@ int glgpu_batch_create(glgpu_handle* const* handles, int32_t n, glgpu_batch** ou
     b->natiles = (int)atiles.size();
     std::vector<Item> litems, aitems;
     if (b->dtype == 4) {
-        b->loop_rows = choose_loop_rows(geos.data(), n);
-        const int arows = choose_A_rows(geos.data(), n);
+        const int rows = choose_loop_rows(geos.data(), n), arows = choose_A_rows(geos.data(), n);
         for (int q = 0; q < n; ++q) {
-            add_loop_items(litems, handles[q]->g, q, b->loop_rows, kWideCols);
+            add_loop_items(litems, handles[q]->g, q, rows, kWideCols);
             add_loop_items(aitems, handles[q]->g, q, arows, kACols);
         }
         b->nlitems = (int)litems.size();

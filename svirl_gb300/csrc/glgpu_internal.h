@@ -231,8 +231,8 @@ struct glgpu_handle {
     glgpu::Item* items = nullptr;
     int nitems = 0;
     int strip_rows = 0;                 // strip height of the psi sweep items
-    glgpu::Item* litems = nullptr;      // FP32: items of the cooperative psi loop and their height
-    int nlitems = 0, loop_rows = 0;
+    glgpu::Item* litems = nullptr;      // FP32: items of the cooperative psi loop
+    int nlitems = 0;
     glgpu::Item* aitems = nullptr;      // FP32: items of the cooperative A loop
     int naitems = 0;
     int psi_grid = 0;                   // CTAs of the persistent psi sweep
@@ -299,8 +299,8 @@ struct glgpu_batch {
     glgpu::LoopState* loop_pin = nullptr;
     glgpu::Inst* insts_pin = nullptr;
     int ntiles = 0;
-    glgpu::Item* litems = nullptr;       // FP32: items of the cooperative psi loop and their height
-    int nlitems = 0, loop_rows = 0;
+    glgpu::Item* litems = nullptr;       // FP32: items of the cooperative psi loop
+    int nlitems = 0;
     glgpu::Item* aitems = nullptr;      // FP32: items of the cooperative A loop
     int naitems = 0;
     cudaGraphExec_t td_exec[glgpu::kTDGraphs] = {};

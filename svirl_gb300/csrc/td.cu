@@ -1140,10 +1140,10 @@ static cudaError_t launch_psi_loop(int dtype, int grid, cudaStream_t s, const In
     return cudaLaunchCooperativeKernel(psi_loop_fn(dtype), dim3(grid), dim3(psi_loop_threads(dtype)), a, 0, s);
 }
 
+// The cooperative A loop (tdl.cu), or one round of it to time.
 static cudaError_t launch_A_loop(int grid, cudaStream_t s, const Inst* insts, int ninst, const Item* items, int nitems,
-                                 LoopState* loop) {
-    int zero = 0;
-    void* a[] = {&insts, &ninst, &items, &nitems, &loop, &zero};
+                                 LoopState* loop, int once) {
+    void* a[] = {&insts, &ninst, &items, &nitems, &loop, &once};
     return cudaLaunchCooperativeKernel(A_loop_fn(), dim3(grid), dim3(psi_loop_threads(4)), a, 0, s);
 }
 
@@ -1331,7 +1331,7 @@ static cudaError_t run_host_loop(const TDLaunch& L, int eqn, int Nt, cudaStream_
                 if (e != cudaSuccess) return e;
             }
             if (part == 1 && L.A_grid > 0) {
-                const cudaError_t e = launch_A_loop(L.A_grid, s, L.insts, L.ninst, L.aitems, L.naitems, L.loop);
+                const cudaError_t e = launch_A_loop(L.A_grid, s, L.insts, L.ninst, L.aitems, L.naitems, L.loop, 0);
                 if (e != cudaSuccess) return e;
             }
             for (; (part == 0 ? L.loop_grid : L.A_grid) == 0;) {
@@ -1458,7 +1458,7 @@ int time_sweeps(glgpu_handle* h, int which, int nrep, double* avg_ms) {
                                  h->nitems, h->loop);
             } else {
                 if (h->dtype == 8) k_A_sweep<<<h->natiles, kThreads, 0, h->stream>>>(h->inst, h->atiles, h->loop, none, 0);
-                else e = launch_A_loop(A_loop_grid(h->naitems), h->stream, h->inst, 1, h->aitems, h->naitems, h->loop);
+                else e = launch_A_loop(A_loop_grid(h->naitems), h->stream, h->inst, 1, h->aitems, h->naitems, h->loop, 1);
             }
             cudaEventRecord(e1, h->stream);
             if (e == cudaSuccess) e = cudaEventSynchronize(e1);

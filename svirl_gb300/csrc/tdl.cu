@@ -102,7 +102,8 @@ template <int K> struct ClosePsi {
     __device__ __forceinline__ int operator()(const Inst& I, InstState* st) const {
         const int R = *(volatile const int*)&st->rhs, redo = *(volatile const int*)&st->redo;
         const int k = K * (round - (redo ? 1 : 0)), base = K * first;
-        const int stop = redo ? redo : stop_level<K>(st, k, I.thr_psi, guard + base);
+        int stop = redo ? redo : stop_level<K>(st, k, I.thr_psi, guard + base);
+        if (first > 0) stop = 0;  // a timed loop runs for `guard` sweeps whatever they find
         if (!stop || (!redo && stop < K && !*(volatile const int*)&st->keep)) {
             st->redo = stop;
             // the next round keeps every sweep if the step before stopped within it
@@ -551,13 +552,14 @@ __device__ __forceinline__ int delta_of(int R, int k) { return (R + 1 + ((k / 2 
 
 struct CloseA {
     int guard;  // in sweeps
+    int once;   // a timed loop: one round
     __device__ __forceinline__ int operator()(const Inst& I, InstState* st) const {
         const int R = *(volatile const int*)&st->rhsA, redo = *(volatile const int*)&st->redo, k = *(volatile const int*)&st->sweep;
         const int stored = *(volatile const int*)&st->keep;  // the sweep that the round stored
         int stop = redo == 3 ? 0 : redo, go = redo == 3;
         if (!redo) {
             stop = stop_level<2>(st, k, I.thr_A, guard);
-            if (!stop && k + 2 >= guard) return 3;
+            if (once || (!stop && k + 2 >= guard)) return 3;
             if (stop != stored && (stop || stored != 2)) {
                 st->redo = stop ? stop : 3;
                 return 1;
@@ -584,7 +586,7 @@ struct CloseA {
 
 constexpr int kAMinB = 6;  // CTAs per SM that the registers must allow (7: spills, 56 us a sweep against 43)
 __global__ void __launch_bounds__(kPsiThreads, kAMinB)
-k_A_loop_f32(const Inst* __restrict__ insts, int ninst, const Item* __restrict__ items, int nitems, LoopState* loop, int) {
+k_A_loop_f32(const Inst* __restrict__ insts, int ninst, const Item* __restrict__ items, int nitems, LoopState* loop, int once) {
     constexpr int NS = kWideStages;
     __shared__ AStage s_st[kPsiWarps][NS];
     __shared__ int s_word;
@@ -775,7 +777,7 @@ k_A_loop_f32(const Inst* __restrict__ insts, int ninst, const Item* __restrict__
             if (!own) wmax[0] = wmax[1] = wnan[0] = wnan[1] = 0.f;  // the halo lanes' columns are other strips'
         }
         if (cur_inst >= 0 && !done && !quiet) strip_flush<2>(insts[cur_inst], wmax, wnan);
-        if (!end_round(insts, ninst, loop, seq, s_word, CloseA{min(loop->guard, kLoopGuard)})) break;
+        if (!end_round(insts, ninst, loop, seq, s_word, CloseA{min(loop->guard, kLoopGuard), once})) break;
     }
 }
 
