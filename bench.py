@@ -189,21 +189,21 @@ def peaks():
     return 6800.0, "fallback"
 
 
-def ncu_traffic(dtype_name, fuse):
+def ncu_traffic(dtype_name, fuse, rows):
     """DRAM bytes per psi-sweep round from the committed ncu summary of the same
-    kernel build (same sweeps per round), or None."""
+    kernel build (same sweeps per round and strip height of the handle), or None."""
     p = os.path.join(ROOT, "profiles", "psi_loop_%s_2049.md" % dtype_name)
     if not os.path.exists(p):
         return None
     vals = {}
     for line in open(p):
-        if ":" in line and line.split(":", 1)[0] in ("traffic_bytes_per_launch", "sweeps_per_launch"):
+        if ":" in line and line.split(":", 1)[0] in ("traffic_bytes_per_launch", "sweeps_per_launch", "strip_rows"):
             k, v = line.split(":", 1)
             try:
                 vals[k] = float(v.strip())
             except ValueError:
                 return None
-    if int(vals.get("sweeps_per_launch", 1)) != fuse:
+    if int(vals.get("sweeps_per_launch", 1)) != fuse or int(vals.get("strip_rows", 0)) != rows:
         return None
     return vals.get("traffic_bytes_per_launch")
 
@@ -828,6 +828,8 @@ def main():
     # the right-hand side and two link values of A, write psi^(k+1) (32 B FP32,
     # 64 B FP64), +1 B for the material mask.
     fuse = int(h.lib.glgpu_psi_sweeps_per_launch())
+    if tuned["kernel"] == 0:
+        h.set_psi_strip_rows(0)  # the loop has heights of its own: the handle's is the model's
     rows = int(h.lib.glgpu_psi_strip_rows(h.h))
     sweep_ms = h.time_sweeps(0, 20)
     bytes_per_node_sweep = (32 if dtype == np.float32 else 64) + 1
@@ -914,7 +916,7 @@ def main():
                                            "measured_us": tuned["measured"]}},
             "roofline": {"bound": "hbm", "achieved": achieved, "peak": peak, "unit": "GB/s",
                          "frac": achieved / peak,
-                         "traffic": ncu_traffic(args.dtype, fuse) if tuned["kernel"] == 0 else None,
+                         "traffic": ncu_traffic(args.dtype, fuse, rows) if tuned["kernel"] == 0 else None,
                          "kernel": ("k_psi_loop_f32" if dtype == np.float32 else "k_psi_loop_f64") if tuned["kernel"] == 0 else "k_psi_sweep_bulk",
                          "sweeps_per_launch": fuse, "strip_rows": rows,
                          "bytes_per_node_sweep": bytes_per_node_sweep, "bytes_per_launch": alg_bytes,
