@@ -104,7 +104,6 @@ static void free_all(glgpu_handle* h) {
         if (h->ab[q]) cudaFree(h->ab[q]);
     for (int q = 0; q < kTDGraphs; ++q)
         if (h->td_exec[q]) cudaGraphExecDestroy(h->td_exec[q]);
-    if (h->st_gather) cudaFree(h->st_gather);
     if (h->cbits) cudaFree(h->cbits);
     if (h->vpi) cudaFree(h->vpi);
     if (h->lock) cudaFree(h->lock);
@@ -168,7 +167,6 @@ int glgpu_create(const glgpu_grid* grid, int32_t device, glgpu_handle** out) {
     ok = ok && cudaMalloc(&h->code, (size_t)h->g.N + 64) == cudaSuccess;
     ok = ok && cudaMalloc(&h->dinv, (size_t)h->g.N * rs) == cudaSuccess;
     ok = ok && cudaMalloc(&h->st, sizeof(InstState)) == cudaSuccess;
-    ok = ok && cudaMalloc(&h->st_gather, sizeof(InstState)) == cudaSuccess;
     ok = ok && cudaMalloc(&h->inst, sizeof(Inst)) == cudaSuccess;
     ok = ok && cudaMalloc(&h->tiles, sizeof(Tile) * (size_t)h->ntiles) == cudaSuccess;
     h->natiles = atiles_of(h->g.Nx, h->g.Ny);
@@ -583,7 +581,6 @@ int glgpu_batch_create(glgpu_handle* const* handles, int32_t n, glgpu_batch** ou
     b->gather_h.resize(n);
     bool ok = cudaStreamCreateWithFlags(&b->stream, cudaStreamNonBlocking) == cudaSuccess;
     ok = ok && cudaMalloc(&b->insts, sizeof(Inst) * (size_t)n) == cudaSuccess;
-    ok = ok && cudaMalloc(&b->gather, sizeof(InstState) * (size_t)n) == cudaSuccess;
     ok = ok && cudaMalloc(&b->tiles, sizeof(Tile) * tiles.size()) == cudaSuccess;
     ok = ok && cudaMalloc(&b->atiles, sizeof(ATile) * atiles.size()) == cudaSuccess;
     if (b->nlitems > 0) ok = ok && cudaMalloc(&b->litems, sizeof(Item) * litems.size()) == cudaSuccess;
@@ -618,7 +615,7 @@ int glgpu_batch_destroy(glgpu_batch* b) {
         if (b->td_exec[q]) cudaGraphExecDestroy(b->td_exec[q]);
     if (b->cg_exec) cudaGraphExecDestroy(b->cg_exec);
     res_free(&b->res);
-    void* ptrs[] = {b->insts, b->gather, b->tiles, b->atiles, b->litems, b->aitems, b->loop, b->cg_partials, b->cg_loop, b->cg_tiles, b->cg_states};
+    void* ptrs[] = {b->insts, b->tiles, b->atiles, b->litems, b->aitems, b->loop, b->cg_partials, b->cg_loop, b->cg_tiles, b->cg_states};
     for (void* p : ptrs)
         if (p) cudaFree(p);
     void* pins[] = {b->gather_pin, b->loop_pin, b->insts_pin};

@@ -258,7 +258,6 @@ struct glgpu_handle {
     uint8_t* cbits = nullptr;           // batched CG: cell bits per node, written at the start of a call
     // TD graphs, one per (equation mode, kappa finite)
     cudaGraphExec_t td_exec[glgpu::kTDGraphs] = {};
-    glgpu::InstState* st_gather = nullptr;  // device copy target of the loop state
     bool td_graph_failed = false;
     bool use_graphs = true;
     int loop_guard = 0;                 // Jacobi loop guard in sweep launches (0: kLoopGuard)
@@ -276,8 +275,7 @@ struct glgpu_handle {
 // one device) advanced together.  Their descriptors, item and tile tables are
 // concatenated, so one sweep launch covers every instance and each instance
 // keeps its own Jacobi stop rule.
-// Pinned host staging of a handle's per-call copies (descriptor up, loop state and
-// statistics down).
+// Pinned host staging of a handle's calls (descriptor up, loop state and statistics down).
 struct PinStage {
     glgpu::Inst inst;
     glgpu::InstState st;
@@ -293,7 +291,6 @@ struct glgpu_batch {
     glgpu::ATile* atiles = nullptr;     // A-sweep tiles
     int natiles = 0;
     glgpu::LoopState* loop = nullptr;
-    glgpu::InstState* gather = nullptr;
     std::vector<glgpu::InstState> gather_h;
     glgpu::InstState* gather_pin = nullptr;  // pinned host copies of the per-call transfers
     glgpu::LoopState* loop_pin = nullptr;

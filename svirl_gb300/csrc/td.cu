@@ -1396,10 +1396,13 @@ __global__ void k_bench_prep(const Inst* __restrict__ insts, int ninst, LoopStat
     }
 }
 
-// Per-call counters of every instance back to zero.
-// With `loop`, also the time loop's state for a call of Nt steps (written here rather
-// than copied from the host, which saves a transfer per call).
-__global__ void k_reset_counters(const Inst* __restrict__ insts, int ninst, LoopState* loop, int Nt, int guard) {
+// Start of a call, a CTA per instance: its descriptor from pinned host memory, its per-call
+// counters back to zero and, if given, its barrier of the resident loop; with `loop` also
+// the time loop's state for a call of Nt steps.  One launch where the copies, the memset and
+// a kernel took four operations of the stream, as did the end (65^2, 5 steps, states set and read: 163 -> 153 us).
+__global__ void k_call_begin(const Inst* host, Inst* __restrict__ insts, int ninst, ResGroup* groups, LoopState* loop, int Nt,
+                             int guard) {
+    static_assert(sizeof(Inst) % 8 == 0 && sizeof(ResGroup) % 8 == 0, "copied in 8-byte words");
     if (loop && blockIdx.x == 0 && threadIdx.x == 0) {
         LoopState ls;
         memset(&ls, 0, sizeof(ls));
@@ -1408,7 +1411,14 @@ __global__ void k_reset_counters(const Inst* __restrict__ insts, int ninst, Loop
         ls.guard = guard;
         *loop = ls;
     }
-    for (int q = blockIdx.x * blockDim.x + threadIdx.x; q < ninst; q += gridDim.x * blockDim.x) {
+    const int q = blockIdx.x;
+    const unsigned long long* src = (const unsigned long long*)(host + q);
+    unsigned long long* dst = (unsigned long long*)(insts + q);
+    for (int w = threadIdx.x; w < (int)(sizeof(Inst) / 8); w += blockDim.x) dst[w] = *(const volatile unsigned long long*)(src + w);
+    if (groups)
+        for (int w = threadIdx.x; w < (int)(sizeof(ResGroup) / 8); w += blockDim.x) ((unsigned long long*)(groups + q))[w] = 0ull;
+    __syncthreads();
+    if (threadIdx.x == 0) {
         InstState* st = insts[q].st;
         st->nan_seen = 0;
         st->last_sweeps_psi = st->last_sweeps_A = st->max_sweeps_psi = st->max_sweeps_A = 0;
@@ -1417,9 +1427,15 @@ __global__ void k_reset_counters(const Inst* __restrict__ insts, int ninst, Loop
     }
 }
 
-// The instances' loop states gathered into one array (one copy to the host).
-__global__ void k_gather_states(const Inst* __restrict__ insts, int ninst, InstState* out) {
-    for (int q = blockIdx.x * blockDim.x + threadIdx.x; q < ninst; q += gridDim.x * blockDim.x) out[q] = *insts[q].st;
+// End of a call: the instances' states and the loop's into pinned host memory.
+__global__ void k_call_end(const Inst* __restrict__ insts, int ninst, InstState* out, const LoopState* loop, LoopState* loop_out) {
+    static_assert(sizeof(InstState) % 8 == 0 && sizeof(LoopState) % 8 == 0, "copied in 8-byte words");
+    const int q = blockIdx.x;
+    const unsigned long long* src = (const unsigned long long*)insts[q].st;
+    for (int w = threadIdx.x; w < (int)(sizeof(InstState) / 8); w += blockDim.x) ((unsigned long long*)(out + q))[w] = src[w];
+    if (q == 0)
+        for (int w = threadIdx.x; w < (int)(sizeof(LoopState) / 8); w += blockDim.x)
+            ((unsigned long long*)loop_out)[w] = ((const unsigned long long*)loop)[w];
 }
 
 int time_sweeps(glgpu_handle* h, int which, int nrep, double* avg_ms) {
@@ -1535,13 +1551,16 @@ struct TDOutcome {
 // One TD call over the instances of L: per-call counters reset, the graph (built
 // once per eqn mode and kappa mix) or the host-driven loop, then the instances'
 // loop states gathered to the host.
-// gather_host and hl: pinned host memory (the call's last copies are asynchronous)
+// insts_host, gather_host and hl_pinned: pinned host memory, which the call's first and last
+// kernels read and write
 static TDOutcome td_core(cudaStream_t s, const TDLaunch& L, int Nt, int eqn, cudaGraphExec_t* execs, bool* graph_failed,
-                         bool use_graphs, int guard, bool timed, InstState* gather_dev, InstState* gather_host,
-                         LoopState* hl_pinned) {
+                         bool use_graphs, int guard, bool timed, const Inst* insts_host, Inst* insts_dev,
+                         InstState* gather_host, LoopState* hl_pinned) {
     TDOutcome o = {cudaSuccess, 0, 0, 0, 0.f, 0};
-    k_reset_counters<<<(L.ninst + 127) / 128, 128, 0, s>>>(L.insts, L.ninst, Nt > 0 ? L.loop : nullptr, Nt,
-                                                           guard > 0 ? guard : kLoopGuard);
+    k_call_begin<<<L.ninst, 128, 0, s>>>(insts_host, insts_dev, L.ninst, L.res ? L.res->groups : nullptr,
+                                         Nt > 0 ? L.loop : nullptr, Nt, guard > 0 ? guard : kLoopGuard);
+    o.err = cudaGetLastError();
+    if (o.err != cudaSuccess) return o;
     cudaEvent_t ev0 = nullptr, ev1 = nullptr;
     if (timed) {
         cudaEventCreate(&ev0);
@@ -1578,9 +1597,8 @@ static TDOutcome td_core(cudaStream_t s, const TDLaunch& L, int Nt, int eqn, cud
         }
         if (ev1) cudaEventRecord(ev1, s);
     }
-    k_gather_states<<<(L.ninst + 127) / 128, 128, 0, s>>>(L.insts, L.ninst, gather_dev);
-    o.err = cudaMemcpyAsync(gather_host, gather_dev, sizeof(InstState) * (size_t)L.ninst, cudaMemcpyDeviceToHost, s);
-    if (o.err == cudaSuccess) o.err = cudaMemcpyAsync(hl_pinned, L.loop, sizeof(hl), cudaMemcpyDeviceToHost, s);
+    k_call_end<<<L.ninst, 32, 0, s>>>(L.insts, L.ninst, gather_host, L.loop, hl_pinned);
+    o.err = cudaGetLastError();
     if (o.err == cudaSuccess) o.err = cudaStreamSynchronize(s);
     if (ev0) {
         if (o.err == cudaSuccess && Nt > 0) cudaEventElapsedTime(&o.ms, ev0, ev1);
@@ -1625,12 +1643,10 @@ int td_run(glgpu_handle* h, double dt, int Nt, int eqn, glgpu_td_stats* stats, d
     // dt of the order-parameter iterator; the A kernel also receives it (td.py:278)
     h->inst_h.dt = dt;
     h->inst_h.fdt = (float)dt;
-    // pinned staging: the descriptor upload and the statistics download of a call are
-    // asynchronous copies (the stream is synchronised before td_core returns)
+    // pinned staging of the descriptor and the statistics (the stream is synchronised before
+    // td_core returns)
     PinStage* ps = (PinStage*)h->pin;
     ps->inst = h->inst_h;
-    cudaError_t e = cudaMemcpyAsync(h->inst, &ps->inst, sizeof(Inst), cudaMemcpyHostToDevice, h->stream);
-    if (e != cudaSuccess) return cuda_check(h, e, "td: write descriptor");
     TDLaunch L;
     L.insts = h->inst; L.tiles = h->tiles; L.items = h->items; L.loop = h->loop;
     L.atiles = h->atiles; L.natiles = h->natiles;
@@ -1648,7 +1664,7 @@ int td_run(glgpu_handle* h, double dt, int Nt, int eqn, glgpu_td_stats* stats, d
     L.loop_grid = resident || h->psi_scheme != 0 || bulk_selected(h) ? 0 : psi_loop_grid(h->dtype, L.nwork);
     TDOutcome o = td_core(h->stream, L, Nt, eqn, h->td_exec, &h->td_graph_failed, h->use_graphs, h->loop_guard,
                           elapsed_ms != nullptr,
-                          h->st_gather, &ps->st, &ps->loop);
+                          &ps->inst, h->inst, &ps->st, &ps->loop);
     const InstState hs = ps->st;
     if (o.err != cudaSuccess) return cuda_check(h, o.err, "td");
     if (elapsed_ms) *elapsed_ms = o.ms;
@@ -1682,8 +1698,6 @@ int batch_td(glgpu_batch* b, double dt, int Nt, int eqn, glgpu_td_stats* stats, 
         any_fv = any_fv || h->vpi != nullptr || h->lock_n > 0;
     }
     memcpy(b->insts_pin, insts.data(), sizeof(Inst) * insts.size());
-    cudaError_t e = cudaMemcpyAsync(b->insts, b->insts_pin, sizeof(Inst) * insts.size(), cudaMemcpyHostToDevice, b->stream);
-    if (e != cudaSuccess) return batch_error(b, GLGPU_E_CUDA, std::string("batch_td: ") + cudaGetErrorString(e));
     TDLaunch L;
     L.insts = b->insts; L.tiles = b->tiles; L.items = nullptr; L.loop = b->loop;
     L.atiles = b->atiles; L.natiles = b->natiles;
@@ -1700,7 +1714,7 @@ int batch_td(glgpu_batch* b, double dt, int Nt, int eqn, glgpu_td_stats* stats, 
     L.loop_grid = resident ? 0 : psi_loop_grid(b->dtype, L.nwork);
     TDOutcome o = td_core(b->stream, L, Nt, eqn, b->td_exec, &b->td_graph_failed, b->use_graphs, b->loop_guard,
                           elapsed_ms != nullptr,
-                          b->gather, b->gather_pin, b->loop_pin);
+                          b->insts_pin, b->insts, b->gather_pin, b->loop_pin);
     if (o.err == cudaSuccess) memcpy(b->gather_h.data(), b->gather_pin, sizeof(InstState) * (size_t)b->ninst);
     if (o.err != cudaSuccess) return batch_error(b, GLGPU_E_CUDA, std::string("batch_td: ") + cudaGetErrorString(o.err));
     if (elapsed_ms) *elapsed_ms = o.ms;

@@ -770,8 +770,6 @@ void res_free(ResState* r) {
 }
 
 cudaError_t res_launch(const ResState& r, const Inst* insts, int ninst, LoopState* loop, int Nt, int eqn, cudaStream_t s) {
-    cudaError_t e = cudaMemsetAsync(r.groups, 0, sizeof(ResGroup) * (size_t)ninst, s);
-    if (e != cudaSuccess) return e;
     int do_psi = eqn != 2, do_A = eqn != 1, more = ninst > 1 ? 1 : 0;
     const ResTile* tiles = r.tiles;
     const int *first = r.first, *owner = r.owner;
