@@ -132,8 +132,9 @@ template <int K> struct ClosePsi {
 // buffers follow from its number, and of the loop state only `done` is read again.
 // Only whether a residual meets the stop rule counts, so where a CTA already holds one
 // that does not, the differences (two of the FP64 instructions) are left out.
-// Sweep at 1025 x 1025: 45 us, 38 of them FP64 pipe, against 72 for a third of a strip
-// launch of three sweeps inside a conditional graph node (513^2: 19 against 23, 65^2: 7.4
+// Sweep at 1025 x 1025: 43 us, 38 of them FP64 pipe (46 with the descriptor and the tile
+// table read again from L2 in every round), against 72 for a third of a strip
+// launch of three sweeps inside a conditional graph node (513^2: 18.8 against 23, 65^2: 7.4
 // against 15; as a launch per sweep in the conditional node 61, 26 and 14).
 __device__ __forceinline__ void flush_f64(const Inst& I, unsigned long long rmax, bool nan, unsigned long long* s_max) {
     const int lane = threadIdx.x & 31;
@@ -159,7 +160,8 @@ k_psi_loop_f64(const Inst* __restrict__ insts, int ninst, const Tile* __restrict
     using T = double;
     __shared__ int s_word, s_big;
     __shared__ unsigned long long s_max[kWarps];
-    __shared__ C2<T>* s_psi[kPsiBufs];
+    __shared__ Inst s_inst;  // a round's barrier empties L1: the descriptor stays here
+    const Inst& I = s_inst;
     int cur_inst = -1, R = 0, done = 1;
     uint32_t rt = 0;
     for (int round = first;; ++round) {
@@ -169,31 +171,30 @@ k_psi_loop_f64(const Inst* __restrict__ insts, int ninst, const Tile* __restrict
         unsigned long long rmax = 0ull, thr = 0ull;
         bool rnan = false, fresh = true;
         for (int it = blockIdx.x; it < ntiles; it += gridDim.x) {
-            const Tile t = tiles[it];
+            const Tile t = ninst == 1 ? Tile{0, it * kThreads} : tiles[it];
             if (fresh || t.inst != cur_inst) {
-                if (!fresh && !done) flush_f64(insts[cur_inst], rmax, rnan, s_max);
+                if (!fresh && !done) flush_f64(I, rmax, rnan, s_max);
                 // an instance's `done` changes only at the end of a round
-                const InstState* st = insts[t.inst].st;
                 if (t.inst != cur_inst || ninst > 1) {
-                    const Inst& I = insts[t.inst];
+                    const InstState* st = insts[t.inst].st;
+                    for (int w = threadIdx.x; w < (int)(sizeof(Inst) / 8); w += kThreads)
+                        ((unsigned long long*)&s_inst)[w] = ((const unsigned long long*)(insts + t.inst))[w];
                     done = *(volatile const int*)&st->done;
                     R = *(volatile const int*)&st->rhs;
                     rt = *(volatile const uint32_t*)&st->rand_t;
-                    if (threadIdx.x < kPsiBufs) s_psi[threadIdx.x] = (C2<T>*)I.psi[threadIdx.x];
                 }
                 if (threadIdx.x == 0) s_big = 0;
                 cur_inst = t.inst;
                 fresh = false;
                 __syncthreads();
-                cur = s_psi[ring_of(R, round)];
-                rhs = s_psi[R];
-                nxt = s_psi[ring_of(R, round + 1)];
-                thr = insts[cur_inst].thr_psi;
+                cur = (const C2<T>*)I.psi[ring_of(R, round)];
+                rhs = (const C2<T>*)I.psi[R];
+                nxt = (C2<T>*)I.psi[ring_of(R, round + 1)];
+                thr = I.thr_psi;
                 rmax = 0ull;
                 rnan = false;
             }
             const int n = t.n0 + (int)threadIdx.x;
-            const Inst& I = insts[cur_inst];
             const Geo& g = I.g;
             if (done || n >= g.N) continue;
             const int Nx = g.Nx, j = n / Nx, i = n - j * Nx;
@@ -243,7 +244,7 @@ k_psi_loop_f64(const Inst* __restrict__ insts, int ninst, const Tile* __restrict
                 if (rmax > thr) *(volatile int*)&s_big = 1;
             }
         }
-        if (!fresh && !done) flush_f64(insts[cur_inst], rmax, rnan, s_max);
+        if (!fresh && !done) flush_f64(I, rmax, rnan, s_max);
         if (!end_round(insts, ninst, loop, round - first + 1, s_word, ClosePsi<1>{round, first, kFuse * min(loop->guard, kLoopGuard)}))
             break;
     }
