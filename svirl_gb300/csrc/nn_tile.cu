@@ -328,9 +328,11 @@ k_conv_tile(const __grid_constant__ CUtensorMap ta1, const __grid_constant__ CUt
 // ---------------------------------------------------------------------------
 // Weight gradient, as k_conv_wgrad_tma (nn_tc.cu: M = two taps x 64 input channels, N =
 // output channels, K = pixels, MN-major boxes of 64 pixels, split-K), with 8 x 8-pixel
-// boxes, so that images of any size are covered (outside the image dy is filled with
-// zeros, which drops those pixels), and channels beyond the counts filled with zeros and
-// not stored.  NB: output channels of a CTA (an MMA's N).
+// boxes, so that images of any size are covered, and channels beyond the counts filled with
+// zeros and not stored.  Pixels of a box outside the image count as zero in both operands:
+// the copy engine fills dy with zeros there, and the rows of x, which its shift may take from
+// inside the image, are cleared before the MMAs (0 times an infinite x is NaN).  NB: output
+// channels of a CTA (an MMA's N).
 // ---------------------------------------------------------------------------
 constexpr int WT_BOX = 64 * 128;        // 64 pixels x 64 channels
 constexpr int WT_STAGE = 3 * WT_BOX;    // two tap boxes of x, dy
@@ -345,8 +347,8 @@ constexpr int WT_SMEM = WT_STAGES * WT_STAGE + 1024 + (2 * WT_STAGES + 2) * 8;
 template <int NB>
 __global__ void __launch_bounds__(WT_THREADS)
 k_conv_wgrad_tile(const __grid_constant__ CUtensorMap tx1, const __grid_constant__ CUtensorMap tx2,
-                  const __grid_constant__ CUtensorMap tdy, float* __restrict__ ws, int C1, int C2, int Cout, int nck1,
-                  int nck, int ntx, int nty, int nboxes, int chunk, int* err) {
+                  const __grid_constant__ CUtensorMap tdy, float* __restrict__ ws, int C1, int C2, int Cout, int H, int W,
+                  int nck1, int nck, int ntx, int nty, int nboxes, int chunk, int* err) {
     constexpr int ACCS = kWtAcc<NB>;
     constexpr uint32_t kCols = ACCS * NB;
     constexpr uint32_t kIdescT = (1u << 4) | (1u << 7) | (1u << 10) | (1u << 15) | (1u << 16) |
@@ -410,11 +412,27 @@ k_conv_wgrad_tile(const __grid_constant__ CUtensorMap tx1, const __grid_constant
             }
             __syncwarp();
         } else if (warp == 1) {
+            int bx = q0 % ntx, by = q0 / ntx % nty;  // the box's place in its image
             for (int kc = 0; kc < nk; ++kc) {
                 const int st = kc % WT_STAGES, use = kc / WT_STAGES;
                 if (!wait_parity_warp(saddr(full + st), (uint32_t)(use & 1))) {
                     ok = false;
                     break;
+                }
+                const int y1 = H - by * 8, x1 = W - bx * 8;  // rows and columns of the box inside the image
+                if (y1 < 8 || x1 < 8) {                      // (uniform)
+                    for (int p = lane; p < 128; p += 32) {   // 64 pixels of each tap, a row of 128 bytes each
+                        if ((p >> 3 & 7) < y1 && (p & 7) < x1) continue;
+                        uint4* row = (uint4*)(smem + st * WT_STAGE + p * 128);
+#pragma unroll
+                        for (int v = 0; v < 8; ++v) row[v] = make_uint4(0u, 0u, 0u, 0u);
+                    }
+                    asm volatile("fence.proxy.async.shared::cta;\n" ::: "memory");
+                    __syncwarp();
+                }
+                if (++bx == ntx) {
+                    bx = 0;
+                    if (++by == nty) by = 0;
                 }
                 asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
                 const uint32_t a = desc_lo_mn(saddr(smem + st * WT_STAGE), WT_BOX), b = a + ((2 * WT_BOX) >> 4);
@@ -631,7 +649,8 @@ int glnn_tile_wgrad(const void* dy, const void* x1, int c1, const void* x2, int 
         cudaFuncSetAttribute(k_conv_wgrad_tile<64>, cudaFuncAttributeMaxDynamicSharedMemorySize, WT_SMEM) == cudaSuccess;
     if (!ready) return 0;
     auto go = [&](auto kernel) {
-        kernel<<<grid, WT_THREADS, WT_SMEM, s>>>(t1, t2, td, ws, c1, c2, cout, nck1, nck, ntx, nty, n * ntx * nty, chunk, err);
+        kernel<<<grid, WT_THREADS, WT_SMEM, s>>>(t1, t2, td, ws, c1, c2, cout, h, w, nck1, nck, ntx, nty, n * ntx * nty,
+                                                   chunk, err);
         return 1;
     };
     return nb == 16 ? go(k_conv_wgrad_tile<16>) : (nb == 32 ? go(k_conv_wgrad_tile<32>) : go(k_conv_wgrad_tile<64>));

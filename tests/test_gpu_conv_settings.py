@@ -1,0 +1,63 @@
+"""The convolutions under the settings of glnn_set_conv_tma: tile kernels (2, the default)
+against the thread-gather and mma.sync kernels (0)."""
+import ctypes as C
+
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+torch = pytest.importorskip("torch")
+
+
+def _layer(setting, x1, x2, w, b, dy):
+    """y, dx1, dx2, dW, db of one layer (ReLU forward, dy as it is)."""
+    from svirl_gb300 import _lib
+    lib = _lib.load()
+    p = lambda t: None if t is None else C.c_void_p(t.data_ptr())  # noqa: E731
+    n, h, wd, c1 = x1.shape
+    c2, cout = 0 if x2 is None else x2.shape[3], w.shape[0]
+    dev = {"device": "cuda"}
+    err = torch.zeros(1, dtype=torch.int32, **dev)
+    wb, wt = [torch.empty(cout * 9 * (c1 + c2), dtype=torch.bfloat16, **dev) for _ in range(2)]
+    y = torch.empty((n, h, wd, cout), dtype=torch.bfloat16, **dev)
+    dx1, dx2 = torch.empty_like(x1), None if x2 is None else torch.empty_like(x2)
+    dw, db = torch.empty((cout, 3, 3, c1 + c2), **dev), torch.empty(cout, **dev)
+    nwork = lib.glnn_conv3x3_bwd_weight_work(n, h, wd, c1 + c2, cout)
+    work = torch.empty(nwork, **dev)
+    s = C.c_void_p(torch.cuda.current_stream().cuda_stream)
+    try:
+        assert lib.glnn_set_conv_tma(setting) == 0
+        assert lib.glnn_prep_weights(p(w), p(wb), p(wt), cout, c1 + c2, s) == 0
+        assert lib.glnn_conv3x3_fwd(p(x1), c1, p(x2), c2, p(wb), p(b), p(y), n, h, wd, cout, 1, p(err), s) == 0
+        assert lib.glnn_conv3x3_bwd_data(p(dy), p(y), 0, p(wt), p(dx1), c1, p(dx2), c2, n, h, wd, cout, p(err), s) == 0
+        assert lib.glnn_conv3x3_bwd_weight(p(dy), p(y), 0, p(x1), c1, p(x2), c2, p(dw), p(db), p(work), nwork, n, h, wd,
+                                           cout, p(err), s) == 0
+    finally:
+        lib.glnn_set_conv_tma(2)
+    assert int(err.item()) == 0
+    return y, dx1, dx2, dw, db
+
+
+def _inputs(shape, seed):
+    g = torch.Generator(device="cuda").manual_seed(seed)
+    n, h, w, c1, c2, cout = shape
+    r = lambda *s: torch.randn(s, generator=g, device="cuda")  # noqa: E731
+    return (r(n, h, w, c1).bfloat16(), r(n, h, w, c2).bfloat16() if c2 else None, 0.1 * r(cout, 3, 3, c1 + c2), r(cout),
+            r(n, h, w, cout).bfloat16())
+
+
+@pytest.mark.parametrize("shape", [(1, 1, 1, 8, 0, 8), (1, 17, 9, 8, 0, 32), (2, 31, 23, 64, 32, 32), (1, 12, 10, 96, 40, 64),
+                                   (1, 10, 10, 24, 0, 200), (1, 16, 13, 32, 0, 32), (1, 13, 16, 32, 0, 32)])
+def test_pixels_outside_the_image_add_nothing_to_the_weight_gradient(shape):
+    """Infinite activations on the image's last row and column: a weight gets an infinity or a
+    NaN exactly where a pixel of the image brings it one."""
+    x1, x2, w, b, dy = _inputs(shape, 11)
+    x1[:, -1, :, 0] = float("inf")
+    x1[:, :, -1, -1] = float("-inf")
+    if x2 is not None:
+        x2[:, -1, -1, 3] = float("inf")
+    got, ref = [_layer(s, x1, x2, w, b, dy)[3] for s in (2, 0)]
+    assert torch.equal(torch.isnan(got), torch.isnan(ref))
+    assert torch.equal(torch.where(torch.isinf(got), got, 0.0), torch.where(torch.isinf(ref), ref, 0.0))
+    f = torch.isfinite(ref)
+    assert torch.allclose(got[f], ref[f], rtol=0.0, atol=5e-3 * float(ref[f].abs().max()) if f.any() else 0.0)
