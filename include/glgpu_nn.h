@@ -44,15 +44,18 @@ int glnn_conv3x3_fwd(const void* x1, int32_t c1, const void* x2, int32_t c2, con
  * the epilogue of one tile under the MMAs of the next (c1, c2, cout multiples of 64; w
  * a multiple of 128 or a divisor of 128; h*w a multiple of 128).  1 = by TMA, one
  * output tile per CTA, for the latter shapes.  The thread gather otherwise;
- * 0 = always the thread gather.  Every setting computes the same values bitwise.
- * Nonzero also selects the tcgen05 weight gradient (0: the mma.sync one).
+ * 0 = always the thread gather.  Every setting computes the same values bitwise, but for
+ * the data gradient of the input-box kernel where cout is no multiple of 16: its K steps
+ * take one tap each there, so the FP32 sums are grouped differently before they are
+ * rounded to bfloat16.
+ * Weight gradient: see glnn_conv3x3_bwd_weight.
  * Process-wide. */
 int glnn_set_conv_tma(int32_t enable);
 /* [dx1|dx2] = conv3x3^T(dy * relu'(y), Wt), on tcgen05 like the forward.  y may be
  * NULL when relu = 0.  With relu = 0 and the shapes of the TMA forward (roles of
- * input and output channels exchanged) the operands are loaded by TMA (dy as the
- * 4-D activation tensor, Wt as the 3-D tensor [9][cin][cout]); else the threads
- * gather them (and apply the ReLU derivative).  Callers that have both gradients
+ * input and output channels exchanged; cout any multiple of 8) the operands are loaded
+ * by TMA (dy as the 4-D activation tensor, Wt as the 3-D tensor [9][cin][cout]); else
+ * the threads gather them (and apply the ReLU derivative).  Callers that have both gradients
  * to compute mask dy once with glnn_relu_mask and pass relu = 0. */
 int glnn_relu_mask(const void* dy, const void* y, void* out, int64_t count, void* stream); /* out = dy * (y > 0), bf16, count % 8 == 0 */
 int glnn_conv3x3_bwd_data(const void* dy, const void* y, int32_t relu, const void* wt, void* dx1, int32_t c1,
@@ -62,11 +65,12 @@ int glnn_conv3x3_bwd_data(const void* dy, const void* y, int32_t relu, const voi
 /* dW[cout][9*cin] and db[cout] (float32, overwritten) from dy * relu'(y) and
  * the input [x1|x2].  work: float32 scratch of glnn_conv3x3_bwd_weight_work()
  * floats, 16-byte aligned (split-K partial sums, reduced in a fixed order:
- * deterministic).  With glnn_set_conv_tma(1) and c1, c2, cout multiples of 64,
+ * deterministic).  With glnn_set_conv_tma(1) or (2) and c1, c2, cout multiples of 64,
  * w a multiple or a divisor of 64 and h*w a multiple of 64, it runs on tcgen05
  * (M = two taps x 64 input channels, N = 64 output channels, K = pixels, both
- * operands MN-major boxes loaded by TMA, FP32 accumulator in tensor memory); else
- * on mma.sync.  *err (a device int) is set to 1 if a CTA's bounded wait ran out
+ * operands MN-major boxes loaded by TMA, FP32 accumulator in tensor memory); with (2)
+ * the other shapes too (8 x 8-pixel boxes, N = 16, 32 or 64); else on mma.sync.  The
+ * kernels' sums are grouped differently: equal up to FP32 rounding.  *err (a device int) is set to 1 if a CTA's bounded wait ran out
  * (its partial sums are then NaN). */
 int64_t glnn_conv3x3_bwd_weight_work(int32_t n, int32_t h, int32_t w, int32_t cin, int32_t cout);
 int glnn_conv3x3_bwd_weight(const void* dy, const void* y, int32_t relu, const void* x1, int32_t c1, const void* x2,

@@ -61,3 +61,29 @@ def test_pixels_outside_the_image_add_nothing_to_the_weight_gradient(shape):
     assert torch.equal(torch.where(torch.isinf(got), got, 0.0), torch.where(torch.isinf(ref), ref, 0.0))
     f = torch.isfinite(ref)
     assert torch.allclose(got[f], ref[f], rtol=0.0, atol=5e-3 * float(ref[f].abs().max()) if f.any() else 0.0)
+
+
+@pytest.mark.parametrize("shape", [(1, 1, 1, 8, 0, 8), (2, 16, 8, 32, 0, 32), (1, 17, 9, 8, 0, 32), (2, 31, 23, 64, 32, 32),
+                                   (3, 24, 56, 16, 0, 48), (1, 9, 11, 128, 0, 128), (1, 20, 18, 128, 128, 128),
+                                   (1, 33, 7, 32, 16, 96), (24, 48, 40, 32, 0, 64), (2, 64, 64, 64, 0, 64),
+                                   (8, 128, 128, 32, 0, 8), (2, 64, 60, 32, 0, 72), (2, 40, 33, 40, 24, 24)])
+def test_settings_give_the_same_values(shape):
+    """The forward bit for bit; the data gradient too where cout is a multiple of 16 (a K
+    step of the tile kernel then holds the products that it holds in the gather kernel).
+    Elsewhere its FP32 sums are grouped differently: at most the rounding of the sums
+    (K = 9 cout terms, each side off by K 2^-24 times the terms' sum) and one rounding to
+    bfloat16 (2^-8 of a value, either side) apart."""
+    x1, x2, w, b, dy = _inputs(shape, 3)
+    tile, gather = [_layer(s, x1, x2, w, b, dy) for s in (2, 0)]
+    assert torch.equal(tile[0], gather[0])
+    cout = shape[5]
+    k = 9 * cout
+    terms = k * float(dy.float().abs().max()) * float(w.abs().max())
+    for t, g in zip(tile[1:3], gather[1:3]):
+        if t is None:
+            continue
+        if cout % 16 == 0:
+            assert torch.equal(t, g)
+        else:
+            t, g = t.float(), g.float()
+            assert bool(((t - g).abs() <= 2.0 ** -7 * g.abs().maximum(t.abs()) + 2 * k * 2.0 ** -24 * terms).all())
