@@ -34,7 +34,7 @@ extern "C" {
 #define GLGPU_E_ARG (-1)      /* bad argument (sizes, dtype, NULL) */
 #define GLGPU_E_CUDA (-2)     /* CUDA runtime error */
 #define GLGPU_E_OOM (-3)      /* device allocation failed */
-#define GLGPU_E_TIMEOUT (-4)  /* a device loop hit its iteration guard */
+#define GLGPU_E_TIMEOUT (-4)  /* a device loop hit its iteration guard, or a wait its limit */
 #define GLGPU_E_NAN (-5)      /* NaN residual seen (state still updated like the reference) */
 #define GLGPU_E_NOROOT (-6)   /* no real non-negative line-search root */
 
@@ -150,6 +150,13 @@ int glgpu_set_use_graphs(glgpu_handle* h, int32_t enable);
  * the loop also applies, so by default the guard fires only if that cap fails.
  * The reference's host loop has no guard. */
 int glgpu_set_loop_guard(glgpu_handle* h, int32_t launches);
+/* Safety net of the loops whose CTAs wait for one another (one cooperative launch per
+ * call or per Jacobi loop): polls of a barrier, about a microsecond each, after which a
+ * CTA gives up; the others then leave too and the call returns GLGPU_E_TIMEOUT without
+ * doing its remaining steps.  0 (the default) = 2^22.  After this error the order
+ * parameter, the vector potential and the Langevin seed are those of no one step: set
+ * them anew (the handle itself stays usable). */
+int glgpu_set_wait_limit(glgpu_handle* h, int32_t polls);
 
 /* --- timing (CUDA events on the handle's stream; no counterpart in the reference,
  *     which has no timing code: its profiler calls are commented out,
@@ -214,6 +221,7 @@ const char* glgpu_batch_last_error(const glgpu_batch* b);
 int glgpu_batch_td(glgpu_batch* b, double dt, int32_t Nt, int32_t eqn, glgpu_td_stats* stats, double* elapsed_ms);
 int glgpu_batch_set_use_graphs(glgpu_batch* b, int32_t enable);
 int glgpu_batch_set_loop_guard(glgpu_batch* b, int32_t launches);  /* as glgpu_set_loop_guard */
+int glgpu_batch_set_wait_limit(glgpu_batch* b, int32_t polls);     /* as glgpu_set_wait_limit, for every instance */
 /* Free-energy minimisation of every instance of the batch with the step
  * length, beta and stop test decided on the device (one graph launch for the
  * whole run).  No counterpart in the reference; each instance follows the

@@ -69,6 +69,7 @@ _SIGNATURES = {
     "glgpu_td": (C.c_int, [_H, C.c_double, C.c_int32, C.c_int32, C.POINTER(TDStats)]),
     "glgpu_set_use_graphs": (C.c_int, [_H, C.c_int32]),
     "glgpu_set_loop_guard": (C.c_int, [_H, C.c_int32]),
+    "glgpu_set_wait_limit": (C.c_int, [_H, C.c_int32]),
     "glgpu_td_timed": (C.c_int, [_H, C.c_double, C.c_int32, C.c_int32, C.POINTER(TDStats), C.POINTER(C.c_double)]),
     "glgpu_time_sweeps": (C.c_int, [_H, C.c_int32, C.c_int32, C.POINTER(C.c_double)]),
     "glgpu_free_energy": (C.c_int, [_H, C.POINTER(C.c_double)]),
@@ -90,6 +91,7 @@ _SIGNATURES = {
     "glgpu_batch_td": (C.c_int, [_H, C.c_double, C.c_int32, C.c_int32, C.POINTER(TDStats), C.POINTER(C.c_double)]),
     "glgpu_batch_set_use_graphs": (C.c_int, [_H, C.c_int32]),
     "glgpu_batch_set_loop_guard": (C.c_int, [_H, C.c_int32]),
+    "glgpu_batch_set_wait_limit": (C.c_int, [_H, C.c_int32]),
     "glgpu_batch_set_energy_targets": (C.c_int, [_H, _P, C.c_double]),
     "glgpu_batch_set_cg_window": (C.c_int, [_H, C.c_int32, C.c_double]),
     "glgpu_batch_cg": (C.c_int, [_H, C.c_int32, C.c_double, C.c_double, C.c_int32, C.POINTER(C.c_int32), C.POINTER(C.c_double),
@@ -292,6 +294,10 @@ class Handle:
 
     def set_loop_guard(self, launches):
         check(self.lib.glgpu_set_loop_guard(self.h, int(launches)), self.h, "set_loop_guard")
+
+    def set_wait_limit(self, polls):
+        """Polls of a barrier between CTAs before a time loop gives up (0: the default of 2^22)."""
+        check(self.lib.glgpu_set_wait_limit(self.h, int(polls)), self.h, "set_wait_limit")
 
     # TD ------------------------------------------------------------------------
     def td(self, dt, Nt, eqn=0):

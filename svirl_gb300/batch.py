@@ -76,6 +76,10 @@ class HandleBatch:
         """Jacobi loop guard in sweep launches (0: the default of 1088)."""
         self._check(self.lib.glgpu_batch_set_loop_guard(self.b, int(launches)), "set_loop_guard")
 
+    def set_wait_limit(self, polls):
+        """As ``Handle.set_wait_limit``, for every instance."""
+        self._check(self.lib.glgpu_batch_set_wait_limit(self.b, int(polls)), "set_wait_limit")
+
     def td_raw(self, dt, Nt, eqn=0, timed=False):
         """``glgpu_batch_td``: eqn 0 = both equations, 1 = psi only, 2 = A only."""
         st = _lib.TDStats()

@@ -346,6 +346,13 @@ int glgpu_set_loop_guard(glgpu_handle* h, int32_t launches) {
     return GLGPU_OK;
 }
 
+int glgpu_set_wait_limit(glgpu_handle* h, int32_t polls) {
+    if (check_handle(h)) return GLGPU_E_ARG;
+    if (polls < 0) return set_error(h, GLGPU_E_ARG, "set_wait_limit: polls must be >= 0");
+    h->wait_limit = polls;
+    return GLGPU_OK;
+}
+
 static void drop_td_graphs(glgpu_handle* h) {
     for (int q = 0; q < kTDGraphs; ++q)
         if (h->td_exec[q]) {
@@ -661,6 +668,13 @@ int glgpu_batch_set_loop_guard(glgpu_batch* b, int32_t launches) {
     if (!b) return GLGPU_E_ARG;
     if (launches < 0) return batch_error(b, GLGPU_E_ARG, "batch_set_loop_guard: launches must be >= 0");
     b->loop_guard = launches;
+    return GLGPU_OK;
+}
+
+int glgpu_batch_set_wait_limit(glgpu_batch* b, int32_t polls) {
+    if (!b) return GLGPU_E_ARG;
+    if (polls < 0) return batch_error(b, GLGPU_E_ARG, "batch_set_wait_limit: polls must be >= 0");
+    b->wait_limit = polls;
     return GLGPU_OK;
 }
 

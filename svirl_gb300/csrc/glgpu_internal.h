@@ -113,14 +113,15 @@ struct LoopState {
     int ninst;
     long long total_launches;  // sweep kernel launches (psi and A) in the current call
     int guard;                // launches after which a Jacobi loop is stopped with kErrLoopGuard
-    unsigned arrived, round;  // cooperative Jacobi loop (grid_round): CTAs arrived; 2 x finished sweeps + go on
+    unsigned arrived, round;  // cooperative Jacobi loop (end_round): CTAs arrived; 2 x finished rounds + go on
+    unsigned spins;           // polls of a barrier between CTAs before one gives up (kErrBarrier)
 };
 
 constexpr int kErrLoopGuard = 1;
 constexpr int kErrCopyWait = 2;  // a wait for a bulk copy into shared memory ran out (psi sweep)
-constexpr int kErrBarrier = 4;   // a wait at an instance's barrier ran out (resident time loop)
+constexpr int kErrBarrier = 4;   // a wait at a barrier between CTAs ran out (cooperative loops)
 
-// Polls of a barrier between CTAs before one gives up (about a microsecond each: seconds).
+// LoopState::spins by default (a poll takes about a microsecond: seconds).
 constexpr unsigned kBarrierSpins = 1u << 22;
 
 // Resident time loop (tdr.cu).  An instance's barrier: CTAs arrived so far in the
@@ -261,6 +262,7 @@ struct glgpu_handle {
     bool td_graph_failed = false;
     bool use_graphs = true;
     int loop_guard = 0;                 // Jacobi loop guard in sweep launches (0: kLoopGuard)
+    int wait_limit = 0;                 // polls of a barrier between CTAs (0: kBarrierSpins)
     int psi_select = 0;                 // psi sweep kernel (bulk_selected)
     int psi_scheme = 0;                 // psi time stepping: 0 backward Euler, 1 Crank-Nicolson, 2 as written
     std::string last_error;
@@ -303,6 +305,7 @@ struct glgpu_batch {
     cudaGraphExec_t td_exec[glgpu::kTDGraphs] = {};
     bool td_graph_failed = false, use_graphs = true;
     int loop_guard = 0;                  // Jacobi loop guard in sweep launches (0: kLoopGuard)
+    int wait_limit = 0;                  // polls of a barrier between CTAs (0: kBarrierSpins)
     // batched device CG (allocated on first use)
     void* cg_tiles = nullptr;            // CG tile table (larger tiles than the TD one)
     int cg_ntiles = 0;

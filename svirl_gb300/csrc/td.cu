@@ -906,9 +906,10 @@ k_fv_A(const Inst* __restrict__ insts, const Tile* __restrict__ tiles, int post)
 __global__ void k_loop_begin(const Inst* __restrict__ insts, int ninst, LoopState* loop,
                              cudaGraphConditionalHandle cond, int use_cond, int which) {
     int active = 0;
+    const bool cut = (loop->err & kErrBarrier) != 0;  // a loop of this call was given up: no further one runs
     for (int q = threadIdx.x; q < ninst; q += blockDim.x) {
         InstState* st = insts[q].st;
-        const bool part = which == 0 || insts[q].solveA;
+        const bool part = !cut && (which == 0 || insts[q].solveA);
         st->sweep = 0;
         st->done = part ? 0 : 1;
         if (which == 1) st->commitA = 0;
@@ -965,9 +966,14 @@ __global__ void __launch_bounds__(kThreads) k_A_commit(const Inst* __restrict__ 
     }
 }
 
-// End of a time step: count it and decide whether the time loop goes on.
+// End of a time step: count it and decide whether the time loop goes on (not after a
+// barrier wait that ran out: that step's loops are unfinished).
 __global__ void k_step_end(const Inst* __restrict__ insts, int ninst, LoopState* loop,
                            cudaGraphConditionalHandle cond, int use_cond) {
+    if (loop->err & kErrBarrier) {
+        if (threadIdx.x == 0 && use_cond) cudaGraphSetConditional(cond, 0u);
+        return;
+    }
     for (int q = threadIdx.x; q < ninst; q += blockDim.x) insts[q].st->steps += 1;
     if (threadIdx.x == 0) {
         int s = loop->step + 1;
@@ -1392,6 +1398,7 @@ __global__ void k_bench_prep(const Inst* __restrict__ insts, int ninst, LoopStat
         loop->arrived = 0u;
         loop->round = 0u;
         loop->guard = 1;
+        loop->spins = kBarrierSpins;
         loop->cont = 1;
     }
 }
@@ -1401,7 +1408,7 @@ __global__ void k_bench_prep(const Inst* __restrict__ insts, int ninst, LoopStat
 // the time loop's state for a call of Nt steps.  One launch where the copies, the memset and
 // a kernel took four operations of the stream, as did the end (65^2, 5 steps, states set and read: 163 -> 153 us).
 __global__ void k_call_begin(const Inst* host, Inst* __restrict__ insts, int ninst, ResGroup* groups, LoopState* loop, int Nt,
-                             int guard) {
+                             int guard, int wait_limit) {
     static_assert(sizeof(Inst) % 8 == 0 && sizeof(ResGroup) % 8 == 0, "copied in 8-byte words");
     if (loop && blockIdx.x == 0 && threadIdx.x == 0) {
         LoopState ls;
@@ -1409,6 +1416,7 @@ __global__ void k_call_begin(const Inst* host, Inst* __restrict__ insts, int nin
         ls.Nt = Nt;
         ls.ninst = ninst;
         ls.guard = guard;
+        ls.spins = wait_limit > 0 ? (unsigned)wait_limit : kBarrierSpins;
         *loop = ls;
     }
     const int q = blockIdx.x;
@@ -1554,11 +1562,11 @@ struct TDOutcome {
 // insts_host, gather_host and hl_pinned: pinned host memory, which the call's first and last
 // kernels read and write
 static TDOutcome td_core(cudaStream_t s, const TDLaunch& L, int Nt, int eqn, cudaGraphExec_t* execs, bool* graph_failed,
-                         bool use_graphs, int guard, bool timed, const Inst* insts_host, Inst* insts_dev,
+                         bool use_graphs, int guard, int wait_limit, bool timed, const Inst* insts_host, Inst* insts_dev,
                          InstState* gather_host, LoopState* hl_pinned) {
     TDOutcome o = {cudaSuccess, 0, 0, 0, 0.f, 0};
     k_call_begin<<<L.ninst, 128, 0, s>>>(insts_host, insts_dev, L.ninst, L.res ? L.res->groups : nullptr,
-                                         Nt > 0 ? L.loop : nullptr, Nt, guard > 0 ? guard : kLoopGuard);
+                                         Nt > 0 ? L.loop : nullptr, Nt, guard > 0 ? guard : kLoopGuard, wait_limit);
     o.err = cudaGetLastError();
     if (o.err != cudaSuccess) return o;
     cudaEvent_t ev0 = nullptr, ev1 = nullptr;
@@ -1663,7 +1671,7 @@ int td_run(glgpu_handle* h, double dt, int Nt, int eqn, glgpu_td_stats* stats, d
     L.nwork = h->dtype == 8 ? h->ntiles : h->nlitems;
     L.loop_grid = resident || h->psi_scheme != 0 || bulk_selected(h) ? 0 : psi_loop_grid(h->dtype, L.nwork);
     TDOutcome o = td_core(h->stream, L, Nt, eqn, h->td_exec, &h->td_graph_failed, h->use_graphs, h->loop_guard,
-                          elapsed_ms != nullptr,
+                          h->wait_limit, elapsed_ms != nullptr,
                           &ps->inst, h->inst, &ps->st, &ps->loop);
     const InstState hs = ps->st;
     if (o.err != cudaSuccess) return cuda_check(h, o.err, "td");
@@ -1713,7 +1721,7 @@ int batch_td(glgpu_batch* b, double dt, int Nt, int eqn, glgpu_td_stats* stats, 
     L.nwork = b->dtype == 8 ? b->ntiles : b->nlitems;
     L.loop_grid = resident ? 0 : psi_loop_grid(b->dtype, L.nwork);
     TDOutcome o = td_core(b->stream, L, Nt, eqn, b->td_exec, &b->td_graph_failed, b->use_graphs, b->loop_guard,
-                          elapsed_ms != nullptr,
+                          b->wait_limit, elapsed_ms != nullptr,
                           b->insts_pin, b->insts, b->gather_pin, b->loop_pin);
     if (o.err == cudaSuccess) memcpy(b->gather_h.data(), b->gather_pin, sizeof(InstState) * (size_t)b->ninst);
     if (o.err != cudaSuccess) return batch_error(b, GLGPU_E_CUDA, std::string("batch_td: ") + cudaGetErrorString(o.err));

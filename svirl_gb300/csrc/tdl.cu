@@ -63,10 +63,11 @@ __device__ __forceinline__ bool end_round(const Inst* insts, int ninst, LoopStat
         }
     } else if (threadIdx.x == 0) {
         unsigned word, it = 0;
+        const unsigned spins = *(volatile const unsigned*)&loop->spins;
         for (;;) {
             asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(word) : "l"(&loop->round) : "memory");
             if (word >> 1 == (unsigned)seq) break;
-            if (++it >= kBarrierSpins || ((it & 1023u) == 0u && (*(volatile int*)&loop->err & kErrBarrier))) {
+            if (++it >= spins || ((it & 1023u) == 0u && (*(volatile int*)&loop->err & kErrBarrier))) {
                 atomicOr(&loop->err, kErrBarrier);
                 word = 0u;
                 break;

@@ -69,10 +69,11 @@ __device__ __forceinline__ bool res_barrier(ResGroup* g, unsigned& target, unsig
         __threadfence();
         atomicAdd(&g->arrived, 1u);
         unsigned seen, it = 0;
+        const unsigned spins = *(volatile const unsigned*)&loop->spins;
         for (;;) {
             asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(seen) : "l"(&g->arrived) : "memory");
             if ((int)(seen - target) >= 0) break;
-            if (++it >= kBarrierSpins || ((it & 1023u) == 0u && (*(volatile int*)&loop->err & kErrBarrier))) {
+            if (++it >= spins || ((it & 1023u) == 0u && (*(volatile int*)&loop->err & kErrBarrier))) {
                 atomicOr(&loop->err, kErrBarrier);
                 s_broken = 1;
                 break;
