@@ -61,19 +61,36 @@ template <int BX, int BY, int R, int K, int KA> struct ResShape {
 };
 
 // One round of the instance's barrier: everything this CTA wrote is visible to the
-// CTAs that pass it.  false: the wait ran out (or another CTA's did).
-__device__ __forceinline__ bool res_barrier(ResGroup* g, unsigned& target, unsigned ncta, LoopState* loop, int& s_broken) {
+// CTAs that pass it.  false: the wait ran out (or another CTA's did).  Where instances run
+// in waves (`more`), the first barrier of an instance waits for CTAs that may have most of
+// another instance's call before them, as long as any call: that wait runs out only when
+// nothing has arrived at any instance's barrier during `spins` polls.
+__device__ __forceinline__ bool res_barrier(ResGroup* g, unsigned& target, unsigned ncta, LoopState* loop, const ResGroup* groups,
+                                            int more, int& s_broken) {
     __syncthreads();
     if (threadIdx.x == 0) {
+        const bool patient = more && target == 0u;
         target += ncta;
         __threadfence();
         atomicAdd(&g->arrived, 1u);
-        unsigned seen, it = 0;
+        unsigned seen, it = 0, progress = 0;
         const unsigned spins = *(volatile const unsigned*)&loop->spins;
         for (;;) {
             asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(seen) : "l"(&g->arrived) : "memory");
             if ((int)(seen - target) >= 0) break;
-            if (++it >= spins || ((it & 1023u) == 0u && (*(volatile int*)&loop->err & kErrBarrier))) {
+            if (++it >= spins || (it & 1023u) == 0u) {
+                const bool cut = (*(volatile int*)&loop->err & kErrBarrier) != 0;
+                if (!cut) {
+                    if (it < spins) continue;
+                    unsigned all = 0;
+#pragma unroll 1
+                    for (int q = patient ? loop->ninst : 0; q-- > 0;) all += *(volatile unsigned*)&groups[q].arrived;
+                    if (all != progress) {
+                        progress = all;
+                        it = 0;
+                        continue;
+                    }
+                }
                 atomicOr(&loop->err, kErrBarrier);
                 s_broken = 1;
                 break;
@@ -238,7 +255,7 @@ k_td_resident(const Inst* __restrict__ insts, const ResTile* __restrict__ tiles,
                     U[2 * node(r)] = va;
                     U[2 * node(r) + 1] = vb;
                 }
-            if (!res_barrier(grp, target, ncta, loop, sm.broken)) return false;
+            if (!res_barrier(grp, target, ncta, loop, groups, more, sm.broken)) return false;
             ud0 = z;
 #pragma unroll
             for (int r = 0; r < R; ++r) {
@@ -375,7 +392,7 @@ k_td_resident(const Inst* __restrict__ insts, const ResTile* __restrict__ tiles,
                         store_rim(&sp[l][0][0], out + (l - 1) * SLOT);
                     }
                     post_round(K);
-                    if (!(ok = res_barrier(grp, target, ncta, loop, sm.broken))) break;
+                    if (!(ok = res_barrier(grp, target, ncta, loop, groups, more, sm.broken))) break;
                     fetch_round(K);
                     const C2<T>* const in = scratch + (size_t)flip * K * SLOT;
 #pragma unroll
@@ -506,7 +523,7 @@ k_td_resident(const Inst* __restrict__ insts, const ResTile* __restrict__ tiles,
                     }
                     store_rim(&sp[1 + KA][0][0], mine + (2 * K + flipA) * SLOT);
                     post_round(KA);
-                    if (!(ok = res_barrier(grp, target, ncta, loop, sm.broken))) break;
+                    if (!(ok = res_barrier(grp, target, ncta, loop, groups, more, sm.broken))) break;
                     fetch_round(KA);
                     const C2<T>* const in = scratch + (2 * K + flipA) * SLOT;
 #pragma unroll
@@ -554,7 +571,7 @@ k_td_resident(const Inst* __restrict__ insts, const ResTile* __restrict__ tiles,
                 if (do_psi) {
                     ok = refresh_links(a0, b0);
                 } else {
-                    ok = res_barrier(grp, target, ncta, loop, sm.broken);
+                    ok = res_barrier(grp, target, ncta, loop, groups, more, sm.broken);
                     ud0 = z;
 #pragma unroll
                     for (int r = 0; r < R; ++r) ua[r] = ub[r] = ul[r] = z;
@@ -582,7 +599,7 @@ k_td_resident(const Inst* __restrict__ insts, const ResTile* __restrict__ tiles,
             }
         }
         // a CTA's exchange slots are free for its next instance once all have read them
-        if (more && ok) ok = res_barrier(grp, target, ncta, loop, sm.broken);
+        if (more && ok) ok = res_barrier(grp, target, ncta, loop, groups, more, sm.broken);
         __syncthreads();
         if (sm.broken) return;
     }

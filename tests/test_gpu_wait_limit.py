@@ -71,3 +71,34 @@ def test_wait_limit_of_a_batch(sizes):
     with pytest.raises(GLGPUError):
         batch.set_wait_limit(-1)
     batch.close()
+
+
+def test_a_film_waits_for_the_films_before_it():
+    """Films in waves, of which one takes many sweeps a step and its neighbours one: their
+    CTAs wait at the next film's first barrier for nearly the whole call, far beyond the
+    limit of a wait inside a film, and the call is none the worse for it."""
+    from svirl_gb300.batch import HandleBatch
+    # tiles of 58 x 26: 36 (random start), 260 (uniform, at rest in zero field: a sweep a step), 288
+    shapes, steps, polls = [(348, 156), (754, 520), (696, 624)], 1500, 4000
+
+    def films():
+        out = []
+        for q, (nx, ny) in enumerate(shapes):
+            g = make_pair(Nx=nx, Ny=ny, dx=0.5, dy=0.5, sigma=150.0, H=0.0 if q else 0.3, kappa=np.inf, seed=q, dtype=np.float32)[0]
+            if q:
+                g._h.set_psi(np.ones(nx * ny, dtype=np.complex64))
+            out.append(g)
+        return out
+
+    gls, refs = films(), films()
+    batch = HandleBatch([g._h for g in gls])
+    batch.set_wait_limit(polls)
+    st, ms = batch.td_raw(0.1, steps, timed=True)
+    assert st.sweep_launches == 1 and st.steps == steps
+    for g, r in zip(gls, refs):
+        r._h.td(0.1, steps, 0)
+        assert _same(g, r)
+    # the wait: the first film's time but for the second's, a poll being a microsecond or less
+    alone = [r._h.td_timed(0.1, 100, 0)[1] * steps / 100 for r in refs]
+    assert alone[0] - alone[1] > 2e-3 * polls, alone
+    batch.close()
