@@ -347,6 +347,7 @@ int psi_loop_grid(int dtype, int n);
 constexpr int kWideCols = 56, kACols = 60;  // output columns of an FP32 item of the psi loop, of the A loop
 int choose_loop_rows(const Geo* const* geos, int n);
 int choose_A_rows(const Geo* const* geos, int n);
+double loops_step_us(const Geo* const* geos, int n, bool any_A);
 void add_loop_items(std::vector<Item>& items, const Geo& g, int inst, int rows, int cols);
 const void* A_loop_fn();  // the cooperative A loop (FP32), its CTAs over n items
 int A_loop_grid(int n);

@@ -611,12 +611,12 @@ k_td_resident(const Inst* __restrict__ insts, const ResTile* __restrict__ tiles,
 
 struct ResCfg {
     int dtype, nt, iw, ih, nodes, K, smem, most;  // nodes: of a tile, with its halo
-    bool waves;
+    double wave_us;  // a time step of a film among films in waves (0: the shape takes no waves)
     size_t scratch;  // exchange slots of a CTA, bytes
     void* fn;
 };
-template <typename T, class S, int MINB> static ResCfg res_cfg(int most, bool waves) {
-    return ResCfg{(int)sizeof(T), S::NT, S::IW, S::IH, S::kBX * S::H, S::kK, (int)sizeof(ResSmem<T, S>), most, waves,
+template <typename T, class S, int MINB> static ResCfg res_cfg(int most, double wave_us) {
+    return ResCfg{(int)sizeof(T), S::NT, S::IW, S::IH, S::kBX * S::H, S::kK, (int)sizeof(ResSmem<T, S>), most, wave_us,
                   sizeof(C2<T>) * S::kSlots * S::SLOT, (void*)k_td_resident<T, S, MINB>};
 }
 // Shapes in the order they are tried.  A single FP32 domain takes the first in which it
@@ -624,8 +624,9 @@ template <typename T, class S, int MINB> static ResCfg res_cfg(int most, bool wa
 // res_sweep_us finds fastest: small tiles with many
 // sweeps per round, where the barrier and the halo's way through L2 (2.6 us a round)
 // are most of a step, then larger ones.  Batches whose tiles do not all fit run in
-// waves on a shape marked `waves`.  Measured, us per time step (22 psi sweeps), by the
-// launch-per-sweep loop and by the shapes here (own nodes per tile):
+// waves on a shape with a wave_us, or in the loops of tdl.cu (res_schedule).  Measured, us
+// per time step (22 psi sweeps), by the launch-per-sweep loop and by the shapes here (own
+// nodes per tile):
 //   FP32, kappa = inf:  129^2 145, 16x16 19;  513^2 164, 58x26 52;  700^2 172, 60x60 72
 //   FP32, kappa = 4:    257^2 22x22 39 (16x16 42);  385^2 250, 24x24 53 (58x26 55);
 //                       449^2 58x26 56, two CTAs per SM 73
@@ -635,17 +636,17 @@ template <typename T, class S, int MINB> static ResCfg res_cfg(int most, bool wa
 //   (60x60: 16.0)
 static const ResCfg* res_cfgs(int* n) {
     static const ResCfg c[] = {
-        res_cfg<float, ResShape<32, 16, 2, 8, 4>, 2>(240, false),   // 16 x 16
-        res_cfg<float, ResShape<32, 8, 4, 5, 4>, 2>(0, false),      // 22 x 22
-        res_cfg<float, ResShape<32, 8, 4, 4, 4>, 2>(0, false),      // 24 x 24
-        res_cfg<float, ResShape<64, 8, 4, 3, 2>, 1>(0, false),      // 58 x 26, a CTA per SM (128 registers)
-        res_cfg<float, ResShape<64, 8, 4, 3, 2>, 2>(0, true),       // 58 x 26, two (64 registers, spills)
-        res_cfg<float, ResShape<64, 8, 8, 2, 2>, 1>(0, true),       // 60 x 60
-        res_cfg<double, ResShape<16, 16, 1, 2, 1>, 2>(230, false),  // 12 x 12
-        res_cfg<double, ResShape<32, 8, 2, 2, 1>, 2>(0, false),     // 28 x 12
-        res_cfg<double, ResShape<32, 16, 2, 2, 1>, 1>(0, false),    // 28 x 28
-        res_cfg<double, ResShape<64, 4, 4, 1, 1>, 2>(0, false),     // 62 x 14
-        res_cfg<double, ResShape<64, 8, 4, 1, 1>, 1>(0, false),     // 62 x 30
+        res_cfg<float, ResShape<32, 16, 2, 8, 4>, 2>(240, 0.0),   // 16 x 16
+        res_cfg<float, ResShape<32, 8, 4, 5, 4>, 2>(0, 0.0),      // 22 x 22
+        res_cfg<float, ResShape<32, 8, 4, 4, 4>, 2>(0, 0.0),      // 24 x 24
+        res_cfg<float, ResShape<64, 8, 4, 3, 2>, 1>(0, 0.0),      // 58 x 26, a CTA per SM (128 registers)
+        res_cfg<float, ResShape<64, 8, 4, 3, 2>, 2>(0, 49.0),     // 58 x 26, two (64 registers, spills)
+        res_cfg<float, ResShape<64, 8, 8, 2, 2>, 1>(0, 66.0),     // 60 x 60
+        res_cfg<double, ResShape<16, 16, 1, 2, 1>, 2>(230, 0.0),  // 12 x 12
+        res_cfg<double, ResShape<32, 8, 2, 2, 1>, 2>(0, 0.0),     // 28 x 12
+        res_cfg<double, ResShape<32, 16, 2, 2, 1>, 1>(0, 0.0),    // 28 x 28
+        res_cfg<double, ResShape<64, 4, 4, 1, 1>, 2>(0, 0.0),     // 62 x 14
+        res_cfg<double, ResShape<64, 8, 4, 1, 1>, 1>(0, 0.0),     // 62 x 30
     };
     *n = (int)(sizeof(c) / sizeof(c[0]));
     return c;
@@ -669,7 +670,14 @@ static int res_tiles_of(const ResCfg& c, const Geo& g) {
 // 1.8 times as long.  Instances start in one order, the same in every CTA's list, so
 // the first unfinished instance always has all its CTAs at work or on the way to it,
 // and no barrier waits for a CTA that waits for another.
-// false: no shape takes the call.
+// Waves or the loops of tdl.cu: a film in a wave takes wave_us a step whatever share of the
+// CTAs it uses, so large films (two of 512^2 do not fit together) lose in waves and small ones
+// gain, and A costs more there.  us per step, waves / loops: 2 films of 512^2 95 / 166, 4:
+// 200 / 207, 8: 375 / 314, 16: 796 / 523; kappa = 4: 171 / 239, 360 / 315, 678 / 473, 1358 /
+// 803; 200 of 128^2 482 / 595, kappa = 4 900 / 883; 32 of 65 .. 496, mixed kappa, 520 / 609.
+// (0.95: near the line the estimates are as far off, and films in waves do not wait for the
+// one with the most sweeps.)
+// false: no shape takes the call, or the loops are expected to be faster.
 static bool res_schedule(int dtype, glgpu_handle* const* hs, int n, ResPlan* plan) {
     int nc = 0, dev = 0, sms = 0, coop = 0;
     const ResCfg* cs = res_cfgs(&nc);
@@ -679,6 +687,7 @@ static bool res_schedule(int dtype, glgpu_handle* const* hs, int n, ResPlan* pla
     if (!coop) return false;
     int best = -1, best_cap = 0;
     double best_us = 0.0;
+    bool in_waves = false;
     for (int c = 0; c < nc; ++c) {
         if (cs[c].dtype != dtype) continue;
         int per = 0;
@@ -694,12 +703,13 @@ static bool res_schedule(int dtype, glgpu_handle* const* hs, int n, ResPlan* pla
             largest = std::max(largest, t);
         }
         const bool fits = all <= (cs[c].most > 0 ? std::min(cs[c].most, cap) : cap);
-        if (!fits && !(n > 1 && cs[c].waves && largest <= cap)) continue;
+        if (!fits && !(n > 1 && cs[c].wave_us > 0.0 && largest <= cap)) continue;
         const double us = res_sweep_us(cs[c], all, sms);
         if (best >= 0 && us >= best_us) continue;
         best = c;
         best_cap = cap;
         best_us = us;
+        in_waves = !fits;
         if (dtype == 4) break;  // in order
     }
     if (best < 0) return false;
@@ -744,6 +754,15 @@ static bool res_schedule(int dtype, glgpu_handle* const* hs, int n, ResPlan* pla
             busy[ctas[t]] = now + (hs[q]->inst_h.solveA ? 1.8 : 1.0);
         }
         plan->owner.insert(plan->owner.end(), ctas.begin(), ctas.begin() + nt);
+    }
+    if (in_waves) {
+        std::vector<const Geo*> geos(n);
+        bool any_A = false;
+        for (int q = 0; q < n; ++q) {
+            geos[q] = &hs[q]->g;
+            any_A = any_A || hs[q]->inst_h.solveA != 0;
+        }
+        if (loops_step_us(geos.data(), n, any_A) < 0.95 * c.wave_us * *std::max_element(busy.begin(), busy.end())) return false;
     }
     plan->first.assign(1, 0);
     for (int k = 0; k < grid; ++k) {
