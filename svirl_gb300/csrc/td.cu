@@ -1638,16 +1638,16 @@ static void fill_stats(glgpu_td_stats* stats, const InstState* hs, int n, const 
     }
 }
 
-// The resident loop runs backward Euler with the default sweep kernel selection; the
-// fixed-vortex steps, the Crank-Nicolson schemes, a loop guard in launches and the
-// host-driven loop keep a launch per sweep.
+// The resident loop runs backward Euler; the fixed-vortex steps, the Crank-Nicolson
+// schemes, a loop guard in launches and the host-driven loop keep a launch per Jacobi loop
+// or sweep, as does a single handle for which the bulk-copy sweep is selected.
 static bool resident_ok(const glgpu_handle* h, bool use_graphs, int guard) {
-    return use_graphs && guard == 0 && h->psi_scheme == 0 && h->psi_select == 0 && !h->vpi && h->lock_n == 0;
+    return use_graphs && guard == 0 && h->psi_scheme == 0 && !h->vpi && h->lock_n == 0;
 }
 
 int td_run(glgpu_handle* h, double dt, int Nt, int eqn, glgpu_td_stats* stats, double* elapsed_ms) {
     if (eqn < 0 || eqn > 2 || Nt < 0) return set_error(h, GLGPU_E_ARG, "glgpu_td: bad eqn or Nt");
-    const bool resident = Nt > 0 && resident_ok(h, h->use_graphs, h->loop_guard) && res_prepare(&h->res, &h, 1);
+    const bool resident = Nt > 0 && resident_ok(h, h->use_graphs, h->loop_guard) && !bulk_selected(h) && res_prepare(&h->res, &h, 1);
     // dt of the order-parameter iterator; the A kernel also receives it (td.py:278)
     h->inst_h.dt = dt;
     h->inst_h.fdt = (float)dt;

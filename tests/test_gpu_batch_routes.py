@@ -27,3 +27,19 @@ def test_waves_or_loops(sizes, kappas, waves):
         b._h.td(0.1, 2, 0)
         assert all(np.array_equal(x, y) for x, y in zip(gpu_state(a), gpu_state(b)))
     batch.close()
+
+
+def test_selected_sweep_kernel_concerns_fp32_handles_alone():
+    """The bulk-copy sweep exists in FP32 and for single handles: selecting it changes the
+    route of nothing else."""
+    from svirl_gb300.batch import HandleBatch
+    for dtype, launch in ((np.float64, True), (np.float32, False)):
+        gl = make_pair(Nx=97, Ny=64, H=0.2, dtype=dtype)[0]
+        assert gl._h.td(0.1, 2).sweep_launches == 1
+        gl._h.set_psi_sweep_kernel(1)
+        assert (gl._h.td(0.1, 2).sweep_launches == 1) == launch
+    films = _films((64, 97), (np.inf, 4.0))
+    films[0]._h.set_psi_sweep_kernel(1)
+    batch = HandleBatch([g._h for g in films])
+    assert batch.td_raw(0.1, 2).sweep_launches == 1
+    batch.close()
