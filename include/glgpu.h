@@ -100,6 +100,9 @@ int glgpu_set_psi_strip_rows(glgpu_handle* h, int32_t rows);
  * (TMA), four strips per CTA, measured slower on GB300 (172 us per launch against 59 for
  * three sweeps on the 2049^2 workload).  Both compute the same values bitwise. */
 int glgpu_set_psi_sweep_kernel(glgpu_handle* h, int32_t select);
+/* 1: with the present settings glgpu_td runs the whole call as one launch with the state
+ * on chip, and no psi sweep kernel at all, unless kernel 1 is selected; 0: it does not. */
+int glgpu_td_resident(glgpu_handle* h);
 /* Time stepping of the order parameter: 0 (default) = backward Euler, the
  * reference's scheme (svirl/cuda/td.h:4-133); 1 = Crank-Nicolson of the
  * reference's commented-out kernel (iterate_order_parameter_jacobi_step_CN,

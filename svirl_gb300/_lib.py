@@ -50,6 +50,7 @@ _SIGNATURES = {
     "glgpu_psi_strip_rows": (C.c_int, [_H]),
     "glgpu_set_psi_strip_rows": (C.c_int, [_H, C.c_int32]),
     "glgpu_set_psi_sweep_kernel": (C.c_int, [_H, C.c_int32]),
+    "glgpu_td_resident": (C.c_int, [_H]),
     "glgpu_set_psi_scheme": (C.c_int, [_H, C.c_int32]),
     "glgpu_set_irregular_vector_potential": (C.c_int, [_H, _P, C.c_int32]),
     "glgpu_get_irregular_vector_potential": (C.c_int, [_H, _P]),
@@ -286,8 +287,12 @@ class Handle:
         check(self.lib.glgpu_set_psi_scheme(self.h, int(scheme)), self.h, "set_psi_scheme")
 
     def set_psi_sweep_kernel(self, select):
-        """FP32 psi sweep kernel: 0 = register strip (default), 1 = bulk-copy ring."""
+        """FP32 psi sweep kernel: 0 = cooperative loop (default), 1 = bulk-copy ring."""
         check(self.lib.glgpu_set_psi_sweep_kernel(self.h, int(select)), self.h, "set_psi_sweep_kernel")
+
+    def td_resident(self):
+        """Whether TD calls run as one launch with the state on chip (unless sweep kernel 1 is selected)."""
+        return int(self.lib.glgpu_td_resident(self.h)) == 1
 
     def set_use_graphs(self, enable):
         check(self.lib.glgpu_set_use_graphs(self.h, 1 if enable else 0), self.h, "set_use_graphs")

@@ -6,10 +6,12 @@ height follows from the size) and the bulk-copy ring, compiled for the heights i
 for the ring the height an item-count model picks.  ``tune(handle)`` measures instead:
 it times one sweep launch (``glgpu_time_sweeps``: CUDA events, L2 flushed
 before each launch) for every (kernel, height) pair, applies the fastest, and
-stores it in a JSON cache keyed by (dtype, Nx, Ny, kappa finite), so that later
-handles with the same key take the stored choice without measuring.  Results
-do not depend on the choice: every pair computes the same values bitwise
-(tests/test_gpu_strip_rows.py, tests/test_gpu_psi_kernels.py).
+stores it in a JSON cache keyed by (dtype, Nx, Ny, kappa finite, kernel set), so that
+later handles with the same key take the stored choice without measuring.  (The heights
+make no difference to kernel 0.)  Domains that fit on chip run no sweep kernel but the
+resident loop, which selecting kernel 1 would switch off: they keep kernel 0 whatever the
+sweeps measure.  Results do not depend on the choice: every pair computes the same values
+bitwise (tests/test_gpu_strip_rows.py, tests/test_gpu_psi_kernels.py).
 
 The cache file is ``$SVIRL_GB300_TUNE_CACHE`` or ``~/.cache/svirl_gb300/psi_sweep.json``.
 No counterpart in the reference, whose kernels have one fixed launch shape
@@ -22,6 +24,7 @@ import numpy as np
 
 STRIP_ROWS = (8, 12, 17)  # the heights libglgpu compiles the sweep for
 KERNELS_FP32 = (0, 1)     # 0 cooperative loop, 1 bulk-copy ring (glgpu_set_psi_sweep_kernel)
+KERNEL_SET = 2            # of the key: choices among other kernels than these are not taken over
 
 
 def cache_path():
@@ -32,8 +35,8 @@ def cache_path():
 
 
 def key_of(handle):
-    return "%s:%dx%d:%s" % (np.dtype(handle.dtype).name, handle.Nx, handle.Ny,
-                            "finite" if handle.kappa_finite() else "inf")
+    return "%s:%dx%d:%s:%d" % (np.dtype(handle.dtype).name, handle.Nx, handle.Ny,
+                               "finite" if handle.kappa_finite() else "inf", KERNEL_SET)
 
 
 def _load(path):
@@ -65,9 +68,13 @@ def tune(handle, reps=5, path=None, force=False):
     path = path or cache_path()
     table = _load(path)
     key = key_of(handle)
+    on_chip = getattr(handle, "td_resident", lambda: False)()
     if not force and key in table:
-        apply(handle, table[key])
-        return dict(table[key], cached=True)
+        choice = dict(table[key], cached=True)
+        if on_chip:
+            choice["kernel"] = 0
+        apply(handle, choice)
+        return choice
     kernels = KERNELS_FP32 if np.dtype(handle.dtype) == np.float32 else (0,)
     measured = {}
     for kern in kernels:
@@ -76,7 +83,7 @@ def tune(handle, reps=5, path=None, force=False):
             handle.set_psi_strip_rows(rows)
             handle.time_sweeps(0, 1)  # warm-up launch
             measured["%d/%d" % (kern, rows)] = 1e3 * handle.time_sweeps(0, reps)
-    best = min(measured, key=measured.get)
+    best = min((k for k in measured if not on_chip or k.startswith("0/")), key=measured.get)
     kern, rows = (int(x) for x in best.split("/"))
     choice = {"kernel": kern, "rows": rows, "us": measured[best], "measured": measured}
     apply(handle, choice)

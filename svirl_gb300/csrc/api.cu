@@ -385,6 +385,12 @@ int glgpu_set_psi_sweep_kernel(glgpu_handle* h, int32_t select) {
     return GLGPU_OK;
 }
 
+int glgpu_td_resident(glgpu_handle* h) {
+    if (check_handle(h)) return GLGPU_E_ARG;
+    cudaSetDevice(h->device);
+    return td_resident(h) ? 1 : 0;
+}
+
 int glgpu_set_psi_strip_rows(glgpu_handle* h, int32_t rows) {
     if (check_handle(h)) return GLGPU_E_ARG;
     cudaSetDevice(h->device);

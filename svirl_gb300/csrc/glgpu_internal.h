@@ -335,6 +335,7 @@ size_t real_size(const glgpu_handle* h);
 // td.cu
 int td_run(glgpu_handle* h, double dt, int Nt, int eqn, glgpu_td_stats* stats, double* elapsed_ms);
 int time_sweeps(glgpu_handle* h, int which, int nrep, double* avg_ms);
+bool td_resident(glgpu_handle* h);  // its TD calls run as one resident launch (unless the bulk-copy sweep is selected)
 int choose_strip_rows(const Geo& g);
 // the FP32 bulk-copy psi sweep is selected (glgpu_set_psi_sweep_kernel)
 inline bool bulk_selected(const glgpu_handle* h) { return h->dtype == 4 && h->psi_select == 1; }

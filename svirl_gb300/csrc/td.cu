@@ -1645,9 +1645,13 @@ static bool resident_ok(const glgpu_handle* h, bool use_graphs, int guard) {
     return use_graphs && guard == 0 && h->psi_scheme == 0 && !h->vpi && h->lock_n == 0;
 }
 
+bool td_resident(glgpu_handle* h) {
+    return resident_ok(h, h->use_graphs, h->loop_guard) && res_prepare(&h->res, &h, 1);
+}
+
 int td_run(glgpu_handle* h, double dt, int Nt, int eqn, glgpu_td_stats* stats, double* elapsed_ms) {
     if (eqn < 0 || eqn > 2 || Nt < 0) return set_error(h, GLGPU_E_ARG, "glgpu_td: bad eqn or Nt");
-    const bool resident = Nt > 0 && resident_ok(h, h->use_graphs, h->loop_guard) && !bulk_selected(h) && res_prepare(&h->res, &h, 1);
+    const bool resident = Nt > 0 && !bulk_selected(h) && td_resident(h);
     // dt of the order-parameter iterator; the A kernel also receives it (td.py:278)
     h->inst_h.dt = dt;
     h->inst_h.fdt = (float)dt;

@@ -43,3 +43,11 @@ def test_selected_sweep_kernel_concerns_fp32_handles_alone():
     batch = HandleBatch([g._h for g in films])
     assert batch.td_raw(0.1, 2).sweep_launches == 1
     batch.close()
+
+
+def test_td_resident_says_what_a_call_does():
+    for dtype, n in ((np.float32, 97), (np.float64, 97), (np.float32, 900)):
+        gl = make_pair(Nx=n, Ny=n - 3, H=0.2, dtype=dtype)[0]
+        for guard in (0, 1000):
+            gl._h.set_loop_guard(guard)
+            assert gl._h.td_resident() == (gl._h.td(0.1, 2).sweep_launches == 1)
