@@ -817,26 +817,25 @@ cudaError_t res_launch(const ResState& r, const Inst* insts, int ninst, LoopStat
                                        (size_t)r.plan.smem, s);
 }
 
-// The largest residual that meets the stop rule 1e-4 max(code) < 1 (jacobi_converged,
-// monotone in the residual), as IEEE bits, so that the device loop compares integers
+// The largest residual that meets the stop rule (jacobi_converged, monotone in the
+// residual), as IEEE bits, so that the device loop compares integers
 // (the rule's FP64 division takes the GPU about a microsecond).
 unsigned long long res_threshold(int dtype, double stop) {
+    // (int)x < 10000 in the rule; a NaN x (an infinite residual against an infinite
+    // criterion) becomes 0 there
     auto conv = [&](unsigned long long b) {
         if (dtype == 4) {
             float r;
             const uint32_t u = (uint32_t)b;
             memcpy(&r, &u, 4);
-            float x = (float)((1.0e4 * (double)r) / (double)(float)stop);
-            if (x > 1.0e8) x = 1.0e8f;
-            return (int)x < 10000;
+            return !((float)((1.0e4 * (double)r) / (double)(float)stop) >= 10000.0f);
         }
         double r;
         memcpy(&r, &b, 8);
-        double x = (1.0e4 * r) / stop;
-        if (x > 1.0e8) x = 1.0e8;
-        return (int)x < 10000;
+        return !((1.0e4 * r) / stop >= 10000.0);
     };
-    unsigned long long lo = 0, hi = dtype == 4 ? 0x7f800000ull : 0x7ff0000000000000ull;  // conv(0), not conv(inf)
+    unsigned long long lo = 0, hi = dtype == 4 ? 0x7f800000ull : 0x7ff0000000000000ull;  // conv(0)
+    if (conv(hi)) return hi;
     while (hi - lo > 1) {
         const unsigned long long m = lo + (hi - lo) / 2;
         if (conv(m)) lo = m;
