@@ -24,8 +24,10 @@
 // filled or not, 1440 cycles a box (MMAs alone: about 50 cycles each).  64 images of
 // 128^2, us, thread-gather kernel / this one (copies of the input and output alone at the
 // measured HBM rate): 8 -> 32 channels 201 / 31 (13), 32 -> 32 390 / 41 (20), 64 + 32 -> 32
-// 966 / 90 (40), 32 -> 8 358 / 37 (13); the 64 + 32 -> 32 layer forward and backward, 32
-// images: 1555 / 320.
+// 966 / 90 (40), 32 -> 8 358 / 37 (13) (back to back; 10 us more each as single calls from a
+// flushed L2); the 64 + 32 -> 32 layer forward and backward, 32 images: 1555 / 320.
+#include <type_traits>
+
 #include "nn_tc.cuh"
 
 #include "../../include/glgpu.h"
@@ -51,30 +53,27 @@ constexpr int BOX8_BYTES = BOXW * BOXH * 16, ZERO8_BYTES = (TH - 1) * BOXW * 16 
 // A views of a box: the tile's rows, eight pixels each, are ROW_BYTES apart
 constexpr uint32_t kBoxHi = desc_hi(ROW_BYTES), kWeightHi = desc_hi(1024);
 
-// The MMAs of one tap and chunk, KS K steps, from the box at a and the weights at b (low
-// descriptor halves); `acc`: whether the first adds to the accumulator.
-template <int KS> __device__ __forceinline__ void tap_mmas(uint32_t d, uint32_t a, uint32_t b, uint32_t idesc, uint32_t acc) {
-#pragma unroll
-    for (int j = 0; j < KS; ++j) mma_f16(d, a + 2 * j, kBoxHi, b + 2 * j, kWeightHi, idesc, j > 0 ? 1u : acc);
-}
 template <int MODE> __device__ __forceinline__ constexpr uint32_t tap_off(int tap) {
     return (uint32_t)(((MODE == 0 ? tap / 3 : 2 - tap / 3) * ROW_BYTES + (MODE == 0 ? tap % 3 : 2 - tap % 3) * 128) >> 4);
 }
 
-// All taps of a tile of one chunk, KS K steps each, or of two chunks, tap by tap.
-template <int MODE, int WB, int KS>
-__device__ __forceinline__ void tile_mmas(uint32_t d, uint32_t a, uint32_t w, uint32_t idesc) {
+// The MMAs of a tile, tap by tap and through the NCK chunks of a tap: chunk c takes ks[c]
+// K steps (KS, if not 0) from the box at a[c]; w: the weights (low descriptor halves).
+// Unrolled, with the steps that a chunk lacks skipped: the operands are then constants away
+// from the bases.  64 images of 128^2 to 32 channels, us, by a loop over chunks with a branch
+// on their steps / this: 32 + 32 189 / 90, 64 + 32 154 / 99, 64 + 48 181 / 109, 64 + 64 150 /
+// 117, 96 183 / 99; one chunk of 32, steps skipped / known at compile time: 52 / 48.
+template <int MODE, int WB, int NCK, int KS = 0>
+__device__ __forceinline__ void tile_mmas(uint32_t d, const uint32_t (&a)[NCK], const int (&ks)[NCK], uint32_t w, uint32_t idesc) {
 #pragma unroll
     for (int tap = 0; tap < 9; ++tap)
-        tap_mmas<KS>(d, a + tap_off<MODE>(tap), w + (uint32_t)((tap * WB) >> 4), idesc, tap > 0 ? 1u : 0u);
-}
-template <int MODE, int WB, int KS0, int KS1>
-__device__ __forceinline__ void tile_mmas2(uint32_t d, uint32_t a0, uint32_t a1, uint32_t w, uint32_t idesc) {
 #pragma unroll
-    for (int tap = 0; tap < 9; ++tap) {
-        tap_mmas<KS0>(d, a0 + tap_off<MODE>(tap), w + (uint32_t)((tap * WB) >> 4), idesc, tap > 0 ? 1u : 0u);
-        tap_mmas<KS1>(d, a1 + tap_off<MODE>(tap), w + (uint32_t)(((9 + tap) * WB) >> 4), idesc, 1u);
-    }
+        for (int c = 0; c < NCK; ++c)
+#pragma unroll
+            for (int j = 0; j < 4; ++j)
+                if (KS > 0 ? j < KS : j < ks[c])
+                    mma_f16(d, a[c] + tap_off<MODE>(tap) + 2 * j, kBoxHi, w + (uint32_t)(((c * 9 + tap) * WB) >> 4) + 2 * j, kWeightHi,
+                            idesc, tap > 0 || c > 0 || j > 0 ? 1u : 0u);
 }
 
 // MODE 0 (forward): A = [x1 | x2] (C1 + C2 channels), B = Wb as [cout][9][cin], out =
@@ -226,33 +225,28 @@ k_conv_tile(const __grid_constant__ CUtensorMap ta1, const __grid_constant__ CUt
                     }
                 }
                 asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
-                if (!ok) {  // (a copy did not arrive: nothing is multiplied, the tile is committed as it is)
-                } else if (sh.nck == 1) {
-                    const uint32_t a = box0 + (uint32_t)st * (BOX_BYTES >> 4);
-                    if (C1 > 48) tile_mmas<MODE, WB, 4>(d, a, w0, kIdescT);
-                    else if (C1 > 32) tile_mmas<MODE, WB, 3>(d, a, w0, kIdescT);
-                    else if (C1 > 16) tile_mmas<MODE, WB, 2>(d, a, w0, kIdescT);
-                    else tile_mmas<MODE, WB, 1>(d, a, w0, kIdescT);
-                } else if (sh.nck == 2 && (C1 == 128 || (C1 == 64 && (C2 == 64 || C2 == 32)))) {
-                    const uint32_t a0 = box0 + (uint32_t)st * (BOX_BYTES >> 4);
-                    const uint32_t a1 = box0 + (uint32_t)(st + 1 < S ? st + 1 : 0) * (BOX_BYTES >> 4);
-                    if (C2 == 32) tile_mmas2<MODE, WB, 4, 2>(d, a0, a1, w0, kIdescT);
-                    else tile_mmas2<MODE, WB, 4, 4>(d, a0, a1, w0, kIdescT);
-                } else {
-                    for (int tap = 0; tap < 9; ++tap) {
-                        const uint32_t off = tap_off<MODE>(tap);
-                        int sc = st;
-                        for (int ck = 0; ck < sh.nck; ++ck) {
-                            const int left = ck < sh.nck1 ? C1 - ck * 64 : C2 - (ck - sh.nck1) * 64;
-                            const uint32_t a = box0 + (uint32_t)sc * (BOX_BYTES >> 4) + off;
-                            const uint32_t b = w0 + (uint32_t)((ck * 9 + tap) * (WB >> 4)), more = tap > 0 || ck > 0 ? 1u : 0u;
-                            if (left > 48) tap_mmas<4>(d, a, b, kIdescT, more);
-                            else if (left > 32) tap_mmas<3>(d, a, b, kIdescT, more);
-                            else if (left > 16) tap_mmas<2>(d, a, b, kIdescT, more);
-                            else tap_mmas<1>(d, a, b, kIdescT, more);
-                            if (++sc == S) sc = 0;
-                        }
+                // (a copy did not arrive: nothing is multiplied, the tile is committed as it is)
+                auto go = [&](auto nck, auto steps) {
+                    constexpr int NCK = decltype(nck)::value;
+                    uint32_t a[NCK];
+                    int ks[NCK];
+#pragma unroll
+                    for (int c = 0; c < NCK; ++c) {
+                        const int left = c < sh.nck1 ? C1 - c * 64 : C2 - (c - sh.nck1) * 64;
+                        ks[c] = (left + 15) / 16;
+                        a[c] = box0 + (uint32_t)(st + c < S ? st + c : st + c - S) * (BOX_BYTES >> 4);
                     }
+                    tile_mmas<MODE, WB, NCK, decltype(steps)::value>(d, a, ks, w0, kIdescT);
+                };
+                if (ok) {
+                    using std::integral_constant;
+                    if (sh.nck == 1 && C1 > 48) go(integral_constant<int, 1>{}, integral_constant<int, 4>{});
+                    else if (sh.nck == 1 && C1 > 32) go(integral_constant<int, 1>{}, integral_constant<int, 3>{});
+                    else if (sh.nck == 1 && C1 > 16) go(integral_constant<int, 1>{}, integral_constant<int, 2>{});
+                    else if (sh.nck == 1) go(integral_constant<int, 1>{}, integral_constant<int, 1>{});
+                    else if (sh.nck == 2) go(integral_constant<int, 2>{}, integral_constant<int, 0>{});
+                    else if (sh.nck == 3) go(integral_constant<int, 3>{}, integral_constant<int, 0>{});
+                    else go(integral_constant<int, 4>{}, integral_constant<int, 0>{});
                 }
                 for (int ck = 0; ck < sh.nck; ++ck) mma_commit(empty0 + 8 * (st + ck < S ? st + ck : st + ck - S));
                 st = s1;

@@ -87,3 +87,14 @@ def test_settings_give_the_same_values(shape):
         else:
             t, g = t.float(), g.float()
             assert bool(((t - g).abs() <= 2.0 ** -7 * g.abs().maximum(t.abs()) + 2 * k * 2.0 ** -24 * terms).all())
+
+
+@pytest.mark.parametrize("c1,c2", [(16, 16), (32, 32), (48, 16), (64, 16), (64, 48), (80, 0), (112, 0), (32, 96), (96, 64), (48, 80),
+                                   (144, 0), (240, 0), (64, 176)])
+def test_chunks_of_any_length_in_any_order(c1, c2):
+    """Input channels in two to four chunks of one to four K steps: the same bits as the
+    gather kernel's."""
+    x1, x2, w, b, dy = _inputs((1, 19, 12, c1, c2, 32), 5)
+    tile, gather = [_layer(s, x1, x2, w, b, dy) for s in (2, 0)]
+    for t, g in zip(tile[:3], gather[:3]):
+        assert t is None or torch.equal(t, g)
