@@ -406,6 +406,7 @@ k_conv_wgrad_tile(const __grid_constant__ CUtensorMap tx1, const __grid_constant
             }
             __syncwarp();
         } else if (warp == 1) {
+            const bool ragged = (H & 7) != 0 || (W & 7) != 0;
             int bx = q0 % ntx, by = q0 / ntx % nty;  // the box's place in its image
             for (int kc = 0; kc < nk; ++kc) {
                 const int st = kc % WT_STAGES, use = kc / WT_STAGES;
@@ -413,20 +414,22 @@ k_conv_wgrad_tile(const __grid_constant__ CUtensorMap tx1, const __grid_constant
                     ok = false;
                     break;
                 }
-                const int y1 = H - by * 8, x1 = W - bx * 8;  // rows and columns of the box inside the image
-                if (y1 < 8 || x1 < 8) {                      // (uniform)
-                    for (int p = lane; p < 128; p += 32) {   // 64 pixels of each tap, a row of 128 bytes each
-                        if ((p >> 3 & 7) < y1 && (p & 7) < x1) continue;
-                        uint4* row = (uint4*)(smem + st * WT_STAGE + p * 128);
+                if (ragged) {
+                    const int y1 = H - by * 8, x1 = W - bx * 8;  // rows and columns of the box inside the image
+                    if (y1 < 8 || x1 < 8) {                      // (uniform)
+                        for (int p = lane; p < 128; p += 32) {   // 64 pixels of each tap, a row of 128 bytes each
+                            if ((p >> 3 & 7) < y1 && (p & 7) < x1) continue;
+                            uint4* row = (uint4*)(smem + st * WT_STAGE + p * 128);
 #pragma unroll
-                        for (int v = 0; v < 8; ++v) row[v] = make_uint4(0u, 0u, 0u, 0u);
+                            for (int v = 0; v < 8; ++v) row[v] = make_uint4(0u, 0u, 0u, 0u);
+                        }
+                        asm volatile("fence.proxy.async.shared::cta;\n" ::: "memory");
+                        __syncwarp();
                     }
-                    asm volatile("fence.proxy.async.shared::cta;\n" ::: "memory");
-                    __syncwarp();
-                }
-                if (++bx == ntx) {
-                    bx = 0;
-                    if (++by == nty) by = 0;
+                    if (++bx == ntx) {
+                        bx = 0;
+                        if (++by == nty) by = 0;
+                    }
                 }
                 asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
                 const uint32_t a = desc_lo_mn(saddr(smem + st * WT_STAGE), WT_BOX), b = a + ((2 * WT_BOX) >> 4);
