@@ -91,13 +91,16 @@ int glgpu_psi_sweeps_per_launch(void);
  * compiled strip heights, by the item-count model of the persistent sweep), or what
  * glgpu_set_psi_strip_rows set; 0 if h is NULL. */
 int glgpu_psi_strip_rows(const glgpu_handle* h);
+/* Rows per warp strip of the cooperative FP32 psi loop, chosen by the size; 0 for FP64 and if
+ * h is NULL. */
+int glgpu_psi_loop_rows(const glgpu_handle* h);
 /* Force the bulk-copy sweep's strip height (one of the compiled heights; 0 = the model's
  * choice); the default sweep has heights of its own, chosen by the size.
  * Results do not depend on it: every node gets the same arithmetic. */
 int glgpu_set_psi_strip_rows(glgpu_handle* h, int32_t rows);
 /* The FP32 psi sweep kernel: 0 (default) = the whole Jacobi loop as one cooperative
  * launch; 1 = a launch per three sweeps, inputs staged in shared memory by bulk copies
- * (TMA), four strips per CTA, measured slower on GB300 (172 us per launch against 59 for
+ * (TMA), four strips per CTA, measured slower on GB300 (133 us per launch against 60 for
  * three sweeps on the 2049^2 workload).  Both compute the same values bitwise. */
 int glgpu_set_psi_sweep_kernel(glgpu_handle* h, int32_t select);
 /* 1: with the present settings glgpu_td runs the whole call as one launch with the state

@@ -47,6 +47,7 @@ _P = C.c_void_p
 _SIGNATURES = {
     "glgpu_version": (C.c_int, []),
     "glgpu_psi_sweeps_per_launch": (C.c_int, []),
+    "glgpu_psi_loop_rows": (C.c_int, [_H]),
     "glgpu_psi_strip_rows": (C.c_int, [_H]),
     "glgpu_set_psi_strip_rows": (C.c_int, [_H, C.c_int32]),
     "glgpu_set_psi_sweep_kernel": (C.c_int, [_H, C.c_int32]),

@@ -177,7 +177,8 @@ int glgpu_create(const glgpu_grid* grid, int32_t device, glgpu_handle** out) {
     std::vector<Item> litems, aitems;
     if (h->dtype == 4) {
         const Geo* gp = &h->g;
-        add_loop_items(litems, h->g, 0, choose_loop_rows(&gp, 1), kWideCols);
+        h->loop_rows = choose_loop_rows(&gp, 1);
+        add_loop_items(litems, h->g, 0, h->loop_rows, kWideCols);
         add_loop_items(aitems, h->g, 0, choose_A_rows(&gp, 1), kACols);
         h->nlitems = (int)litems.size();
         h->naitems = (int)aitems.size();
@@ -390,6 +391,8 @@ int glgpu_td_resident(glgpu_handle* h) {
     cudaSetDevice(h->device);
     return td_resident(h) ? 1 : 0;
 }
+
+int glgpu_psi_loop_rows(const glgpu_handle* h) { return h ? h->loop_rows : 0; }
 
 int glgpu_set_psi_strip_rows(glgpu_handle* h, int32_t rows) {
     if (check_handle(h)) return GLGPU_E_ARG;

@@ -95,11 +95,6 @@ struct CGLoop {
     double wtol;   // ... stop unless E fell by more than wtol |E| since the last mark
 };
 
-template <typename T>
-__device__ __forceinline__ void store_partials(const double* v, int nv, double* out) {
-    for (int k = 0; k < nv; ++k) out[k] = v[k];
-}
-
 // Sums of P per-thread values over the CTA into out[0 .. NV - 1], by the threads that hold
 // them.  A warp halves the number of values that a lane carries at each exchange: the
 // lanes of one half keep the first half of the values and hand over the rest, and so on,

@@ -14,15 +14,16 @@
 
 namespace glgpu {
 
-// Temporal blocking of the psi Jacobi loop: one launch of the psi sweep kernel
-// does kFuse consecutive sweeps and writes every one of them, so the loop can
-// stop after any of them exactly where the one-sweep-per-launch loop stops.
+// Temporal blocking of the FP32 psi Jacobi loop: a round (a launch, for the bulk-copy
+// kernel) does kFuse consecutive sweeps, and the loop can stop after any of them exactly
+// where a loop of single sweeps stops: the bulk-copy kernel stores every sweep, a round of
+// k_psi_loop_f32 (tdl.cu) its last, or all, or is repeated up to the sweep that it lacks.
 #ifndef GLGPU_FUSE
 #define GLGPU_FUSE 3
 #endif
 constexpr int kFuse = GLGPU_FUSE;
 static_assert(kFuse >= 1 && kFuse <= 4, "1 <= GLGPU_FUSE <= 4");
-constexpr int kPsiBufs = kFuse + 2;  // right-hand side + input + kFuse outputs
+constexpr int kPsiBufs = kFuse + 2;  // right-hand side, input, the kFuse outputs
 // TD graphs cached per handle / batch: eqn mode (3) x any finite kappa (2) x any
 // fixed vortices (2)
 constexpr int kTDGraphs = 12;
@@ -161,10 +162,10 @@ struct Tile {
     int inst, n0;
 };
 
-// A tile of the A sweep: kATX x kATY nodes of one instance from node (i0, j0)
+// A tile of the FP64 A sweep: kATX x kATY nodes of one instance from node (i0, j0)
 // (a CTA of 256 threads covers 256 / kATX rows of the tile per pass).  64 x 32:
-// 0.084 ms per sweep at 2049^2 and kappa = 4; 32 x 32, 64 x 16 and 128 x 8 tiles
-// 0.090-0.091 ms, 32 x 64 and 128 x 16 0.084-0.085.
+// 0.65 ms per sweep at 2049^2 and kappa = 4; 32 x 32, 64 x 16 and 128 x 8 tiles
+// 0.70-0.71 ms, 32 x 64 0.65, 128 x 16 0.67.
 #ifndef GLGPU_ATX
 #define GLGPU_ATX 64
 #endif
@@ -234,6 +235,7 @@ struct glgpu_handle {
     int strip_rows = 0;                 // strip height of the psi sweep items
     glgpu::Item* litems = nullptr;      // FP32: items of the cooperative psi loop
     int nlitems = 0;
+    int loop_rows = 0;                  // their strip height
     glgpu::Item* aitems = nullptr;      // FP32: items of the cooperative A loop
     int naitems = 0;
     int psi_grid = 0;                   // CTAs of the persistent psi sweep

@@ -1,5 +1,5 @@
-// Node arithmetic of the TDGL Jacobi sweeps, shared by the sweep kernels of td.cu
-// (one launch per sweep or three) and the resident time loop of tdr.cu, so that a
+// Node arithmetic of the TDGL Jacobi sweeps, shared by the sweep kernels of td.cu, the
+// cooperative loops of tdl.cu and the resident time loop of tdr.cu, so that a
 // node gets the same operations in the same order on every path.  Fused multiply-adds
 // are written out (and mul_rn keeps other products unfused): left to the compiler, the
 // choice differs between kernels.
@@ -97,7 +97,9 @@ template <typename T> __device__ __forceinline__ T A_fixed(T first, T dt_rho, T 
 // num / den with rden = 1 / den, den in [1, 2) or a few times that.  FP32 multiplies.
 // FP64: one correction of num * rden by its remainder (Markstein 1990: the correctly
 // rounded quotient from a correctly rounded reciprocal), three FP64 instructions
-// instead of a division's dozen; infinities and NaN pass through.
+// instead of a division's dozen; infinities and NaN pass through.  On 2e8 random operands
+// the division's bits, but for quotients below 1e-290 (a subnormal remainder) and the sign
+// of a zero.
 __device__ __forceinline__ float div_by(float num, float, float rden) { return num * rden; }
 __device__ __forceinline__ double div_by(double num, double den, double rden) {
     const double q = num * rden;

@@ -1,16 +1,18 @@
-// TDGL time stepping on the GPU: the Jacobi sweeps of the backward-Euler psi step
-// and of the A step, and the time/Jacobi loops themselves, which run entirely on
-// the device (a CUDA graph with nested conditional WHILE nodes; the sweep kernel
-// that finishes last decides whether the loop continues).
+// TDGL time stepping on the GPU: the time loop of the calls that the resident loop (tdr.cu)
+// does not take, as one CUDA graph (conditional WHILE nodes) or driven by the host, around
+// the cooperative Jacobi loops of tdl.cu; and the sweeps that still take a launch each, in
+// a WHILE of their own whose last CTA decides whether it continues: FP64 A, Crank-Nicolson
+// and the bulk-copy psi sweep (kFuse sweeps a launch).
 //
 // Reference: svirl/cuda/td.h:4-133 (psi sweep), td.h:310-463 (A sweep),
 // svirl/solvers/td.py:157-218,252-325,342-377 (host loops, stop rule, swaps).
 //
 // Buffer rotation.  The reference copies psi into a separate right-hand-side
 // buffer each step and ping-pongs psi/psi_next.  Here psi^(0) (the right-hand
-// side) stays in buffer R and the other kFuse+1 buffers rotate: a launch reads
-// psi^(k) and writes psi^(k+1) .. psi^(k+kFuse) (pbuf below), so no copy is
-// needed, the loop can end after any sweep, and the values are those of the
+// side) stays in buffer R and the others take turns: in the loops of tdl.cu two for the
+// states between rounds and two for sweeps inside a round that are kept (ring_of, mid_of);
+// the launches here read psi^(k) and write all of psi^(k+1) .. psi^(k+kFuse) (pbuf below).
+// So no copy is needed, a loop can end after any sweep, and the values are those of the
 // reference.  A uses three buffers, psi^(k) in (R+1+((k-1)&1))%3; this
 // rotation also reproduces the reference's aliasing of the supercurrent
 // argument (svirl/solvers/td.py:266,303): sweep k sees A^(2*floor(k/2)), which is
@@ -73,9 +75,7 @@ __device__ void finish_instance_A(const Inst& I, LoopState* loop, int k) {
 // Buffer of psi^(s) in a psi Jacobi loop whose right-hand side psi^(0) is in
 // buffer R: the kFuse + 1 other buffers rotate, so the input of a launch and its
 // kFuse outputs are always distinct.
-// A launch of K sweeps needs K + 1 of them.
-template <int K = kFuse>
-__device__ __forceinline__ int pbuf(int R, int s) { return s == 0 ? R : (R + 1 + (s - 1) % (K + 1)) % kPsiBufs; }
+__device__ __forceinline__ int pbuf(int R, int s) { return s == 0 ? R : (R + 1 + (s - 1) % (kFuse + 1)) % kPsiBufs; }
 
 // Called by the warp that finishes the last strip of an instance in a psi
 // launch that did sweeps k+1 .. k+kFuse: the loop stops after the first of them
@@ -561,16 +561,16 @@ k_psi_sweep_cn(const Inst* __restrict__ insts, const Tile* __restrict__ tiles, L
 }
 
 // One Jacobi sweep of the A step (svirl/cuda/td.h:310-463) in FP64 (FP32: k_A_loop_f32,
-// tdl.cu): each thread owns the
-// x link and the y link that start at its node.  A CTA takes a 2-D tile of
+// tdl.cu): each thread owns the x link and the y link that start at its node.  What bounds
+// it: the FP64 pipe (0.65 ms per sweep at 2049^2, a pair of sweeps averaged; 51 us at the
+// HBM rate).  A CTA takes a 2-D tile of
 // kATX x kATY nodes (ATile) and first stages the current iterate of the links its
 // nodes read (x links of rows j0-1 .. j0+kATY and columns i0-1 .. i0+kATX-1, y links
 // of rows j0-1 .. j0+kATY-1 and columns i0-1 .. i0+kATX) into shared memory with
 // coalesced row loads; the twelve neighbour values of a node's two link updates
 // then come from shared memory.  One prologue, one block reduction and one set of
-// atomics per tile (2,048 nodes; per 256 they made each CTA's life a chain of
-// dependent loads and atomics; that version took 0.202 ms per sweep at 2049^2,
-// 0.125 ms with four 256-node tiles per CTA).  The arithmetic of a link is unchanged.
+// atomics per tile (2,048 nodes; per 256 they make each CTA's life a chain of dependent
+// loads and atomics).
 __global__ void __launch_bounds__(kThreads)
 k_A_sweep(const Inst* __restrict__ insts, const ATile* __restrict__ atiles, LoopState* loop,
           cudaGraphConditionalHandle cond, int use_cond) {
