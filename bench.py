@@ -189,21 +189,24 @@ def peaks():
     return 6800.0, "fallback"
 
 
-def ncu_traffic(dtype_name, fuse, rows):
-    """DRAM bytes per psi-sweep round from the committed ncu summary of the same
-    kernel build (same sweeps per round and strip height of the handle), or None."""
+def ncu_traffic(dtype_name, fuse, rows, loop_rows=None):
+    """DRAM bytes per psi-sweep round from the committed ncu summary of the same kernel
+    (same sweeps per round, strip height of the handle and, if given, of the loop), or
+    None."""
     p = os.path.join(ROOT, "profiles", "psi_loop_%s_2049.md" % dtype_name)
     if not os.path.exists(p):
         return None
     vals = {}
     for line in open(p):
-        if ":" in line and line.split(":", 1)[0] in ("traffic_bytes_per_launch", "sweeps_per_launch", "strip_rows"):
+        if ":" in line and line.split(":", 1)[0] in ("traffic_bytes_per_launch", "sweeps_per_launch", "strip_rows", "loop_rows"):
             k, v = line.split(":", 1)
             try:
                 vals[k] = float(v.strip())
             except ValueError:
                 return None
     if int(vals.get("sweeps_per_launch", 1)) != fuse or int(vals.get("strip_rows", 0)) != rows:
+        return None
+    if loop_rows is not None and int(vals.get("loop_rows", 0)) != loop_rows:
         return None
     return vals.get("traffic_bytes_per_launch")
 
@@ -734,7 +737,7 @@ def main():
     ap.add_argument("--kappa", type=float, default=float("inf"),
                     help="GL parameter of the TDGL workload (inf: the headline workload; finite: adds the A step)")
     ap.add_argument("--psi-kernel", type=int, choices=[0, 1], default=None,
-                    help="FP32 psi sweep kernel (0 register strip, 1 bulk-copy ring); default: the autotuner's choice")
+                    help="FP32 psi sweep kernel (0 cooperative loop, 1 bulk-copy ring); default: the autotuner's choice")
     ap.add_argument("--no-graphs", action="store_true",
                     help="host-driven Jacobi loop (same kernels); ncu cannot profile kernels inside conditional graphs")
     ap.add_argument("--workload", choices=["tdgl", "states", "serve", "learned", "c1", "conv", "cg"], default="tdgl",
@@ -836,6 +839,12 @@ def main():
     alg_bytes = N * bytes_per_node_sweep * fuse
     peak, peak_kind = peaks()
     achieved = alg_bytes / (sweep_ms * 1e-3) / 1e9
+    # what the round moves over DRAM (the committed ncu summary of this kernel): the fused
+    # sweeps read their inputs once and keep most writes in L2, so well below the
+    # algorithmic bytes; where it does not come near the peak, latency is the bound
+    loop_rows = int(h.lib.glgpu_psi_loop_rows(h.h))
+    traffic = ncu_traffic(args.dtype, fuse, rows, loop_rows) if tuned["kernel"] == 0 and args.size == N_SIDE else None
+    dram = None if traffic is None else traffic / (sweep_ms * 1e-3) / 1e9
     # finite kappa: the A sweep timed alone as well (pairs of sweeps 0 and 1, L2
     # flushed before each pair); algorithmic bytes per node-sweep: psi, the
     # right-hand side, the supercurrent argument, A^(k), the write (8 B each in FP32,
@@ -914,11 +923,11 @@ def main():
                        "psi_sweep_shape": {"kernel": ["cooperative loop", "bulk-copy ring"][tuned["kernel"]],
                                            "strip_rows": tuned["rows"], "from_cache": tuned["cached"],
                                            "measured_us": tuned["measured"]}},
-            "roofline": {"bound": "hbm", "achieved": achieved, "peak": peak, "unit": "GB/s",
-                         "frac": achieved / peak,
-                         "traffic": ncu_traffic(args.dtype, fuse, rows) if tuned["kernel"] == 0 else None,
+            "roofline": {"bound": "latency" if dram is not None and dram < 0.7 * peak else "hbm", "achieved": achieved,
+                         "peak": peak, "unit": "GB/s", "frac": achieved / peak, "basis": "algorithmic bytes",
+                         "traffic": traffic, "dram_GBps": dram, "dram_frac": None if dram is None else dram / peak,
                          "kernel": ("k_psi_loop_f32" if dtype == np.float32 else "k_psi_loop_f64") if tuned["kernel"] == 0 else "k_psi_sweep_bulk",
-                         "sweeps_per_launch": fuse, "strip_rows": rows,
+                         "sweeps_per_launch": fuse, "strip_rows": rows, "loop_rows": loop_rows,
                          "bytes_per_node_sweep": bytes_per_node_sweep, "bytes_per_launch": alg_bytes,
                          "launch_ms": sweep_ms, "peak_kind": peak_kind},
             "e2e": {"value": e2e_value, "unit": "node-steps/s",
