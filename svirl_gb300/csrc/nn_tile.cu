@@ -57,23 +57,61 @@ template <int MODE> __device__ __forceinline__ constexpr uint32_t tap_off(int ta
     return (uint32_t)(((MODE == 0 ? tap / 3 : 2 - tap / 3) * ROW_BYTES + (MODE == 0 ? tap % 3 : 2 - tap % 3) * 128) >> 4);
 }
 
-// The MMAs of a tile, tap by tap and through the NCK chunks of a tap: chunk c takes ks[c]
-// K steps (KS, if not 0) from the box at a[c]; w: the weights (low descriptor halves).
-// Unrolled, with the steps that a chunk lacks skipped: the operands are then constants away
-// from the bases.  64 images of 128^2 to 32 channels, us, by a loop over chunks with a branch
-// on their steps / this: 32 + 32 189 / 90, 64 + 32 154 / 99, 64 + 48 181 / 109, 64 + 64 150 /
-// 117, 96 183 / 99; one chunk of 32, steps skipped / known at compile time: 52 / 48.
-template <int MODE, int WB, int NCK, int KS = 0>
-__device__ __forceinline__ void tile_mmas(uint32_t d, const uint32_t (&a)[NCK], const int (&ks)[NCK], uint32_t w, uint32_t idesc) {
+// The MMAs of a tile, tap by tap and through the chunks of a tap: chunk c takes KS[c] K steps
+// (ks[c] where that is 0) from the box at a[c]; w: the weights (low descriptor halves).  The
+// operands are constants away from the bases, which a loop over chunks with a branch on
+// their steps moved for every MMA.  64 images of 128^2 to 32 channels, us, by that loop /
+// this: 32 + 32 189 / 81, 64 + 32 154 / 91, 64 + 48 181 / 101, 64 + 64 150 / 109, 96 183 / 91.
+// One chunk unrolled over all taps, more over a row of taps (one chunk by rows: 48 against
+// 46 us at 32 channels, 68 against 64 at 64; two unrolled over all taps: 97).
+template <int MODE, int WB, int... KS>
+__device__ __forceinline__ void tile_mmas(uint32_t d, const uint32_t (&a)[sizeof...(KS)], const int (&ks)[sizeof...(KS)],
+                                          uint32_t w, uint32_t idesc) {
+    constexpr int kSteps[] = {KS...}, NCK = sizeof...(KS);
+    if constexpr (NCK == 1) {
 #pragma unroll
-    for (int tap = 0; tap < 9; ++tap)
+        for (int tap = 0; tap < 9; ++tap)
 #pragma unroll
-        for (int c = 0; c < NCK; ++c)
+            for (int j = 0; j < kSteps[0]; ++j)
+                mma_f16(d, a[0] + tap_off<MODE>(tap) + 2 * j, kBoxHi, w + (uint32_t)((tap * WB) >> 4) + 2 * j, kWeightHi, idesc,
+                        tap > 0 || j > 0 ? 1u : 0u);
+    } else {
+        uint32_t row = tap_off<MODE>(MODE == 0 ? 0 : 2);  // the tap row's place in a box
+#pragma unroll 1
+        for (int ky = 0; ky < 3; ++ky) {
 #pragma unroll
-            for (int j = 0; j < 4; ++j)
-                if (KS > 0 ? j < KS : j < ks[c])
-                    mma_f16(d, a[c] + tap_off<MODE>(tap) + 2 * j, kBoxHi, w + (uint32_t)(((c * 9 + tap) * WB) >> 4) + 2 * j, kWeightHi,
-                            idesc, tap > 0 || c > 0 || j > 0 ? 1u : 0u);
+            for (int kx = 0; kx < 3; ++kx)
+#pragma unroll
+                for (int c = 0; c < NCK; ++c)
+#pragma unroll
+                    for (int j = 0; j < 4; ++j)
+                        if (kSteps[c] > 0 ? j < kSteps[c] : j < ks[c])
+                            mma_f16(d, a[c] + row + (uint32_t)((MODE == 0 ? kx : 2 - kx) * (128 >> 4) + 2 * j), kBoxHi,
+                                    w + (uint32_t)(((c * 9 + kx) * WB) >> 4) + 2 * j, kWeightHi, idesc,
+                                    kx > 0 || c > 0 || j > 0 ? 1u : (uint32_t)(ky > 0));
+            row += MODE == 0 ? (uint32_t)(ROW_BYTES >> 4) : 0u - (uint32_t)(ROW_BYTES >> 4);
+            w += (uint32_t)((3 * WB) >> 4);
+        }
+    }
+}
+
+// The K steps of one or two chunks as compile-time numbers.
+template <int MODE, int WB, int... KS>
+__device__ __forceinline__ void tile_mmas1(uint32_t d, const uint32_t (&a)[sizeof...(KS) + 1], const int (&ks)[sizeof...(KS) + 1],
+                                           uint32_t w, uint32_t idesc) {
+    const int k = ks[sizeof...(KS)];
+    if (k > 3) tile_mmas<MODE, WB, KS..., 4>(d, a, ks, w, idesc);
+    else if (k > 2) tile_mmas<MODE, WB, KS..., 3>(d, a, ks, w, idesc);
+    else if (k > 1) tile_mmas<MODE, WB, KS..., 2>(d, a, ks, w, idesc);
+    else tile_mmas<MODE, WB, KS..., 1>(d, a, ks, w, idesc);
+}
+template <int MODE, int WB>
+__device__ __forceinline__ void tile_mmas2(uint32_t d, const uint32_t (&a)[2], const int (&ks)[2], uint32_t w, uint32_t idesc) {
+    const int k = MODE == 1 ? 4 : ks[0];  // (the data gradient has one input: its first chunk is full)
+    if (k > 3) tile_mmas1<MODE, WB, 4>(d, a, ks, w, idesc);
+    else if (k > 2) tile_mmas1<MODE, WB, 3>(d, a, ks, w, idesc);
+    else if (k > 1) tile_mmas1<MODE, WB, 2>(d, a, ks, w, idesc);
+    else tile_mmas1<MODE, WB, 1>(d, a, ks, w, idesc);
 }
 
 // MODE 0 (forward): A = [x1 | x2] (C1 + C2 channels), B = Wb as [cout][9][cin], out =
@@ -226,27 +264,26 @@ k_conv_tile(const __grid_constant__ CUtensorMap ta1, const __grid_constant__ CUt
                 }
                 asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
                 // (a copy did not arrive: nothing is multiplied, the tile is committed as it is)
-                auto go = [&](auto nck, auto steps) {
+                auto go = [&](auto nck) {
                     constexpr int NCK = decltype(nck)::value;
                     uint32_t a[NCK];
                     int ks[NCK];
 #pragma unroll
                     for (int c = 0; c < NCK; ++c) {
-                        const int left = c < sh.nck1 ? C1 - c * 64 : C2 - (c - sh.nck1) * 64;
-                        ks[c] = (left + 15) / 16;
-                        a[c] = box0 + (uint32_t)(st + c < S ? st + c : st + c - S) * (BOX_BYTES >> 4);
+                        const int left = c == 0 || c < sh.nck1 ? C1 - c * 64 : C2 - (c - sh.nck1) * 64;
+                        ks[c] = min(4, (left + 15) / 16);
+                        a[c] = box0 + (uint32_t)(c == 0 || st + c < S ? st + c : st + c - S) * (BOX_BYTES >> 4);
                     }
-                    tile_mmas<MODE, WB, NCK, decltype(steps)::value>(d, a, ks, w0, kIdescT);
+                    if constexpr (NCK == 1) tile_mmas1<MODE, WB>(d, a, ks, w0, kIdescT);
+                    else if constexpr (NCK == 2) tile_mmas2<MODE, WB>(d, a, ks, w0, kIdescT);
+                    else if constexpr (NCK == 3) tile_mmas<MODE, WB, 0, 0, 0>(d, a, ks, w0, kIdescT);
+                    else tile_mmas<MODE, WB, 0, 0, 0, 0>(d, a, ks, w0, kIdescT);
                 };
                 if (ok) {
-                    using std::integral_constant;
-                    if (sh.nck == 1 && C1 > 48) go(integral_constant<int, 1>{}, integral_constant<int, 4>{});
-                    else if (sh.nck == 1 && C1 > 32) go(integral_constant<int, 1>{}, integral_constant<int, 3>{});
-                    else if (sh.nck == 1 && C1 > 16) go(integral_constant<int, 1>{}, integral_constant<int, 2>{});
-                    else if (sh.nck == 1) go(integral_constant<int, 1>{}, integral_constant<int, 1>{});
-                    else if (sh.nck == 2) go(integral_constant<int, 2>{}, integral_constant<int, 0>{});
-                    else if (sh.nck == 3) go(integral_constant<int, 3>{}, integral_constant<int, 0>{});
-                    else go(integral_constant<int, 4>{}, integral_constant<int, 0>{});
+                    if (sh.nck == 1) go(std::integral_constant<int, 1>{});
+                    else if (sh.nck == 2) go(std::integral_constant<int, 2>{});
+                    else if (sh.nck == 3) go(std::integral_constant<int, 3>{});
+                    else go(std::integral_constant<int, 4>{});
                 }
                 for (int ck = 0; ck < sh.nck; ++ck) mma_commit(empty0 + 8 * (st + ck < S ? st + ck : st + ck - S));
                 st = s1;
