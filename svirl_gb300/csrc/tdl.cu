@@ -264,7 +264,7 @@ k_psi_loop_f64(const Inst* __restrict__ insts, int ninst, const Tile* __restrict
 // the round; a stop elsewhere repeats the round up to there.
 // What bounds it: latency, at 12 warps per SM (168 registers); 25 M warp instructions a
 // round at 2049^2 where strips of 32 columns, one a lane, took 37 M.  A round at 2049^2:
-// 52 us from a flushed L2 (59 as a timed launch), against 78 for a timed launch of those
+// 54 us from a flushed L2 (60 as a timed launch), against 78 for a timed launch of those
 // strips, which also held their rows in registers two ahead; 79 with two columns a lane
 // and rows one ahead in registers.  Tiles of 64 x 32 nodes in shared memory, a column of
 // 8 nodes a thread: 66 us with bulk copies for the next tile (the copy engine takes 60
