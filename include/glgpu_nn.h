@@ -42,8 +42,9 @@ int glnn_conv3x3_fwd(const void* x1, int32_t c1, const void* x2, int32_t c2, con
  * channels, one box of input per 16 x 8 pixel tile for all nine taps (any image size;
  * c1 and c2 multiples of 16, or c1 = 8 alone); more input channels, a box per tap with
  * the epilogue of one tile under the MMAs of the next (c1, c2, cout multiples of 64; w
- * a multiple of 128 or a divisor of 128; h*w a multiple of 128).  1 = by TMA, one
- * output tile per CTA, for the latter shapes.  The thread gather otherwise;
+ * a multiple of 128 or a divisor of 128; h*w a multiple of 128), or the input boxes again
+ * up to 256 channels where the shape is another.  1 = by TMA, one output tile per CTA, for
+ * the shapes of the box per tap.  The thread gather otherwise;
  * 0 = always the thread gather.  Every setting computes the same values bitwise, but for
  * the data gradient of the input-box kernel where cout is no multiple of 16: its K steps
  * take one tap each there, so the FP32 sums are grouped differently before they are
